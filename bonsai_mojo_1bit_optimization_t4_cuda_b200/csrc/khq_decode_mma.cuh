@@ -14,7 +14,7 @@
 //     query finish it.
 // V is accumulated in the rotated domain exactly as the first-generation kernel does:
 //   O^T[dim, head] += V^T[dim, token] P^T[token, head], V^T = raw fp16 codebook entries (exact),
-//   the per-token scales (alpha_v*v_norm*energy etc.) folded into three variants of P.
+//   the per-token scales (alpha_v*v_norm*energy etc.) folded into three variants of P (dim 3: see M2State).
 //
 // Thread mapping (mma.sync.m16n8k16 fragments): lane = 4*g + t.  K side: token rows g and g+8,
 // thread t owns the 64-dim quarter [64t, 64t+64) of both rows (mask words 4t..4t+3), k-step s
@@ -46,20 +46,18 @@ constexpr int M2_OFF_VSM = M2_OFF_VRN + M2_ROWS * 2;
 constexpr int M2_STAGE_BYTES = M2_OFF_VSM + M2_ROWS * 4;  // 28160
 
 constexpr int M2_SM_STAGES = 0;
-// V codebook, split so that it fits beside everything else: (d0, d1) as one 32-bit word per
-// (code, patch) and d2 as one half.  Rows of 65 words / 65 halfs instead of 64: the bank of a
-// look-up then depends on the code as well as on the patch, which spreads the warp's 32
-// look-ups (8 patches x 4 tokens per instruction) over the banks.
-constexpr int M2_VQA_STRIDE = 65;                                    // words per code row
-constexpr int M2_VQB_STRIDE = 130;                                   // bytes per code row
-constexpr int M2_SM_VQ = M2_SM_STAGES + M2_NSTAGE * M2_STAGE_BYTES;  // (d0, d1): 256 x 65 x 4 B
-constexpr int M2_SM_VQB = M2_SM_VQ + 256 * M2_VQA_STRIDE * 4;        // d2: 256 x 130 B
-constexpr int M2_SM_ROPE = M2_SM_VQB + 256 * M2_VQB_STRIDE;          // 2 x M2_TT tokens x 32 float2
+// V codebook, one row per code: for every pair of patches the two (d0, d1) words, then the two d2 halfs
+// (12 bytes), so that both look-ups of a (code, patch) share one address computation.  A row has one word of
+// padding: the bank of a look-up then depends on the code as well as on the patch, which spreads the
+// warp's 32 look-ups (8 patches x 4 tokens per instruction) over the banks.
+constexpr int M2_VQ_ROW = (NP / 2) * 12 + 4;                         // 388 bytes per code
+constexpr int M2_SM_VQ = M2_SM_STAGES + M2_NSTAGE * M2_STAGE_BYTES;
+constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // 2 x M2_TT tokens x 32 float2
 constexpr int M2_SM_BROT = M2_SM_ROPE + 2 * M2_TT * 32 * 8;          // 4 kinds x 16 steps x 32 lanes x 8 B
 constexpr int M2_SM_FREQ = M2_SM_BROT + 4 * 16 * 32 * 8;
 constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats
 constexpr int M2_SM_BARS = M2_SM_DINV + 256;
-constexpr int M2_SM_C3 = M2_SM_BARS + 64;              // 64 patches x float2: dim-3 centroids x alpha_v
+constexpr int M2_SM_C3 = M2_SM_BARS + 64;              // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
 constexpr int M2_SM_RSTEP = M2_SM_C3 + NP * 8;                          // 32 x float2: cos / sin of one tile's worth (32 positions) of each rotary pair
 constexpr int M2_SM_QR = M2_SM_RSTEP + 32 * 8;                             // raw rotary query fragments: 4 kv-heads x 4 k-steps x 32 lanes x 8 B
 constexpr int M2_SM_TOTAL = M2_SM_QR + HKV * 4 * 32 * 8;
@@ -72,13 +70,13 @@ constexpr int M2_SM_TOTAL = M2_SM_QR + HKV * 4 * 32 * 8;
 // Warp w owns lanes 32 (w & 3) .. +31, which it shares with the other warps of its kv-head.  Columns: 0 .. 127 =
 // the kv-head's query fragments (eight per k-step: q1.x, q1.y, q2.x, q2.y and their low-order halves; written by
 // the kv-head's first warp), 128 .. 255 = the rotor fragments of the lane quadrant (eight per k-step: b1.x, b1.y,
-// b2.x, b2.y and their low-order halves; the same values in all four quadrants), 256 + 64 (w >> 2) .. +63 = the
-// warp's O^T accumulators, which are in registers only while the V side of a block runs.
-constexpr uint32_t M2_TM_COLS = 512, M2_TM_ROT = 128, M2_TM_ACC = 256;
-static_assert(M2_TM_ACC + 64 * M2_WPK <= M2_TM_COLS, "tensor-memory columns");
-static_assert(M2_SM_TOTAL <= 227 * 1024 && M2_SM_C3 % 16 == 0 && M2_SM_ROPE % 16 == 0 && M2_SM_VQB % 16 == 0,
+// b2.x, b2.y and their low-order halves; the same values in all four quadrants), 256 + 80 (w >> 2) .. +79 = the
+// warp's O^T accumulators, twenty per pair of patches, which are in registers only while the V side of that pair runs.
+constexpr uint32_t M2_TM_COLS = 512, M2_TM_ROT = 128, M2_TM_ACC = 256, M2_TM_ACC_WARP = 80;
+static_assert(M2_TM_ACC + M2_TM_ACC_WARP * M2_WPK <= M2_TM_COLS, "tensor-memory columns");
+static_assert(M2_SM_TOTAL <= 227 * 1024 && M2_SM_C3 % 16 == 0 && M2_SM_ROPE % 16 == 0 && M2_SM_VQ % 16 == 0,
               "shared memory budget");
-static_assert(HKV * MERGE_FLOATS * 4 <= 256 * M2_VQA_STRIDE * 4, "cluster export records alias the codebook");
+static_assert(HKV * MERGE_FLOATS * 4 <= 256 * M2_VQ_ROW, "cluster export records alias the codebook");
 static_assert(HKV * M2_WPK * MERGE_FLOATS * 4 <= M2_NSTAGE * M2_STAGE_BYTES, "records alias the stages");
 static_assert(HKV * NREP * D * 4 <= M2_NSTAGE * M2_STAGE_BYTES, "prologue scratch aliases the stages");
 static_assert(M2_STAGE_BYTES % 16 == 0 && M2_OFF_KPAY % 16 == 0 && M2_OFF_VPAY % 16 == 0 && M2_OFF_KN % 16 == 0 &&
@@ -177,18 +175,34 @@ __device__ __forceinline__ void m2_step_rope(float2* dst, const float2* src, con
     }
 }
 
+// The layer's V codebook (entry (patch, code) starts at half 3 (256 patch + code)) into its shared-memory rows.  Two
+// codes (three words) per thread and iteration, eight iterations' loads in flight: bound by load latency.
+__device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __half* __restrict__ vq, int tid) {
+    const unsigned int* src = reinterpret_cast<const unsigned int*>(vq);
+#pragma unroll 8
+    for (int u = tid; u < NP * 256 / 2; u += M2_THREADS) {
+        const unsigned int w0 = __ldg(src + 3 * u), w1 = __ldg(src + 3 * u + 1), w2 = __ldg(src + 3 * u + 2);
+        const int patch = u >> 7, code = 2 * (u & 127);  // the pair never straddles a patch (256 codes)
+        unsigned char* e = dst + code * M2_VQ_ROW + (patch >> 1) * 12;
+        *reinterpret_cast<unsigned int*>(e + 4 * (patch & 1)) = w0;
+        *reinterpret_cast<unsigned short*>(e + 8 + 2 * (patch & 1)) = (unsigned short)(w1 & 0xFFFFu);
+        e += M2_VQ_ROW;
+        *reinterpret_cast<unsigned int*>(e + 4 * (patch & 1)) = (w1 >> 16) | (w2 << 16);
+        *reinterpret_cast<unsigned short*>(e + 8 + 2 * (patch & 1)) = (unsigned short)(w2 >> 16);
+    }
+}
+
 // Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, the rotor B fragments (with and without the centroid factor) and the V
 // codebook.  Must be followed by __syncthreads().
 __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const CompressedKV& P, int tid) {
     float* freq_s = reinterpret_cast<float*>(smem + M2_SM_FREQ);
     float* dinv_s = reinterpret_cast<float*>(smem + M2_SM_DINV);
     uint2* brot = reinterpret_cast<uint2*>(smem + M2_SM_BROT);
-    unsigned short* vqa = reinterpret_cast<unsigned short*>(smem + M2_SM_VQ);
-    unsigned short* vqb = reinterpret_cast<unsigned short*>(smem + M2_SM_VQB);
     if (tid < 32) freq_s[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
-    if (tid >= 128 && tid < 128 + NP)
-        reinterpret_cast<float2*>(smem + M2_SM_C3)[tid - 128] = make_float2(__half2float(P.cents_v[0 * D + 4 * (tid - 128) + 3]) * P.alpha_v,
-                                                                             __half2float(P.cents_v[1 * D + 4 * (tid - 128) + 3]) * P.alpha_v);
+    if (tid >= 128 && tid < 128 + NP) {
+        const float c0 = __half2float(P.cents_v[0 * D + 4 * (tid - 128) + 3]), c1 = __half2float(P.cents_v[1 * D + 4 * (tid - 128) + 3]);
+        reinterpret_cast<float2*>(smem + M2_SM_C3)[tid - 128] = make_float2(c0 * P.alpha_v, (c1 - c0) * P.alpha_v);
+    }
     if (tid < 64) dinv_s[tid] = (1.0f / 256.0f) / (__half2float(P.d_k[tid]) + 1e-8f);
     if (tid >= 192 && tid < 224) {
         const int m = tid - 192;
@@ -228,7 +242,7 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
         brot[512 + e] = hi;    // rotor (residual operand), fp16 hi
         brot[1536 + e] = lo;   //   and what fp16 lost
     }
-    stage_vq_codebook<M2_THREADS, M2_VQA_STRIDE, M2_VQB_STRIDE>(P.vq, reinterpret_cast<unsigned int*>(vqa), vqb, tid);
+    m2_stage_codebook(smem + M2_SM_VQ, P.vq, tid);
 }
 
 // Query-side operands of one (sequence, layer, kv-head): this warp's B fragments.
@@ -237,12 +251,12 @@ struct M2Query {
     uint32_t rot;  // ... and of its lane quadrant's rotor fragments
 };
 
-__device__ __forceinline__ void m2_tm_st4(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};" ::"r"(a), "r"(b), "r"(c), "r"(d), "r"(taddr) : "memory");
+__device__ __forceinline__ void m2_tm_st4f(uint32_t taddr, const float* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};" ::"f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void m2_tm_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+__device__ __forceinline__ void m2_tm_ld4f(uint32_t taddr, float* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
                  : "r"(taddr)
                  : "memory");
 }
@@ -410,21 +424,32 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
 }
 
 // Running attention state of a warp in fragment layout: thread (g, t) holds heads 2t, 2t+1.
+//
+// O^T lives in tensor memory, twenty columns per pair of patches (2pp, 2pp + 1) of the thread's patch group g: three
+// accumulator tiles of the dims 0..2 (rows idx = 2 jj + r of the pair's six (patch, dim) rows), one of the dim-3 residual
+// fields, one of the dim-3 centroid bits.  Dim 3 of a patch is centroid[bit] * alpha_v * s2 + (field - 8) * s3 per token
+// with per-token scales s2, s3; both sums over tokens are taken over the raw bit fields as they lie in the payload,
+//     sum p s2 bit  and  sum p s3 field   (exact fp16 operands: a bit field is a subnormal fp16 number),
+// and the centroids, their difference and the -8 enter once per item, with sum p s2 and sum p s3 kept per head.
 struct M2State {
-    uint32_t tm_o;  // tensor-memory address of the warp's 64 accumulator columns: O^T tiles [0..11] dims 0..2 of the
-                    // patches, [12..15] dim 3 of the patches, four registers each; in registers only during the V side
-    float m[2], l[2];
+    uint32_t tm_o;
+    float m[2], l[2], p2[2], p3[2];  // reference maximum, sum of weights, sums of p s2 and p s3 (per lane)
     __device__ __forceinline__ void init() {  // whole warp
         float z[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) z[i] = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) m2_tm_st16f(tm_o + 16 * c, z);
+        for (int c = 0; c < (int)M2_TM_ACC_WARP / 16; ++c) m2_tm_st16f(tm_o + 16 * c, z);
         m2_tm_st_wait();
         m[0] = m[1] = NEG_BIG;
-        l[0] = l[1] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) l[e] = p2[e] = p3[e] = 0.0f;
     }
 };
+// What a unit of the two dim-3 accumulators of patch parity u stands for: the fields sit at bits 0..3 (even patch) or
+// 4..7 (odd), the centroid bit at 7 or 3, of a subnormal fp16 number (units of 2^-24).
+__device__ __forceinline__ constexpr float m2_field_unit(int u) { return u ? 1048576.0f : 16777216.0f; }
+__device__ __forceinline__ constexpr float m2_bit_unit(int u) { return u ? 2097152.0f : 131072.0f; }
 
 // Packed pairs of fp32 (one instruction for two neighbouring accumulator registers; each half is
 // rounded like the scalar operation).
@@ -451,9 +476,6 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
                                          M2State& st) {
     const int g = lane >> 2, t = lane & 3;
     const float* dinv_s = reinterpret_cast<const float*>(smem + M2_SM_DINV);
-    const unsigned char* vqa = smem + M2_SM_VQ;
-    const unsigned char* vqb = smem + M2_SM_VQB;
-    const float2* c3s = reinterpret_cast<const float2*>(smem + M2_SM_C3) + 8 * g;
     const uint2* qr_s = reinterpret_cast<const uint2*>(smem + M2_SM_QR) + kvh * 4 * 32;
 
     // ================================ K side: scores ==========================================
@@ -612,8 +634,13 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             const float en = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VRN)[row]);
             const float sm = reinterpret_cast<const float*>(S + M2_OFF_VSM)[row];
             s1[x] = valid[x] ? P.alpha_v * vn * en : 0.0f;     // dims 0..2: codebook entry
-            s2[x] = valid[x] ? vn : 0.0f;                      // dim 3: centroid * alpha_v (folded in c3)
-            s3[x] = valid[x] ? sm * vn * (1.0f / 7.0f) : 0.0f;  // dim 3: (dump - 8)
+            s2[x] = valid[x] ? vn : 0.0f;                      // dim 3: centroid bit
+            s3[x] = valid[x] ? sm * vn * (1.0f / 7.0f) : 0.0f;  // dim 3: residual field
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            st.p2[e] = fmaf(pw[1][e], s2[1], fmaf(pw[0][e], s2[0], st.p2[e] * corr[e]));
+            st.p3[e] = fmaf(pw[1][e], s3[1], fmaf(pw[0][e], s3[0], st.p3[e] * corr[e]));
         }
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
@@ -630,58 +657,38 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
         }
     }
     // ================================ V side: O^T += V^T P^T ====================================
-    // the accumulators come out of tensor memory for this part only
-    float o[16][4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) m2_tm_ld16f(st.tm_o + 16 * c, &o[4 * c][0]);
-    m2_tm_ld_wait();
-    if (rescale) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            o[i][0] *= corr[0];
-            o[i][1] *= corr[1];
-            o[i][2] *= corr[0];
-            o[i][3] *= corr[1];
-        }
-    }
-    // thread (g, t): patch group g of tokens 2t, 2t+1, 2t+8, 2t+9
+    // thread (g, t): patch group g of tokens 2t, 2t+1, 2t+8, 2t+9; per pass two patches = 24 bits of each token's
+    // fields, and the accumulators of that pair come out of tensor memory
     uint32_t vw[4][3], hb[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int tok = 2 * t + (i & 1) + 8 * (i >> 1);
-        const uint32_t* vp = reinterpret_cast<const uint32_t*>(S + M2_OFF_VPAY + ((r0 + tok) * HKV + kvh) * V_PAY);
-        vw[i][0] = vp[3 * g];
-        vw[i][1] = vp[3 * g + 1];
-        vw[i][2] = vp[3 * g + 2];
-        hb[i] = ((vp[24 + (g >> 2)] >> (8 * (g & 3))) & 0xFFu) << 7;  // bit 7 + pl = high code bit of patch pl
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(S + M2_OFF_VPAY + ((r0 + tok) * HKV + kvh) * V_PAY);
+#pragma unroll
+        for (int w = 0; w < 3; ++w) vw[i][w] = row[3 * g + w];
+        hb[i] = ((row[24 + (g >> 2)] >> (8 * (g & 3))) & 0xFFu) << 7;  // bit 7 + pl = high code bit of patch pl
     }
+    const unsigned char* vq = smem + M2_SM_VQ + 48 * g;
 #pragma unroll
-    for (int pp = 0; pp < 4; ++pp) {  // patch pairs (2pp, 2pp+1) -> tiles 3pp .. 3pp+2
+    for (int pp = 0; pp < 4; ++pp) {
+        float o[5][4];
+        m2_tm_ld16f(st.tm_o + 20 * pp, &o[0][0]);
+        m2_tm_ld4f(st.tm_o + 20 * pp + 16, &o[4][0]);
+        uint32_t f24[4];  // the pair's two 12-bit fields: code bits 0..6, centroid bit 7, residual 8..11
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            f24[i] = pp == 0 ? vw[i][0] : pp == 1 ? __funnelshift_r(vw[i][0], vw[i][1], 24)
+                   : pp == 2 ? __funnelshift_r(vw[i][1], vw[i][2], 16) : vw[i][2] >> 8;
         uint32_t ex[2][4], ey[2][4];  // [patch of the pair][token i]: (d0,d1), (d2,-)
-        uint32_t f3[2][4];            // 12-bit fields
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int pl = 2 * pp + u;
+        for (int u = 0; u < 2; ++u)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                uint32_t f;
-                switch (pl) {
-                    case 0: f = vw[i][0]; break;
-                    case 1: f = vw[i][0] >> 12; break;
-                    case 2: f = (vw[i][0] >> 24) | (vw[i][1] << 8); break;
-                    case 3: f = vw[i][1] >> 4; break;
-                    case 4: f = vw[i][1] >> 16; break;
-                    case 5: f = (vw[i][1] >> 28) | (vw[i][2] << 4); break;
-                    case 6: f = vw[i][2] >> 8; break;
-                    default: f = vw[i][2] >> 20; break;
-                }
-                f &= 0xFFFu;
-                f3[u][i] = f;
-                const uint32_t code = (f & 0x7Fu) | ((hb[i] >> pl) & 0x80u);
-                ex[u][i] = *reinterpret_cast<const uint32_t*>(vqa + (code * M2_VQA_STRIDE + 8 * g + pl) * 4);
-                ey[u][i] = *reinterpret_cast<const unsigned short*>(vqb + code * M2_VQB_STRIDE + (8 * g + pl) * 2);
+                const uint32_t code = ((u ? f24[i] >> 12 : f24[i]) & 0x7Fu) | ((hb[i] >> (2 * pp + u)) & 0x80u);
+                const unsigned char* e = vq + code * M2_VQ_ROW + 12 * pp;
+                ex[u][i] = *reinterpret_cast<const uint32_t*>(e + 4 * u);
+                ey[u][i] = *reinterpret_cast<const unsigned short*>(e + 8 + 2 * u);
             }
-        }
         // rows: idx = 2j + r -> (patch idx/3, dim idx%3); the pair's six (patch, dim) rows in order
         uint32_t lo[6], hi[6];  // token pairs (2t, 2t+1) and (2t+8, 2t+9)
 #pragma unroll
@@ -693,41 +700,37 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             hi[3 * u + 1] = __byte_perm(ex[u][2], ex[u][3], 0x7632);
             hi[3 * u + 2] = __byte_perm(ey[u][2], ey[u][3], 0x5410);
         }
+        // dim 3 of the two patches: byte 1 (even patch) or 2 (odd) of a token's 24 bits holds the residual field, and for
+        // the odd patch the centroid bit too; the even patch's centroid bit is the top bit of byte 0.  The masks leave
+        // nothing of the neighbouring bits.
+        const uint32_t b01l = __byte_perm(f24[0], f24[1], 0x5410), b01h = __byte_perm(f24[2], f24[3], 0x5410);
+        const uint32_t b1l = b01l >> 8, b1h = b01h >> 8;
+        const uint32_t b2l = __byte_perm(f24[0], f24[1], 0x7632), b2h = __byte_perm(f24[2], f24[3], 0x7632);
+        const uint32_t da[4] = {b1l & 0x000F000Fu, b2l & 0x00F000F0u, b1h & 0x000F000Fu, b2h & 0x00F000F0u};
+        const uint32_t ca[4] = {b01l & 0x00800080u, b2l & 0x00080008u, b01h & 0x00800080u, b2h & 0x00080008u};
+        m2_tm_ld_wait();
+        if (rescale) {
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                o[i][0] *= corr[0];
+                o[i][1] *= corr[1];
+                o[i][2] *= corr[0];
+                o[i][3] *= corr[1];
+            }
+        }
 #pragma unroll
         for (int jj = 0; jj < 3; ++jj) {
             const uint32_t a[4] = {lo[2 * jj], lo[2 * jj + 1], hi[2 * jj], hi[2 * jj + 1]};
-            m2_mma(o[3 * pp + jj], a, pb[0][0], pb[0][1]);
-            m2_mma_lo(o[3 * pp + jj], a, pl_[0][0], pl_[0][1]);
+            m2_mma(o[jj], a, pb[0][0], pb[0][1]);
+            m2_mma_lo(o[jj], a, pl_[0][0], pl_[0][1]);
         }
-        // dim 3 of the two patches (rows 0, 1 of tile 12 + pp): centroid choice and (dump - 8)
-        uint32_t ca[4], da[4];  // a0..a3 of the two extra MMAs
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int pl = 2 * pp + u;
-            float cv[4];
-            uint32_t dv[4];
-            const float2 c3p = c3s[pl];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                cv[i] = ((f3[u][i] >> 7) & 1u) ? c3p.y : c3p.x;
-                dv[i] = 0x6400u | (f3[u][i] >> 8);  // fp16 bits of 1024 + dump
-            }
-            ca[u] = m2_pack(cv[0], cv[1]);
-            ca[2 + u] = m2_pack(cv[2], cv[3]);
-            const uint32_t bias = 0x64086408u;  // fp16x2 (1032, 1032): (1024 + dump) - 1032 = dump - 8
-            const uint32_t plo = dv[0] | (dv[1] << 16), phi = dv[2] | (dv[3] << 16);
-            const __half2 d_lo = __hsub2(*reinterpret_cast<const __half2*>(&plo), *reinterpret_cast<const __half2*>(&bias));
-            const __half2 d_hi = __hsub2(*reinterpret_cast<const __half2*>(&phi), *reinterpret_cast<const __half2*>(&bias));
-            da[u] = *reinterpret_cast<const uint32_t*>(&d_lo);
-            da[2 + u] = *reinterpret_cast<const uint32_t*>(&d_hi);
-        }
-        m2_mma(o[12 + pp], ca, pb[1][0], pb[1][1]);
-        m2_mma_lo(o[12 + pp], ca, pl_[1][0], pl_[1][1]);
-        m2_mma(o[12 + pp], da, pb[2][0], pb[2][1]);
-        m2_mma_lo(o[12 + pp], da, pl_[2][0], pl_[2][1]);
+        m2_mma(o[3], da, pb[2][0], pb[2][1]);
+        m2_mma_lo(o[3], da, pl_[2][0], pl_[2][1]);
+        m2_mma(o[4], ca, pb[1][0], pb[1][1]);
+        m2_mma_lo(o[4], ca, pl_[1][0], pl_[1][1]);
+        m2_tm_st16f(st.tm_o + 20 * pp, &o[0][0]);
+        m2_tm_st4f(st.tm_o + 20 * pp + 16, &o[4][0]);
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) m2_tm_st16f(st.tm_o + 16 * c, &o[4 * c][0]);
     m2_tm_st_wait();
 }
 
@@ -765,7 +768,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
     }
     __syncthreads();
     M2State st;
-    st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + 64u * (uint32_t)sub;
+    st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + M2_TM_ACC_WARP * (uint32_t)sub;
     st.init();
 #pragma unroll 1
     for (int i = 0; i < ntiles; ++i) {
@@ -793,26 +796,39 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
 
     // ---- per-warp record in the first generation's layout, then merge + inverse V transform --------
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], 4);
-        st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], 8);
-        st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], 16);
-    }
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int m = 4; m <= 16; m <<= 1) {
+            st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], m);
+            st.p2[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p2[e], m);
+            st.p3[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p3[e], m);
+        }
     float* rec = reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * MERGE_FLOATS;
-    float o[16][4];
+    const float2* c3s = reinterpret_cast<const float2*>(smem + M2_SM_C3) + 8 * g;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) m2_tm_ld16f(st.tm_o + 16 * c, &o[4 * c][0]);
-    m2_tm_ld_wait();
-    if (t < 3) {
+    for (int pp = 0; pp < 4; ++pp) {
+        float o[5][4];
+        m2_tm_ld16f(st.tm_o + 20 * pp, &o[0][0]);
+        m2_tm_ld4f(st.tm_o + 20 * pp + 16, &o[4][0]);
+        m2_tm_ld_wait();
+        if (t < 3) {
+            float* rp = rec + 2 * t * D + 4 * (8 * g + 2 * pp);  // head 2t, dim 0 of patch 2pp; head 2t + 1 is D further
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int idx = 2 * j + r;
-                const int dim = j < 12 ? 4 * (8 * g + idx / 3) + idx % 3 : 4 * (8 * g + 2 * (j - 12) + r) + 3;
-                rec[(2 * t) * D + dim] = o[j][2 * r];
-                rec[(2 * t + 1) * D + dim] = o[j][2 * r + 1];
+            for (int idx = 0; idx < 6; ++idx) {
+                rp[4 * (idx / 3) + idx % 3] = o[idx >> 1][2 * (idx & 1)];
+                rp[D + 4 * (idx / 3) + idx % 3] = o[idx >> 1][2 * (idx & 1) + 1];
             }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float2 c = c3s[2 * pp + u];
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    rp[e * D + 4 * u + 3] = fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
+                                            fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]);
+            }
+        }
+    }
+    if (t < 3) {
         if (g == 0) {
             rec[NREP * D + 2 * t] = st.m[0];
             rec[NREP * D + 2 * t + 1] = st.m[1];
