@@ -7,7 +7,8 @@
 // Everything left of y is linear, so it moves to the query side once per (sequence, layer):
 //   * non-rotary output dims (>= 64):  q.K^ = y . q~,  q~ = R^T H256 (q * dinv * [dim >= 64])
 //     -> one GEMM  S_pass[token, head] = T[token, dim] Q1[dim, head] + C[token, dim] Q2[dim, head]
-//        with T = ternary symbols (exact in fp16), C = sign*code*(rs/mult), Q1 = q~*c, Q2 = q~;
+//        with T = ternary symbols, C = sign*code (both exact in fp16), Q1 = q~*c, Q2 = q~, each accumulated by itself
+//        and scaled by its row's factor afterwards;
 //   * rotary output dims (< 64): the first 64 outputs of H256 are H64 of the sum of the four
 //     64-dim blocks, so u[token, 64] = T * (R c)-blocks + C * R-blocks is a second GEMM with the
 //     same A operands; H64, /d, the rotation by the token's angle, and a 64-deep GEMM with the raw
@@ -52,9 +53,11 @@ constexpr int M2_SM_STAGES = 0;
 // warp's 32 look-ups (8 patches x 4 tokens per instruction) over the banks.
 constexpr int M2_VQ_ROW = (NP / 2) * 12 + 4;                         // 388 bytes per code
 constexpr int M2_SM_VQ = M2_SM_STAGES + M2_NSTAGE * M2_STAGE_BYTES;
-constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // 2 x M2_TT tokens x 32 float2
-constexpr int M2_SM_BROT = M2_SM_ROPE + 2 * M2_TT * 32 * 8;          // 4 kinds x 16 steps x 32 lanes x 8 B
+constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // 2 x M2_TT tokens x 64 floats
+constexpr int M2_SM_BROT = M2_SM_ROPE + 2 * M2_TT * 64 * 4;          // 4 kinds x 16 steps x 32 lanes x 8 B: set-up only,
+constexpr int M2_SM_RSC = M2_SM_BROT;                                //   then 16 rows x 2 float4 per warp: scalars of a block's rows
 constexpr int M2_SM_FREQ = M2_SM_BROT + 4 * 16 * 32 * 8;
+static_assert(M2_THREADS / 32 * 16 * 32 <= 4 * 16 * 32 * 8, "row scalars alias the rotor fragments' staging");
 constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats
 constexpr int M2_SM_BARS = M2_SM_DINV + 256;
 constexpr int M2_SM_C3 = M2_SM_BARS + 64;              // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
@@ -93,6 +96,13 @@ __device__ __forceinline__ uint32_t m2_movmatrix_t(uint32_t x) {
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
     return r;
 }
+// d = a b (nothing to add: no registers to clear)
+__device__ __forceinline__ void m2_mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
 // low-order ("what fp16 lost") products go through the same instruction
 #define m2_mma_lo(c, a, b0, b1) m2_mma(c, a, b0, b1)
 __device__ __forceinline__ uint32_t m2_pack(float lo, float hi) {
@@ -105,16 +115,6 @@ __device__ __forceinline__ void m2_pack_hilo(float a, float b, uint32_t& hi, uin
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = m2_pack(a - __low2float(h), b - __high2float(h));
 }
-__device__ __forceinline__ uint32_t m2_hfma2(uint32_t a, uint32_t b, uint32_t c) {
-    const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b),
-                              *reinterpret_cast<const __half2*>(&c));
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ uint32_t m2_hmul2(uint32_t a, uint32_t b) {
-    const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&r);
-}
-
 // Stage `ntok` tokens starting at `tok0` (same contract as stage_tile of the first generation).
 __device__ __forceinline__ void m2_stage_tile(const CompressedKV& P, unsigned char* stage, uint64_t* bar, int tok0,
                                               int ntok, int tid) {
@@ -151,14 +151,17 @@ __device__ __forceinline__ void m2_stage_tile(const CompressedKV& P, unsigned ch
     }
 }
 
-__device__ __forceinline__ void m2_fill_rope(float2* tab, const float* freq, const CompressedKV& P, int tok0, int tid) {
+// RoPE table of a tile: 64 floats per token; pairs 2i and 2i + 1 are the four floats cos, cos, sin, sin at 4i.
+__device__ __forceinline__ void m2_fill_rope(float* tab, const float* freq, const CompressedKV& P, int tok0, int tid) {
     for (int e = tid; e < M2_TT * 32; e += M2_THREADS) {
         const int t = e >> 5, m = e & 31;
         double th = (double)token_pos(P, tok0 + t) * (double)freq[m];
         th -= rint(th * 0.15915494309189535) * 6.283185307179586;
         float s, c;
         __sincosf((float)th, &s, &c);
-        tab[e] = make_float2(c, s);
+        float* o = tab + 64 * t + 4 * (m >> 1) + (m & 1);
+        o[0] = c;
+        o[2] = s;
     }
 }
 
@@ -167,11 +170,12 @@ __device__ __forceinline__ void m2_fill_rope(float2* tab, const float* freq, con
 // tiles, so that rounding never accumulates over more than that many turns (< 4e-6), and whenever the
 // positions are not contiguous.
 constexpr int M2_ROPE_RESEED = 64;
-__device__ __forceinline__ void m2_step_rope(float2* dst, const float2* src, const float2* step, int tid) {
+__device__ __forceinline__ void m2_step_rope(float* dst, const float* src, const float* step, int tid) {
 #pragma unroll
-    for (int e = tid; e < M2_TT * 32; e += M2_THREADS) {
-        const float2 a = src[e], d = step[e & 31];
-        dst[e] = make_float2(a.x * d.x - a.y * d.y, a.y * d.x + a.x * d.y);
+    for (int e = tid; e < M2_TT * 16; e += M2_THREADS) {
+        const float4 a = reinterpret_cast<const float4*>(src)[e], d = reinterpret_cast<const float4*>(step)[e & 15];
+        reinterpret_cast<float4*>(dst)[e] =
+            make_float4(a.x * d.x - a.z * d.z, a.y * d.y - a.w * d.w, a.z * d.x + a.x * d.z, a.w * d.y + a.y * d.w);
     }
 }
 
@@ -208,7 +212,9 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
         const int m = tid - 192;
         double th = (double)M2_TT * (double)powf(P.rope_base, -2.0f * (float)m / 64.0f);
         th -= rint(th * 0.15915494309189535) * 6.283185307179586;
-        reinterpret_cast<float2*>(smem + M2_SM_RSTEP)[m] = make_float2((float)cos(th), (float)sin(th));
+        float* o = reinterpret_cast<float*>(smem + M2_SM_RSTEP) + 4 * (m >> 1) + (m & 1);
+        o[0] = (float)cos(th);
+        o[2] = (float)sin(th);
     }
     // Rotor B fragments with the three low index bits of the 64-point Hadamard transform folded
     // in: u[8j + n] is produced by step s = 2j + (n >> 2) as rotor output c = n & 3, and
@@ -433,7 +439,8 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
 // and the centroids, their difference and the -8 enter once per item, with sum p s2 and sum p s3 kept per head.
 struct M2State {
     uint32_t tm_o;
-    float m[2], l[2], p2[2], p3[2];  // reference maximum, sum of weights, sums of p s2 and p s3 (per lane)
+    float m[2], l[2], p2[2], p3[2];  // reference of the weights, sum of weights, sums of p s2 and p s3 (per lane)
+    float top[2];                    // largest score (per lane)
     __device__ __forceinline__ void init() {  // whole warp
         float z[16];
 #pragma unroll
@@ -441,11 +448,12 @@ struct M2State {
 #pragma unroll
         for (int c = 0; c < (int)M2_TM_ACC_WARP / 16; ++c) m2_tm_st16f(tm_o + 16 * c, z);
         m2_tm_st_wait();
-        m[0] = m[1] = NEG_BIG;
+        m[0] = m[1] = top[0] = top[1] = NEG_BIG;
 #pragma unroll
         for (int e = 0; e < 2; ++e) l[e] = p2[e] = p3[e] = 0.0f;
     }
 };
+constexpr float M2_SLACK = 2.0f;
 // What a unit of the two dim-3 accumulators of patch parity u stands for: the fields sit at bits 0..3 (even patch) or
 // 4..7 (odd), the centroid bit at 7 or 3, of a subnormal fp16 number (units of 2^-24).
 __device__ __forceinline__ constexpr float m2_field_unit(int u) { return u ? 1048576.0f : 16777216.0f; }
@@ -461,6 +469,10 @@ __device__ __forceinline__ void m2_sub2(float& d0, float& d1, float a0, float a1
     asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
         : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
+__device__ __forceinline__ void m2_mul2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
 __device__ __forceinline__ void m2_fma2(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0,
                                         float c1) {
     asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7};"
@@ -468,67 +480,81 @@ __device__ __forceinline__ void m2_fma2(float& d0, float& d1, float a0, float a1
         : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
 }
 
-// One block of 16 tokens (rows r0..r0+15 of the staged tile) of kv-head `kvh`.
-// valid_lo/valid_hi: block-relative range of tokens that belong to the caller's range.
-__device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, const unsigned char* __restrict__ smem,
-                                         const float2* __restrict__ rope, int r0, int kvh, int lane, int valid_lo,
-                                         int valid_hi, const M2Query& Q, const CompressedKV& P, float scale,
-                                         M2State& st) {
-    const int g = lane >> 2, t = lane & 3;
-    const float* dinv_s = reinterpret_cast<const float*>(smem + M2_SM_DINV);
-    const uint2* qr_s = reinterpret_cast<const uint2*>(smem + M2_SM_QR) + kvh * 4 * 32;
+// The two rows of a lane (g and g + 8 of the block), its 64-dim quarter of each.
+struct M2KRows {
+    const uint32_t* kp[2];      // payload words of the row
+    uint4 mw[2];                // the quarter's mask words
+    khq3::KQuarter kq[2];
+    uint32_t wc[2], first[2];   // outliers of the four words, eight bits each; ordinal of the quarter's first one
+};
+// What the K side of a block leaves: pass-part scores (rows g (0, 1) and g + 8 (2, 3), heads 2t, 2t + 1) of the ternary and
+// of the residual part, and the rotor block sums u[token, 8j + n].
+struct M2KSums {
+    float cs[4], cs2[4], cu[8][4];
+};
 
-    // ================================ K side: scores ==========================================
-    const uint32_t* kp[2];
-    uint4 mw[2];
-    uint32_t wbase[2];
-    float sp[2], sp2[2];
-    float ratio[2];  // rs / mult of rows g, g + 8: scales the residual part of the rotor sums after their GEMM
+// Returns whether a word of the lane needs another path than the common one.
+__device__ __forceinline__ bool m2_open_rows(M2KRows& kr, const unsigned char* __restrict__ S, int r0, int kvh, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    bool odd = false;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         const int row = (r0 + g + 8 * x) * HKV + kvh;
-        kp[x] = reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY);
-        mw[x] = *reinterpret_cast<const uint4*>(S + M2_OFF_MASK + row * 64 + 16 * t);
+        kr.kp[x] = reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY);
+        const uint4 m = *reinterpret_cast<const uint4*>(S + M2_OFF_MASK + row * 64 + 16 * t);
+        kr.mw[x] = m;
         // outliers of this thread's quarter, then the ordinal of its first one (scan over the quad)
-        int cnt = (int)(khq3::k3_count(mw[x].x) + khq3::k3_count(mw[x].y) + khq3::k3_count(mw[x].z) + khq3::k3_count(mw[x].w));
-        int incl = cnt;
-        int up = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+        const uint32_t wc = khq3::k3_count(m.x) + (khq3::k3_count(m.y) << 8) + (khq3::k3_count(m.z) << 16) + (khq3::k3_count(m.w) << 24);
+        const uint32_t cnt = (wc * 0x01010101u) >> 24;
+        uint32_t incl = cnt;
+        uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
         if (t >= 1) incl += up;
         up = __shfl_up_sync(0xFFFFFFFFu, incl, 2);
         if (t >= 2) incl += up;
-        wbase[x] = (uint32_t)(incl - cnt);
-        float mult = (float)kp[x][0] / 1000.0f;
-        if (mult < 0.1f || mult > 10.0f || isnan(mult)) mult = 1.0f;
-        const float rs = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_KRN)[row]);
-        const float kn = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_KN)[row]);
-        sp[x] = P.alpha_k * kn * mult * scale;
-        sp2[x] = P.alpha_k * kn * rs * scale;
-        ratio[x] = rs / mult;
+        kr.wc[x] = wc;
+        kr.first[x] = incl - cnt;
+        khq3::kq_open(kr.kq[x], kr.kp[x], kr.first[x], cnt);
+        odd = odd || cnt > khq3::KQ_MAX || ((wc + 0x07070707u) & 0x10101010u) != 0u;  // a word with 9 .. 16 outliers
     }
-    const uint32_t neg1024 = 0xE400E400u;  // fp16x2 (-1024, -1024)
-    float cs[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // pass-part scores, ternary part: rows g (0,1), g+8 (2,3); heads 2t, 2t+1
-    float cs2[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // pass-part scores, residual part (exact integer operand)
-    float cu[8][4];                          // rotor block sums u[token, 8j + n]
-    float cur[4];                            // their residual part, before the row scale
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cu[j][0] = cu[j][1] = cu[j][2] = cu[j][3] = 0.0f;
+    return odd;
+}
+
+// Mask word wi of row x into operand words.  ANY: words with more than eight outliers and quarters with more than the
+// window holds come up.
+template <bool ANY>
+__device__ __forceinline__ void m2_word(M2KRows& kr, int x, int wi, uint32_t (&t2)[8], uint32_t (&c2)[8]) {
+    const uint32_t w = wi == 0 ? kr.mw[x].x : wi == 1 ? kr.mw[x].y : wi == 2 ? kr.mw[x].z : kr.mw[x].w;
+    const uint32_t cnt = (kr.wc[x] >> (8 * wi)) & 0xFFu;
+    if (!ANY) {
+        khq3::kq_word(kr.kq[x], w, cnt, t2, c2);
+    } else if (((kr.wc[x] * 0x01010101u) >> 24) > khq3::KQ_MAX) {
+        khq3::kq_word_slow(w, kr.first[x] + (((wi ? kr.wc[x] << (32 - 8 * wi) : 0u) * 0x01010101u) >> 24), kr.kp[x], t2, c2);
+    } else if (cnt > 8u) {
+        khq3::kq_word_dense(kr.kq[x], w, t2, c2);
+    } else {
+        khq3::kq_word(kr.kq[x], w, cnt, t2, c2);
+    }
+}
+
+template <bool ANY>
+__device__ __forceinline__ void m2_k_gemm(M2KRows& kr, const M2Query& Q, const float (&ratio)[2], M2KSums& ks) {
+    float (&cs)[4] = ks.cs, (&cs2)[4] = ks.cs2, (&cu)[8][4] = ks.cu;
+    float cur[4];  // residual part of a rotor tile, before the row scale
     uint32_t qf[2][8], rf[2][8];  // this and the next k-step's query and rotor fragments
     m2_tm_ld8(Q.tm, qf[0]);
     m2_tm_ld8(Q.rot, rf[0]);
 #pragma unroll
     for (int wi = 0; wi < 4; ++wi) {
-        const uint32_t wa = wi == 0 ? mw[0].x : wi == 1 ? mw[0].y : wi == 2 ? mw[0].z : mw[0].w;
-        const uint32_t wb = wi == 0 ? mw[1].x : wi == 1 ? mw[1].y : wi == 2 ? mw[1].z : mw[1].w;
         // a whole mask word (16 dims = this thread's share of four k-steps) of each of the two rows at once
-        uint32_t ta[8], ha[8], tb[8], hb[8];
-        wbase[0] += khq3::k3_word(wa, wbase[0], kp[0], ta, ha);
-        wbase[1] += khq3::k3_word(wb, wbase[1], kp[1], tb, hb);
+        uint32_t ta[8], xa[8], tb[8], xb[8];
+        m2_word<ANY>(kr, 0, wi, ta, xa);
+        m2_word<ANY>(kr, 1, wi, tb, xb);
+        if (ANY) __syncwarp();
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int s = wi * 4 + q;
             const uint32_t a1[4] = {ta[q], tb[q], ta[4 + q], tb[4 + q]};  // dims (4q, 4q + 2) and (4q + 1, 4q + 3) of rows g, g + 8
-            const uint32_t ax[4] = {m2_hfma2(ta[q], neg1024, ha[q]), m2_hfma2(tb[q], neg1024, hb[q]),
-                                    m2_hfma2(ta[4 + q], neg1024, ha[4 + q]), m2_hfma2(tb[4 + q], neg1024, hb[4 + q])};  // sign*code, exact
+            const uint32_t ax[4] = {xa[q], xb[q], xa[4 + q], xb[4 + q]};  // sign * code
             m2_tm_ld_wait();
             if (s + 1 < 16) {
                 m2_tm_ld8(Q.tm + 8 * (s + 1), qf[(s + 1) & 1]);
@@ -536,16 +562,25 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             }
             const uint32_t(&qq)[8] = qf[s & 1];  // q1.x, q1.y, q2.x, q2.y, then their low-order halves
             const uint32_t(&rr)[8] = rf[s & 1];  // b1.x, b1.y, b2.x, b2.y, then their low-order halves
-            m2_mma(cs, a1, qq[0], qq[1]);
+            if (s == 0) {
+                m2_mma0(cs, a1, qq[0], qq[1]);
+                m2_mma0(cs2, ax, qq[2], qq[3]);
+            } else {
+                m2_mma(cs, a1, qq[0], qq[1]);
+                m2_mma(cs2, ax, qq[2], qq[3]);
+            }
+            // residual part of the rotor sums: exact operand first, the row's scale in fp32 after the two k-steps that
+            // feed this tile
+            if ((s & 1) == 0) {
+                m2_mma0(cu[s >> 1], a1, rr[0], rr[1]);
+                m2_mma0(cur, ax, rr[2], rr[3]);
+            } else {
+                m2_mma(cu[s >> 1], a1, rr[0], rr[1]);
+                m2_mma(cur, ax, rr[2], rr[3]);
+            }
             m2_mma_lo(cs, a1, qq[4], qq[5]);  // low-order halves of the query operands: the code operands are exact
-            m2_mma(cs2, ax, qq[2], qq[3]);
             m2_mma_lo(cs2, ax, qq[6], qq[7]);
-            m2_mma(cu[s >> 1], a1, rr[0], rr[1]);
             m2_mma_lo(cu[s >> 1], a1, rr[4], rr[5]);
-            // residual part of the same rotor sums: exact integer operand first, the row's rs / mult in fp32 after the
-            // two k-steps that feed this tile
-            if ((s & 1) == 0) cur[0] = cur[1] = cur[2] = cur[3] = 0.0f;
-            m2_mma(cur, ax, rr[2], rr[3]);
             m2_mma_lo(cur, ax, rr[6], rr[7]);
             if (s & 1) {
                 float* c = cu[s >> 1];
@@ -554,8 +589,63 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             }
         }
     }
+}
+// Blocks with a word off the common path (about one in 300 at 11 % outliers), out of line: as branches inside the common
+// path the rare words cost copies of all operand registers (MOVs were 15 % of the instructions).
+__device__ __noinline__ void m2_k_gemm_odd(const M2KRows& kr0, const M2Query& Q0, float ratio0, float ratio1, M2KSums& out) {
+    M2KRows kr = kr0;
+    const M2Query Q = Q0;
+    M2KSums ks;
+    const float ratio[2] = {ratio0, ratio1};
+    m2_k_gemm<true>(kr, Q, ratio, ks);
+    out = ks;
+}
+
+// One block of 16 tokens (rows r0..r0+15 of the staged tile) of kv-head `kvh`.
+// valid_lo/valid_hi: block-relative range of tokens that belong to the caller's range.
+__device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, const unsigned char* __restrict__ smem,
+                                         const float* __restrict__ rope, int r0, int kvh, int lane, int valid_lo,
+                                         int valid_hi, const M2Query& Q, const CompressedKV& P, float scale,
+                                         M2State& st) {
+    const int g = lane >> 2, t = lane & 3;
+    const float* dinv_s = reinterpret_cast<const float*>(smem + M2_SM_DINV);
+    const uint2* qr_s = reinterpret_cast<const uint2*>(smem + M2_SM_QR) + kvh * 4 * 32;
+    float4* rsc = reinterpret_cast<float4*>(const_cast<unsigned char*>(smem) + M2_SM_RSC) + 32 * (threadIdx.x >> 5);
+
+    // ---- the block's row scalars, one row per lane ---------------------------------------------
+    // {score scale of the ternary part, of the residual part, residual / ternary scale of the rotor sums, -} and the three
+    // V scales {dims 0..2, dim-3 centroid bit, dim-3 residual field, -}; the residual operand is in units of 2^-24
+    if (lane < 16) {
+        const int row = (r0 + lane) * HKV + kvh;
+        float mult = (float)*reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY) / 1000.0f;
+        if (mult < 0.1f || mult > 10.0f || isnan(mult)) mult = 1.0f;
+        const float rs = 16777216.0f * hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_KRN)[row]);
+        const float kn = P.alpha_k * scale * hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_KN)[row]);
+        const float vn = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VN)[row]);
+        const float en = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VRN)[row]);
+        const float sm = reinterpret_cast<const float*>(S + M2_OFF_VSM)[row];
+        const bool in = lane >= valid_lo && lane < valid_hi;
+        rsc[2 * lane] = make_float4(kn * mult, kn * rs, rs / mult, 0.0f);
+        rsc[2 * lane + 1] = in ? make_float4(P.alpha_v * vn * en, vn, sm * vn * (1.0f / 7.0f), 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    // ================================ K side: scores ==========================================
+    M2KRows kr;
+    const bool odd = m2_open_rows(kr, S, r0, kvh, lane);
+    __syncwarp();
+    const float ratio[2] = {rsc[2 * g].z, rsc[2 * (g + 8)].z};
+    M2KSums ks;
+    if (!__any_sync(0xFFFFFFFFu, odd)) {
+        m2_k_gemm<false>(kr, Q, ratio, ks);
+    } else {  // only these have their address taken
+        const M2KRows krm = kr;
+        const M2Query Qm = Q;
+        M2KSums ksm;
+        m2_k_gemm_odd(krm, Qm, ratio[0], ratio[1], ksm);
+        ks = ksm;
+    }
+    float (&cs)[4] = ks.cs, (&cs2)[4] = ks.cs2, (&cu)[8][4] = ks.cu;
     // ---- rotary part: rest of H64 over idx = 8j + 2t + e, /d, rotation, dot with the raw query ----
-    float cr[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float cr[4];
     {
         // index bits 0..2 were transformed inside the GEMM (folded into the rotor operand)
         // bits 3, 4, 5 (j)
@@ -570,20 +660,22 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
                         m2_add2(cu[j][e], cu[j][e + 1], a0, a1, b0, b1);
                         m2_sub2(cu[j | m][e], cu[j | m][e + 1], a0, a1, b0, b1);
                     }
-        // scale by dinv, rotate pairs (idx, idx + 32) = tiles (j, j + 4)
+        // scale by dinv, rotate pairs (idx, idx + 32) = tiles (j, j + 4): two neighbouring pairs per packed operation
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 dlo = *reinterpret_cast<const float2*>(dinv_s + 8 * j + 2 * t);
             const float2 dhi = *reinterpret_cast<const float2*>(dinv_s + 32 + 8 * j + 2 * t);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const float4 rc = *reinterpret_cast<const float4*>(rope + (r0 + g + 8 * x) * 32 + 8 * j + 2 * t);
-                const float z0 = cu[j][2 * x] * dlo.x, z1 = cu[j][2 * x + 1] * dlo.y;
-                const float w0 = cu[j + 4][2 * x] * dhi.x, w1 = cu[j + 4][2 * x + 1] * dhi.y;
-                cu[j][2 * x] = z0 * rc.x - w0 * rc.y;
-                cu[j + 4][2 * x] = z0 * rc.y + w0 * rc.x;
-                cu[j][2 * x + 1] = z1 * rc.z - w1 * rc.w;
-                cu[j + 4][2 * x + 1] = z1 * rc.w + w1 * rc.z;
+                const float4 rc = *reinterpret_cast<const float4*>(rope + (r0 + g + 8 * x) * 64 + 16 * j + 4 * t);  // cos, cos, sin, sin
+                float *a = &cu[j][2 * x], *b = &cu[j + 4][2 * x];
+                float z0, z1, w0, w1, u0, u1;
+                m2_mul2(z0, z1, a[0], a[1], dlo.x, dlo.y);
+                m2_mul2(w0, w1, b[0], b[1], dhi.x, dhi.y);
+                m2_mul2(u0, u1, w0, w1, -rc.z, -rc.w);
+                m2_fma2(a[0], a[1], z0, z1, rc.x, rc.y, u0, u1);
+                m2_mul2(u0, u1, w0, w1, rc.x, rc.y);
+                m2_fma2(b[0], b[1], z0, z1, rc.z, rc.w, u0, u1);
             }
         }
 #pragma unroll
@@ -594,53 +686,66 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             m2_pack_hilo(cu[2 * kk + 1][0], cu[2 * kk + 1][1], a[2], al[2]);
             m2_pack_hilo(cu[2 * kk + 1][2], cu[2 * kk + 1][3], a[3], al[3]);
             const uint2 qrk = qr_s[kk * 32 + lane];
-            m2_mma(cr, a, qrk.x, qrk.y);
+            if (kk == 0) m2_mma0(cr, a, qrk.x, qrk.y);
+            else m2_mma(cr, a, qrk.x, qrk.y);
             m2_mma_lo(cr, al, qrk.x, qrk.y);
         }
     }
     // ================================ softmax over the block ====================================
     float sc[2][2], pw[2][2];  // [row x: g, g+8][head e: 2t, 2t+1]
     bool valid[2];
+    bool raise = false;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         valid[x] = (g + 8 * x) >= valid_lo && (g + 8 * x) < valid_hi;
+        const float2 sp = *reinterpret_cast<const float2*>(rsc + 2 * (g + 8 * x));
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            sc[x][e] = valid[x] ? fmaf(sp[x], cs[2 * x + e] + cr[2 * x + e], sp2[x] * cs2[2 * x + e]) : -1e30f;
+        for (int e = 0; e < 2; ++e) {
+            sc[x][e] = valid[x] ? fmaf(sp.x, cs[2 * x + e] + cr[2 * x + e], sp.y * cs2[2 * x + e]) : -1e30f;
+            st.top[e] = fmaxf(st.top[e], sc[x][e]);
+            raise = raise || sc[x][e] > st.m[e] + M2_SLACK;
+        }
     }
-    float corr[2];
+    // The reference the weights are taken against follows the maximum only when a score is M2_SLACK above it: the weights
+    // stay below e^2, and most blocks need no reduction over the warp and no pass over the accumulators.
+    float corr[2] = {1.0f, 1.0f};
+    const bool rescale = __any_sync(0xFFFFFFFFu, raise);
+    if (rescale) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float bm = fmaxf(sc[0][e], sc[1][e]);
+            bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 4));
+            bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 8));
+            bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 16));
+            const float mn = fmaxf(st.m[e], bm);
+            corr[e] = __expf(st.m[e] - mn);
+            st.m[e] = mn;
+            st.l[e] *= corr[e];
+            st.p2[e] *= corr[e];
+            st.p3[e] *= corr[e];
+        }
+    }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        float bm = fmaxf(sc[0][e], sc[1][e]);
-        bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 4));
-        bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 8));
-        bm = fmaxf(bm, __shfl_xor_sync(0xFFFFFFFFu, bm, 16));
-        const float mn = fmaxf(st.m[e], bm);
-        corr[e] = __expf(st.m[e] - mn);
-        st.m[e] = mn;
-        pw[0][e] = valid[0] ? __expf(sc[0][e] - mn) : 0.0f;
-        pw[1][e] = valid[1] ? __expf(sc[1][e] - mn) : 0.0f;
-        st.l[e] = st.l[e] * corr[e] + pw[0][e] + pw[1][e];
+        pw[0][e] = valid[0] ? __expf(sc[0][e] - st.m[e]) : 0.0f;
+        pw[1][e] = valid[1] ? __expf(sc[1][e] - st.m[e]) : 0.0f;
+        st.l[e] += pw[0][e] + pw[1][e];
     }
-    const bool rescale = __any_sync(0xFFFFFFFFu, corr[0] != 1.0f || corr[1] != 1.0f);
     // three scaled variants of P, transposed into B fragments (tokens = k, heads = n)
     uint32_t pb[3][2], pl_[3][2];  // fp16 hi and the fp16 of what hi lost
     {
         float s1[2], s2[2], s3[2];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-            const int row = (r0 + g + 8 * x) * HKV + kvh;
-            const float vn = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VN)[row]);
-            const float en = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VRN)[row]);
-            const float sm = reinterpret_cast<const float*>(S + M2_OFF_VSM)[row];
-            s1[x] = valid[x] ? P.alpha_v * vn * en : 0.0f;     // dims 0..2: codebook entry
-            s2[x] = valid[x] ? vn : 0.0f;                      // dim 3: centroid bit
-            s3[x] = valid[x] ? sm * vn * (1.0f / 7.0f) : 0.0f;  // dim 3: residual field
+            const float4 v = rsc[2 * (g + 8 * x) + 1];
+            s1[x] = v.x;  // dims 0..2: codebook entry
+            s2[x] = v.y;  // dim 3: centroid bit
+            s3[x] = v.z;  // dim 3: residual field
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            st.p2[e] = fmaf(pw[1][e], s2[1], fmaf(pw[0][e], s2[0], st.p2[e] * corr[e]));
-            st.p3[e] = fmaf(pw[1][e], s3[1], fmaf(pw[0][e], s3[0], st.p3[e] * corr[e]));
+            st.p2[e] = fmaf(pw[1][e], s2[1], fmaf(pw[0][e], s2[0], st.p2[e]));
+            st.p3[e] = fmaf(pw[1][e], s3[1], fmaf(pw[0][e], s3[0], st.p3[e]));
         }
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
@@ -745,7 +850,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
                                                     float scale, unsigned& tiles_done, WarpState& ws, uint32_t tmem) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
-    float2* rope_tab = reinterpret_cast<float2*>(smem + M2_SM_ROPE);
+    float* rope_tab = reinterpret_cast<float*>(smem + M2_SM_ROPE);
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
 
@@ -779,16 +884,16 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
             m2_stage_tile(P, smem + M2_SM_STAGES + ((gi + 1) % M2_NSTAGE) * M2_STAGE_BYTES, &bars[(gi + 1) % M2_NSTAGE],
                           tok0, min(M2_TT, P.c_len - tok0), tid);
             if (P.pos_chunk == 0 && ((i + 1) % M2_ROPE_RESEED) != 0)
-                m2_step_rope(rope_tab + ((i + 1) & 1) * M2_TT * 32, rope_tab + (i & 1) * M2_TT * 32,
-                             reinterpret_cast<const float2*>(smem + M2_SM_RSTEP), tid);
+                m2_step_rope(rope_tab + ((i + 1) & 1) * M2_TT * 64, rope_tab + (i & 1) * M2_TT * 64,
+                             reinterpret_cast<const float*>(smem + M2_SM_RSTEP), tid);
             else
-                m2_fill_rope(rope_tab + ((i + 1) & 1) * M2_TT * 32, freq_s, P, tok0, tid);
+                m2_fill_rope(rope_tab + ((i + 1) & 1) * M2_TT * 64, freq_s, P, tok0, tid);
         }
         mbar_wait_bounded(&bars[stg], (uint32_t)((gi / M2_NSTAGE) & 1), &g_status);
         const int blk0 = base + i * M2_TT + 16 * sub;
         const int vlo = max(my_lo - blk0, 0), vhi = min(my_hi - blk0, 16);
         if (vhi > vlo)
-            m2_block(smem + M2_SM_STAGES + stg * M2_STAGE_BYTES, smem, rope_tab + (i & 1) * M2_TT * 32, 16 * sub, kvh,
+            m2_block(smem + M2_SM_STAGES + stg * M2_STAGE_BYTES, smem, rope_tab + (i & 1) * M2_TT * 64, 16 * sub, kvh,
                      lane, vlo, vhi, Q, P, scale, st);
         __syncthreads();  // stage and rope buffer free for the tile after next
     }
@@ -803,6 +908,15 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
             st.p2[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p2[e], m);
             st.p3[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p3[e], m);
         }
+    // the record is relative to the largest score itself
+    float fin[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int m = 4; m <= 16; m <<= 1) st.top[e] = fmaxf(st.top[e], __shfl_xor_sync(0xFFFFFFFFu, st.top[e], m));
+        fin[e] = __expf(st.m[e] - st.top[e]);
+        st.l[e] *= fin[e];
+    }
     float* rec = reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * MERGE_FLOATS;
     const float2* c3s = reinterpret_cast<const float2*>(smem + M2_SM_C3) + 8 * g;
 #pragma unroll
@@ -815,23 +929,23 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
             float* rp = rec + 2 * t * D + 4 * (8 * g + 2 * pp);  // head 2t, dim 0 of patch 2pp; head 2t + 1 is D further
 #pragma unroll
             for (int idx = 0; idx < 6; ++idx) {
-                rp[4 * (idx / 3) + idx % 3] = o[idx >> 1][2 * (idx & 1)];
-                rp[D + 4 * (idx / 3) + idx % 3] = o[idx >> 1][2 * (idx & 1) + 1];
+                rp[4 * (idx / 3) + idx % 3] = fin[0] * o[idx >> 1][2 * (idx & 1)];
+                rp[D + 4 * (idx / 3) + idx % 3] = fin[1] * o[idx >> 1][2 * (idx & 1) + 1];
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const float2 c = c3s[2 * pp + u];
 #pragma unroll
                 for (int e = 0; e < 2; ++e)
-                    rp[e * D + 4 * u + 3] = fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
-                                            fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]);
+                    rp[e * D + 4 * u + 3] = fin[e] * (fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
+                                                      fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]));
             }
         }
     }
     if (t < 3) {
         if (g == 0) {
-            rec[NREP * D + 2 * t] = st.m[0];
-            rec[NREP * D + 2 * t + 1] = st.m[1];
+            rec[NREP * D + 2 * t] = st.top[0];
+            rec[NREP * D + 2 * t + 1] = st.top[1];
             rec[NREP * D + NREP + 2 * t] = st.l[0];
             rec[NREP * D + NREP + 2 * t + 1] = st.l[1];
         }

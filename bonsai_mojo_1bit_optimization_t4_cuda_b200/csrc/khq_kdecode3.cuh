@@ -62,6 +62,14 @@ KHQ3_HD uint32_t k3_funnel_r(uint32_t lo, uint32_t hi, uint32_t sh) {
     return sh ? ((lo >> sh) | (hi << (32 - sh))) : lo;
 #endif
 }
+// the same for shifts up to 32
+KHQ3_HD uint32_t k3_funnel_rc(uint32_t lo, uint32_t hi, uint32_t sh) {
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_rc(lo, hi, sh);
+#else
+    return sh >= 32u ? hi : k3_funnel_r(lo, hi, sh);
+#endif
+}
 KHQ3_HD uint32_t k3_popc(uint32_t x) {
 #if defined(__CUDA_ARCH__)
     return (uint32_t)__popc(x);
@@ -170,6 +178,96 @@ KHQ3_HD uint32_t k3_word(uint32_t w, uint32_t ob, const uint32_t* kp, uint32_t (
         h2[2 * q + 1] = k3_prmt(hq, gc, 0x3726u);
     }
     return cnt;
+}
+
+// ---- the same decode for the mma.sync kernel: a lane walks the four mask words of a 64-dim quarter of a row ----
+// Differences from k3_word: the residual operand is c = sign * code as a subnormal fp16 number (low byte = the code
+// itself, units of 2^-24; no bias to take off afterwards), the quarter's codes and signs are fetched once and shifted
+// along, and the prefix sums, the ordinals and the selectors come out of a few multiply-adds.
+struct KQuarter {
+    uint32_t c0, c1, c2;  // the next 24 residual codes, four bits each
+    uint32_t neg;         // the signs of at least 24 entries, 1 = negative
+};
+constexpr uint32_t KQ_MAX = 24;  // outliers of a quarter that the window holds; more: kq_word_slow for its words
+
+// `ob` = ordinal of the quarter's first outlier, `cnt` = its outliers, `kp` = the row's ten payload words (up to 29 words
+// from kp are read for rows with more outlier symbols than the format holds).
+KHQ3_HD void kq_open(KQuarter& q, const uint32_t* kp, uint32_t ob, uint32_t cnt) {
+    const uint32_t* c = kp + 1 + (ob >> 3);
+    const uint32_t sh = (4u * ob) & 31u;
+    q.c0 = k3_funnel_r(c[0], c[1], sh);
+    q.c1 = k3_funnel_r(c[1], c[2], sh);
+    q.c2 = k3_funnel_r(c[2], c[3], sh);
+    const uint32_t sb = 232u + ob;
+    q.neg = ~k3_funnel_r(kp[sb >> 5], kp[(sb >> 5) + 1u], sb & 31u);
+    if (ob + cnt > 50u) {  // entries past the 50 of the format read as code 0, negative
+        const uint32_t left = ob < 50u ? 50u - ob : 0u;
+        q.c0 &= left >= 8u ? ~0u : (1u << (4u * left)) - 1u;
+        q.c1 &= left >= 16u ? ~0u : left <= 8u ? 0u : (1u << (4u * (left - 8u))) - 1u;
+        q.c2 &= left >= 24u ? ~0u : left <= 16u ? 0u : (1u << (4u * (left - 16u))) - 1u;
+        q.neg |= left >= 32u ? 0u : ~0u << left;
+    }
+}
+KHQ3_HD void kq_advance(KQuarter& q, uint32_t n) {  // n <= 8
+    q.c0 = k3_funnel_rc(q.c0, q.c1, 4u * n);
+    q.c1 = k3_funnel_rc(q.c1, q.c2, 4u * n);
+    q.c2 = k3_funnel_rc(q.c2, 0u, 4u * n);
+    q.neg >>= n;
+}
+// Decodes the quarter's next mask word, which has cnt <= 8 outliers: operand words as in k3_word, t and c.
+KHQ3_HD void kq_word(KQuarter& q, uint32_t w, uint32_t cnt, uint32_t (&t2)[8], uint32_t (&c2)[8]) {
+    const uint32_t E = w & 0x33333333u, O = (w >> 2) & 0x33333333u;  // even / odd symbols, one per nibble
+    const uint32_t b = w & (w >> 1);
+    const uint32_t e3 = b & 0x11111111u, o3 = (b >> 2) & 0x11111111u;  // outliers
+    // ordinal of every dim inside the word (nibble-wise prefix sums, at most 8: no carries), with bit 3 set where there is no
+    // outlier: a permute selector that replicates the (clear) top bit of a table byte, i.e. zero
+    const uint32_t ordO = e3 * 0x11111111u + o3 * 0x11111110u;
+    const uint32_t selE = (ordO - e3) | (0x88888888u - 8u * e3), selO = ordO | (0x88888888u - 8u * o3);
+    // tables of eight bytes: residual codes and signs (bit 6) of the next entries
+    const uint32_t ev = q.c0 & 0x0F0F0F0Fu, od = (q.c0 >> 4) & 0x0F0F0F0Fu;
+    const uint32_t ca = k3_prmt(ev, od, 0x5140u), cb = k3_prmt(ev, od, 0x7362u);
+    const uint32_t sa = ((q.neg & 0x0Fu) * 0x08102040u) & 0x40404040u, sb = ((q.neg & 0xF0u) * 0x00810204u) & 0x40404040u;
+    kq_advance(q, cnt);
+    const uint32_t lut = 0x3C3CBC00u;  // fp16 high bytes of 0, -1, +1, +1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t sel = i == 0 ? selE : i == 1 ? selE >> 16 : i == 2 ? selO : selO >> 16;
+        const uint32_t sym = i == 0 ? E : i == 1 ? E >> 16 : i == 2 ? O : O >> 16;
+        const uint32_t g = k3_prmt(ca, cb, sel), s = 2u * k3_prmt(sa, sb, sel);
+        const uint32_t t = k3_prmt(lut, 0u, sym) + s;  // negative outliers: 0x3C -> 0xBC
+        t2[2 * i] = k3_prmt(t, 0u, 0x1404u);
+        t2[2 * i + 1] = k3_prmt(t, 0u, 0x3424u);
+        c2[2 * i] = k3_prmt(g, s, 0x5140u);
+        c2[2 * i + 1] = k3_prmt(g, s, 0x7362u);
+    }
+}
+// The same for a word with more than eight outliers, four dims at a time (about one word in 80 000 at 11 % outliers).
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__
+#else
+inline
+#endif
+void kq_word_dense(KQuarter& q, uint32_t w, uint32_t (&t2)[8], uint32_t (&c2)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t2[j] = c2[j] = 0u;
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t part = w & (0xFFu << (8 * i));
+        uint32_t t[8], c[8];
+        kq_word(q, part, k3_count(part), t, c);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // the other dims of the word come out as zero
+            t2[j] |= t[j];
+            c2[j] |= c[j];
+        }
+    }
+}
+// Per-dim path: any word, any ordinal.
+KHQ3_HD void kq_word_slow(uint32_t w, uint32_t ob, const uint32_t* kp, uint32_t (&t2)[8], uint32_t (&c2)[8]) {
+    uint32_t hs[8];
+    k3_word_slow(w, ob, kp, t2, hs);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c2[j] = hs[j] & 0x800F800Fu;  // the sign and the code of sign * (1024 + code)
 }
 
 // The eight 12-bit fields of one three-word group of a V payload row.
