@@ -32,10 +32,12 @@
 namespace khq {
 
 constexpr int M2_WPK = 3;           // warps per kv-head (12 warps: three per scheduler, at most 168 registers each)
-constexpr int M2_TT = 16 * M2_WPK;  // tokens per tile: every warp of a kv-head takes 16
+constexpr int M2_BT = 16;           // tokens per block: one warp's share of a stage
+constexpr int M2_TT = M2_BT * M2_WPK;  // tokens that the CTA's three groups advance together
 constexpr int M2_THREADS = 32 * HKV * M2_WPK;
-constexpr int M2_NSTAGE = 2;
-constexpr int M2_ROWS = M2_TT * HKV;
+constexpr int M2_GTHREADS = 32 * HKV;  // a group: the four warps (one per kv-head) that share a block
+constexpr int M2_NSTAGE = 2;           // stages per group
+constexpr int M2_ROWS = M2_BT * HKV;
 constexpr int M2_OFF_MASK = 0;
 constexpr int M2_OFF_KPAY = M2_OFF_MASK + M2_ROWS * 64;
 constexpr int M2_OFF_VPAY = M2_OFF_KPAY + M2_ROWS * K_PAY;
@@ -44,7 +46,8 @@ constexpr int M2_OFF_KRN = M2_OFF_KN + M2_ROWS * 2;
 constexpr int M2_OFF_VN = M2_OFF_KRN + M2_ROWS * 2;
 constexpr int M2_OFF_VRN = M2_OFF_VN + M2_ROWS * 2;
 constexpr int M2_OFF_VSM = M2_OFF_VRN + M2_ROWS * 2;
-constexpr int M2_STAGE_BYTES = M2_OFF_VSM + M2_ROWS * 4;  // 28160
+constexpr int M2_STAGE_BYTES = M2_OFF_VSM + M2_ROWS * 4;  // 14080
+constexpr int M2_STAGES_BYTES = M2_WPK * M2_NSTAGE * M2_STAGE_BYTES;
 
 constexpr int M2_SM_STAGES = 0;
 // V codebook, one row per code: for every pair of patches the two (d0, d1) words, then the two d2 halfs
@@ -52,8 +55,8 @@ constexpr int M2_SM_STAGES = 0;
 // padding: the bank of a look-up then depends on the code as well as on the patch, which spreads the
 // warp's 32 look-ups (8 patches x 4 tokens per instruction) over the banks.
 constexpr int M2_VQ_ROW = (NP / 2) * 12 + 4;                         // 388 bytes per code
-constexpr int M2_SM_VQ = M2_SM_STAGES + M2_NSTAGE * M2_STAGE_BYTES;
-constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // 2 x M2_TT tokens x 64 floats
+constexpr int M2_SM_VQ = M2_SM_STAGES + M2_STAGES_BYTES;
+constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // per group two buffers of M2_BT tokens x 64 floats
 constexpr int M2_SM_BROT = M2_SM_ROPE + 2 * M2_TT * 64 * 4;          // 4 kinds x 16 steps x 32 lanes x 8 B: set-up only,
 constexpr int M2_SM_RSC = M2_SM_BROT;                                //   then 16 rows x 2 float4 per warp: scalars of a block's rows
 constexpr int M2_SM_FREQ = M2_SM_BROT + 4 * 16 * 32 * 8;
@@ -80,8 +83,8 @@ static_assert(M2_TM_ACC + M2_TM_ACC_WARP * M2_WPK <= M2_TM_COLS, "tensor-memory 
 static_assert(M2_SM_TOTAL <= 227 * 1024 && M2_SM_C3 % 16 == 0 && M2_SM_ROPE % 16 == 0 && M2_SM_VQ % 16 == 0,
               "shared memory budget");
 static_assert(HKV * MERGE_FLOATS * 4 <= 256 * M2_VQ_ROW, "cluster export records alias the codebook");
-static_assert(HKV * M2_WPK * MERGE_FLOATS * 4 <= M2_NSTAGE * M2_STAGE_BYTES, "records alias the stages");
-static_assert(HKV * NREP * D * 4 <= M2_NSTAGE * M2_STAGE_BYTES, "prologue scratch aliases the stages");
+static_assert(HKV * M2_WPK * MERGE_FLOATS * 4 <= M2_STAGES_BYTES, "records alias the stages");
+static_assert(HKV * NREP * D * 4 <= M2_STAGES_BYTES, "prologue scratch aliases the stages");
 static_assert(M2_STAGE_BYTES % 16 == 0 && M2_OFF_KPAY % 16 == 0 && M2_OFF_VPAY % 16 == 0 && M2_OFF_KN % 16 == 0 &&
                   M2_OFF_VSM % 16 == 0, "bulk copy alignment");
 
@@ -115,9 +118,16 @@ __device__ __forceinline__ void m2_pack_hilo(float a, float b, uint32_t& hi, uin
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = m2_pack(a - __low2float(h), b - __high2float(h));
 }
-// Stage `ntok` tokens starting at `tok0` (same contract as stage_tile of the first generation).
+// The CTA's three groups (warps of the same warp >> 2) walk their own blocks at their own pace: a barrier of the whole CTA
+// per tile made the twelve warps run through the same phase together, all of them on the same pipe, and wait for the slowest.
+__device__ __forceinline__ void m2_group_sync(int sub) {
+    asm volatile("bar.sync %0, %1;" ::"r"(2 + HKV + sub), "n"(M2_GTHREADS) : "memory");
+}
+
+// Stage `ntok` tokens starting at `tok0` for group `sub` (tid: thread inside the group; same contract as stage_tile of the
+// first generation).
 __device__ __forceinline__ void m2_stage_tile(const CompressedKV& P, unsigned char* stage, uint64_t* bar, int tok0,
-                                              int ntok, int tid) {
+                                              int ntok, int tid, int sub) {
     const size_t r0 = (size_t)tok0 * HKV;
     const int rows = ntok * HKV;
     const unsigned char* src[8] = {reinterpret_cast<const unsigned char*>(P.k_mask) + r0 * 64,
@@ -143,17 +153,17 @@ __device__ __forceinline__ void m2_stage_tile(const CompressedKV& P, unsigned ch
             const int words = rows * bpr[a] / 4;
             const unsigned int* s = reinterpret_cast<const unsigned int*>(src[a]);
             unsigned int* d = reinterpret_cast<unsigned int*>(stage + dst[a]);
-            for (int i = tid; i < words; i += M2_THREADS) d[i] = s[i];
+            for (int i = tid; i < words; i += M2_GTHREADS) d[i] = s[i];
         }
         fence_proxy_async();
-        __syncthreads();
+        m2_group_sync(sub);
         if (tid == 0) mbar_arrive(bar);
     }
 }
 
-// RoPE table of a tile: 64 floats per token; pairs 2i and 2i + 1 are the four floats cos, cos, sin, sin at 4i.
+// RoPE table of a block: 64 floats per token; pairs 2i and 2i + 1 are the four floats cos, cos, sin, sin at 4i.
 __device__ __forceinline__ void m2_fill_rope(float* tab, const float* freq, const CompressedKV& P, int tok0, int tid) {
-    for (int e = tid; e < M2_TT * 32; e += M2_THREADS) {
+    for (int e = tid; e < M2_BT * 32; e += M2_GTHREADS) {
         const int t = e >> 5, m = e & 31;
         double th = (double)token_pos(P, tok0 + t) * (double)freq[m];
         th -= rint(th * 0.15915494309189535) * 6.283185307179586;
@@ -165,14 +175,14 @@ __device__ __forceinline__ void m2_fill_rope(float* tab, const float* freq, cons
     }
 }
 
-// The next tile's RoPE table from this tile's: every entry turns by 32 positions of its pair (four FMAs
+// A group's next RoPE table from its last: every entry turns by M2_TT positions of its pair (four FMAs
 // instead of a range reduction and a sincos).  The caller re-seeds with m2_fill_rope every M2_ROPE_RESEED
-// tiles, so that rounding never accumulates over more than that many turns (< 4e-6), and whenever the
+// blocks, so that rounding never accumulates over more than that many turns (< 4e-6), and whenever the
 // positions are not contiguous.
 constexpr int M2_ROPE_RESEED = 64;
 __device__ __forceinline__ void m2_step_rope(float* dst, const float* src, const float* step, int tid) {
 #pragma unroll
-    for (int e = tid; e < M2_TT * 16; e += M2_THREADS) {
+    for (int e = tid; e < M2_BT * 16; e += M2_GTHREADS) {
         const float4 a = reinterpret_cast<const float4*>(src)[e], d = reinterpret_cast<const float4*>(step)[e & 15];
         reinterpret_cast<float4*>(dst)[e] =
             make_float4(a.x * d.x - a.z * d.z, a.y * d.y - a.w * d.w, a.z * d.x + a.x * d.z, a.w * d.y + a.y * d.w);
@@ -494,12 +504,12 @@ struct M2KSums {
 };
 
 // Returns whether a word of the lane needs another path than the common one.
-__device__ __forceinline__ bool m2_open_rows(M2KRows& kr, const unsigned char* __restrict__ S, int r0, int kvh, int lane) {
+__device__ __forceinline__ bool m2_open_rows(M2KRows& kr, const unsigned char* __restrict__ S, int kvh, int lane) {
     const int g = lane >> 2, t = lane & 3;
     bool odd = false;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
-        const int row = (r0 + g + 8 * x) * HKV + kvh;
+        const int row = (g + 8 * x) * HKV + kvh;
         kr.kp[x] = reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY);
         const uint4 m = *reinterpret_cast<const uint4*>(S + M2_OFF_MASK + row * 64 + 16 * t);
         kr.mw[x] = m;
@@ -601,11 +611,11 @@ __device__ __noinline__ void m2_k_gemm_odd(const M2KRows& kr0, const M2Query& Q0
     out = ks;
 }
 
-// One block of 16 tokens (rows r0..r0+15 of the staged tile) of kv-head `kvh`.
+// One staged block of 16 tokens of kv-head `kvh`.
 // valid_lo/valid_hi: block-relative range of tokens that belong to the caller's range.
 __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, const unsigned char* __restrict__ smem,
-                                         const float* __restrict__ rope, int r0, int kvh, int lane, int valid_lo,
-                                         int valid_hi, const M2Query& Q, const CompressedKV& P, float scale,
+                                         const float* __restrict__ rope, int kvh, int lane, int valid_lo, int valid_hi,
+                                         const M2Query& Q, const CompressedKV& P, float scale,
                                          M2State& st) {
     const int g = lane >> 2, t = lane & 3;
     const float* dinv_s = reinterpret_cast<const float*>(smem + M2_SM_DINV);
@@ -616,7 +626,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     // {score scale of the ternary part, of the residual part, residual / ternary scale of the rotor sums, -} and the three
     // V scales {dims 0..2, dim-3 centroid bit, dim-3 residual field, -}; the residual operand is in units of 2^-24
     if (lane < 16) {
-        const int row = (r0 + lane) * HKV + kvh;
+        const int row = lane * HKV + kvh;
         float mult = (float)*reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY) / 1000.0f;
         if (mult < 0.1f || mult > 10.0f || isnan(mult)) mult = 1.0f;
         const float rs = 16777216.0f * hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_KRN)[row]);
@@ -630,7 +640,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     }
     // ================================ K side: scores ==========================================
     M2KRows kr;
-    const bool odd = m2_open_rows(kr, S, r0, kvh, lane);
+    const bool odd = m2_open_rows(kr, S, kvh, lane);
     __syncwarp();
     const float ratio[2] = {rsc[2 * g].z, rsc[2 * (g + 8)].z};
     M2KSums ks;
@@ -667,7 +677,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             const float2 dhi = *reinterpret_cast<const float2*>(dinv_s + 32 + 8 * j + 2 * t);
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const float4 rc = *reinterpret_cast<const float4*>(rope + (r0 + g + 8 * x) * 64 + 16 * j + 4 * t);  // cos, cos, sin, sin
+                const float4 rc = *reinterpret_cast<const float4*>(rope + (g + 8 * x) * 64 + 16 * j + 4 * t);  // cos, cos, sin, sin
                 float *a = &cu[j][2 * x], *b = &cu[j + 4][2 * x];
                 float z0, z1, w0, w1, u0, u1;
                 m2_mul2(z0, z1, a[0], a[1], dlo.x, dlo.y);
@@ -768,7 +778,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int tok = 2 * t + (i & 1) + 8 * (i >> 1);
-        const uint32_t* row = reinterpret_cast<const uint32_t*>(S + M2_OFF_VPAY + ((r0 + tok) * HKV + kvh) * V_PAY);
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(S + M2_OFF_VPAY + (tok * HKV + kvh) * V_PAY);
 #pragma unroll
         for (int w = 0; w < 3; ++w) vw[i][w] = row[3 * g + w];
         hb[i] = ((row[24 + (g >> 2)] >> (8 * (g & 3))) & 0xFFu) << 7;  // bit 7 + pl = high code bit of patch pl
@@ -840,19 +850,17 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
 }
 
 // Attention of all 24 query heads over compressed tokens [my_lo, my_hi) of P; the CTA's 12 warps
-// are (kv-head = warp & 3) x (16-token third of each 48-token tile = warp >> 2).  On return,
+// are (kv-head = warp & 3) x (group = warp >> 2: every third 16-token block).  On return,
 // warps 0..3 hold in `ws` the merged state of their kv-head's six heads in the first generation's
 // layout (lane = 8 dims, rotated V domain), ready for merge_from / v_epilogue_store.  Tables must
 // be set up; all M2_THREADS threads call it.
 template <bool ALL_WARPS_MERGE = false>  // true: every warp of a kv-head returns the kv-head's merged state
 __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const __half* __restrict__ q,
                                                     size_t q_head_stride, const CompressedKV& P, int my_lo, int my_hi,
-                                                    float scale, unsigned& tiles_done, WarpState& ws, uint32_t tmem) {
+                                                    float scale, unsigned& blocks_done, WarpState& ws, uint32_t tmem) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
-    float* rope_tab = reinterpret_cast<float*>(smem + M2_SM_ROPE);
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
 
     M2Query Q;
     Q.tm = tmem + ((uint32_t)(32 * kvh) << 16);
@@ -863,41 +871,43 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
     __syncthreads();  // the query scratch aliases the stages
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the query and rotor fragments other warps stored
 
-    const int base = my_lo & ~1;
-    const int ntiles = (my_hi > my_lo) ? (my_hi - base + M2_TT - 1) / M2_TT : 0;
-    const unsigned t0 = tiles_done;
-    if (ntiles > 0) {
-        m2_fill_rope(rope_tab, freq_s, P, base, tid);
-        m2_stage_tile(P, smem + M2_SM_STAGES + (t0 % M2_NSTAGE) * M2_STAGE_BYTES, &bars[t0 % M2_NSTAGE], base,
-                      min(M2_TT, P.c_len - base), tid);
+    // group `sub` takes blocks sub, sub + M2_WPK, ... of M2_BT tokens
+    const int base = (my_lo & ~1) + M2_BT * sub, gtid = 32 * kvh + lane;
+    const int nblk = (my_hi > base) ? (my_hi - base + M2_TT - 1) / M2_TT : 0;
+    const unsigned t0 = blocks_done;
+    unsigned char* stages = smem + M2_SM_STAGES + sub * M2_NSTAGE * M2_STAGE_BYTES;
+    float* rope_tab = reinterpret_cast<float*>(smem + M2_SM_ROPE) + sub * 2 * M2_BT * 64;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS) + sub * M2_NSTAGE;
+    if (nblk > 0) {
+        m2_stage_tile(P, stages + (t0 % M2_NSTAGE) * M2_STAGE_BYTES, &bars[t0 % M2_NSTAGE], base, min(M2_BT, P.c_len - base), gtid, sub);
+        m2_fill_rope(rope_tab, freq_s, P, base, gtid);
     }
-    __syncthreads();
     M2State st;
     st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + M2_TM_ACC_WARP * (uint32_t)sub;
     st.init();
+    m2_group_sync(sub);
 #pragma unroll 1
-    for (int i = 0; i < ntiles; ++i) {
+    for (int i = 0; i < nblk; ++i) {
         const unsigned gi = t0 + i;
         const int stg = gi % M2_NSTAGE;
-        if (i + 1 < ntiles) {
+        if (i + 1 < nblk) {
             const int tok0 = base + (i + 1) * M2_TT;
-            m2_stage_tile(P, smem + M2_SM_STAGES + ((gi + 1) % M2_NSTAGE) * M2_STAGE_BYTES, &bars[(gi + 1) % M2_NSTAGE],
-                          tok0, min(M2_TT, P.c_len - tok0), tid);
+            m2_stage_tile(P, stages + ((gi + 1) % M2_NSTAGE) * M2_STAGE_BYTES, &bars[(gi + 1) % M2_NSTAGE], tok0,
+                          min(M2_BT, P.c_len - tok0), gtid, sub);
+            float* next = rope_tab + ((i + 1) & 1) * M2_BT * 64;
             if (P.pos_chunk == 0 && ((i + 1) % M2_ROPE_RESEED) != 0)
-                m2_step_rope(rope_tab + ((i + 1) & 1) * M2_TT * 64, rope_tab + (i & 1) * M2_TT * 64,
-                             reinterpret_cast<const float*>(smem + M2_SM_RSTEP), tid);
+                m2_step_rope(next, rope_tab + (i & 1) * M2_BT * 64, reinterpret_cast<const float*>(smem + M2_SM_RSTEP), gtid);
             else
-                m2_fill_rope(rope_tab + ((i + 1) & 1) * M2_TT * 64, freq_s, P, tok0, tid);
+                m2_fill_rope(next, freq_s, P, tok0, gtid);
         }
         mbar_wait_bounded(&bars[stg], (uint32_t)((gi / M2_NSTAGE) & 1), &g_status);
-        const int blk0 = base + i * M2_TT + 16 * sub;
-        const int vlo = max(my_lo - blk0, 0), vhi = min(my_hi - blk0, 16);
-        if (vhi > vlo)
-            m2_block(smem + M2_SM_STAGES + stg * M2_STAGE_BYTES, smem, rope_tab + (i & 1) * M2_TT * 64, 16 * sub, kvh,
-                     lane, vlo, vhi, Q, P, scale, st);
-        __syncthreads();  // stage and rope buffer free for the tile after next
+        const int blk0 = base + i * M2_TT;
+        m2_block(stages + stg * M2_STAGE_BYTES, smem, rope_tab + (i & 1) * M2_BT * 64, kvh, lane, max(my_lo - blk0, 0), min(my_hi - blk0, M2_BT), Q,
+                 P, scale, st);
+        m2_group_sync(sub);  // stage and rope buffer free for the block after next
     }
-    tiles_done = t0 + (unsigned)ntiles;
+    blocks_done = t0 + (unsigned)nblk;
+    __syncthreads();  // the records alias the stages
 
     // ---- per-warp record in the first generation's layout, then merge + inverse V transform --------
 #pragma unroll
@@ -969,9 +979,9 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
-    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 32);
+    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
     if (tid == 0) {
-        for (int s = 0; s < M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
@@ -979,7 +989,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tm_slot;
     int cur_table = -1;
-    unsigned tiles_done = 0;
+    unsigned blocks_done = 0;
 #pragma unroll 1
     while (true) {
         __syncthreads();
@@ -1010,7 +1020,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
                 m2_rotor_to_tmem(smem, tmem, warp, lane);
             }
             WarpState ws;
-            m2_compressed_range<true>(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, tiles_done, ws, tmem);
+            m2_compressed_range<true>(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, ws, tmem);
             // the three warps of a kv-head transform and store two heads each
             static_assert(M2_WPK == 3 && NREP == 6, "head split of the item epilogue");
             if (sub == 0) v_epilogue_store<0, 2>(ws, P, lane, ob);
@@ -1057,9 +1067,9 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     const int chunk = (((len + csize - 1) / csize) + 1) & ~1;
     const int my_lo = min(s_lo + crank * chunk, s_hi);
     const int my_hi = min(my_lo + chunk, s_hi);
-    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 32);
+    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
     if (tid == 0) {
-        for (int s = 0; s < M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
@@ -1068,9 +1078,9 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tm_slot;
     m2_rotor_to_tmem(smem, tmem, warp, lane);
-    unsigned tiles_done = 0;
+    unsigned blocks_done = 0;
     WarpState ws;
-    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, tiles_done, ws, tmem);
+    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, ws, tmem);
     // the query fragments are not needed any more; everything below is ordinary memory
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
