@@ -112,11 +112,35 @@ __device__ __forceinline__ uint32_t m2_pack(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// Packed pairs of fp32 (one instruction for two neighbouring accumulator registers; each half is
+// rounded like the scalar operation).
+__device__ __forceinline__ void m2_add2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void m2_sub2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void m2_mul2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void m2_fma2(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0,
+                                        float c1) {
+    asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7};"
+        " fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+
 // fp16x2 of (a, b) and fp16x2 of what that rounding lost: hi + lo carries ~22 mantissa bits.
 __device__ __forceinline__ void m2_pack_hilo(float a, float b, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(a, b);
     hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = m2_pack(a - __low2float(h), b - __high2float(h));
+    const float2 f = __half22float2(h);
+    float ra, rb;
+    m2_sub2(ra, rb, a, b, f.x, f.y);
+    lo = m2_pack(ra, rb);
 }
 // The CTA's three groups (warps of the same warp >> 2) walk their own blocks at their own pace: a barrier of the whole CTA
 // per tile made the twelve warps run through the same phase together, all of them on the same pipe, and wait for the slowest.
@@ -469,26 +493,6 @@ constexpr float M2_SLACK = 2.0f;
 __device__ __forceinline__ constexpr float m2_field_unit(int u) { return u ? 1048576.0f : 16777216.0f; }
 __device__ __forceinline__ constexpr float m2_bit_unit(int u) { return u ? 2097152.0f : 131072.0f; }
 
-// Packed pairs of fp32 (one instruction for two neighbouring accumulator registers; each half is
-// rounded like the scalar operation).
-__device__ __forceinline__ void m2_add2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
-    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ void m2_sub2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
-    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ void m2_mul2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
-    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ void m2_fma2(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0,
-                                        float c1) {
-    asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7};"
-        " fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d;}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
 
 // The two rows of a lane (g and g + 8 of the block), its 64-dim quarter of each.
 struct M2KRows {
@@ -858,7 +862,7 @@ template <bool ALL_WARPS_MERGE = false>  // true: every warp of a kv-head return
 __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const __half* __restrict__ q,
                                                     size_t q_head_stride, const CompressedKV& P, int my_lo, int my_hi,
                                                     float scale, unsigned& blocks_done, WarpState& ws, uint32_t tmem) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
 
@@ -976,7 +980,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
                               float* __restrict__ partials, float scale, float rope_base, int ring_cap) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_next;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int kvh = warp & 3, sub = warp >> 2;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
     uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
@@ -987,7 +991,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     m2_tm_alloc(tm_slot, warp);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tm_slot;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
     int cur_table = -1;
     unsigned blocks_done = 0;
 #pragma unroll 1
@@ -1053,7 +1057,7 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
                                float scale) {
     extern __shared__ __align__(128) unsigned char smem[];
     cg::cluster_group cluster = cg::this_cluster();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     const int split_id = blockIdx.x / csize;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
@@ -1076,7 +1080,7 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     m2_setup_tables(smem, P, tid);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tm_slot;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
     m2_rotor_to_tmem(smem, tmem, warp, lane);
     unsigned blocks_done = 0;
     WarpState ws;
