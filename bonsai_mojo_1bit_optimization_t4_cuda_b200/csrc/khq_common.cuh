@@ -72,6 +72,13 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
         : "memory");
 }
 
+// ---- programmatic dependent launch ------------------------------------------------------------
+// A kernel launched with the attribute may start while the one before it in the stream still runs; wait() returns when
+// that one has completed and its writes are visible.  trigger() lets the next kernel start; it comes after this kernel's
+// own wait(), so that a kernel that has started knows everything before its predecessor to be complete.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- small math helpers ---------------------------------------------------------------------
 __device__ __forceinline__ float h2f(__half h) { return __half2float(h); }
 __device__ __forceinline__ float hbits2f(uint16_t b) { return __half2float(__ushort_as_half(b)); }

@@ -1,5 +1,5 @@
 // khq_decode.cu -- two-region KHQ decode attention for sm_100a:
-//   khq_attn_compressed_kernel  compressed region, split-K partials (acc, max, sum_exp)
+//   khq_attn_compressed_mma_kernel  compressed region, split-K partials (acc, max, sum_exp)
 //   khq_attn_reduce_kernel      LSE merge of the split partials
 //   khq_window_attn_kernel      raw fp16 ring window
 //   khq_merge_gate_kernel       LSE merge of the two regions + sigmoid output gate
@@ -365,60 +365,6 @@ __device__ __forceinline__ void v_epilogue_store(const WarpState& st, const Comp
     }
 }
 
-// grid = num_splits * cluster_size CTAs, cluster (cluster_size,1,1): the CTAs of one cluster
-// share one of the caller's splits and merge through distributed shared memory, so one partial
-// per split leaves the cluster whatever the cluster size.
-template <bool VQS>
-__global__ void __launch_bounds__(DEC_THREADS, 1)
-khq_attn_compressed_kernel(const __half* __restrict__ q, CompressedKV P, float* __restrict__ out_attn,
-                           float* __restrict__ out_partial, int num_splits, int L_q, int l_idx,
-                           int s_limit, float scale) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int kvh = warp & 3, sub = warp >> 2;
-    const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-    const int split_id = blockIdx.x / csize;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM_BARS);
-
-    // ---- token range of this split, then of this CTA inside the split ----------------------
-    int s_lo = 0, s_hi = s_limit;
-    if (num_splits > 1) {
-        const int per = (s_limit + num_splits - 1) / num_splits;
-        s_lo = min(split_id * per, s_limit);
-        s_hi = min(s_lo + per, s_limit);
-    }
-    const int len = s_hi - s_lo;
-    const int chunk = (((len + csize - 1) / csize) + 1) & ~1;
-    const int my_lo = min(s_lo + crank * chunk, s_hi);
-    const int my_hi = min(my_lo + chunk, s_hi);
-
-    if (tid == 0) {
-        for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
-        fence_barrier_init();
-    }
-    setup_tables(smem, P, tid);
-    if (VQS && my_hi > my_lo) load_codebook(reinterpret_cast<unsigned short*>(smem + SM_VQ), P.vq, tid);
-    WarpState st;
-    st.init();
-    unsigned tiles_done = 0;
-    compressed_range<VQS>(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, st,
-                          tiles_done);
-
-    // ---- merge warps -> CTA -> cluster, then the V epilogue on cluster rank 0 ------------------
-    merge_cta_and_cluster(st, reinterpret_cast<float*>(smem + SM_MERGE_A), kvh, sub, lane);
-    if (crank == 0 && sub == 0) {
-        float* ob[NREP];
-#pragma unroll
-        for (int h = 0; h < NREP; ++h) {
-            const int total_id = (kvh * NREP + h) * L_q + l_idx;
-            ob[h] = (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART
-                                     : out_attn + (size_t)total_id * PART;
-        }
-        v_epilogue_store(st, P, lane, ob);
-    }
-}
-
 // LSE merge of `n` partial records `stride` floats apart (acc[D], max, sum) by one block of
 // G * D threads: M = max m_i, num = sum acc_i[dd] e^{m_i - M}, den = sum s_i e^{m_i - M}.
 // Thread (group g, dim dd) adds records g, g + G, ... in order; the groups' sums are then
@@ -481,6 +427,8 @@ template <int G>
 __global__ void __launch_bounds__(G * D) khq_attn_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                                 int num_splits) {
     const int qid = blockIdx.x, d = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     float num, den;
     const float M = lse_merge_records<G>(partial + (size_t)qid * num_splits * PART, (size_t)PART, num_splits, num, den);
     if (d >= D) return;
@@ -496,47 +444,86 @@ __global__ void __launch_bounds__(G * D) khq_attn_reduce_kernel(const float* __r
 // Raw ring window
 // ------------------------------------------------------------------------------------------
 // Window tokens s = first, first+step, ... < win_hi of this warp: slot (win_start + s) % ring_cap,
-// rows token-major (slot*H_kv + kv)*D, K already RoPE'd.
+// rows token-major (slot*H_kv + kv)*D, K already RoPE'd.  U tokens at a time: their 2 U row loads are in flight together
+// and their dot products and warp sums interleave (one token at a time, a token cost a warp a full memory latency plus a
+// chain of six warp sums: 0.75 us).
 // When new_s >= 0, window token new_s is read from new_k / new_v (one token, H_kv*D halfs each)
 // instead of its ring slot: the fused step kernel appends it to the ring while the window runs.
+template <int U>
 __device__ __forceinline__ void window_range(const __half* __restrict__ q, const __half* __restrict__ ring_k,
                                              const __half* __restrict__ ring_v, int win_start, int first,
                                              int step, int win_hi, int ring_cap, float scale, int kvh,
                                              int lane, WarpState& st, int new_s = -1,
                                              const __half* __restrict__ new_k = nullptr,
                                              const __half* __restrict__ new_v = nullptr) {
-    float qv[NREP][8];
+    if (first >= win_hi) return;
+    uint4 qr[NREP];
 #pragma unroll
-    for (int h = 0; h < NREP; ++h) {
-        const uint4 qr = *reinterpret_cast<const uint4*>(q + (size_t)(kvh * NREP + h) * 2 * D + lane * 8);
-        const __half* hq = reinterpret_cast<const __half*>(&qr);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) qv[h][j] = __half2float(hq[j]) * scale;
-    }
+    for (int h = 0; h < NREP; ++h) qr[h] = *reinterpret_cast<const uint4*>(q + (size_t)(kvh * NREP + h) * 2 * D + lane * 8);
 #pragma unroll 1
-    for (int s = first; s < win_hi; s += step) {
-        const int slot = (win_start + s) % ring_cap;
-        const size_t off = ((size_t)slot * HKV + kvh) * D + lane * 8;
-        const bool fresh = (s == new_s);
-        const uint4 kr = *reinterpret_cast<const uint4*>(fresh ? new_k + (size_t)kvh * D + lane * 8 : ring_k + off);
-        const uint4 vr = *reinterpret_cast<const uint4*>(fresh ? new_v + (size_t)kvh * D + lane * 8 : ring_v + off);
-        const __half* hk = reinterpret_cast<const __half*>(&kr);
-        const __half* hv = reinterpret_cast<const __half*>(&vr);
-        float sc[NREP];
+    for (int s0 = first; s0 < win_hi; s0 += U * step) {
+        uint4 kr[U], vr[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int s = s0 + u * step < win_hi ? s0 + u * step : s0;  // past the end: a row that is there, weight 0
+            const size_t off = ((size_t)((win_start + s) % ring_cap) * HKV + kvh) * D + lane * 8;
+            const bool fresh = (s == new_s);
+            kr[u] = *reinterpret_cast<const uint4*>(fresh ? new_k + (size_t)kvh * D + lane * 8 : ring_k + off);
+            vr[u] = *reinterpret_cast<const uint4*>(fresh ? new_v + (size_t)kvh * D + lane * 8 : ring_v + off);
+        }
+        float sc[U][NREP];
+        {
+            float k8[U][8];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) k8[u][j] = __half2float(reinterpret_cast<const __half*>(&kr[u])[j]);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
+                float q8[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) q8[j] = __half2float(reinterpret_cast<const __half*>(&qr[h])[j]) * scale;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    float a = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) a = fmaf(q8[j], k8[u][j], a);
+                    sc[u][h] = a;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) reduce6(sc[u], lane);
+#pragma unroll
+        for (int u = 1; u < U; ++u)
+            if (s0 + u * step >= win_hi)
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) sc[u][h] = -1e30f;
 #pragma unroll
         for (int h = 0; h < NREP; ++h) {
-            float a = 0.0f;
+            float top = sc[0][h];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a = fmaf(qv[h][j], __half2float(hk[j]), a);
-            sc[h] = a;
+            for (int u = 1; u < U; ++u) top = fmaxf(top, sc[u][h]);
+            if (top > st.m[h]) {  // warp-uniform: every lane holds the same scores and maximum
+                const float fac = __expf(st.m[h] - top);
+                st.l[h] *= fac;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) st.acc[h][j] *= fac;
+                st.m[h] = top;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                sc[u][h] = __expf(sc[u][h] - st.m[h]);
+                st.l[h] += sc[u][h];
+            }
         }
-        reduce6(sc, lane);
-        float pw[NREP];
-        softmax_step(st, sc, pw);
-        float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __half2float(hv[j]);
-        accumulate_v(st, pw, v);
+        for (int u = 0; u < U; ++u) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __half2float(reinterpret_cast<const __half*>(&vr[u])[j]);
+            accumulate_v(st, sc[u], v);
+        }
     }
 }
 
@@ -554,7 +541,17 @@ __device__ __forceinline__ void raw_store(const WarpState& st, int lane, float* 
 }
 
 // One cluster: token s is served by warp (kv, sub) of CTA c when
-// s % (cluster_size*DEC_WPK) == c*DEC_WPK + sub.
+// s % (cluster_size*DEC_WPK) == c*DEC_WPK + sub.  The heads of the result are dealt to the cluster's warps, which merge the
+// per-warp records through distributed shared memory.
+constexpr int WIN_SMEM = DEC_WARPS * MERGE_FLOATS * 4;  // one record per warp
+
+// Behind a cluster barrier: head h merged over the records of all warps of the cluster that served its kv-head.
+__device__ __forceinline__ HeadAcc window_head(cg::cluster_group& cluster, const float* rec, int csize, int h, int lane) {
+    return merge_head<true>(DEC_WPK * csize, lane, [&](int i) {
+        return head_of_record(cluster.map_shared_rank(rec, i / DEC_WPK) + (h / NREP + HKV * (i % DEC_WPK)) * MERGE_FLOATS, h % NREP);
+    });
+}
+
 __global__ void __launch_bounds__(DEC_THREADS, 1)
 khq_window_attn_kernel(const __half* __restrict__ q, const __half* __restrict__ ring_k,
                        const __half* __restrict__ ring_v, float* __restrict__ out, int win_start,
@@ -564,17 +561,18 @@ khq_window_attn_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+    float* rec = reinterpret_cast<float*>(smem);
+    pdl_wait();
+    pdl_trigger();
     WarpState st;
     st.init();
-    window_range(q, ring_k, ring_v, win_start, crank * DEC_WPK + sub, csize * DEC_WPK, win_len, ring_cap, scale,
-                 kvh, lane, st);
-    merge_cta_and_cluster(st, reinterpret_cast<float*>(smem), kvh, sub, lane);
-    if (crank == 0 && sub == 0) {
-        float* ob[NREP];
-#pragma unroll
-        for (int h = 0; h < NREP; ++h) ob[h] = out + (size_t)(kvh * NREP + h) * PART;
-        raw_store(st, lane, ob);
-    }
+    window_range<4>(q, ring_k, ring_v, win_start, crank * DEC_WPK + sub, csize * DEC_WPK, win_len, ring_cap, scale,
+                    kvh, lane, st);
+    store_record(st, rec + warp * MERGE_FLOATS, lane);
+    cluster.sync();
+#pragma unroll 1
+    for (int h = crank + csize * warp; h < HQ; h += csize * DEC_WARPS) store_head(window_head(cluster, rec, csize, h, lane), out + (size_t)h * PART, lane);
+    cluster.sync();  // peers must stay resident until their records have been read
 }
 
 // ------------------------------------------------------------------------------------------
@@ -634,8 +632,8 @@ khq_decode_batched_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesD
             merge_cta_and_cluster(st, reinterpret_cast<float*>(smem + SM_MERGE_A), kvh, sub, lane);
             if (sub == 0) v_epilogue_store(st, P, lane, ob);
         } else {
-            window_range(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, DEC_WPK, w.hi, ring_cap, scale, kvh,
-                         lane, st);
+            window_range<4>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, DEC_WPK, w.hi, ring_cap, scale, kvh,
+                            lane, st);
             merge_cta_and_cluster(st, reinterpret_cast<float*>(smem + SM_MERGE_A), kvh, sub, lane);
             if (sub == 0) raw_store(st, lane, ob);
         }
@@ -657,6 +655,8 @@ __global__ void __launch_bounds__(D)
 khq_batched_merge_gate_few_kernel(const KhqSeqDesc* __restrict__ descs, const float* __restrict__ partials) {
     constexpr int CH = 8;
     const int di = blockIdx.x / HQ, h = blockIdx.x % HQ, dd = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     const KhqSeqDesc d = descs[di];
     const float* base = partials + ((size_t)d.first_slot * HQ + h) * PART;
     const float gate = __half2float(d.q_gate[(size_t)h * 2 * D + D + dd]);
@@ -693,6 +693,8 @@ template <int G>
 __global__ void __launch_bounds__(G * D)
 khq_batched_merge_gate_kernel(const KhqSeqDesc* __restrict__ descs, const float* __restrict__ partials) {
     const int di = blockIdx.x / HQ, h = blockIdx.x % HQ, dd = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     const KhqSeqDesc d = descs[di];
     float num, den;
     lse_merge_records<G>(partials + ((size_t)d.first_slot * HQ + h) * PART, (size_t)HQ * PART, d.n_slots, num, den);
@@ -709,6 +711,8 @@ __global__ void __launch_bounds__(G * D)
 khq_batched_merge_partial_kernel(const KhqSeqDesc* __restrict__ descs, const float* __restrict__ partials,
                                  float* __restrict__ out_partials) {
     const int di = blockIdx.x / HQ, h = blockIdx.x % HQ, dd = threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     const KhqSeqDesc d = descs[di];
     float num, den;
     const float M = lse_merge_records<G>(partials + ((size_t)d.first_slot * HQ + h) * PART, (size_t)HQ * PART, d.n_slots, num, den);
@@ -723,21 +727,24 @@ khq_batched_merge_partial_kernel(const KhqSeqDesc* __restrict__ descs, const flo
 
 // Fused tail of a decode step for one sequence: appends the step's token to the three rings (K
 // RoPE'd, V, K un-RoPE'd; CTA 0, while every CTA reads that token straight from the inputs), runs
-// the raw-window attention over win_len tokens (the new one is the last), then the cluster's rank-0
-// CTA merges the window partial with the compressed-region partial attn_c (when has_c), divides by
-// (den + 1e-8), applies the sigmoid gate and stores fp16 -- the math of khq_window_attn_kernel +
-// khq_merge_gate_kernel in one launch.
+// the raw-window attention over win_len tokens (the new one is the last), then the cluster's warps
+// merge the heads they are dealt: the window records, the n_c <= 32 records per head of the compressed region
+// (head-major, PART floats each), /(den + 1e-8), sigmoid gate, fp16 store.
+// With n_c > 0 the launch before it in the stream is the compressed-region kernel of the same step, which starts only when
+// everything before it is complete and writes nothing but those records: the window part runs beside it.
 __global__ void __launch_bounds__(DEC_THREADS, 1)
 khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k, __half* __restrict__ ring_v,
                        __half* __restrict__ ring_u, const __half* __restrict__ new_k, const __half* __restrict__ new_v,
-                       const __half* __restrict__ new_u, const float* __restrict__ attn_c, __half* __restrict__ out,
-                       int win_start, int win_len, int ring_cap, float scale, int has_c) {
+                       const __half* __restrict__ new_u, const float* __restrict__ part_c, __half* __restrict__ out,
+                       int win_start, int win_len, int ring_cap, float scale, int n_c) {
     extern __shared__ __align__(128) unsigned char smem[];
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     const int new_s = win_len - 1;
+    float* rec = reinterpret_cast<float*>(smem);
+    if (n_c == 0) pdl_wait();
     if (crank == 0) {  // ring appends: 3 rows of H_kv*D halfs = 3 x 128 sixteen-byte chunks
         const int slot = (win_start + new_s) % ring_cap;
         const size_t row = (size_t)slot * HKV * D;
@@ -751,42 +758,42 @@ khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k
     }
     WarpState st;
     st.init();
-    window_range(q, ring_k, ring_v, win_start, crank * DEC_WPK + sub, csize * DEC_WPK, win_len, ring_cap, scale, kvh,
-                 lane, st, new_s, new_k, new_v);
-    merge_cta_and_cluster(st, reinterpret_cast<float*>(smem), kvh, sub, lane);
-    if (crank == 0 && sub == 0) {
+    window_range<4>(q, ring_k, ring_v, win_start, crank * DEC_WPK + sub, csize * DEC_WPK, win_len, ring_cap, scale, kvh,
+                    lane, st, new_s, new_k, new_v);
+    store_record(st, rec + warp * MERGE_FLOATS, lane);
+    cluster.sync();
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll 1
+    for (int h = crank + csize * warp; h < HQ; h += csize * DEC_WARPS) {
+        const uint4 gr = *reinterpret_cast<const uint4*>(q + (size_t)h * 2 * D + D + lane * 8);
+        HeadAcc a = window_head(cluster, rec, csize, h, lane);
+        if (n_c > 0) {
+            const HeadAcc c = merge_head<false>(n_c, lane, [&](int i) {
+                const float* p = part_c + ((size_t)h * n_c + i) * PART;
+                return HeadRec{p, p + D, p + D + 1};
+            });
+            const float M = fmaxf(a.m, c.m), wa = __expf(a.m - M), wc = __expf(c.m - M);
+            a.l = a.l * wa + c.l * wc;
 #pragma unroll
-        for (int h = 0; h < NREP; ++h) {
-            const int head = kvh * NREP + h;
-            float wsc = 1.0f, csc = 0.0f, den = st.l[h];
-            const float* cc = attn_c + (size_t)head * PART;
-            if (has_c) {
-                const float mc = cc[D], mw = st.m[h];
-                const float M = fmaxf(mc, mw);
-                csc = __expf(mc - M);
-                wsc = __expf(mw - M);
-                den = cc[D + 1] * csc + st.l[h] * wsc;
-            }
-            const float inv = 1.0f / (den + 1e-8f);
-            const uint4 gr = *reinterpret_cast<const uint4*>(q + (size_t)head * 2 * D + D + lane * 8);
-            const __half* hg = reinterpret_cast<const __half*>(&gr);
-            __half o8[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float num = st.acc[h][j] * wsc;
-                if (has_c) num = cc[lane * 8 + j] * csc + num;
-                const float g = __half2float(hg[j]);
-                o8[j] = __float2half(num * inv * (1.0f / (1.0f + __expf(-g))));
-            }
-            *reinterpret_cast<uint4*>(out + (size_t)head * D + lane * 8) = *reinterpret_cast<const uint4*>(o8);
+            for (int j = 0; j < 8; ++j) a.a[j] = a.a[j] * wa + c.a[j] * wc;
         }
+        const float inv = 1.0f / (a.l + 1e-8f);
+        const __half* hg = reinterpret_cast<const __half*>(&gr);
+        __half o8[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o8[j] = __float2half(a.a[j] * inv * (1.0f / (1.0f + __expf(-__half2float(hg[j])))));
+        *reinterpret_cast<uint4*>(out + (size_t)h * D + lane * 8) = *reinterpret_cast<const uint4*>(o8);
     }
+    cluster.sync();  // peers must stay resident until their records have been read
 }
 
 // LSE merge of the two regions, /(den + 1e-8), sigmoid gate, fp16 store.
 __global__ void khq_merge_gate_kernel(const float* __restrict__ attn_c, const float* __restrict__ attn_w,
                                       const __half* __restrict__ q_gate, __half* __restrict__ out, int H_q,
                                       int d_v, int has_w) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= H_q * d_v) return;
     const int h = i / d_v, d = i % d_v;
@@ -927,21 +934,26 @@ __global__ void khq_gather_q_kernel(const __half* __restrict__ q_gate, __half* _
 // ------------------------------------------------------------------------------------------
 static inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
+// cluster == 0: no cluster attribute.  All kernels launched through here begin with pdl_wait() (or know what they may do
+// before it), so they carry the programmatic-serialisation attribute: their launch latency and prologue overlap the end of
+// the kernel before them.
 template <typename Kernel, typename... Args>
-static cudaError_t launch_cluster(Kernel kernel, unsigned grid, unsigned cluster, size_t smem_bytes,
-                                  cudaStream_t stream, unsigned threads, Args... args) {
+static cudaError_t launch_pdl(Kernel kernel, unsigned grid, unsigned cluster, size_t smem_bytes,
+                              cudaStream_t stream, unsigned threads, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 0 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
@@ -953,17 +965,14 @@ static cudaError_t ensure_smem_attrs() {
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if ((e = cudaFuncSetAttribute(khq_attn_compressed_kernel<false>, attr, SM_TOTAL)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(khq_attn_compressed_kernel<true>, attr, SM_TOTAL_VQ)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_decode_batched_kernel<false>, attr, SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_decode_batched_kernel<true>, attr, SM_TOTAL_VQ)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_decode_batched_mma_kernel, attr, M2_SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_attn_compressed_mma_kernel, attr, M2_SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(m3::khq_decode_batched_tc5_kernel, attr, m3::SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(m3::khq_decode_batched_tc5w_kernel, attr, m3::SM_TOTAL)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(khq_window_attn_kernel, attr, 2 * HKV * MERGE_FLOATS * 4)) != cudaSuccess)
-        return e;
-    if ((e = cudaFuncSetAttribute(khq_window_step_kernel, attr, 2 * HKV * MERGE_FLOATS * 4)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_window_attn_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_window_step_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev] = true;
     return cudaSuccess;
 }
@@ -980,17 +989,17 @@ static int sm_count() {
     return n[dev];
 }
 
-// How many clusters of `c` CTAs of the compressed-attention kernels fit on the device at once.
-static int max_clusters(bool mma, int c) {
-    static int cache[64][2][9] = {};
+// How many clusters of `c` CTAs of the compressed-attention kernel fit on the device at once.
+static int max_clusters(int c) {
+    static int cache[64][9] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || c < 1 || c > 8) return 1;
-    int& slot = cache[dev][mma ? 1 : 0][c];
+    int& slot = cache[dev][c];
     if (slot == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)c, 1, 1);
-        cfg.blockDim = dim3(mma ? (unsigned)M2_THREADS : (unsigned)DEC_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = mma ? (size_t)M2_SM_TOTAL : (size_t)SM_TOTAL;
+        cfg.blockDim = dim3((unsigned)M2_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = (size_t)M2_SM_TOTAL;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)c;
@@ -999,9 +1008,7 @@ static int max_clusters(bool mma, int c) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        const cudaError_t e = mma ? cudaOccupancyMaxActiveClusters(&n, khq_attn_compressed_mma_kernel, &cfg)
-                                  : cudaOccupancyMaxActiveClusters(&n, khq_attn_compressed_kernel<false>, &cfg);
-        if (e != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, khq_attn_compressed_mma_kernel, &cfg) != cudaSuccess || n <= 0) {
             (void)cudaGetLastError();
             n = sm_count() / c > 0 ? sm_count() / c : 1;
         }
@@ -1009,7 +1016,6 @@ static int max_clusters(bool mma, int c) {
     }
     return slot;
 }
-
 
 }  // namespace khq
 
@@ -1024,7 +1030,7 @@ static int attn_launch_impl(const void* q, const void* k_payload, const void* v_
                             void* out_partial, int num_queries, int num_heads, int L_q, int c_len,
                             int n_rep, float scale, float alpha_k, float alpha_v,
                             float rope_base, int start_pos, int num_splits, int pos_chunk, int pos_stride,
-                            cudaStream_t stream) {
+                            bool reduce, cudaStream_t stream) {
     if (num_queries <= 0 || c_len <= 0) return -100;
     if (num_splits < 1) num_splits = 1;
     if (num_splits > 1 && out_partial == nullptr) return -101;
@@ -1070,54 +1076,34 @@ static int attn_launch_impl(const void* q, const void* k_payload, const void* v_
     for (int l = 0; l < L_q; ++l) {
         const int s_limit = (L_q > 1) ? (c_len < l + 1 ? c_len : l + 1) : c_len;
         const int per = (s_limit + num_splits - 1) / num_splits;
-        // CTAs per split (a portable cluster of at most 8) and the kernel generation, by estimated
-        // time in units of 0.23 us: waves x (per-CTA set-up + tokens per CTA x cost per token), waves =
-        // splits / clusters of that size that fit on the GPU at once (clusters are placed inside a GPC, so
-        // fewer than SMs / size fit).  Measured: tensor-core generation set-up ~104 (tables, tensor-memory
-        // allocation, query build, record), 0.63 per token in whole 48-token tiles; CUDA-core generation set-up
-        // ~116, 3.06 per token, ~TT tokens per CTA.
-        int cluster = (per + TT - 1) / TT;
-        if (cluster < 1) cluster = 1;
-        if (cluster > 8) cluster = 8;
-        bool use_mma = false;
-        {
-            const int tpc1 = (per + cluster - 1) / cluster;
-            const long long w1 = (num_splits + max_clusters(false, cluster) - 1) / max_clusters(false, cluster);
-            long long best = w1 * (116 + (tpc1 * 306LL) / 100);
-            for (int c = 1; c <= 8; ++c) {
-                const int tpc = (per + c - 1) / c;
-                const int tiles = (tpc + M2_TT - 1) / M2_TT;
-                const long long waves = (num_splits + max_clusters(true, c) - 1) / max_clusters(true, c);
-                const long long cost = waves * (104 + (tiles * M2_TT * 63LL) / 100);
-                if (cost < best) {
-                    best = cost;
-                    cluster = c;
-                    use_mma = true;
-                }
-                if (tpc <= M2_TT) break;  // more CTAs would only add set-ups
+        // CTAs per split (a portable cluster of at most 8), by estimated time in units of 0.16 us: waves x (per-CTA
+        // set-up + tokens per CTA in whole 48-token rounds), waves = splits / clusters of that size that fit on the GPU at
+        // once (clusters are placed inside a GPC, so fewer than SMs / size fit).
+        int cluster = 1;
+        long long best = -1;
+        for (int c = 1; c <= 8; ++c) {
+            const int tpc = (per + c - 1) / c;
+            const long long waves = (num_splits + max_clusters(c) - 1) / max_clusters(c);
+            const long long cost = waves * (70 + (tpc + M2_TT - 1) / M2_TT * M2_TT);
+            if (best < 0 || cost < best) {
+                best = cost;
+                cluster = c;
             }
+            if (tpc <= M2_TT) break;  // more CTAs would only add set-ups
         }
-        if (use_mma)
-            err = launch_cluster(khq_attn_compressed_mma_kernel, (unsigned)(num_splits * cluster), (unsigned)cluster,
-                                 (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS, static_cast<const __half*>(q), P,
-                                 static_cast<float*>(out_attn), static_cast<float*>(out_partial), num_splits, L_q,
-                                 l, s_limit, scale);
-        else
-            err = launch_cluster(khq_attn_compressed_kernel<false>, (unsigned)(num_splits * cluster),
-                                 (unsigned)cluster, (size_t)SM_TOTAL, stream, (unsigned)DEC_THREADS,
-                                 static_cast<const __half*>(q), P,
-                                 static_cast<float*>(out_attn), static_cast<float*>(out_partial), num_splits, L_q,
-                                 l, s_limit, scale);
+        err = launch_pdl(khq_attn_compressed_mma_kernel, (unsigned)(num_splits * cluster), (unsigned)cluster,
+                         (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS, static_cast<const __half*>(q), P,
+                         static_cast<float*>(out_attn), static_cast<float*>(out_partial), num_splits, L_q,
+                         l, s_limit, scale);
         if (err != cudaSuccess) return static_cast<int>(err);
     }
-    if (num_splits > 1) {
+    if (num_splits > 1 && reduce) {
         if (num_splits > 32)
-            khq_attn_reduce_kernel<MERGE_GROUPS><<<(unsigned)num_queries, MERGE_GROUPS * D, 0, stream>>>(
-                static_cast<const float*>(out_partial), static_cast<float*>(out_attn), num_splits);
+            err = launch_pdl(khq_attn_reduce_kernel<MERGE_GROUPS>, (unsigned)num_queries, 0, 0, stream, MERGE_GROUPS * D,
+                             static_cast<const float*>(out_partial), static_cast<float*>(out_attn), num_splits);
         else
-            khq_attn_reduce_kernel<1><<<(unsigned)num_queries, D, 0, stream>>>(
-                static_cast<const float*>(out_partial), static_cast<float*>(out_attn), num_splits);
-        err = cudaGetLastError();
+            err = launch_pdl(khq_attn_reduce_kernel<1>, (unsigned)num_queries, 0, 0, stream, D,
+                             static_cast<const float*>(out_partial), static_cast<float*>(out_attn), num_splits);
         if (err != cudaSuccess) return static_cast<int>(err);
     }
     return 0;
@@ -1136,7 +1122,7 @@ extern "C" int launch_khq_attn_fp16(const void* q, const void* k_payload, const 
     return attn_launch_impl(q, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
                             centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, out_attn, out_partial,
                             num_queries, num_heads, L_q, c_len, n_rep, scale, alpha_k, alpha_v, rope_base, start_pos,
-                            num_splits, 0, 0, stream);
+                            num_splits, 0, 0, true, stream);
 }
 
 // launch_khq_attn_fp16 over a slice that holds every G-th `pos_chunk`-token chunk of a longer context
@@ -1157,7 +1143,13 @@ extern "C" int launch_khq_attn_strided_fp16(const void* q, const void* k_payload
     return attn_launch_impl(q, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
                             centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, out_attn, out_partial,
                             num_queries, num_heads, L_q, c_len, n_rep, scale, alpha_k, alpha_v, rope_base, start_pos,
-                            num_splits, pos_chunk, pos_stride, stream);
+                            num_splits, pos_chunk, pos_stride, true, stream);
+}
+
+// CTAs of the one cluster that runs a raw window: a warp takes four tokens at a time.
+static unsigned window_cluster(int win_len) {
+    const int c = (win_len + DEC_WPK * 4 - 1) / (DEC_WPK * 4);
+    return (unsigned)(c < 1 ? 1 : c > 8 ? 8 : c);
 }
 
 extern "C" int launch_khq_window_attn_fp16(const void* q, const void* ring_k, const void* ring_v,
@@ -1168,13 +1160,9 @@ extern "C" int launch_khq_window_attn_fp16(const void* q, const void* ring_k, co
     if (!aligned(q, 16) || !aligned(ring_k, 16) || !aligned(ring_v, 16) || !aligned(out_attn, 8)) return -104;
     cudaError_t err = ensure_smem_attrs();
     if (err != cudaSuccess) return static_cast<int>(err);
-    int cluster = (win_len + DEC_WPK * 4 - 1) / (DEC_WPK * 4);
-    if (cluster < 1) cluster = 1;
-    if (cluster > 8) cluster = 8;
-    err = launch_cluster(khq_window_attn_kernel, (unsigned)cluster, (unsigned)cluster,
-                         (size_t)(2 * HKV * MERGE_FLOATS * 4), stream, (unsigned)DEC_THREADS,
-                         static_cast<const __half*>(q), static_cast<const __half*>(ring_k), static_cast<const __half*>(ring_v),
-                         static_cast<float*>(out_attn), win_start, win_len, ring_cap, scale);
+    err = launch_pdl(khq_window_attn_kernel, window_cluster(win_len), window_cluster(win_len), (size_t)WIN_SMEM, stream,
+                     (unsigned)DEC_THREADS, static_cast<const __half*>(q), static_cast<const __half*>(ring_k),
+                     static_cast<const __half*>(ring_v), static_cast<float*>(out_attn), win_start, win_len, ring_cap, scale);
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
@@ -1182,10 +1170,9 @@ extern "C" int launch_khq_merge_gate_fp16(const void* attn_c, const void* attn_w
                                           void* out, int H_q, int d, int has_w, cudaStream_t stream) {
     if (H_q <= 0 || d <= 0) return -100;
     const int total = H_q * d, threads = 256;
-    khq_merge_gate_kernel<<<(total + threads - 1) / threads, threads, 0, stream>>>(
-        static_cast<const float*>(attn_c), static_cast<const float*>(attn_w),
-        static_cast<const __half*>(q_gate), static_cast<__half*>(out), H_q, d, has_w);
-    const cudaError_t err = cudaGetLastError();
+    const cudaError_t err = launch_pdl(khq_merge_gate_kernel, (unsigned)((total + threads - 1) / threads), 0, 0, stream,
+                                       (unsigned)threads, static_cast<const float*>(attn_c), static_cast<const float*>(attn_w),
+                                       static_cast<const __half*>(q_gate), static_cast<__half*>(out), H_q, d, has_w);
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
@@ -1206,24 +1193,22 @@ extern "C" int launch_khq_decode_step_fp16(
     for (const void* p : al)
         if (p && !aligned(p, 16)) return -104;
     if (!aligned(attn_c, 8)) return -104;
+    // the tail merges up to 32 split records per head itself
+    const bool tail_merges = num_splits > 1 && num_splits <= 32;
     if (c_len > 0) {
-        const int rc = launch_khq_attn_fp16(q_gate, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms,
-                                            v_r_norms, centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k,
-                                            d_vec_v, attn_c, attn_partial, HQ, HQ, 1, c_len, c_len, NREP, scale, alpha_k,
-                                            alpha_v, rope_base, 0, num_splits, stream);
+        const int rc = attn_launch_impl(q_gate, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
+                                        centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, attn_c, attn_partial,
+                                        HQ, HQ, 1, c_len, NREP, scale, alpha_k, alpha_v, rope_base, 0, num_splits, 0, 0, !tail_merges, stream);
         if (rc != 0) return rc;
     }
     cudaError_t err = ensure_smem_attrs();
     if (err != cudaSuccess) return static_cast<int>(err);
-    int cluster = (win_len + DEC_WPK * 4 - 1) / (DEC_WPK * 4);
-    if (cluster < 1) cluster = 1;
-    if (cluster > 8) cluster = 8;
-    err = launch_cluster(khq_window_step_kernel, (unsigned)cluster, (unsigned)cluster, (size_t)(2 * HKV * MERGE_FLOATS * 4),
-                         stream, (unsigned)DEC_THREADS, static_cast<const __half*>(q_gate), static_cast<__half*>(ring_k),
-                         static_cast<__half*>(ring_v), static_cast<__half*>(ring_u), static_cast<const __half*>(k_roped),
-                         static_cast<const __half*>(v_new), static_cast<const __half*>(k_unroped),
-                         static_cast<const float*>(attn_c), static_cast<__half*>(out), win_start, win_len, ring_cap, scale,
-                         c_len > 0 ? 1 : 0);
+    const float* part_c = static_cast<const float*>(tail_merges ? attn_partial : attn_c);
+    err = launch_pdl(khq_window_step_kernel, window_cluster(win_len), window_cluster(win_len), (size_t)WIN_SMEM,
+                     stream, (unsigned)DEC_THREADS, static_cast<const __half*>(q_gate), static_cast<__half*>(ring_k),
+                     static_cast<__half*>(ring_v), static_cast<__half*>(ring_u), static_cast<const __half*>(k_roped),
+                     static_cast<const __half*>(v_new), static_cast<const __half*>(k_unroped), part_c, static_cast<__half*>(out),
+                     win_start, win_len, ring_cap, scale, c_len > 0 ? (tail_merges ? num_splits : 1) : 0);
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
@@ -1440,12 +1425,14 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
     if (!aligned(workspace, 256)) return -104;
     cudaError_t err = ensure_smem_attrs();
     if (err != cudaSuccess) return static_cast<int>(err);
-    err = cudaMemsetAsync(workspace, 0, 256, stream);
-    if (err != cudaSuccess) return static_cast<int>(err);
     int* counter = static_cast<int*>(workspace);
     float* partials = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
     const int grid = n_items < sm_count() ? n_items : sm_count();
-    const bool vqs = codebook_in_smem != 0;
+    const bool vqs = codebook_in_smem != 0, mma = codebook_in_smem == 2 || codebook_in_smem < 0;
+    if (!mma || n_items > grid) {  // the default kernel takes its first item without the counter
+        err = cudaMemsetAsync(workspace, 0, 256, stream);
+        if (err != cudaSuccess) return static_cast<int>(err);
+    }
     if (codebook_in_smem == 4)
         m3::khq_decode_batched_tc5w_kernel<<<grid, m3::W_THREADS, m3::SM_TOTAL, stream>>>(
             static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
@@ -1454,10 +1441,10 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
         m3::khq_decode_batched_tc5_kernel<<<grid, m3::THREADS, m3::SM_TOTAL, stream>>>(
             static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
             static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap);
-    else if (codebook_in_smem == 2 || codebook_in_smem < 0)
-        khq_decode_batched_mma_kernel<<<grid, M2_THREADS, M2_SM_TOTAL, stream>>>(
-            static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
-            static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap);
+    else if (mma)
+        err = launch_pdl(khq_decode_batched_mma_kernel, (unsigned)grid, 0, (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS,
+                         static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
+                         static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap);
     else if (vqs)
         khq_decode_batched_kernel<true><<<grid, DEC_THREADS, SM_TOTAL_VQ, stream>>>(
             static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
@@ -1466,18 +1453,18 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
         khq_decode_batched_kernel<false><<<grid, DEC_THREADS, SM_TOTAL, stream>>>(
             static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
             static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap);
-    err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess) return static_cast<int>(err);
     const KhqSeqDesc* dd = static_cast<const KhqSeqDesc*>(descs);
     const bool many = n_items > 32 * n_desc;  // many records per problem
+    const unsigned blocks = (unsigned)(n_desc * HQ);
     if (out_partials) {
-        if (many) khq_batched_merge_partial_kernel<MERGE_GROUPS><<<n_desc * HQ, MERGE_GROUPS * D, 0, stream>>>(dd, partials, out_partials);
-        else khq_batched_merge_partial_kernel<1><<<n_desc * HQ, D, 0, stream>>>(dd, partials, out_partials);
+        if (many) err = launch_pdl(khq_batched_merge_partial_kernel<MERGE_GROUPS>, blocks, 0, 0, stream, MERGE_GROUPS * D, dd, partials, out_partials);
+        else err = launch_pdl(khq_batched_merge_partial_kernel<1>, blocks, 0, 0, stream, D, dd, partials, out_partials);
     } else {
-        if (many) khq_batched_merge_gate_kernel<MERGE_GROUPS><<<n_desc * HQ, MERGE_GROUPS * D, 0, stream>>>(dd, partials);
-        else khq_batched_merge_gate_few_kernel<<<n_desc * HQ, D, 0, stream>>>(dd, partials);
+        if (many) err = launch_pdl(khq_batched_merge_gate_kernel<MERGE_GROUPS>, blocks, 0, 0, stream, MERGE_GROUPS * D, dd, partials);
+        else err = launch_pdl(khq_batched_merge_gate_few_kernel, blocks, 0, 0, stream, D, dd, partials);
     }
-    err = cudaGetLastError();
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 

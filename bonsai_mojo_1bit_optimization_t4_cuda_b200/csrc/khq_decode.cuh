@@ -239,6 +239,92 @@ __device__ __forceinline__ void store_record(const WarpState& st, float* rec, in
         }
 }
 
+// One query head's merged state: the lane's 8 dims, maximum and sum of exps.
+struct HeadAcc {
+    float a[8], m, l;
+};
+// Where a record keeps a head: its 256 accumulators (16-byte aligned if V4, else 8-byte), maximum and sum.
+struct HeadRec {
+    const float *acc, *m, *l;
+};
+// LSE merge of one head over records at(0) .. at(n - 1), n <= 32, by a warp: lane i fetches the maximum and the sum of
+// record i, so the n weights cost one exchange, and the accumulators of four records are in flight together.  The records
+// may lie in this CTA's or a peer CTA's shared memory or in global memory.
+template <bool V4, class At>
+__device__ __forceinline__ HeadAcc merge_head(int n, int lane, At at) {
+    HeadAcc r;
+    float m = NEG_BIG, l = 0.0f;
+    if (lane < n) {
+        const HeadRec h = at(lane);
+        m = *h.m;
+        l = *h.l;
+    }
+    r.m = m;
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) r.m = fmaxf(r.m, __shfl_xor_sync(0xFFFFFFFFu, r.m, k));
+    const float w = __expf(m - r.m);
+    r.l = l * w;
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) r.l += __shfl_xor_sync(0xFFFFFFFFu, r.l, k);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r.a[j] = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) {
+        const float wi = __shfl_sync(0xFFFFFFFFu, w, i);
+        const float* p = at(i).acc + lane * 8;
+        float v[8];
+        if (V4) {
+            *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(p);
+            *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<const float4*>(p + 4);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) *reinterpret_cast<float2*>(&v[j]) = *reinterpret_cast<const float2*>(p + j);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) r.a[j] = fmaf(v[j], wi, r.a[j]);
+    }
+    return r;
+}
+// Head `hh` of its kv-head in a per-warp record (see store_record).
+__device__ __forceinline__ HeadRec head_of_record(const float* rec, int hh) {
+    return {rec + hh * D, rec + NREP * D + hh, rec + NREP * D + NREP + hh};
+}
+// The inverse V transform of a head (rotor, FWHT-256, 1 / (16 d)): the lane's constants, then the transform.
+struct VInverse {
+    uint4 rotor[4], d;
+    __device__ __forceinline__ void load(const CompressedKV& P, int lane) {
+        const uint4* rp = reinterpret_cast<const uint4*>(P.v_rotor + lane * 32);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rotor[i] = rp[i];
+        d = *reinterpret_cast<const uint4*>(P.d_v + lane * 8);
+    }
+    __device__ __forceinline__ void apply(float (&a)[8], int lane) const {
+        const __half* hr = reinterpret_cast<const __half*>(rotor);
+        const __half* hd = reinterpret_cast<const __half*>(&d);
+        float z[8];
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float x = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x = fmaf(a[p * 4 + k], __half2float(hr[p * 16 + c * 4 + k]), x);
+                z[p * 4 + c] = x;
+            }
+        fwht256_lane8(z, lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = z[j] * ((1.0f / 16.0f) / (__half2float(hd[j]) + 1e-8f));
+    }
+};
+__device__ __forceinline__ void store_head(const HeadAcc& h, float* o, int lane) {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) *reinterpret_cast<float2*>(o + lane * 8 + j) = make_float2(h.a[j], h.a[j + 1]);
+    if (lane == 0) {
+        o[D] = h.m;
+        o[D + 1] = h.l;
+    }
+}
+
 // Merge the DEC_WPK warps of each kv-head inside the CTA, then the CTAs of the cluster.  On
 // return the sub==0 warps of cluster rank 0 hold the merged state.  `area` is shared memory no
 // longer used for anything else (>= 2*HKV*MERGE_FLOATS floats).  Must be called by all threads

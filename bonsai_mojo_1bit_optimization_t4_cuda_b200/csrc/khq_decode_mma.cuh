@@ -84,7 +84,7 @@ static_assert(M2_SM_TOTAL <= 227 * 1024 && M2_SM_C3 % 16 == 0 && M2_SM_ROPE % 16
               "shared memory budget");
 static_assert(HKV * MERGE_FLOATS * 4 <= 256 * M2_VQ_ROW, "cluster export records alias the codebook");
 static_assert(HKV * M2_WPK * MERGE_FLOATS * 4 <= M2_STAGES_BYTES, "records alias the stages");
-static_assert(HKV * NREP * D * 4 <= M2_STAGES_BYTES, "prologue scratch aliases the stages");
+static_assert(HKV * NREP * D * 4 <= M2_SM_BROT - M2_SM_ROPE, "the query build's scratch aliases the RoPE buffers");
 static_assert(M2_STAGE_BYTES % 16 == 0 && M2_OFF_KPAY % 16 == 0 && M2_OFF_VPAY % 16 == 0 && M2_OFF_KN % 16 == 0 &&
                   M2_OFF_VSM % 16 == 0, "bulk copy alignment");
 
@@ -214,10 +214,10 @@ __device__ __forceinline__ void m2_step_rope(float* dst, const float* src, const
 }
 
 // The layer's V codebook (entry (patch, code) starts at half 3 (256 patch + code)) into its shared-memory rows.  Two
-// codes (three words) per thread and iteration, eight iterations' loads in flight: bound by load latency.
+// codes (three words) per thread and iteration, eleven iterations' loads in flight: bound by load latency.
 __device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __half* __restrict__ vq, int tid) {
     const unsigned int* src = reinterpret_cast<const unsigned int*>(vq);
-#pragma unroll 8
+#pragma unroll 11
     for (int u = tid; u < NP * 256 / 2; u += M2_THREADS) {
         const unsigned int w0 = __ldg(src + 3 * u), w1 = __ldg(src + 3 * u + 1), w2 = __ldg(src + 3 * u + 2);
         const int patch = u >> 7, code = 2 * (u & 127);  // the pair never straddles a patch (256 codes)
@@ -230,8 +230,8 @@ __device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __ha
     }
 }
 
-// Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, the rotor B fragments (with and without the centroid factor) and the V
-// codebook.  Must be followed by __syncthreads().
+// Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, dim-3 centroids, the rotor B
+// fragments (with and without the centroid factor) and the V codebook.  Must be followed by __syncthreads().
 __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const CompressedKV& P, int tid) {
     float* freq_s = reinterpret_cast<float*>(smem + M2_SM_FREQ);
     float* dinv_s = reinterpret_cast<float*>(smem + M2_SM_DINV);
@@ -244,11 +244,11 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
     if (tid < 64) dinv_s[tid] = (1.0f / 256.0f) / (__half2float(P.d_k[tid]) + 1e-8f);
     if (tid >= 192 && tid < 224) {
         const int m = tid - 192;
-        double th = (double)M2_TT * (double)powf(P.rope_base, -2.0f * (float)m / 64.0f);
-        th -= rint(th * 0.15915494309189535) * 6.283185307179586;
+        // half turns of M2_TT positions: reduced in double, so the fp32 sine and cosine get an exact small argument
+        double th = (double)M2_TT * (double)powf(P.rope_base, -2.0f * (float)m / 64.0f) * 0.3183098861837907;
+        th -= 2.0 * rint(0.5 * th);
         float* o = reinterpret_cast<float*>(smem + M2_SM_RSTEP) + 4 * (m >> 1) + (m & 1);
-        o[0] = (float)cos(th);
-        o[2] = (float)sin(th);
+        sincospif((float)th, &o[2], &o[0]);
     }
     // Rotor B fragments with the three low index bits of the 64-point Hadamard transform folded
     // in: u[8j + n] is produced by step s = 2j + (n >> 2) as rotor output c = n & 3, and
@@ -259,6 +259,10 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
         const int g = lane >> 2, t = lane & 3;
         const int patch = 16 * t + s;
         const int kk[4] = {0, 2, 1, 3};  // dims 64t+4s + {0, 2, 1, 3}
+        __half hr[16], hc[4];
+        *reinterpret_cast<uint4*>(&hr[0]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16);
+        *reinterpret_cast<uint4*>(&hr[8]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16 + 8);
+        *reinterpret_cast<uint2*>(&hc[0]) = *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s);
         float rc[4], r1[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -267,10 +271,10 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
             for (int c = 0; c < 4; ++c) {
                 const int n = 4 * (s & 1) + c;
                 const float sgn = (__popc(n & g) & 1) ? -1.0f : 1.0f;
-                acc += sgn * __half2float(P.k_rotor[patch * 16 + c * 4 + kk[i]]);
+                acc += sgn * __half2float(hr[c * 4 + kk[i]]);
             }
             r1[i] = acc;
-            rc[i] = acc * __half2float(P.cents_k[2 * D + 64 * t + 4 * s + kk[i]]);
+            rc[i] = acc * __half2float(hc[kk[i]]);
         }
         uint2 hi, lo;
         m2_pack_hilo(rc[0], rc[1], hi.x, lo.x);
@@ -419,7 +423,7 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
     for (int i = 0; i < HPW; ++i) {
         const int h = sub + M2_WPK * i;
         const __half* hq = reinterpret_cast<const __half*>(&qraw[i]);
-        float x[8];
+        float x[8], y[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = __half2float(hq[j]) * dv[j];
         fwht256_lane8(x, lane);
@@ -430,8 +434,10 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
                 float a = 0.0f;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) a = fmaf(rr[p][c * 4 + k], x[p * 4 + c], a);
-                scratch[h * D + lane * 8 + p * 4 + k] = a;
+                y[p * 4 + k] = a;
             }
+        *reinterpret_cast<float4*>(scratch + h * D + lane * 8) = make_float4(y[0], y[1], y[2], y[3]);
+        *reinterpret_cast<float4*>(scratch + h * D + lane * 8 + 4) = make_float4(y[4], y[5], y[6], y[7]);
     }
     asm volatile("bar.sync %0, %1;" ::"r"(2 + kvh), "n"(32 * M2_WPK) : "memory");  // the kv-head's warps: all six heads are in the scratch
 #pragma unroll
@@ -854,38 +860,34 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
 }
 
 // Attention of all 24 query heads over compressed tokens [my_lo, my_hi) of P; the CTA's 12 warps
-// are (kv-head = warp & 3) x (group = warp >> 2: every third 16-token block).  On return,
-// warps 0..3 hold in `ws` the merged state of their kv-head's six heads in the first generation's
-// layout (lane = 8 dims, rotated V domain), ready for merge_from / v_epilogue_store.  Tables must
-// be set up; all M2_THREADS threads call it.
-template <bool ALL_WARPS_MERGE = false>  // true: every warp of a kv-head returns the kv-head's merged state
+// are (kv-head = warp & 3) x (group = warp >> 2: every third 16-token block).  On return (behind a CTA barrier) the
+// stages hold one record per warp (store_record's layout, rotated V domain).  Tables must be set up (the CTA barrier after
+// m2_setup_tables may still be outstanding); all M2_THREADS threads call it.
 __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const __half* __restrict__ q,
                                                     size_t q_head_stride, const CompressedKV& P, int my_lo, int my_hi,
-                                                    float scale, unsigned& blocks_done, WarpState& ws, uint32_t tmem) {
+                                                    float scale, unsigned& blocks_done, uint32_t tmem) {
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
-
-    M2Query Q;
-    Q.tm = tmem + ((uint32_t)(32 * kvh) << 16);
-    Q.rot = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ROT;
-    m2_build_query(Q, q, q_head_stride, P, kvh, sub, lane, reinterpret_cast<float*>(smem + M2_SM_STAGES) + kvh * NREP * D,
-                   reinterpret_cast<uint2*>(smem + M2_SM_QR) + kvh * 4 * 32);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();  // the query scratch aliases the stages
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the query and rotor fragments other warps stored
-
-    // group `sub` takes blocks sub, sub + M2_WPK, ... of M2_BT tokens
+    // group `sub` takes blocks sub, sub + M2_WPK, ... of M2_BT tokens; the first one is on its way during the query build
     const int base = (my_lo & ~1) + M2_BT * sub, gtid = 32 * kvh + lane;
     const int nblk = (my_hi > base) ? (my_hi - base + M2_TT - 1) / M2_TT : 0;
     const unsigned t0 = blocks_done;
     unsigned char* stages = smem + M2_SM_STAGES + sub * M2_NSTAGE * M2_STAGE_BYTES;
     float* rope_tab = reinterpret_cast<float*>(smem + M2_SM_ROPE) + sub * 2 * M2_BT * 64;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS) + sub * M2_NSTAGE;
-    if (nblk > 0) {
+    if (nblk > 0)
         m2_stage_tile(P, stages + (t0 % M2_NSTAGE) * M2_STAGE_BYTES, &bars[t0 % M2_NSTAGE], base, min(M2_BT, P.c_len - base), gtid, sub);
-        m2_fill_rope(rope_tab, freq_s, P, base, gtid);
-    }
+
+    M2Query Q;
+    Q.tm = tmem + ((uint32_t)(32 * kvh) << 16);
+    Q.rot = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ROT;
+    m2_build_query(Q, q, q_head_stride, P, kvh, sub, lane, reinterpret_cast<float*>(smem + M2_SM_ROPE) + kvh * NREP * D,
+                   reinterpret_cast<uint2*>(smem + M2_SM_QR) + kvh * 4 * 32);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();  // the query scratch aliases the RoPE buffers
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the query and rotor fragments other warps stored
+    if (nblk > 0) m2_fill_rope(rope_tab, freq_s, P, base, gtid);
     M2State st;
     st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + M2_TM_ACC_WARP * (uint32_t)sub;
     st.init();
@@ -965,22 +967,17 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
         }
     }
     __syncthreads();
-    ws.init();
-    if (ALL_WARPS_MERGE || warp < 4) {
-#pragma unroll
-        for (int r = 0; r < M2_WPK; ++r)
-            merge_from(ws, reinterpret_cast<const float*>(smem + M2_SM_STAGES) + (kvh + 4 * r) * MERGE_FLOATS, lane);
-    }
 }
 
-// Persistent batched kernel, second generation (same contract as khq_decode_batched_kernel).
+// Persistent batched kernel, second generation (same contract as khq_decode_batched_kernel, except that CTA b's first item is
+// item b and the counter hands out the ones from gridDim.x on: a launch of one item per CTA needs no counter at all).
 __global__ void __launch_bounds__(M2_THREADS, 1)
 khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesDesc* __restrict__ tables,
                               const KhqWorkItem* __restrict__ items, int n_items, int* __restrict__ counter,
                               float* __restrict__ partials, float scale, float rope_base, int ring_cap) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_next;
-    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
     uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
@@ -992,57 +989,53 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
+    pdl_wait();
+    pdl_trigger();
     int cur_table = -1;
     unsigned blocks_done = 0;
+    const float* rec = reinterpret_cast<const float*>(smem + M2_SM_STAGES);
 #pragma unroll 1
-    while (true) {
-        __syncthreads();
-        if (tid == 0) s_next = atomicAdd(counter, 1);
-        __syncthreads();
-        const int it = s_next;
-        if (it >= n_items) break;
+    for (int it = blockIdx.x; it < n_items;) {
         const KhqWorkItem w = items[it];
         const KhqSeqDesc d = descs[w.desc];
-        float* ob[NREP];
-#pragma unroll
-        for (int h = 0; h < NREP; ++h) ob[h] = partials + ((size_t)w.slot * HQ + kvh * NREP + h) * PART;
+        const KhqTablesDesc tb = tables[d.table_id];
+        CompressedKV P;
+        P.k_payload = d.k_payload; P.v_payload = d.v_payload; P.v_shared_meta = d.v_shared_meta;
+        P.k_mask = d.k_mask; P.k_norms = d.k_norms; P.k_r_norms = d.k_r_norms;
+        P.v_norms = d.v_norms; P.v_r_norms = d.v_r_norms;
+        P.cents_k = tb.cents_k; P.cents_v = tb.cents_v; P.vq = tb.vq; P.k_rotor = tb.k_rotor;
+        P.v_rotor = tb.v_rotor; P.d_k = tb.d_k; P.d_v = tb.d_v;
+        P.alpha_k = tb.alpha_k; P.alpha_v = tb.alpha_v; P.rope_base = rope_base;
+        P.start_pos = d.start_pos; P.c_len = d.c_len; P.bulk_ok = 1;
+        unpack_pos(d.pos_pack, P);
+        VInverse inv;
         if (w.kind == 0) {
-            const KhqTablesDesc tb = tables[d.table_id];
-            CompressedKV P;
-            P.k_payload = d.k_payload; P.v_payload = d.v_payload; P.v_shared_meta = d.v_shared_meta;
-            P.k_mask = d.k_mask; P.k_norms = d.k_norms; P.k_r_norms = d.k_r_norms;
-            P.v_norms = d.v_norms; P.v_r_norms = d.v_r_norms;
-            P.cents_k = tb.cents_k; P.cents_v = tb.cents_v; P.vq = tb.vq; P.k_rotor = tb.k_rotor;
-            P.v_rotor = tb.v_rotor; P.d_k = tb.d_k; P.d_v = tb.d_v;
-            P.alpha_k = tb.alpha_k; P.alpha_v = tb.alpha_v; P.rope_base = rope_base;
-            P.start_pos = d.start_pos; P.c_len = d.c_len; P.bulk_ok = 1;
-            unpack_pos(d.pos_pack, P);
             if (d.table_id != cur_table) {
                 m2_setup_tables(smem, P, tid);
                 cur_table = d.table_id;
                 __syncthreads();
                 m2_rotor_to_tmem(smem, tmem, warp, lane);
             }
-            WarpState ws;
-            m2_compressed_range<true>(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, ws, tmem);
-            // the three warps of a kv-head transform and store two heads each
-            static_assert(M2_WPK == 3 && NREP == 6, "head split of the item epilogue");
-            if (sub == 0) v_epilogue_store<0, 2>(ws, P, lane, ob);
-            else if (sub == 1) v_epilogue_store<2, 4>(ws, P, lane, ob);
-            else v_epilogue_store<4, 6>(ws, P, lane, ob);
+            m2_compressed_range(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, tmem);
+            inv.load(P, lane);
         } else {
             WarpState ws;
             ws.init();
-            window_range(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, M2_WPK, w.hi, ring_cap, scale, kvh, lane, ws);
-            float* rec = reinterpret_cast<float*>(smem + M2_SM_STAGES);
-            if (sub > 0) store_record(ws, rec + (kvh + 4 * (sub - 1)) * MERGE_FLOATS, lane);
+            window_range<4>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, M2_WPK, w.hi, ring_cap, scale, kvh, lane, ws);
+            store_record(ws, reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * MERGE_FLOATS, lane);
             __syncthreads();
-            if (sub == 0) {
-#pragma unroll
-                for (int r = 0; r < M2_WPK - 1; ++r) merge_from(ws, rec + (kvh + 4 * r) * MERGE_FLOATS, lane);
-                raw_store(ws, lane, ob);
-            }
         }
+        if (tid == 0) s_next = n_items > (int)gridDim.x ? (int)gridDim.x + atomicAdd(counter, 1) : n_items;
+        // two query heads per warp: merge of the three groups' records, inverse V transform, store
+#pragma unroll 1
+        for (int h = warp; h < HQ; h += M2_THREADS / 32) {
+            HeadAcc a = merge_head<true>(M2_WPK, lane, [&](int i) { return head_of_record(rec + (h / NREP + HKV * i) * MERGE_FLOATS, h % NREP); });
+            if (w.kind == 0) inv.apply(a.a, lane);
+            store_head(a, partials + ((size_t)w.slot * HQ + h) * PART, lane);
+        }
+        fence_proxy_async();  // the next item's bulk copies land where the records were
+        __syncthreads();      // the records and s_next
+        it = s_next;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1050,14 +1043,16 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
 }
 
 // Drop-in (single sequence-layer) variant: grid = num_splits * cluster_size CTAs; the CTAs of a
-// cluster share one of the caller's splits and merge through distributed shared memory.
+// cluster share one of the caller's splits.  Their per-warp records stay in each CTA's shared memory; behind a cluster
+// barrier the 24 heads are dealt to the cluster's warps, which merge them through distributed shared memory (one warp per
+// kv-head of rank 0 merging the peers one after the other took 10 us of a 25 us launch).
 __global__ void __launch_bounds__(M2_THREADS, 1)
 khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, float* __restrict__ out_attn,
                                float* __restrict__ out_partial, int num_splits, int L_q, int l_idx, int s_limit,
                                float scale) {
     extern __shared__ __align__(128) unsigned char smem[];
     cg::cluster_group cluster = cg::this_cluster();
-    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     const int split_id = blockIdx.x / csize;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
@@ -1077,40 +1072,32 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
+    pdl_wait();
+    pdl_trigger();
     m2_setup_tables(smem, P, tid);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
     m2_rotor_to_tmem(smem, tmem, warp, lane);
     unsigned blocks_done = 0;
-    WarpState ws;
-    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, ws, tmem);
+    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, tmem);
+    VInverse inv;
+    inv.load(P, lane);
     // the query fragments are not needed any more; everything below is ordinary memory
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    cluster.sync();
     m2_tm_free(tmem, warp);
-    // cluster merge: records exported over the (no longer needed) codebook area
-    float* exp_rec = reinterpret_cast<float*>(smem + M2_SM_VQ) + (warp & 3) * MERGE_FLOATS;
-    if (csize > 1) {
-        __syncthreads();  // every warp is done with the codebook
-        if (warp < 4) store_record(ws, exp_rec, lane);
-        cluster.sync();
-        if (crank == 0 && warp < 4) {
+    const float* rec = reinterpret_cast<const float*>(smem + M2_SM_STAGES);
 #pragma unroll 1
-            for (int r = 1; r < csize; ++r) merge_from(ws, cluster.map_shared_rank(exp_rec, r), lane);
-        }
-        cluster.sync();
+    for (int h = crank + csize * warp; h < HQ; h += csize * (M2_THREADS / 32)) {
+        HeadAcc a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
+            return head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * MERGE_FLOATS, h % NREP);
+        });
+        inv.apply(a.a, lane);
+        const int total_id = h * L_q + l_idx;
+        store_head(a, (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART : out_attn + (size_t)total_id * PART, lane);
     }
-    if (crank == 0 && warp < 4) {
-        float* ob[NREP];
-#pragma unroll
-        for (int h = 0; h < NREP; ++h) {
-            const int total_id = (warp * NREP + h) * L_q + l_idx;
-            ob[h] = (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART
-                                     : out_attn + (size_t)total_id * PART;
-        }
-        v_epilogue_store(ws, P, lane, ob);
-    }
+    cluster.sync();  // peers must stay resident until their records have been read
 }
 
 }  // namespace khq

@@ -856,7 +856,7 @@ khq_decode_batched_tc5_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
         } else if (warp < 8) {
             WarpState ws;
             ws.init();
-            window_range(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, 2, w.hi, ring_cap, scale, kvh, lane, ws);
+            window_range<1>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, 2, w.hi, ring_cap, scale, kvh, lane, ws);
             float* rec = reinterpret_cast<float*>(smem + SM_V) + kvh * MERGE_FLOATS;
             if (sub == 1) store_record(ws, rec, lane);
             dec_barrier();

@@ -67,7 +67,7 @@ __device__ __noinline__ void w_window_item(const KhqSeqDesc& d, const KhqWorkIte
     const int kvh = warp & 3, sub = warp >> 2;
     WarpState ws;
     ws.init();
-    window_range(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, 2, w.hi, ring_cap, scale, kvh, lane, ws);
+    window_range<1>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, 2, w.hi, ring_cap, scale, kvh, lane, ws);
     float* rec = reinterpret_cast<float*>(smem + SM_V) + kvh * MERGE_FLOATS;
     if (sub == 1) store_record(ws, rec, lane);
     dec_barrier();
