@@ -365,6 +365,8 @@ __device__ __forceinline__ void v_epilogue_store(const WarpState& st, const Comp
     }
 }
 
+// Records of the kernel before are read around L1 (__ldcg): with a dependent launch this kernel may have started before
+// they were written.
 // LSE merge of `n` partial records `stride` floats apart (acc[D], max, sum) by one block of
 // G * D threads: M = max m_i, num = sum acc_i[dd] e^{m_i - M}, den = sum s_i e^{m_i - M}.
 // Thread (group g, dim dd) adds records g, g + G, ... in order; the groups' sums are then
@@ -382,7 +384,7 @@ __device__ __forceinline__ float lse_merge_records(const float* __restrict__ bas
     __shared__ float s_num[G > 1 ? G - 1 : 1][D], s_den[G > 1 ? G - 1 : 1];
     const int tid = threadIdx.x, dd = tid & (D - 1), grp = tid / D;
     float M = NEG_BIG;
-    for (int s = tid; s < n; s += NT) M = fmaxf(M, base[s * stride + D]);
+    for (int s = tid; s < n; s += NT) M = fmaxf(M, __ldcg(base + s * stride + D));
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, m));
     if ((tid & 31) == 0) s_red[tid >> 5] = M;
@@ -395,14 +397,14 @@ __device__ __forceinline__ float lse_merge_records(const float* __restrict__ bas
     for (int s0 = 0; s0 < n; s0 += NT) {
         const int cnt = min(NT, n - s0);
         __syncthreads();
-        if (tid < cnt) s_w[tid] = __expf(base[(s0 + tid) * stride + D] - M);
+        if (tid < cnt) s_w[tid] = __expf(__ldcg(base + (s0 + tid) * stride + D) - M);
         __syncthreads();
 #pragma unroll 4
         for (int j = grp; j < cnt; j += G) {
             const float* p = base + (s0 + j) * stride;
             const float w = s_w[j];
-            num = fmaf(p[dd], w, num);
-            den = fmaf(p[D + 1], w, den);
+            num = fmaf(__ldcg(p + dd), w, num);
+            den = fmaf(__ldcg(p + D + 1), w, den);
         }
     }
     if (G > 1) {
@@ -543,11 +545,11 @@ __device__ __forceinline__ void raw_store(const WarpState& st, int lane, float* 
 // One cluster: token s is served by warp (kv, sub) of CTA c when
 // s % (cluster_size*DEC_WPK) == c*DEC_WPK + sub.  The heads of the result are dealt to the cluster's warps, which merge the
 // per-warp records through distributed shared memory.
-constexpr int WIN_SMEM = DEC_WARPS * MERGE_FLOATS * 4;  // one record per warp
+constexpr int WIN_SMEM = (DEC_WARPS * MERGE_FLOATS + HQ * PART) * 4;  // one record per warp; the CTA's own heads
 
 // Behind a cluster barrier: head h merged over the records of all warps of the cluster that served its kv-head.
 __device__ __forceinline__ HeadAcc window_head(cg::cluster_group& cluster, const float* rec, int csize, int h, int lane) {
-    return merge_head<true>(DEC_WPK * csize, lane, [&](int i) {
+    return merge_head<false>(DEC_WPK * csize, lane, [&](int i) {
         return head_of_record(cluster.map_shared_rank(rec, i / DEC_WPK) + (h / NREP + HKV * (i % DEC_WPK)) * MERGE_FLOATS, h % NREP);
     });
 }
@@ -667,9 +669,9 @@ khq_batched_merge_gate_few_kernel(const KhqSeqDesc* __restrict__ descs, const fl
         for (int i = 0; i < CH; ++i) {
             const bool in = s0 + i < d.n_slots;
             const float* p = base + (size_t)(in ? s0 + i : s0) * HQ * PART;
-            m[i] = in ? p[D] : NEG_BIG;
-            l[i] = in ? p[D + 1] : 0.0f;
-            a[i] = in ? p[dd] : 0.0f;
+            m[i] = in ? __ldcg(p + D) : NEG_BIG;
+            l[i] = in ? __ldcg(p + D + 1) : 0.0f;
+            a[i] = in ? __ldcg(p + dd) : 0.0f;
         }
         float cm = M;
 #pragma unroll
@@ -762,30 +764,37 @@ khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k
                     lane, st, new_s, new_k, new_v);
     store_record(st, rec + warp * MERGE_FLOATS, lane);
     cluster.sync();
+    // the window part of the heads dealt to this CTA (every csize-th), while the compressed-region kernel may still run
+    float* own = rec + DEC_WARPS * MERGE_FLOATS;
+#pragma unroll 1
+    for (int k = warp; crank + csize * k < HQ; k += DEC_WARPS) store_head(window_head(cluster, rec, csize, crank + csize * k, lane), own + k * PART, lane);
+    cluster.sync();  // peers must stay resident until their records have been read
     pdl_wait();
     pdl_trigger();
-#pragma unroll 1
-    for (int h = crank + csize * warp; h < HQ; h += csize * DEC_WARPS) {
-        const uint4 gr = *reinterpret_cast<const uint4*>(q + (size_t)h * 2 * D + D + lane * 8);
-        HeadAcc a = window_head(cluster, rec, csize, h, lane);
-        if (n_c > 0) {
-            const HeadAcc c = merge_head<false>(n_c, lane, [&](int i) {
-                const float* p = part_c + ((size_t)h * n_c + i) * PART;
-                return HeadRec{p, p + D, p + D + 1};
-            });
-            const float M = fmaxf(a.m, c.m), wa = __expf(a.m - M), wc = __expf(c.m - M);
-            a.l = a.l * wa + c.l * wc;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) a.a[j] = a.a[j] * wa + c.a[j] * wc;
+    // a thread finishes two dims of one head: all its loads of the split records are in flight together
+    for (int e = tid; e < (HQ - crank + csize - 1) / csize * (D / 2); e += DEC_THREADS) {
+        const int k = e / (D / 2), h = crank + csize * k, d = 2 * (e % (D / 2));
+        const float2 aw = *reinterpret_cast<const float2*>(own + k * PART + d);
+        float M = own[k * PART + D];
+        const float mw = M, lw = own[k * PART + D + 1];
+        const __half2 hg = *reinterpret_cast<const __half2*>(q + (size_t)h * 2 * D + D + d);
+        const float* pc = part_c + (size_t)h * n_c * PART;
+        for (int i = 0; i < n_c; ++i) M = fmaxf(M, __ldcg(pc + i * PART + D));
+        const float w0 = __expf(mw - M);
+        float num0 = aw.x * w0, num1 = aw.y * w0, den = lw * w0;
+#pragma unroll 8
+        for (int i = 0; i < n_c; ++i) {
+            const float w = __expf(__ldcg(pc + i * PART + D) - M);
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(pc + i * PART + d));
+            num0 = fmaf(v.x, w, num0);
+            num1 = fmaf(v.y, w, num1);
+            den = fmaf(__ldcg(pc + i * PART + D + 1), w, den);
         }
-        const float inv = 1.0f / (a.l + 1e-8f);
-        const __half* hg = reinterpret_cast<const __half*>(&gr);
-        __half o8[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o8[j] = __float2half(a.a[j] * inv * (1.0f / (1.0f + __expf(-__half2float(hg[j])))));
-        *reinterpret_cast<uint4*>(out + (size_t)h * D + lane * 8) = *reinterpret_cast<const uint4*>(o8);
+        const float inv = 1.0f / (den + 1e-8f);
+        const float2 gf = __half22float2(hg);
+        *reinterpret_cast<__half2*>(out + (size_t)h * D + d) =
+            __floats2half2_rn(num0 * inv * (1.0f / (1.0f + __expf(-gf.x))), num1 * inv * (1.0f / (1.0f + __expf(-gf.y))));
     }
-    cluster.sync();  // peers must stay resident until their records have been read
 }
 
 // LSE merge of the two regions, /(den + 1e-8), sigmoid gate, fp16 store.
@@ -798,14 +807,14 @@ __global__ void khq_merge_gate_kernel(const float* __restrict__ attn_c, const fl
     if (i >= H_q * d_v) return;
     const int h = i / d_v, d = i % d_v;
     const float* cc = attn_c + (size_t)h * (d_v + 2);
-    float num = cc[d], den = cc[d_v + 1];
+    float num = __ldcg(cc + d), den = __ldcg(cc + d_v + 1);
     if (has_w) {
         const float* cw = attn_w + (size_t)h * (d_v + 2);
-        const float mc = cc[d_v], mw = cw[d_v];
+        const float mc = __ldcg(cc + d_v), mw = __ldcg(cw + d_v);
         const float M = fmaxf(mc, mw);
         const float wc = __expf(mc - M), ww = __expf(mw - M);
-        num = num * wc + cw[d] * ww;
-        den = den * wc + cw[d_v + 1] * ww;
+        num = num * wc + __ldcg(cw + d) * ww;
+        den = den * wc + __ldcg(cw + d_v + 1) * ww;
     }
     const float val = num / (den + 1e-8f);
     const float g = __half2float(q_gate[(size_t)h * 2 * d_v + d_v + d]);

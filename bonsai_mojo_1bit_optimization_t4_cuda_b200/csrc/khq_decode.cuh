@@ -243,14 +243,15 @@ __device__ __forceinline__ void store_record(const WarpState& st, float* rec, in
 struct HeadAcc {
     float a[8], m, l;
 };
-// Where a record keeps a head: its 256 accumulators (16-byte aligned if V4, else 8-byte), maximum and sum.
+// Where a record keeps a head: its 256 accumulators, maximum and sum.
 struct HeadRec {
     const float *acc, *m, *l;
 };
 // LSE merge of one head over records at(0) .. at(n - 1), n <= 32, by a warp: lane i fetches the maximum and the sum of
 // record i, so the n weights cost one exchange, and the accumulators of four records are in flight together.  The records
-// may lie in this CTA's or a peer CTA's shared memory or in global memory.
-template <bool V4, class At>
+// may lie in this CTA's or a peer CTA's shared memory or in global memory.  PAD: the accumulators skip four floats after
+// every 32 (see m2_compressed_range).
+template <bool PAD, class At>
 __device__ __forceinline__ HeadAcc merge_head(int n, int lane, At at) {
     HeadAcc r;
     float m = NEG_BIG, l = 0.0f;
@@ -271,15 +272,10 @@ __device__ __forceinline__ HeadAcc merge_head(int n, int lane, At at) {
 #pragma unroll 4
     for (int i = 0; i < n; ++i) {
         const float wi = __shfl_sync(0xFFFFFFFFu, w, i);
-        const float* p = at(i).acc + lane * 8;
+        const float* p = at(i).acc + lane * 8 + (PAD ? 4 * (lane >> 2) : 0);
         float v[8];
-        if (V4) {
-            *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(p);
-            *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<const float4*>(p + 4);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) *reinterpret_cast<float2*>(&v[j]) = *reinterpret_cast<const float2*>(p + j);
-        }
+        *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<const float4*>(p);
+        *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<const float4*>(p + 4);
 #pragma unroll
         for (int j = 0; j < 8; ++j) r.a[j] = fmaf(v[j], wi, r.a[j]);
     }

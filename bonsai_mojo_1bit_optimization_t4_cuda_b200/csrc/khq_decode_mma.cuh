@@ -57,10 +57,8 @@ constexpr int M2_SM_STAGES = 0;
 constexpr int M2_VQ_ROW = (NP / 2) * 12 + 4;                         // 388 bytes per code
 constexpr int M2_SM_VQ = M2_SM_STAGES + M2_STAGES_BYTES;
 constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // per group two buffers of M2_BT tokens x 64 floats
-constexpr int M2_SM_BROT = M2_SM_ROPE + 2 * M2_TT * 64 * 4;          // 4 kinds x 16 steps x 32 lanes x 8 B: set-up only,
-constexpr int M2_SM_RSC = M2_SM_BROT;                                //   then 16 rows x 2 float4 per warp: scalars of a block's rows
-constexpr int M2_SM_FREQ = M2_SM_BROT + 4 * 16 * 32 * 8;
-static_assert(M2_THREADS / 32 * 16 * 32 <= 4 * 16 * 32 * 8, "row scalars alias the rotor fragments' staging");
+constexpr int M2_SM_RSC = M2_SM_ROPE + 2 * M2_TT * 64 * 4;           // 16 rows x 2 float4 per warp: scalars of a block's rows
+constexpr int M2_SM_FREQ = M2_SM_RSC + M2_THREADS / 32 * 16 * 32;
 constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats
 constexpr int M2_SM_BARS = M2_SM_DINV + 256;
 constexpr int M2_SM_C3 = M2_SM_BARS + 64;              // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
@@ -82,9 +80,27 @@ constexpr uint32_t M2_TM_COLS = 512, M2_TM_ROT = 128, M2_TM_ACC = 256, M2_TM_ACC
 static_assert(M2_TM_ACC + M2_TM_ACC_WARP * M2_WPK <= M2_TM_COLS, "tensor-memory columns");
 static_assert(M2_SM_TOTAL <= 227 * 1024 && M2_SM_C3 % 16 == 0 && M2_SM_ROPE % 16 == 0 && M2_SM_VQ % 16 == 0,
               "shared memory budget");
-static_assert(HKV * MERGE_FLOATS * 4 <= 256 * M2_VQ_ROW, "cluster export records alias the codebook");
-static_assert(HKV * M2_WPK * MERGE_FLOATS * 4 <= M2_STAGES_BYTES, "records alias the stages");
-static_assert(HKV * NREP * D * 4 <= M2_SM_BROT - M2_SM_ROPE, "the query build's scratch aliases the RoPE buffers");
+// Per-warp record: six heads of 256 floats, four floats of padding after every 32 (none after the last), then the maxima and
+// sums.  A thread stores eight consecutive dims of two heads; with this padding the float4 stores of a quarter-warp hit
+// distinct banks (unpadded, all 24 lanes of a store hit one bank and the records cost 7.5 us of a 25 us launch).
+constexpr int M2_REC_HEAD = D + 28, M2_REC_FLOATS = NREP * M2_REC_HEAD + 2 * NREP;
+static_assert(HKV * M2_WPK * M2_REC_FLOATS * 4 <= M2_STAGES_BYTES, "records alias the stages");
+__device__ __forceinline__ HeadRec m2_head_of_record(const float* rec, int hh) {
+    return {rec + hh * M2_REC_HEAD, rec + NREP * M2_REC_HEAD + hh, rec + NREP * M2_REC_HEAD + NREP + hh};
+}
+__device__ __forceinline__ void m2_store_record(const WarpState& st, float* rec, int lane) {
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) {
+        float* p = rec + h * M2_REC_HEAD + lane * 8 + 4 * (lane >> 2);
+        *reinterpret_cast<float4*>(p) = make_float4(st.acc[h][0], st.acc[h][1], st.acc[h][2], st.acc[h][3]);
+        *reinterpret_cast<float4*>(p + 4) = make_float4(st.acc[h][4], st.acc[h][5], st.acc[h][6], st.acc[h][7]);
+        if (lane == h) {  // static indices keep the state in registers
+            rec[NREP * M2_REC_HEAD + h] = st.m[h];
+            rec[NREP * M2_REC_HEAD + NREP + h] = st.l[h];
+        }
+    }
+}
+static_assert(HKV * NREP * D * 4 <= M2_SM_RSC - M2_SM_ROPE, "the query build's scratch aliases the RoPE buffers");
 static_assert(M2_STAGE_BYTES % 16 == 0 && M2_OFF_KPAY % 16 == 0 && M2_OFF_VPAY % 16 == 0 && M2_OFF_KN % 16 == 0 &&
                   M2_OFF_VSM % 16 == 0, "bulk copy alignment");
 
@@ -230,12 +246,11 @@ __device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __ha
     }
 }
 
-// Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, dim-3 centroids, the rotor B
-// fragments (with and without the centroid factor) and the V codebook.  Must be followed by __syncthreads().
+// Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, dim-3 centroids and the V codebook.
+// Must be followed by __syncthreads().
 __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const CompressedKV& P, int tid) {
     float* freq_s = reinterpret_cast<float*>(smem + M2_SM_FREQ);
     float* dinv_s = reinterpret_cast<float*>(smem + M2_SM_DINV);
-    uint2* brot = reinterpret_cast<uint2*>(smem + M2_SM_BROT);
     if (tid < 32) freq_s[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
     if (tid >= 128 && tid < 128 + NP) {
         const float c0 = __half2float(P.cents_v[0 * D + 4 * (tid - 128) + 3]), c1 = __half2float(P.cents_v[1 * D + 4 * (tid - 128) + 3]);
@@ -249,42 +264,6 @@ __device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const Compr
         th -= 2.0 * rint(0.5 * th);
         float* o = reinterpret_cast<float*>(smem + M2_SM_RSTEP) + 4 * (m >> 1) + (m & 1);
         sincospif((float)th, &o[2], &o[0]);
-    }
-    // Rotor B fragments with the three low index bits of the 64-point Hadamard transform folded
-    // in: u[8j + n] is produced by step s = 2j + (n >> 2) as rotor output c = n & 3, and
-    // H64 = H8 (bits 0..2, inside a tile) x H8 (bits 3..5, across tiles), so column n' of the
-    // folded operand is sum_n H8[n][n'] * (column n of the plain one).
-    for (int e = tid; e < 16 * 32; e += M2_THREADS) {
-        const int s = e >> 5, lane = e & 31;
-        const int g = lane >> 2, t = lane & 3;
-        const int patch = 16 * t + s;
-        const int kk[4] = {0, 2, 1, 3};  // dims 64t+4s + {0, 2, 1, 3}
-        __half hr[16], hc[4];
-        *reinterpret_cast<uint4*>(&hr[0]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16);
-        *reinterpret_cast<uint4*>(&hr[8]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16 + 8);
-        *reinterpret_cast<uint2*>(&hc[0]) = *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s);
-        float rc[4], r1[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int n = 4 * (s & 1) + c;
-                const float sgn = (__popc(n & g) & 1) ? -1.0f : 1.0f;
-                acc += sgn * __half2float(hr[c * 4 + kk[i]]);
-            }
-            r1[i] = acc;
-            rc[i] = acc * __half2float(hc[kk[i]]);
-        }
-        uint2 hi, lo;
-        m2_pack_hilo(rc[0], rc[1], hi.x, lo.x);
-        m2_pack_hilo(rc[2], rc[3], hi.y, lo.y);
-        brot[e] = hi;          // rotor * centroid (ternary operand), fp16 hi
-        brot[1024 + e] = lo;   //   and what fp16 lost
-        m2_pack_hilo(r1[0], r1[1], hi.x, lo.x);
-        m2_pack_hilo(r1[2], r1[3], hi.y, lo.y);
-        brot[512 + e] = hi;    // rotor (residual operand), fp16 hi
-        brot[1536 + e] = lo;   //   and what fp16 lost
     }
     m2_stage_codebook(smem + M2_SM_VQ, P.vq, tid);
 }
@@ -350,23 +329,49 @@ __device__ __forceinline__ void m2_tm_free(uint32_t tmem, int warp) {
     }
 }
 
-// The layer's rotor fragments from their shared-memory staging table into the tensor memory of every lane
-// quadrant (warps 0..3, one quadrant each).  After the CTA barrier that follows m2_setup_tables; the readers
-// pass another CTA barrier and a tcgen05 fence before their first load.
-__device__ __forceinline__ void m2_rotor_to_tmem(const unsigned char* smem, uint32_t tmem, int warp, int lane) {
-    if (warp < 4) {
-        const uint2* brot = reinterpret_cast<const uint2*>(smem + M2_SM_BROT);
-        const uint32_t dst = tmem + ((uint32_t)(32 * warp) << 16) + M2_TM_ROT;
-#pragma unroll 4
-        for (int s = 0; s < 16; ++s) {
-            const uint2 b1 = brot[s * 32 + lane], b2 = brot[512 + s * 32 + lane], b1l = brot[1024 + s * 32 + lane],
-                        b2l = brot[1536 + s * 32 + lane];
-            m2_tm_st8(dst + 8 * s, b1.x, b1.y, b2.x, b2.y, b1l.x, b1l.y, b2l.x, b2l.y);
+// The layer's rotor fragments (with and without the centroid factor) into the tensor memory of every lane quadrant; the
+// M2_WPK warps of a quadrant share the k-steps.  The readers pass a CTA barrier and a tcgen05 fence before their first load.
+// The three low index bits of the 64-point Hadamard transform are folded in: u[8j + n] is produced by step s = 2j + (n >> 2)
+// as rotor output c = n & 3, and H64 = H8 (bits 0..2, inside a tile) x H8 (bits 3..5, across tiles), so column n' of the
+// folded operand is sum_n H8[n][n'] * (column n of the plain one).
+__device__ __forceinline__ void m2_rotor_to_tmem(const CompressedKV& P, uint32_t tmem, int warp, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + M2_TM_ROT;
+#pragma unroll 2
+    for (int s = warp >> 2; s < 16; s += M2_WPK) {
+        const int patch = 16 * t + s;
+        __half hr[16], hc[4];
+        *reinterpret_cast<uint4*>(&hr[0]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16);
+        *reinterpret_cast<uint4*>(&hr[8]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16 + 8);
+        *reinterpret_cast<uint2*>(&hc[0]) = *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s);
+        const int kk[4] = {0, 2, 1, 3};  // dims 64t+4s + {0, 2, 1, 3}
+        float rc[4], r1[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int n = 4 * (s & 1) + c;
+                const float v = __half2float(hr[c * 4 + kk[i]]);
+                acc += (__popc(n & g) & 1) ? -v : v;
+            }
+            r1[i] = acc;
+            rc[i] = acc * __half2float(hc[kk[i]]);
         }
-        m2_tm_st_wait();
+        uint2 b1, b1l, b2, b2l;  // rotor * centroid (ternary operand), rotor (residual operand): fp16 and what fp16 lost
+        m2_pack_hilo(rc[0], rc[1], b1.x, b1l.x);
+        m2_pack_hilo(rc[2], rc[3], b1.y, b1l.y);
+        m2_pack_hilo(r1[0], r1[1], b2.x, b2l.x);
+        m2_pack_hilo(r1[2], r1[3], b2.y, b2l.y);
+        m2_tm_st8(dst + 8 * s, b1.x, b1.y, b2.x, b2.y, b1l.x, b1l.y, b2l.x, b2l.y);
     }
+    m2_tm_st_wait();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
+
+// Where the query build's scratch keeps the four dims 4c .. 4c + 3 of head h: swizzled so that the eight lanes (two heads, four
+// 64-dim quarters) of a float4 phase read distinct banks.
+__device__ __forceinline__ int m2_q_chunk(int h, int c) { return 4 * (c ^ ((c >> 4) & 3) ^ ((h & 1) << 2)); }
 
 // q: (H_q, ..) with `q_head_stride` halfs between heads.  scratch: this warp's NREP*D floats.
 __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restrict__ q, size_t q_head_stride,
@@ -436,8 +441,8 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
                 for (int c = 0; c < 4; ++c) a = fmaf(rr[p][c * 4 + k], x[p * 4 + c], a);
                 y[p * 4 + k] = a;
             }
-        *reinterpret_cast<float4*>(scratch + h * D + lane * 8) = make_float4(y[0], y[1], y[2], y[3]);
-        *reinterpret_cast<float4*>(scratch + h * D + lane * 8 + 4) = make_float4(y[4], y[5], y[6], y[7]);
+        *reinterpret_cast<float4*>(scratch + h * D + m2_q_chunk(h, 2 * lane)) = make_float4(y[0], y[1], y[2], y[3]);
+        *reinterpret_cast<float4*>(scratch + h * D + m2_q_chunk(h, 2 * lane + 1)) = make_float4(y[4], y[5], y[6], y[7]);
     }
     asm volatile("bar.sync %0, %1;" ::"r"(2 + kvh), "n"(32 * M2_WPK) : "memory");  // the kv-head's warps: all six heads are in the scratch
 #pragma unroll
@@ -447,7 +452,7 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
             const int d0 = 64 * t + 4 * s;
             float v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if (g < NREP) {
-                const float4 qq = *reinterpret_cast<const float4*>(scratch + g * D + d0);
+                const float4 qq = *reinterpret_cast<const float4*>(scratch + g * D + m2_q_chunk(g, d0 >> 2));
                 const __half* hc = reinterpret_cast<const __half*>(&cck[i]);
                 v[0] = qq.x; v[1] = qq.z; v[2] = qq.y; v[3] = qq.w;  // dims d0 + {0, 2, 1, 3}
                 c[0] = __half2float(hc[0]); c[1] = __half2float(hc[2]); c[2] = __half2float(hc[1]); c[3] = __half2float(hc[3]);
@@ -514,14 +519,15 @@ struct M2KSums {
 };
 
 // Returns whether a word of the lane needs another path than the common one.
-__device__ __forceinline__ bool m2_open_rows(M2KRows& kr, const unsigned char* __restrict__ S, int kvh, int lane) {
+__device__ __forceinline__ bool m2_open_rows(M2KRows& kr, const unsigned char* __restrict__ S, int kvh, int lane, int valid_hi) {
     const int g = lane >> 2, t = lane & 3;
     bool odd = false;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         const int row = (g + 8 * x) * HKV + kvh;
         kr.kp[x] = reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY);
-        const uint4 m = *reinterpret_cast<const uint4*>(S + M2_OFF_MASK + row * 64 + 16 * t);
+        uint4 m = *reinterpret_cast<const uint4*>(S + M2_OFF_MASK + row * 64 + 16 * t);
+        if (g + 8 * x >= valid_hi) m = make_uint4(0u, 0u, 0u, 0u);  // nothing may be staged there: leftovers would take the rare paths
         kr.mw[x] = m;
         // outliers of this thread's quarter, then the ordinal of its first one (scan over the quad)
         const uint32_t wc = khq3::k3_count(m.x) + (khq3::k3_count(m.y) << 8) + (khq3::k3_count(m.z) << 16) + (khq3::k3_count(m.w) << 24);
@@ -650,7 +656,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     }
     // ================================ K side: scores ==========================================
     M2KRows kr;
-    const bool odd = m2_open_rows(kr, S, kvh, lane);
+    const bool odd = m2_open_rows(kr, S, kvh, lane, valid_hi);
     __syncwarp();
     const float ratio[2] = {rsc[2 * g].z, rsc[2 * (g + 8)].z};
     M2KSums ks;
@@ -861,11 +867,11 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
 
 // Attention of all 24 query heads over compressed tokens [my_lo, my_hi) of P; the CTA's 12 warps
 // are (kv-head = warp & 3) x (group = warp >> 2: every third 16-token block).  On return (behind a CTA barrier) the
-// stages hold one record per warp (store_record's layout, rotated V domain).  Tables must be set up (the CTA barrier after
-// m2_setup_tables may still be outstanding); all M2_THREADS threads call it.
+// stages hold one record per warp (store_record's layout, rotated V domain).  The set-up of the tables may still be
+// under way (the barrier after the query build covers it); all M2_THREADS threads call it.
 __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const __half* __restrict__ q,
                                                     size_t q_head_stride, const CompressedKV& P, int my_lo, int my_hi,
-                                                    float scale, unsigned& blocks_done, uint32_t tmem) {
+                                                    float scale, unsigned& blocks_done, uint32_t tmem, VInverse& inv) {
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
@@ -914,6 +920,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
     }
     blocks_done = t0 + (unsigned)nblk;
     __syncthreads();  // the records alias the stages
+    inv.load(P, lane);  // for the caller, in flight behind the records
 
     // ---- per-warp record in the first generation's layout, then merge + inverse V transform --------
 #pragma unroll
@@ -933,7 +940,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
         fin[e] = __expf(st.m[e] - st.top[e]);
         st.l[e] *= fin[e];
     }
-    float* rec = reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * MERGE_FLOATS;
+    float* rec = reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * M2_REC_FLOATS;
     const float2* c3s = reinterpret_cast<const float2*>(smem + M2_SM_C3) + 8 * g;
 #pragma unroll
     for (int pp = 0; pp < 4; ++pp) {
@@ -942,28 +949,30 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
         m2_tm_ld4f(st.tm_o + 20 * pp + 16, &o[4][0]);
         m2_tm_ld_wait();
         if (t < 3) {
-            float* rp = rec + 2 * t * D + 4 * (8 * g + 2 * pp);  // head 2t, dim 0 of patch 2pp; head 2t + 1 is D further
+            // heads 2t and 2t + 1, dims 32 g + 8 pp .. + 7
 #pragma unroll
-            for (int idx = 0; idx < 6; ++idx) {
-                rp[4 * (idx / 3) + idx % 3] = fin[0] * o[idx >> 1][2 * (idx & 1)];
-                rp[D + 4 * (idx / 3) + idx % 3] = fin[1] * o[idx >> 1][2 * (idx & 1) + 1];
-            }
+            for (int e = 0; e < 2; ++e) {
+                float* rp = rec + (2 * t + e) * M2_REC_HEAD + 36 * g + 8 * pp;
+                float v[8];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float2 c = c3s[2 * pp + u];
+                for (int idx = 0; idx < 6; ++idx) v[4 * (idx / 3) + idx % 3] = fin[e] * o[idx >> 1][2 * (idx & 1) + e];
 #pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    rp[e * D + 4 * u + 3] = fin[e] * (fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
-                                                      fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]));
+                for (int u = 0; u < 2; ++u) {
+                    const float2 c = c3s[2 * pp + u];
+                    v[4 * u + 3] = fin[e] * (fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
+                                             fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]));
+                }
+                *reinterpret_cast<float4*>(rp) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4*>(rp + 4) = make_float4(v[4], v[5], v[6], v[7]);
             }
         }
     }
     if (t < 3) {
         if (g == 0) {
-            rec[NREP * D + 2 * t] = st.top[0];
-            rec[NREP * D + 2 * t + 1] = st.top[1];
-            rec[NREP * D + NREP + 2 * t] = st.l[0];
-            rec[NREP * D + NREP + 2 * t + 1] = st.l[1];
+            rec[NREP * M2_REC_HEAD + 2 * t] = st.top[0];
+            rec[NREP * M2_REC_HEAD + 2 * t + 1] = st.top[1];
+            rec[NREP * M2_REC_HEAD + NREP + 2 * t] = st.l[0];
+            rec[NREP * M2_REC_HEAD + NREP + 2 * t + 1] = st.l[1];
         }
     }
     __syncthreads();
@@ -1013,23 +1022,21 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
             if (d.table_id != cur_table) {
                 m2_setup_tables(smem, P, tid);
                 cur_table = d.table_id;
-                __syncthreads();
-                m2_rotor_to_tmem(smem, tmem, warp, lane);
+                m2_rotor_to_tmem(P, tmem, warp, lane);
             }
-            m2_compressed_range(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, tmem);
-            inv.load(P, lane);
+            m2_compressed_range(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, tmem, inv);
         } else {
             WarpState ws;
             ws.init();
             window_range<4>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, M2_WPK, w.hi, ring_cap, scale, kvh, lane, ws);
-            store_record(ws, reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * MERGE_FLOATS, lane);
+            m2_store_record(ws, reinterpret_cast<float*>(smem + M2_SM_STAGES) + warp * M2_REC_FLOATS, lane);
             __syncthreads();
         }
         if (tid == 0) s_next = n_items > (int)gridDim.x ? (int)gridDim.x + atomicAdd(counter, 1) : n_items;
         // two query heads per warp: merge of the three groups' records, inverse V transform, store
 #pragma unroll 1
         for (int h = warp; h < HQ; h += M2_THREADS / 32) {
-            HeadAcc a = merge_head<true>(M2_WPK, lane, [&](int i) { return head_of_record(rec + (h / NREP + HKV * i) * MERGE_FLOATS, h % NREP); });
+            HeadAcc a = merge_head<true>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
             if (w.kind == 0) inv.apply(a.a, lane);
             store_head(a, partials + ((size_t)w.slot * HQ + h) * PART, lane);
         }
@@ -1074,15 +1081,14 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     m2_tm_alloc(tm_slot, warp);
     pdl_wait();
     pdl_trigger();
-    m2_setup_tables(smem, P, tid);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
-    m2_rotor_to_tmem(smem, tmem, warp, lane);
+    m2_setup_tables(smem, P, tid);
+    m2_rotor_to_tmem(P, tmem, warp, lane);
     unsigned blocks_done = 0;
-    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, tmem);
     VInverse inv;
-    inv.load(P, lane);
+    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, tmem, inv);
     // the query fragments are not needed any more; everything below is ordinary memory
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster.sync();
@@ -1091,7 +1097,7 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
 #pragma unroll 1
     for (int h = crank + csize * warp; h < HQ; h += csize * (M2_THREADS / 32)) {
         HeadAcc a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
-            return head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * MERGE_FLOATS, h % NREP);
+            return m2_head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * M2_REC_FLOATS, h % NREP);
         });
         inv.apply(a.a, lane);
         const int total_id = h * L_q + l_idx;
