@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "khq_decode.cuh"
+#include "khq_launch.cuh"
 
 namespace khq {
 
@@ -744,11 +745,11 @@ khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-    const int new_s = win_len - 1;
+    const int new_s = new_k != nullptr ? win_len - 1 : -1;  // -1: the token's rows are in the rings already
     float* rec = reinterpret_cast<float*>(smem);
     if (n_c == 0) pdl_wait();
     if (crank == 0) {  // ring appends: 3 rows of H_kv*D halfs = 3 x 128 sixteen-byte chunks
-        const int slot = (win_start + new_s) % ring_cap;
+        const int slot = (win_start + win_len - 1) % ring_cap;
         const size_t row = (size_t)slot * HKV * D;
         for (int c = tid; c < 3 * (HKV * D / 8); c += DEC_THREADS) {
             const int which = c / (HKV * D / 8), i = c % (HKV * D / 8);
@@ -942,29 +943,6 @@ __global__ void khq_gather_q_kernel(const __half* __restrict__ q_gate, __half* _
 // Host side
 // ------------------------------------------------------------------------------------------
 static inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
-
-// cluster == 0: no cluster attribute.  All kernels launched through here begin with pdl_wait() (or know what they may do
-// before it), so they carry the programmatic-serialisation attribute: their launch latency and prologue overlap the end of
-// the kernel before them.
-template <typename Kernel, typename... Args>
-static cudaError_t launch_pdl(Kernel kernel, unsigned grid, unsigned cluster, size_t smem_bytes,
-                              cudaStream_t stream, unsigned threads, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem_bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = cluster > 0 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 // Opt in to >48 KB of dynamic shared memory, once per device.
 static cudaError_t ensure_smem_attrs() {
@@ -1189,15 +1167,14 @@ extern "C" int launch_khq_merge_gate_fp16(const void* attn_c, const void* attn_w
 // c_len tokens (launch_khq_attn_fp16 with its arguments; skipped when c_len == 0), then the fused
 // ring append + window attention + merge + gate kernel.  win_len counts the step's own token,
 // which is appended at slot (win_start + win_len - 1) % ring_cap.
-extern "C" int launch_khq_decode_step_fp16(
+// k_roped == v_new == NULL: the token's rows are in the rings already (a pre-step appended them).
+static int decode_step_impl(
     const void* q_gate, const void* k_roped, const void* v_new, const void* k_unroped, void* ring_k, void* ring_v,
     void* ring_u, const void* k_payload, const void* v_payload, const void* v_shared_meta, const void* k_mask,
     const void* k_norms, const void* k_r_norms, const void* v_norms, const void* v_r_norms, const void* centroids_k,
     const void* centroids_v, const void* vq_centroids, const void* k_rotor, const void* v_rotor, const void* d_vec_k,
     const void* d_vec_v, void* attn_c, void* attn_partial, void* out, int c_len, int win_start, int win_len, int ring_cap,
     int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, cudaStream_t stream) {
-    if (!q_gate || !k_roped || !v_new || !ring_k || !ring_v || !attn_c || !out || win_len <= 0 || c_len < 0) return -100;
-    if (ring_cap <= 0 || win_len > ring_cap) return -103;
     const void* al[] = {q_gate, k_roped, v_new, k_unroped, ring_k, ring_v, ring_u, out};
     for (const void* p : al)
         if (p && !aligned(p, 16)) return -104;
@@ -1219,6 +1196,66 @@ extern "C" int launch_khq_decode_step_fp16(
                      static_cast<const __half*>(v_new), static_cast<const __half*>(k_unroped), part_c, static_cast<__half*>(out),
                      win_start, win_len, ring_cap, scale, c_len > 0 ? (tail_merges ? num_splits : 1) : 0);
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
+}
+
+extern "C" int launch_khq_decode_step_fp16(
+    const void* q_gate, const void* k_roped, const void* v_new, const void* k_unroped, void* ring_k, void* ring_v,
+    void* ring_u, const void* k_payload, const void* v_payload, const void* v_shared_meta, const void* k_mask,
+    const void* k_norms, const void* k_r_norms, const void* v_norms, const void* v_r_norms, const void* centroids_k,
+    const void* centroids_v, const void* vq_centroids, const void* k_rotor, const void* v_rotor, const void* d_vec_k,
+    const void* d_vec_v, void* attn_c, void* attn_partial, void* out, int c_len, int win_start, int win_len, int ring_cap,
+    int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, cudaStream_t stream) {
+    if (!q_gate || !k_roped || !v_new || !ring_k || !ring_v || !attn_c || !out || win_len <= 0 || c_len < 0) return -100;
+    if (ring_cap <= 0 || win_len > ring_cap) return -103;
+    return decode_step_impl(q_gate, k_roped, v_new, k_unroped, ring_k, ring_v, ring_u, k_payload, v_payload, v_shared_meta, k_mask,
+                            k_norms, k_r_norms, v_norms, v_r_norms, centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor,
+                            d_vec_k, d_vec_v, attn_c, attn_partial, out, c_len, win_start, win_len, ring_cap, num_splits, scale,
+                            alpha_k, alpha_v, rope_base, stream);
+}
+
+// One decode step of one layer from a context that keeps the layer's addresses: compression event if due, compressed-region
+// attention, and the fused tail (mirrored in include/khq_b200.h).
+struct khq_layer_ctx {
+    const void *d_k, *cents_k, *rotor_k, *d_v, *cents_v, *rotor_v, *vq;
+    void *ring_k, *ring_v, *ring_u;
+    void *k_mask, *k_payload, *k_norms, *k_r_norms, *v_payload, *v_norms, *v_r_norms, *v_shared_meta;
+    void *attn_c, *attn_partial;
+    float ts_k, alpha_k, ts_v, alpha_v, rope_base;
+    int ring_cap;
+};
+static_assert(sizeof(khq_layer_ctx) == 20 * 8 + 24, "ABI");
+extern "C" int launch_khq_compress_fp16(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
+                                        void*, int, int, float, float, int, cudaStream_t);
+
+extern "C" int launch_khq_layer_step(const khq_layer_ctx* L, const void* q_gate, const void* k_roped, const void* v_new,
+                                     const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits,
+                                     float scale, cudaStream_t stream) {
+    constexpr int CHUNK = 128;
+    if (!L || !q_gate || !out || win_len <= 0 || c_len < 0 || !L->attn_c || (k_roped == nullptr) != (v_new == nullptr)) return -100;
+    if (L->ring_cap <= 0 || win_len > L->ring_cap) return -103;
+    if (compress) {  // the 128 oldest raw tokens, contiguous in the ring; the step's own token is not among them
+        const int s0 = c_len % L->ring_cap, row = c_len * HKV;
+        if (win_len <= CHUNK || s0 + CHUNK > L->ring_cap) return -103;
+        const auto at = [](void* p, size_t bytes) { return static_cast<void*>(static_cast<char*>(p) + bytes); };
+        const size_t src = (size_t)s0 * HKV * D * sizeof(__half);
+        // K first: it zeroes the shared meta rows that the V launch then fills
+        int rc = launch_khq_compress_fp16(at(L->ring_u, src), L->d_k, L->rotor_k, L->cents_k, L->cents_k, at(L->k_mask, (size_t)row * 64),
+                                          at(L->k_norms, (size_t)row * 2), at(L->k_r_norms, (size_t)row * 2),
+                                          at(L->k_payload, (size_t)row * K_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
+                                          L->ts_k, L->alpha_k, 0, stream);
+        if (rc != 0) return rc;
+        rc = launch_khq_compress_fp16(at(L->ring_v, src), L->d_v, L->rotor_v, L->cents_v, L->vq, at(L->k_mask, (size_t)row * 64),
+                                      at(L->v_norms, (size_t)row * 2), at(L->v_r_norms, (size_t)row * 2),
+                                      at(L->v_payload, (size_t)row * V_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
+                                      L->ts_v, L->alpha_v, 1, stream);
+        if (rc != 0) return rc;
+        c_len += CHUNK;
+        win_len -= CHUNK;
+    }
+    return decode_step_impl(q_gate, k_roped, v_new, k_unroped, L->ring_k, L->ring_v, L->ring_u, L->k_payload, L->v_payload,
+                            L->v_shared_meta, L->k_mask, L->k_norms, L->k_r_norms, L->v_norms, L->v_r_norms, L->cents_k, L->cents_v,
+                            L->vq, L->rotor_k, L->rotor_v, L->d_k, L->d_v, L->attn_c, L->attn_partial, out, c_len,
+                            c_len % L->ring_cap, win_len, L->ring_cap, num_splits, scale, L->alpha_k, L->alpha_v, L->rope_base, stream);
 }
 
 extern "C" int launch_khq_gather_q_fp16(const void* q_gate, void* q_out, int H_q, int d,

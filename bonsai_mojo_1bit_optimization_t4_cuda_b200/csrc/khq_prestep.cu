@@ -13,6 +13,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "khq_common.cuh"
+#include "khq_launch.cuh"
+
 namespace khq_prestep {
 
 __device__ __forceinline__ void norm_head(__half* x, const float* w, int dim, float eps, int lane) {
@@ -60,6 +63,8 @@ khq_prestep_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, const __
                    __half* __restrict__ ring_v, __half* __restrict__ ring_u, int H_q, int d, int rotary_dim, int pos,
                    float theta, float eps, int has_norms) {
     const int h = blockIdx.x, lane = threadIdx.x;
+    khq::pdl_wait();
+    khq::pdl_trigger();
     if (h < H_q) {
         __half* x = q_gate + (size_t)h * 2 * d;
         norm_head(x, has_norms ? q_norm_w : nullptr, d, eps, lane);
@@ -87,6 +92,8 @@ khq_prestep_batched_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, 
                            int H_q, int H_kv, int d, int rotary_dim, float theta, float eps, int has_norms) {
     const int per = H_q + H_kv;
     const int b = blockIdx.x / per, h = blockIdx.x % per, lane = threadIdx.x;
+    khq::pdl_wait();
+    khq::pdl_trigger();
     const int pos = positions[b];
     if (h < H_q) {
         __half* x = q_gate + ((size_t)b * H_q + h) * 2 * d;
@@ -116,12 +123,11 @@ extern "C" int launch_khq_prestep_fp16(void* q_gate, void* k, const void* v, con
     const void* ptrs[] = {q_gate, k, v, ring_k_slot, ring_v_slot, ring_u_slot};
     for (const void* p : ptrs)
         if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return -104;
-    khq_prestep::khq_prestep_kernel<<<H_q + H_kv, 32, 0, stream>>>(
-        static_cast<__half*>(q_gate), static_cast<__half*>(k), static_cast<const __half*>(v),
+    const cudaError_t err = khq::launch_pdl(
+        khq_prestep::khq_prestep_kernel, (unsigned)(H_q + H_kv), 0, 0, stream, 32, static_cast<__half*>(q_gate), static_cast<__half*>(k), static_cast<const __half*>(v),
         static_cast<const float*>(q_norm_w), static_cast<const float*>(k_norm_w), static_cast<__half*>(ring_k_slot),
         static_cast<__half*>(ring_v_slot), static_cast<__half*>(ring_u_slot), H_q, d, rotary_dim, pos, rope_theta,
         rms_eps, has_norms);
-    const cudaError_t err = cudaGetLastError();
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
@@ -139,11 +145,10 @@ extern "C" int launch_khq_prestep_batched_fp16(void* q_gate, void* k, const void
     for (const void* p : ptrs)
         if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return -104;
     if ((ring_seq_stride & 7) != 0) return -104;
-    khq_prestep::khq_prestep_batched_kernel<<<(unsigned)(batch * (H_q + H_kv)), 32, 0, stream>>>(
-        static_cast<__half*>(q_gate), static_cast<__half*>(k), static_cast<const __half*>(v),
+    const cudaError_t err = khq::launch_pdl(
+        khq_prestep::khq_prestep_batched_kernel, (unsigned)(batch * (H_q + H_kv)), 0, 0, stream, 32, static_cast<__half*>(q_gate), static_cast<__half*>(k), static_cast<const __half*>(v),
         static_cast<const float*>(q_norm_w), static_cast<const float*>(k_norm_w), static_cast<__half*>(ring_k),
         static_cast<__half*>(ring_v), static_cast<__half*>(ring_u), ring_seq_stride, static_cast<const int*>(slots),
         static_cast<const int*>(positions), H_q, H_kv, d, rotary_dim, rope_theta, rms_eps, has_norms);
-    const cudaError_t err = cudaGetLastError();
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }

@@ -15,13 +15,15 @@ ring appends of ALL sequences (``launch_khq_prestep_batched_fp16``), one K and o
 launch over the sequences whose event is due (``launch_khq_compress_batched_fp16``), and one
 batched attention launch (``launch_khq_decode_batched_fp16``); the work items are re-planned
 on the host every step and the step-dependent descriptor fields of every layer are rewritten by
-one small launch (``launch_khq_update_descs``).
+one small launch (``launch_khq_update_descs``).  All of it is issued by one native call
+(``launch_khq_engine_step``).
 
 State layout: one contiguous device buffer per payload array and per layer, each sequence's
 slice sized for its capacity and starting on a 128-row boundary.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Sequence
 
 import numpy as np
@@ -39,6 +41,7 @@ CHUNK = 128
 WATERMARK = 256
 KV = H_KV * D  # halfs per token row group
 ROTARY_DIM = 64
+COPY_BYTES = 256 * 1024
 SEQ_DYN = np.dtype([("c_len", "<i4"), ("start_pos", "<i4"), ("win_start", "<i4"), ("win_len", "<i4"),
                     ("first_slot", "<i4"), ("n_slots", "<i4"), ("r0", "<i4"), ("r1", "<i4")])
 COMPRESS_SEG = np.dtype([("x", "<u8"), ("row0", "<i8")])
@@ -105,12 +108,12 @@ class BatchEngine:
         self.ring_k = [ring() for _ in range(self.L)]
         self.ring_v = [ring() for _ in range(self.L)]
         self.ring_u = [ring() for _ in range(self.L)]
-        self.q_gate = [z(self.B * H_Q * 2 * D, torch.float16).view(self.B, H_Q * 2 * D) for _ in range(self.L)]
-        self.out = [z(self.B * H_Q * D, torch.float16).view(self.B, H_Q * D) for _ in range(self.L)]
-        # two parities of the K / V input rows: the copy stream fills one while the pre-step reads the other
-        self.d_k = [z(self.B * KV, torch.float16).view(self.B, KV) for _ in range(2)]
-        self.d_v = [z(self.B * KV, torch.float16).view(self.B, KV) for _ in range(2)]
-        self._copy_stream = torch.cuda.Stream(device=dev) if dev.type == "cuda" else None
+        # inputs and outputs of all layers in one buffer each, so that a copy can take several layers
+        self._q = z(self.L * self.B * H_Q * 2 * D, torch.float16).view(self.L, self.B, H_Q * 2 * D)
+        self._out = z(self.L * self.B * H_Q * D, torch.float16).view(self.L, self.B, H_Q * D)
+        self._k = z(self.L * self.B * KV, torch.float16).view(self.L, self.B, KV)
+        self._v = z(self.L * self.B * KV, torch.float16).view(self.L, self.B, KV)
+        self.q_gate, self.out = list(self._q), list(self._out)
         # ---- descriptors: layer-major, pointers fixed, the step-dependent ints rewritten per step
         d = np.zeros(self.L * self.B, SEQ_DESC)
         for l in range(self.L):
@@ -141,11 +144,17 @@ class BatchEngine:
         self.max_items = int(sum((int(c) + self.tokens_per_item - 1) // self.tokens_per_item + 2 for c in self.cap)) + tail_items
         self.ws_bytes = int(self.lib.khq_b200_decode_workspace_bytes(self.max_items))
         self.workspace = z(self.ws_bytes, torch.uint8)
-        self.d_items = z(self.max_items * WORK_ITEM.itemsize, torch.uint8)
-        self.d_dyn = z(self.B * SEQ_DYN.itemsize, torch.uint8)
-        self.d_slots = z(self.B, torch.int32)
-        self.d_pos = z(self.B, torch.int32)
-        self.d_segs = z(self.L * self.B * COMPRESS_SEG.itemsize, torch.uint8)
+        # a step's control block: per-sequence state, ring slots, positions, work items and, last, the runs that are
+        # compressed this step (copied only when there are some); one copy per step, device and host laid out alike
+        parts = [("dyn", self.B * SEQ_DYN.itemsize), ("slots", self.B * 4), ("pos", self.B * 4), ("items", self.max_items * WORK_ITEM.itemsize),
+                 ("segs", self.L * self.B * COMPRESS_SEG.itemsize)]
+        self._at, n = {}, 0
+        for name, size in parts:
+            self._at[name] = n
+            n = _align(n + size, 128)
+        self.d_control = z(n, torch.uint8)
+        self.d_items = self.d_control[self._at["items"]:]
+        self.d_dyn = self.d_control[self._at["dyn"]:self._at["dyn"] + self.B * SEQ_DYN.itemsize]
         # ---- pinned host staging: two parities of the control block, one set of data buffers ----
         cuda = dev.type == "cuda"
         pin = lambda *shape, dt=torch.float16: (torch.zeros(*shape, dtype=dt).pin_memory() if cuda else torch.zeros(*shape, dtype=dt))
@@ -153,14 +162,61 @@ class BatchEngine:
         self.h_k = pin(self.L, self.B, KV)
         self.h_v = pin(self.L, self.B, KV)
         self.h_out = pin(self.L, self.B, H_Q * D)
-        self._ctl = [dict(items=pin(self.max_items * WORK_ITEM.itemsize, dt=torch.uint8), dyn=pin(self.B * SEQ_DYN.itemsize, dt=torch.uint8),
-                          slots=pin(self.B, dt=torch.int32), pos=pin(self.B, dt=torch.int32),
-                          segs=pin(self.L * self.B * COMPRESS_SEG.itemsize, dt=torch.uint8),
-                          done=(torch.cuda.Event() if cuda else None)) for _ in range(2)]
+        self._ctl = []
+        for _ in range(2):
+            block = pin(n, dt=torch.uint8)
+            raw = block.numpy()
+            part = lambda name, dt, count: raw[self._at[name]:self._at[name] + count * np.dtype(dt).itemsize].view(dt)
+            self._ctl.append(dict(block=block, dyn=part("dyn", SEQ_DYN, self.B), slots=part("slots", np.int32, self.B),
+                                  pos=part("pos", np.int32, self.B), items=part("items", WORK_ITEM, self.max_items),
+                                  segs=part("segs", COMPRESS_SEG, self.L * self.B).reshape(self.L, self.B)))
+        # ---- native side: copy streams and events, the layers' addresses, the step's arguments --------
+        self._native = ctypes.c_void_p()
+        if cuda:
+            with torch.cuda.device(dev):
+                check("khq_b200_engine_create", self.lib.khq_b200_engine_create(ctypes.byref(self._native)))
+        self._layers = (_lib.EngineLayer * self.L)()
+        for l in range(self.L):
+            y, tb = self._layers[l], self.tables[l]
+            for f, src in (("d_k", "d_k"), ("cents_k", "cents_k"), ("rotor_k", "k_rotor"), ("d_v", "d_v"), ("cents_v", "cents_v"),
+                           ("rotor_v", "v_rotor"), ("vq", "vq")):
+                setattr(y, f, tb[src].data_ptr())
+            for f, src in self.pay[l].items():
+                setattr(y, f, src.data_ptr())
+            y.ring_k, y.ring_v, y.ring_u = self.ring_k[l].data_ptr(), self.ring_v[l].data_ptr(), self.ring_u[l].data_ptr()
+            if self.norm_w is not None:
+                y.q_norm, y.k_norm = self.norm_w[l][0].data_ptr(), self.norm_w[l][1].data_ptr()
+            y.ts_k, y.alpha_k, y.ts_v, y.alpha_v = tb["ts_k"], tb["alpha_k"], tb["ts_v"], tb["alpha_v"]
+        self._ring_u_at = np.array([r.data_ptr() for r in self.ring_u], np.uint64)
+        a = self._args = _lib.EngineStep()
+        a.h_q, a.h_k, a.h_v, a.h_out = self.h_q.data_ptr(), self.h_k.data_ptr(), self.h_v.data_ptr(), self.h_out.data_ptr()
+        a.d_q, a.d_k, a.d_v, a.d_out = self._q.data_ptr(), self._k.data_ptr(), self._v.data_ptr(), self._out.data_ptr()
+        base = self.d_control.data_ptr()
+        a.d_control = base
+        for f in ("items", "dyn", "slots", "pos", "segs"):
+            setattr(a, "d_" + f, base + self._at[f])
+        a.descs, a.tables, a.workspace, a.workspace_bytes = (self.d_descs.data_ptr(), self.d_tables.data_ptr(), self.workspace.data_ptr(),
+                                                             self.ws_bytes)
+        a.n_layers, a.n_seq, a.ring_cap, a.rotary_dim, a.codebook_in_smem = self.L, self.B, RING, ROTARY_DIM, int(codebook_in_smem)
+        a.rope_theta, a.rms_eps = self.rope_theta, self.rms_eps
+        # A copy of a few tens of KB takes as long as one of 256 KB (3-4 us): layers are copied in groups of about that
+        # much, at most half of them at once so that copies and kernels still overlap.
+        a.layers_per_chunk = int(min(max(COPY_BYTES // (self.B * (H_Q * 2 * D + 2 * KV) * 2), 1), max(self.L // 2, 1)))
         self._step = 0
         self.n_items = 0
         self.events_fired = 0
-        self._plan_and_upload(self._ctl[0])
+        self._plan(self._ctl[0])
+        if cuda:
+            nb = self._control_bytes(0)
+            self.d_control[:nb].copy_(self._ctl[0]["block"][:nb])
+            check("launch_khq_update_descs", self.lib.launch_khq_update_descs(self.d_descs.data_ptr(), self.d_dyn.data_ptr(), self.B,
+                                                                              self.L, current_stream()))
+
+    def __del__(self):
+        native = getattr(self, "_native", None)
+        if native:
+            self.lib.khq_b200_engine_destroy(native)
+            self._native = None
 
     # ---------------------------------------------------------------------------------- sizes
     @property
@@ -183,36 +239,35 @@ class BatchEngine:
     def h2d_bytes_per_step(self) -> int:
         """Projections of one step for every layer and sequence plus the step's control block
         (work items, per-sequence state, ring slots, positions)."""
-        return self.L * self.B * (H_Q * 2 * D + 2 * KV) * 2 + self.n_items * WORK_ITEM.itemsize + self.B * (SEQ_DYN.itemsize + 8)
+        return self.L * self.B * (H_Q * 2 * D + 2 * KV) * 2 + self._control_bytes(0)
 
     @property
     def d2h_bytes_per_step(self) -> int:
         return self.L * self.B * H_Q * D * 2
 
     # ---------------------------------------------------------------------------------- planning
-    def _plan_and_upload(self, ctl) -> None:
+    def _control_bytes(self, n_events: int) -> int:
+        """Bytes of the control block that a step with n_events compression events copies."""
+        if n_events:
+            return self._at["segs"] + self.L * self.B * COMPRESS_SEG.itemsize
+        return self._at["items"] + self.n_items * WORK_ITEM.itemsize
+
+    def _plan(self, ctl) -> None:
         """Cut the current compressed prefixes and windows into work items (host planner of the
-        library), and send items + per-sequence state to the device; one launch then rewrites the
-        step-dependent fields of all L x B descriptors."""
-        c = np.ascontiguousarray(self.boundary, np.int32)
-        w = np.ascontiguousarray(self.write_pos - self.boundary, np.int32)
-        first = np.zeros(self.B, np.int32)
-        cnt = np.zeros(self.B, np.int32)
-        items = ctl["items"].numpy().view(WORK_ITEM)
-        n = self.lib.khq_b200_plan_decode(c.ctypes.data, w.ctypes.data, self.B, self.tokens_per_item_arg, items.ctypes.data,
-                                          self.max_items, first.ctypes.data, cnt.ctypes.data)
+        library) and write items and per-sequence state into the host control block; one launch then
+        rewrites the step-dependent fields of all L x B descriptors from it."""
+        dyn = ctl["dyn"]
+        c = self.boundary.astype(np.int32)
+        w = (self.write_pos - self.boundary).astype(np.int32)
+        first = np.empty(self.B, np.int32)
+        cnt = np.empty(self.B, np.int32)
+        n = self.lib.khq_b200_plan_decode(c.ctypes.data, w.ctypes.data, self.B, self.tokens_per_item_arg,
+                                          ctl["block"].data_ptr() + self._at["items"], self.max_items, first.ctypes.data, cnt.ctypes.data)
         if n < 0 or n > self.max_items:
             raise _lib.KhqLaunchError("khq_b200_plan_decode", n)
         self.n_items = int(n)
-        dyn = ctl["dyn"].numpy().view(SEQ_DYN)
-        dyn["c_len"], dyn["start_pos"], dyn["win_start"], dyn["win_len"] = c, 0, (self.boundary % RING).astype(np.int32), w
+        dyn["c_len"], dyn["start_pos"], dyn["win_start"], dyn["win_len"] = c, 0, c % RING, w
         dyn["first_slot"], dyn["n_slots"] = first, cnt
-        nb = self.n_items * WORK_ITEM.itemsize
-        self.d_items[:nb].copy_(ctl["items"][:nb], non_blocking=True)
-        self.d_dyn.copy_(ctl["dyn"], non_blocking=True)
-        if self.device.type == "cuda":
-            check("launch_khq_update_descs", self.lib.launch_khq_update_descs(self.d_descs.data_ptr(), self.d_dyn.data_ptr(), self.B,
-                                                                              self.L, current_stream()))
 
     # ---------------------------------------------------------------------------------- loading
     def compress_into(self, layer: int, seq: int, k_unroped: torch.Tensor, v: torch.Tensor, tok0: int = 0) -> None:
@@ -285,88 +340,29 @@ class BatchEngine:
         in pinned host memory.  Every sequence advances by one token: append, compression event if
         due, attention.  The gated outputs land in ``h_out`` (returned; valid once the stream has
         synchronised)."""
-        ctl = self._ctl[self._step & 1]
-        if ctl["done"] is not None:
-            ctl["done"].synchronize()  # the copies that last read this parity's host block have finished
-        self._step += 1
+        parity = self._step & 1
+        ctl, a, lib = self._ctl[parity], self._args, self.lib
+        lib.khq_b200_engine_wait_control(self._native, parity)  # the copy that last read this parity's host block has finished
         # ---- host state machine (src/khq/runtime.mojo:486-553, for every sequence) -----------------
-        slots = (self.write_pos % RING).astype(np.int32)
-        pos = self.write_pos.astype(np.int32)
-        self.write_pos += 1
-        window = self.write_pos - self.boundary
-        due = np.nonzero((window >= WATERMARK) & (self.boundary + CHUNK <= self.cap))[0]
-        if (window[np.setdiff1d(np.arange(self.B), due)] > RING).any():
+        window = self.write_pos + 1 - self.boundary
+        due = (window >= WATERMARK) & (self.boundary + CHUNK <= self.cap)
+        n_ev = int(np.count_nonzero(due))
+        if window.max() > RING and (window[~due] > RING).any():
             raise RuntimeError("a sequence's compressed capacity is exhausted (raise grow_tokens)")
-        ctl["slots"].numpy()[:] = slots
-        ctl["pos"].numpy()[:] = pos
-        n_ev = len(due)
+        self._step += 1
+        ctl["slots"][:] = self.write_pos % RING
+        ctl["pos"][:] = self.write_pos
+        self.write_pos += 1
         if n_ev:
-            segs = ctl["segs"].numpy().view(COMPRESS_SEG).reshape(self.L, self.B)
-            for l in range(self.L):
-                base_u, base_v = self.ring_u[l].data_ptr(), self.ring_v[l].data_ptr()
-                s0 = (self.boundary[due] % RING)
-                off = (due * RING + s0) * KV * 2
-                segs["x"][l, :n_ev] = base_u + off
-                segs["row0"][l, :n_ev] = self.row_off[due] + self.boundary[due] * H_KV
-            # the V launch reads ring_v at the same offsets: keep the byte distance per layer
-            self._v_minus_u = [self.ring_v[l].data_ptr() - self.ring_u[l].data_ptr() for l in range(self.L)]
-        self.boundary[due] += CHUNK
-        self.events_fired += n_ev
-        st = current_stream()
-        self.d_slots.copy_(ctl["slots"], non_blocking=True)
-        self.d_pos.copy_(ctl["pos"], non_blocking=True)
-        if n_ev:
-            self.d_segs.copy_(ctl["segs"], non_blocking=True)
-        self._plan_and_upload(ctl)
-        if ctl["done"] is not None:
-            ctl["done"].record()
-        seg_bytes = self.B * COMPRESS_SEG.itemsize
-        # Host <-> device copies run on their own stream, one layer ahead of (inputs) and behind (outputs) the
-        # kernels: layer l's inputs land while layer l - 1 computes.  Events order the two streams.
-        main, cs = torch.cuda.current_stream(), self._copy_stream
-        cs.wait_stream(main)  # everything queued so far (the previous step's reads of q_gate / d_k / d_v, the control block)
-        in_ready, k_free = [None] * self.L, [None] * self.L
-
-        def stage_inputs(l):
-            with torch.cuda.stream(cs):
-                if l >= 2:
-                    cs.wait_event(k_free[l - 2])  # the pre-step of layer l - 2 has consumed this parity of d_k / d_v
-                self.q_gate[l].copy_(self.h_q[l], non_blocking=True)
-                self.d_k[l & 1].copy_(self.h_k[l], non_blocking=True)
-                self.d_v[l & 1].copy_(self.h_v[l], non_blocking=True)
-                in_ready[l] = cs.record_event()
-
-        stage_inputs(0)
-        for l in range(self.L):
-            if l + 1 < self.L:
-                stage_inputs(l + 1)
-            main.wait_event(in_ready[l])
-            d_k, d_v = self.d_k[l & 1], self.d_v[l & 1]
-            qw, kw = self.norm_w[l] if self.norm_w is not None else (None, None)
-            rc = self.lib.launch_khq_prestep_batched_fp16(
-                self.q_gate[l].data_ptr(), d_k.data_ptr(), d_v.data_ptr(), _lib.ptr(qw), _lib.ptr(kw),
-                self.ring_k[l].data_ptr(), self.ring_v[l].data_ptr(), self.ring_u[l].data_ptr(), RING * KV, self.d_slots.data_ptr(),
-                self.d_pos.data_ptr(), self.B, H_Q, H_KV, D, ROTARY_DIM, self.rope_theta, self.rms_eps, 1 if qw is not None else 0, st)
-            check("launch_khq_prestep_batched_fp16", rc)
-            k_free[l] = main.record_event()
-            if n_ev:
-                tb, P = self.tables[l], self.pay[l]
-                seg_ptr = self.d_segs.data_ptr() + l * seg_bytes
-                rc = self.lib.launch_khq_compress_batched_fp16(
-                    seg_ptr, n_ev, CHUNK * H_KV, tb["d_k"].data_ptr(), tb["k_rotor"].data_ptr(), tb["cents_k"].data_ptr(),
-                    tb["cents_k"].data_ptr(), P["k_mask"].data_ptr(), P["k_norms"].data_ptr(), P["k_r_norms"].data_ptr(),
-                    P["k_payload"].data_ptr(), P["v_shared_meta"].data_ptr(), D, float(tb["ts_k"]), float(tb["alpha_k"]), 0, 0, st)
-                check("launch_khq_compress_batched_fp16", rc)
-                rc = self.lib.launch_khq_compress_batched_fp16(
-                    seg_ptr, n_ev, CHUNK * H_KV, tb["d_v"].data_ptr(), tb["v_rotor"].data_ptr(), tb["cents_v"].data_ptr(),
-                    tb["vq"].data_ptr(), P["k_mask"].data_ptr(), P["v_norms"].data_ptr(), P["v_r_norms"].data_ptr(),
-                    P["v_payload"].data_ptr(), P["v_shared_meta"].data_ptr(), D, float(tb["ts_v"]), float(tb["alpha_v"]), 1,
-                    self._v_minus_u[l], st)
-                check("launch_khq_compress_batched_fp16", rc)
-            self.attention_resident(l, scale)
-            done_l = main.record_event()
-            with torch.cuda.stream(cs):
-                cs.wait_event(done_l)
-                self.h_out[l].copy_(self.out[l], non_blocking=True)
-        main.wait_stream(cs)  # the caller synchronises the current stream before it reads h_out
+            idx = np.nonzero(due)[0]
+            at = self.boundary[idx]
+            # the V launch reads ring_v at the same offsets from its own base
+            ctl["segs"]["x"][:, :n_ev] = self._ring_u_at[:, None] + ((idx * RING + at % RING) * KV * 2).astype(np.uint64)
+            ctl["segs"]["row0"][:, :n_ev] = self.row_off[idx] + at * H_KV
+            self.boundary[idx] += CHUNK
+            self.events_fired += n_ev
+        self._plan(ctl)
+        a.h_control, a.control_bytes, a.parity = ctl["block"].data_ptr(), self._control_bytes(n_ev), parity
+        a.n_items, a.n_events, a.scale = self.n_items, n_ev, float(scale)
+        check("launch_khq_engine_step", lib.launch_khq_engine_step(self._native, self._layers, ctypes.addressof(a), current_stream()))
         return self.h_out

@@ -40,6 +40,11 @@ SIGNATURES = {
     "launch_khq_attn_static_fp16": (
         c_int, [_P] * 17 + [c_int] * 5 + [c_float, c_float, c_float, c_float, c_int, c_int, _P]),
     "launch_khq_merge_slots_gate_fp16": (c_int, [_P, c_int, _P, _P, c_int, c_int, _P]),
+    "launch_khq_layer_step": (c_int, [_P] * 6 + [c_int] * 4 + [c_float, _P]),
+    "khq_b200_engine_create": (c_int, [POINTER(c_void_p)]),
+    "khq_b200_engine_destroy": (c_int, [_P]),
+    "khq_b200_engine_wait_control": (c_int, [_P, c_int]),
+    "launch_khq_engine_step": (c_int, [_P] * 4),
     "launch_khq_decode_step_fp16": (c_int, [_P] * 25 + [c_int] * 5 + [c_float] * 4 + [_P]),
     "launch_khq_gqa_prefill_fp16": (
         c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_float, c_longlong, c_longlong, c_longlong, _P]),
@@ -116,10 +121,56 @@ def ptr(t) -> int:
     return t.data_ptr()
 
 
-def current_stream() -> int:
+class LayerCtx(ctypes.Structure):
+    """``khq_layer_ctx`` of include/khq_b200.h."""
+
+    _fields_ = [(n, c_void_p) for n in (
+        "d_k", "cents_k", "rotor_k", "d_v", "cents_v", "rotor_v", "vq", "ring_k", "ring_v", "ring_u", "k_mask", "k_payload", "k_norms",
+        "k_r_norms", "v_payload", "v_norms", "v_r_norms", "v_shared_meta", "attn_c", "attn_partial")] + [
+        (n, c_float) for n in ("ts_k", "alpha_k", "ts_v", "alpha_v", "rope_base")] + [("ring_cap", c_int)]
+
+
+class EngineLayer(ctypes.Structure):
+    """``khq_engine_layer`` of include/khq_b200.h."""
+
+    _fields_ = [(n, c_void_p) for n in (
+        "d_k", "cents_k", "rotor_k", "d_v", "cents_v", "rotor_v", "vq", "ring_k", "ring_v", "ring_u", "k_mask", "k_payload", "k_norms",
+        "k_r_norms", "v_payload", "v_norms", "v_r_norms", "v_shared_meta", "q_norm", "k_norm")] + [
+        (n, c_float) for n in ("ts_k", "alpha_k", "ts_v", "alpha_v")]
+
+
+class EngineStep(ctypes.Structure):
+    """``khq_engine_step`` of include/khq_b200.h."""
+
+    _fields_ = [(n, c_void_p) for n in (
+        "h_q", "h_k", "h_v", "h_control", "h_out", "d_q", "d_k", "d_v", "d_out", "d_control", "d_items", "d_dyn", "d_slots", "d_pos", "d_segs",
+        "descs", "tables", "workspace")] + [("control_bytes", c_size_t), ("workspace_bytes", c_size_t)] + [
+        (n, c_int) for n in ("n_layers", "n_seq", "n_items", "n_events", "layers_per_chunk", "parity", "ring_cap", "rotary_dim",
+                             "codebook_in_smem")] + [(n, c_float) for n in ("scale", "rope_theta", "rms_eps")]
+
+
+def _stream_getter():
+    """torch's current stream of the current device as an address, without building the Stream object (1 us a call)."""
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    try:
+        raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        return lambda: raw(device())
+    except AttributeError:
+        return lambda: torch.cuda.current_stream().cuda_stream
+
+
+_current_stream = None
+
+
+def current_stream() -> int:
+    global _current_stream
+    if _current_stream is None:
+        import torch
+
+        torch.cuda.init()
+        _current_stream = _stream_getter()
+    return _current_stream()
 
 
 class KhqLaunchError(RuntimeError):

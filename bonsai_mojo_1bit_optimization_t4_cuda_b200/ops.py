@@ -7,6 +7,8 @@ and re-reads ``BONSAI_DISABLE_CUDA_FFI`` on every call), launches go to torch's 
 """
 from __future__ import annotations
 
+import ctypes
+
 from . import lib as _lib
 from .lib import check, current_stream, ptr
 
@@ -92,6 +94,24 @@ class CudaOps:
             ptr(attn_c), ptr(attn_partial), ptr(out), int(c_len), int(win_start), int(win_len), int(ring_cap),
             int(num_splits), float(scale), float(alpha_k), float(alpha_v), float(rope_base), current_stream())
         check("launch_khq_decode_step_fp16", rc)
+
+    # -- launch_khq_layer_step: one layer's step from a context that keeps its addresses -------------
+    def layer_ctx(self, L, ring_cap, rope_base):
+        """The context of a ``runtime.KhqLayer``; it holds raw addresses of the tensors in ``L.t``."""
+        c = _lib.LayerCtx()
+        for field, name in (("d_k", "dk"), ("cents_k", "ck"), ("rotor_k", "rk"), ("d_v", "dv"), ("cents_v", "cv"), ("rotor_v", "rv"),
+                            ("vq", "vq"), ("ring_k", "ring_k"), ("ring_v", "ring_v"), ("ring_u", "ring_u"), ("k_mask", "kmask"),
+                            ("k_payload", "kpay"), ("k_norms", "knorm"), ("k_r_norms", "krn"), ("v_payload", "vpay"), ("v_norms", "vnorm"),
+                            ("v_r_norms", "vrn"), ("v_shared_meta", "vsm"), ("attn_c", "ac"), ("attn_partial", "ap")):
+            setattr(c, field, L.t[name].data_ptr())
+        c.ts_k, c.alpha_k, c.ts_v, c.alpha_v, c.rope_base, c.ring_cap = L.ts_k, L.alpha_k, L.ts_v, L.alpha_v, rope_base, ring_cap
+        return c, ctypes.addressof(c)
+
+    def layer_step(self, ctx, q_gate, k_roped, v_new, k_unroped, out, c_len, win_len, compress, num_splits, scale):
+        rc = self.lib.launch_khq_layer_step(ctx[1], ptr(q_gate), ptr(k_roped), ptr(v_new), ptr(k_unroped), ptr(out), c_len, win_len,
+                                            compress, num_splits, scale, current_stream())
+        if rc != 0:
+            check("launch_khq_layer_step", rc)
 
     # -- peer-memory exchange of context-parallel partials ----------------------------------------
     def publish_partials(self, src, n_records, peer_slots, peer_flags, world, rank, first_slot, parity_offset_records, epoch):

@@ -44,6 +44,16 @@ def _env_int(name: str, fallback: int) -> int:
         return fallback
 
 
+class _Tensors(dict):
+    """A layer's tensors by name.  ``ctx`` is the native context that keeps their addresses; replacing a tensor drops it."""
+
+    ctx = None
+
+    def __setitem__(self, name, value):
+        self.ctx = None
+        dict.__setitem__(self, name, value)
+
+
 class KhqLayer:
     """KHQ state of one attention layer (all tensors live on the runtime's device)."""
 
@@ -58,7 +68,7 @@ class KhqLayer:
         self.write_pos = 0
         # tables: h_dk h_ck h_rk h_dv h_cv h_rv h_vq; rings: h_ring_k h_ring_v h_ring_u;
         # payload: h_kmask h_kpay h_knorm h_krn h_vpay h_vnorm h_vrn h_vsm; scratch: h_ac h_aw h_ap
-        self.t: Dict[str, torch.Tensor] = {}
+        self.t: Dict[str, torch.Tensor] = _Tensors()
 
     def __getattr__(self, name):  # h_xxx accessors, as the reference's fields are named
         t = self.__dict__.get("t")
@@ -196,9 +206,39 @@ class KhqRuntime:
         kv = L.H_kv * L.D
         slot = L.write_pos % KHQ_RING
         T = L.t
-        self.ops.prestep(q_gate_dev, k_dev, v_dev, q_norm_w, k_norm_w, T["ring_k"][slot * kv:(slot + 1) * kv],
-                         T["ring_v"][slot * kv:(slot + 1) * kv], T["ring_u"][slot * kv:(slot + 1) * kv], L.H_q, L.H_kv,
-                         L.D, rotary_dim, pos, rope_theta, rms_eps, has_norms)
+        if hasattr(self.ops, "layer_ctx"):  # addresses will do: no views of the rings
+            off = slot * kv * 2
+            rings = [T[r].data_ptr() + off for r in ("ring_k", "ring_v", "ring_u")]
+        else:
+            rings = [T[r][slot * kv:(slot + 1) * kv] for r in ("ring_k", "ring_v", "ring_u")]
+        self.ops.prestep(q_gate_dev, k_dev, v_dev, q_norm_w, k_norm_w, *rings, L.H_q, L.H_kv, L.D, rotary_dim, pos, rope_theta,
+                         rms_eps, has_norms)
+        return True
+
+    # ------------------------------------------------------------------ native step
+    def _native_step(self, layer_idx: int, L, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, scale: float) -> bool:
+        """The step of one layer (append, event if due, both regions, merge, gate) as one native call.
+        False: a step that only the call-by-call sequence covers (another backend, profiling, debug
+        output, a window beyond the ring)."""
+        window = L.write_pos + 1 - L.boundary
+        if self.prof or self.debug or window > KHQ_RING or window <= 0:
+            return False
+        T = L.t
+        ctx = T.ctx
+        if ctx is None:
+            make = getattr(self.ops, "layer_ctx", None)
+            if make is None or (L.H_q, L.H_kv, L.D) != (24, 4, 256):
+                return False
+            ctx = T.ctx = make(L, KHQ_RING, ROPE_BASE)
+        c_len = L.boundary
+        event = window >= KHQ_WATERMARK and c_len + KHQ_CHUNK <= L.cap
+        c_after = c_len + KHQ_CHUNK if event else c_len
+        self.ops.layer_step(ctx, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, c_len, window, event,
+                            self._khq_split_count(c_after), scale)
+        L.write_pos += 1
+        if event:
+            L.boundary = c_after
+            self.events.append(KhqCompressEvent(layer_idx, c_after // KHQ_CHUNK, c_after, L.write_pos, L.write_pos - c_after))
         return True
 
     # ------------------------------------------------------------------ khq_step
@@ -224,6 +264,9 @@ class KhqRuntime:
         L = self.layers[layer_idx]
         if not L.ready:
             return False
+        if self._native_step(layer_idx, L, q_gate_dev, None if rings_written else k_roped_dev, None if rings_written else v_dev, None,
+                             out_dev, scale):
+            return True
         ops, T = self.ops, L.t
         H_q, H_kv, d = L.H_q, L.H_kv, L.D
         kv = H_kv * d
@@ -299,11 +342,10 @@ class KhqRuntime:
 
     # ------------------------------------------------------------------ fused step (addition)
     def khq_step_fused(self, layer_idx: int, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, scale: float) -> bool:
-        """``khq_capture_unroped`` + ``khq_step`` of one token through ``launch_khq_decode_step_fp16``:
-        the three ring appends, both attention regions, the merge and the gate in two or three
-        launches (and one host call) instead of seven.  A step on which a compression event is due
-        takes the classic sequence (the event sits between the append and the attention), and so does
-        a step whose window would exceed the ring (compressed capacity exhausted: the reference keeps
+        """``khq_capture_unroped`` + ``khq_step`` of one token through ``launch_khq_layer_step``:
+        the compression event if it is due, the three ring appends, both attention regions, the merge and
+        the gate in one host call and two launches (four with an event) instead of seven.  A step whose window
+        would exceed the ring takes the classic sequence (compressed capacity exhausted: the reference keeps
         stepping with window > 256, ``README.md:259``, and so does ``khq_step``).  The state afterwards
         is the one the classic calls leave."""
         if not self.active or not self.ready or layer_idx < 0 or layer_idx >= KHQ_MAX_LAYERS:
@@ -311,23 +353,10 @@ class KhqRuntime:
         L = self.layers[layer_idx]
         if not L.ready:
             return False
-        window_after = L.write_pos + 1 - L.boundary
-        event_due = window_after >= KHQ_WATERMARK and L.boundary + KHQ_CHUNK <= L.cap
-        if event_due or window_after > KHQ_RING or not hasattr(self.ops, "decode_step"):
-            self.khq_capture_unroped(layer_idx, k_unroped_dev)
-            return self.khq_step(layer_idx, q_gate_dev, k_roped_dev, v_dev, out_dev, scale)
-        T = L.t
-        c_len = L.boundary
-        kv = dict(k_payload=T["kpay"], v_payload=T["vpay"], v_shared_meta=T["vsm"], k_mask=T["kmask"], k_norms=T["knorm"],
-                  k_r_norms=T["krn"], v_norms=T["vnorm"], v_r_norms=T["vrn"])
-        tab = dict(cents_k=T["ck"], cents_v=T["cv"], vq=T["vq"], rotor_k=T["rk"], rotor_v=T["rv"], d_k=T["dk"], d_v=T["dv"])
-        t0 = self._tick()
-        self.ops.decode_step(q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, T["ring_k"], T["ring_v"], T["ring_u"], kv, tab,
-                             T["ac"], T["ap"], out_dev, c_len, c_len % KHQ_RING, window_after, KHQ_RING,
-                             self._khq_split_count(c_len) if c_len > 0 else 1, scale, L.alpha_k, L.alpha_v, ROPE_BASE)
-        self._tock(KHQ_P_ATTN, t0)
-        L.write_pos += 1
-        return True
+        if self._native_step(layer_idx, L, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, scale):
+            return True
+        self.khq_capture_unroped(layer_idx, k_unroped_dev)
+        return self.khq_step(layer_idx, q_gate_dev, k_roped_dev, v_dev, out_dev, scale)
 
     # ------------------------------------------------------------------ prompt prefill (addition)
     def khq_prefill(self, layer_idx: int, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, scale: float) -> bool:

@@ -268,6 +268,58 @@ int launch_khq_decode_step_fp16(
     const void* d_vec_v, void* attn_c, void* attn_partial, void* out, int c_len, int win_start, int win_len, int ring_cap,
     int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, khq_stream_t stream);
 
+/* The same step from a context that keeps a layer's addresses (a host that calls once per layer and token fills it once).
+ * In order: when `compress` is nonzero the event of the reference's khq_step (src/khq/runtime.mojo:486-553): the 128 oldest
+ * raw tokens, ring slots c_len % ring_cap .., are compressed to rows c_len * 4 .. and the regions move on by 128; then the
+ * attention over both regions, the ring appends, merge and gate.  c_len / win_len: compressed and raw tokens before the
+ * event, the step's own token included.  k_roped == v_new == NULL: the token's rows are in the rings already (a pre-step
+ * appended them).  attn_partial holds (24, num_splits, 258) fp32.  Returns as launch_khq_decode_step_fp16. */
+typedef struct khq_layer_ctx {
+    const void *d_k, *cents_k, *rotor_k, *d_v, *cents_v, *rotor_v, *vq;
+    void *ring_k, *ring_v, *ring_u;
+    void *k_mask, *k_payload, *k_norms, *k_r_norms, *v_payload, *v_norms, *v_r_norms, *v_shared_meta;
+    void *attn_c, *attn_partial;
+    float ts_k, alpha_k, ts_v, alpha_v, rope_base;
+    int32_t ring_cap;
+} khq_layer_ctx;
+int launch_khq_layer_step(const khq_layer_ctx* ctx, const void* q_gate, const void* k_roped, const void* v_new,
+                          const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits, float scale,
+                          khq_stream_t stream);
+
+/* ---- A batch engine's token step in one call (no counterpart in the reference) -----------------
+ * What a host would issue per layer for n_seq sequences: inputs from pinned host memory (copies on the engine's own
+ * streams, layers_per_chunk layers at a time, one chunk ahead of the kernels), launch_khq_prestep_batched_fp16, the
+ * compression events that are due (segs: n_layers x n_seq khq_compress_seg, the first n_events of each layer), the batched
+ * attention, and the outputs back to pinned host memory; before the layers one copy of the step's control block and one
+ * launch_khq_update_descs.  d_items, d_dyn, d_slots, d_pos and d_segs lie inside the device control block.  h_q (n_layers,
+ * n_seq, 24 * 512), h_k / h_v (n_layers, n_seq, 4 * 256), h_out (n_layers, n_seq, 24 * 256) fp16 and the device buffers of
+ * the same shapes.  The caller's stream waits for the output copies.  Calls on one engine come from one thread at a time;
+ * parity (0 or 1) says which of two control blocks is used, khq_b200_engine_wait_control returns when it may be rewritten. */
+typedef struct khq_engine khq_engine;
+typedef struct khq_engine_layer {
+    const void *d_k, *cents_k, *rotor_k, *d_v, *cents_v, *rotor_v, *vq;
+    void *ring_k, *ring_v, *ring_u;
+    void *k_mask, *k_payload, *k_norms, *k_r_norms, *v_payload, *v_norms, *v_r_norms, *v_shared_meta;
+    const void *q_norm, *k_norm; /* fp32 (256) or NULL */
+    float ts_k, alpha_k, ts_v, alpha_v;
+} khq_engine_layer;
+typedef struct khq_engine_step {
+    const void *h_q, *h_k, *h_v, *h_control;
+    void *h_out;
+    void *d_q, *d_k, *d_v, *d_out, *d_control;
+    const void *d_items, *d_dyn, *d_slots, *d_pos, *d_segs;
+    void *descs;
+    const void *tables;
+    void *workspace;
+    size_t control_bytes, workspace_bytes;
+    int32_t n_layers, n_seq, n_items, n_events, layers_per_chunk, parity, ring_cap, rotary_dim, codebook_in_smem;
+    float scale, rope_theta, rms_eps;
+} khq_engine_step;
+int khq_b200_engine_create(khq_engine** out);
+int khq_b200_engine_destroy(khq_engine* engine);
+int khq_b200_engine_wait_control(khq_engine* engine, int parity);
+int launch_khq_engine_step(khq_engine* engine, const khq_engine_layer* layers, const khq_engine_step* step, khq_stream_t stream);
+
 /* ---- Prefill: causal GQA attention + sigmoid gate over a whole prompt --------------------
  * The math of the reference's fp16-KV attention kernel (gqa_attention_sm75_gpu,
  * src/kernels/elementwise_sm75.mojo:1091-1231), which the reference launches once per prompt
