@@ -83,9 +83,22 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ float h2f(__half h) { return __half2float(h); }
 __device__ __forceinline__ float hbits2f(uint16_t b) { return __half2float(__ushort_as_half(b)); }
 
-// In-lane part of the unnormalised natural-order FWHT-256 when a lane holds the 8 consecutive
-// elements 8*lane..8*lane+7 (stages 1, 2, 4), followed by the cross-lane stages 8..128.
-// Each butterfly computes a+b and a-b exactly as a sequential implementation does.
+// Packed pairs of fp32 (one instruction; each half is rounded like the scalar operation).
+__device__ __forceinline__ void f32x2_addsub(float& s0, float& s1, float& d0, float& d1, float a0, float a1, float b0, float b1) {
+    asm("{.reg .b64 a, b, s, d; mov.b64 a, {%4, %5}; mov.b64 b, {%6, %7}; add.rn.f32x2 s, a, b; sub.rn.f32x2 d, a, b;"
+        " mov.b64 {%0, %1}, s; mov.b64 {%2, %3}, d;}"
+        : "=f"(s0), "=f"(s1), "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+__device__ __forceinline__ void f32x2_fma(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0, float c1) {
+    asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7};"
+        " fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d;}"
+        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+
+// Unnormalised natural-order FWHT-256 when a lane holds the 8 consecutive elements 8*lane..8*lane+7: in-lane stages 1, 2, 4,
+// then the cross-lane stages 8..128.  Each butterfly computes a+b and a-b exactly as a sequential implementation does: across
+// lanes the lower one adds and the upper one subtracts its own value from the other's, which is one multiply-add by +1 or -1
+// (exact products), two elements per instruction (12 instead of 32 instructions a stage).
 __device__ __forceinline__ void fwht256_lane8(float (&v)[8], int lane) {
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
@@ -94,26 +107,16 @@ __device__ __forceinline__ void fwht256_lane8(float (&v)[8], int lane) {
         v[j + 1] = a - b;
     }
 #pragma unroll
-    for (int b4 = 0; b4 < 8; b4 += 4)
+    for (int b4 = 0; b4 < 8; b4 += 4) f32x2_addsub(v[b4], v[b4 + 1], v[b4 + 2], v[b4 + 3], v[b4], v[b4 + 1], v[b4 + 2], v[b4 + 3]);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            float a = v[b4 + k], b = v[b4 + k + 2];
-            v[b4 + k] = a + b;
-            v[b4 + k + 2] = a - b;
-        }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float a = v[j], b = v[j + 4];
-        v[j] = a + b;
-        v[j + 4] = a - b;
-    }
+    for (int j = 0; j < 4; j += 2) f32x2_addsub(v[j], v[j + 1], v[j + 4], v[j + 5], v[j], v[j + 1], v[j + 4], v[j + 5]);
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) {
-        const bool lower = (lane & m) == 0;
+        const float sign = (lane & m) == 0 ? 1.0f : -1.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float other = __shfl_xor_sync(0xFFFFFFFFu, v[j], m);
-            v[j] = lower ? (v[j] + other) : (other - v[j]);
+        for (int j = 0; j < 8; j += 2) {
+            const float o0 = __shfl_xor_sync(0xFFFFFFFFu, v[j], m), o1 = __shfl_xor_sync(0xFFFFFFFFu, v[j + 1], m);
+            f32x2_fma(v[j], v[j + 1], v[j], v[j + 1], sign, sign, o0, o1);
         }
     }
 }

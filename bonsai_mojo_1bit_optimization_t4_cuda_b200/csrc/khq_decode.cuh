@@ -251,8 +251,10 @@ struct HeadRec {
 // record i, so the n weights cost one exchange, and the accumulators of four records are in flight together.  The records
 // may lie in this CTA's or a peer CTA's shared memory or in global memory.  PAD: the accumulators skip four floats after
 // every 32 (see m2_compressed_range).
-template <bool PAD, class At>
-__device__ __forceinline__ HeadAcc merge_head(int n, int lane, At at) {
+// N: the number of records if it is known at compile time (all their loads are then in flight together), else 0.
+template <bool PAD, int N = 0, class At>
+__device__ __forceinline__ HeadAcc merge_head(int n_run, int lane, At at) {
+    const int n = N > 0 ? N : n_run;
     HeadAcc r;
     float m = NEG_BIG, l = 0.0f;
     if (lane < n) {
@@ -269,7 +271,7 @@ __device__ __forceinline__ HeadAcc merge_head(int n, int lane, At at) {
     for (int k = 16; k > 0; k >>= 1) r.l += __shfl_xor_sync(0xFFFFFFFFu, r.l, k);
 #pragma unroll
     for (int j = 0; j < 8; ++j) r.a[j] = 0.0f;
-#pragma unroll 4
+#pragma unroll(N > 0 ? N : 4)
     for (int i = 0; i < n; ++i) {
         const float wi = __shfl_sync(0xFFFFFFFFu, w, i);
         const float* p = at(i).acc + lane * 8 + (PAD ? 4 * (lane >> 2) : 0);
@@ -309,7 +311,7 @@ struct VInverse {
             }
         fwht256_lane8(z, lane);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = z[j] * ((1.0f / 16.0f) / (__half2float(hd[j]) + 1e-8f));
+        for (int j = 0; j < 8; ++j) a[j] = z[j] * __fdividef(1.0f / 16.0f, __half2float(hd[j]) + 1e-8f);
     }
 };
 __device__ __forceinline__ void store_head(const HeadAcc& h, float* o, int lane) {

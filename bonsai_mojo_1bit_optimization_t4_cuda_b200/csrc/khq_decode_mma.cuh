@@ -164,40 +164,53 @@ __device__ __forceinline__ void m2_group_sync(int sub) {
     asm volatile("bar.sync %0, %1;" ::"r"(2 + HKV + sub), "n"(M2_GTHREADS) : "memory");
 }
 
-// Stage `ntok` tokens starting at `tok0` for group `sub` (tid: thread inside the group; same contract as stage_tile of the
-// first generation).
+// Stage `ntok` tokens starting at `tok0` for group `sub` (tid: thread inside the group).  Bulk path: one lane of each of the
+// group's four warps issues two of the eight copies and posts their bytes (the stage's mbarrier counts four arrivals); issued
+// by one lane they held up its warp, and at the next group barrier the other three.  Plain path (odd tail or unaligned
+// arrays): all threads copy with 32-bit loads.
 __device__ __forceinline__ void m2_stage_tile(const CompressedKV& P, unsigned char* stage, uint64_t* bar, int tok0,
                                               int ntok, int tid, int sub) {
     const size_t r0 = (size_t)tok0 * HKV;
     const int rows = ntok * HKV;
-    const unsigned char* src[8] = {reinterpret_cast<const unsigned char*>(P.k_mask) + r0 * 64,
-                                   P.k_payload + r0 * K_PAY,
-                                   P.v_payload + r0 * V_PAY,
-                                   reinterpret_cast<const unsigned char*>(P.k_norms) + r0 * 2,
-                                   reinterpret_cast<const unsigned char*>(P.k_r_norms) + r0 * 2,
-                                   reinterpret_cast<const unsigned char*>(P.v_norms) + r0 * 2,
-                                   reinterpret_cast<const unsigned char*>(P.v_r_norms) + r0 * 2,
-                                   P.v_shared_meta + r0 * 4};
-    const int dst[8] = {M2_OFF_MASK, M2_OFF_KPAY, M2_OFF_VPAY, M2_OFF_KN, M2_OFF_KRN, M2_OFF_VN, M2_OFF_VRN, M2_OFF_VSM};
-    const int bpr[8] = {64, K_PAY, V_PAY, 2, 2, 2, 2, 4};
-    const bool bulk = P.bulk_ok && ((tok0 & 1) == 0) && ((ntok & 1) == 0);
-    if (bulk) {
-        if (tid == 0) {
-            mbar_arrive_expect_tx(bar, (uint32_t)(rows * 220));
-#pragma unroll
-            for (int a = 0; a < 8; ++a) bulk_g2s(stage + dst[a], src[a], (uint32_t)(rows * bpr[a]), bar);
+    const unsigned char* const k_mask = reinterpret_cast<const unsigned char*>(P.k_mask) + r0 * 64;
+    const unsigned char* const k_pay = P.k_payload + r0 * K_PAY;
+    const unsigned char* const v_pay = P.v_payload + r0 * V_PAY;
+    const unsigned char* const kn = reinterpret_cast<const unsigned char*>(P.k_norms) + r0 * 2;
+    const unsigned char* const krn = reinterpret_cast<const unsigned char*>(P.k_r_norms) + r0 * 2;
+    const unsigned char* const vn = reinterpret_cast<const unsigned char*>(P.v_norms) + r0 * 2;
+    const unsigned char* const vrn = reinterpret_cast<const unsigned char*>(P.v_r_norms) + r0 * 2;
+    const unsigned char* const vsm = P.v_shared_meta + r0 * 4;
+    if (P.bulk_ok && ((tok0 & 1) == 0) && ((ntok & 1) == 0)) {
+        if ((tid & 31) == 0) {
+            const auto two = [&](int dst_a, const unsigned char* a, int bytes_a, int dst_b, const unsigned char* b, int bytes_b) {
+                mbar_arrive_expect_tx(bar, (uint32_t)(rows * (bytes_a + bytes_b)));
+                bulk_g2s(stage + dst_a, a, (uint32_t)(rows * bytes_a), bar);
+                bulk_g2s(stage + dst_b, b, (uint32_t)(rows * bytes_b), bar);
+            };
+            switch (tid >> 5) {
+                case 0: two(M2_OFF_MASK, k_mask, 64, M2_OFF_KN, kn, 2); break;
+                case 1: two(M2_OFF_KPAY, k_pay, K_PAY, M2_OFF_KRN, krn, 2); break;
+                case 2: two(M2_OFF_VPAY, v_pay, V_PAY, M2_OFF_VN, vn, 2); break;
+                default: two(M2_OFF_VSM, vsm, 4, M2_OFF_VRN, vrn, 2); break;
+            }
         }
     } else {
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const int words = rows * bpr[a] / 4;
-            const unsigned int* s = reinterpret_cast<const unsigned int*>(src[a]);
-            unsigned int* d = reinterpret_cast<unsigned int*>(stage + dst[a]);
-            for (int i = tid; i < words; i += M2_GTHREADS) d[i] = s[i];
-        }
+        const auto copy = [&](int dst, const unsigned char* src, int bytes) {
+            const unsigned int* s = reinterpret_cast<const unsigned int*>(src);
+            unsigned int* d = reinterpret_cast<unsigned int*>(stage + dst);
+            for (int i = tid; i < rows * bytes / 4; i += M2_GTHREADS) d[i] = s[i];
+        };
+        copy(M2_OFF_MASK, k_mask, 64);
+        copy(M2_OFF_KPAY, k_pay, K_PAY);
+        copy(M2_OFF_VPAY, v_pay, V_PAY);
+        copy(M2_OFF_KN, kn, 2);
+        copy(M2_OFF_KRN, krn, 2);
+        copy(M2_OFF_VN, vn, 2);
+        copy(M2_OFF_VRN, vrn, 2);
+        copy(M2_OFF_VSM, vsm, 4);
         fence_proxy_async();
         m2_group_sync(sub);
-        if (tid == 0) mbar_arrive(bar);
+        if ((tid & 31) == 0) mbar_arrive(bar);
     }
 }
 
@@ -412,7 +425,7 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
         const uint4 r0 = rp[0], r1 = rp[1], r2 = rp[2], r3 = rp[3];
         const __half* hd = reinterpret_cast<const __half*>(&dr);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dv[j] = (lane >= 8) ? (1.0f / 256.0f) / (__half2float(hd[j]) + 1e-8f) : 0.0f;
+        for (int j = 0; j < 8; ++j) dv[j] = (lane >= 8) ? __fdividef(1.0f / 256.0f, __half2float(hd[j]) + 1e-8f) : 0.0f;
         __half hr[32];
         *reinterpret_cast<uint4*>(&hr[0]) = r0;
         *reinterpret_cast<uint4*>(&hr[8]) = r1;
@@ -991,7 +1004,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
     uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
     if (tid == 0) {
-        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], HKV);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
@@ -1036,7 +1049,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
         // two query heads per warp: merge of the three groups' records, inverse V transform, store
 #pragma unroll 1
         for (int h = warp; h < HQ; h += M2_THREADS / 32) {
-            HeadAcc a = merge_head<true>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
+            HeadAcc a = merge_head<true, M2_WPK>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
             if (w.kind == 0) inv.apply(a.a, lane);
             store_head(a, partials + ((size_t)w.slot * HQ + h) * PART, lane);
         }
@@ -1075,7 +1088,7 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     const int my_hi = min(my_lo + chunk, s_hi);
     uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
     if (tid == 0) {
-        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], HKV);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
@@ -1096,9 +1109,13 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     const float* rec = reinterpret_cast<const float*>(smem + M2_SM_STAGES);
 #pragma unroll 1
     for (int h = crank + csize * warp; h < HQ; h += csize * (M2_THREADS / 32)) {
-        HeadAcc a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
-            return m2_head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * M2_REC_FLOATS, h % NREP);
-        });
+        HeadAcc a;
+        if (csize == 1)
+            a = merge_head<true, M2_WPK>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
+        else
+            a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
+                return m2_head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * M2_REC_FLOATS, h % NREP);
+            });
         inv.apply(a.a, lane);
         const int total_id = h * L_q + l_idx;
         store_head(a, (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART : out_attn + (size_t)total_id * PART, lane);
