@@ -47,6 +47,20 @@ def plan(c_len: np.ndarray, win_len: np.ndarray, tokens_per_item: int = 0):
     return items[:n_items], first, cnt
 
 
+def prepare_tables(tables: np.ndarray, rope_base: float, device) -> torch.Tensor:
+    """The decode kernels' images of a TABLES_DESC array (``launch_khq_prepare_tables``), (n, bytes) on
+    the device; complete on return, so any stream may use them."""
+    lib = _lib.load()
+    images = torch.empty(len(tables), int(lib.khq_b200_prepared_bytes()), dtype=torch.uint8, device=device)
+    tables = np.ascontiguousarray(tables)
+    with torch.cuda.device(images.device):
+        for i in range(len(tables)):
+            check("launch_khq_prepare_tables", lib.launch_khq_prepare_tables(
+                tables[i:].ctypes.data, float(rope_base), images[i].data_ptr(), current_stream()))
+        torch.cuda.current_stream().synchronize()
+    return images
+
+
 class BatchedDecode:
     """Device-resident descriptors + workspace for a fixed set of problems.
 

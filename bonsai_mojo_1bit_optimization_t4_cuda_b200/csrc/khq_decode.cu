@@ -624,7 +624,7 @@ khq_decode_batched_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesD
             P.cents_k = t.cents_k; P.cents_v = t.cents_v; P.vq = t.vq; P.k_rotor = t.k_rotor;
             P.v_rotor = t.v_rotor; P.d_k = t.d_k; P.d_v = t.d_v;
             P.alpha_k = t.alpha_k; P.alpha_v = t.alpha_v; P.rope_base = rope_base;
-            P.start_pos = d.start_pos; P.c_len = d.c_len; P.bulk_ok = 1;
+            P.start_pos = d.start_pos; P.c_len = d.c_len; P.bulk_ok = 1; P.image = nullptr;
             unpack_pos(d.pos_pack, P);
             if (d.table_id != cur_table) {
                 setup_tables(smem, P, tid);
@@ -748,6 +748,7 @@ khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k
     const int new_s = new_k != nullptr ? win_len - 1 : -1;  // -1: the token's rows are in the rings already
     float* rec = reinterpret_cast<float*>(smem);
     if (n_c == 0) pdl_wait();
+    pdl_trigger();  // what may start now reads nothing but constants before its own wait
     if (crank == 0) {  // ring appends: 3 rows of H_kv*D halfs = 3 x 128 sixteen-byte chunks
         const int slot = (win_start + win_len - 1) % ring_cap;
         const size_t row = (size_t)slot * HKV * D;
@@ -771,7 +772,6 @@ khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k
     for (int k = warp; crank + csize * k < HQ; k += DEC_WARPS) store_head(window_head(cluster, rec, csize, crank + csize * k, lane), own + k * PART, lane);
     cluster.sync();  // peers must stay resident until their records have been read
     pdl_wait();
-    pdl_trigger();
     // a thread finishes two dims of one head: all its loads of the split records are in flight together
     for (int e = tid; e < (HQ - crank + csize - 1) / csize * (D / 2); e += DEC_THREADS) {
         const int k = e / (D / 2), h = crank + csize * k, d = 2 * (e % (D / 2));
@@ -1017,7 +1017,7 @@ static int attn_launch_impl(const void* q, const void* k_payload, const void* v_
                             void* out_partial, int num_queries, int num_heads, int L_q, int c_len,
                             int n_rep, float scale, float alpha_k, float alpha_v,
                             float rope_base, int start_pos, int num_splits, int pos_chunk, int pos_stride,
-                            bool reduce, cudaStream_t stream) {
+                            bool reduce, const void* image, cudaStream_t stream) {
     if (num_queries <= 0 || c_len <= 0) return -100;
     if (num_splits < 1) num_splits = 1;
     if (num_splits > 1 && out_partial == nullptr) return -101;
@@ -1059,6 +1059,7 @@ static int attn_launch_impl(const void* q, const void* k_payload, const void* v_
     P.bulk_ok = bulk_ok ? 1 : 0;
     P.pos_chunk = pos_chunk;
     P.pos_stride = pos_stride;
+    P.image = static_cast<const unsigned char*>(image);
 
     for (int l = 0; l < L_q; ++l) {
         const int s_limit = (L_q > 1) ? (c_len < l + 1 ? c_len : l + 1) : c_len;
@@ -1109,7 +1110,7 @@ extern "C" int launch_khq_attn_fp16(const void* q, const void* k_payload, const 
     return attn_launch_impl(q, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
                             centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, out_attn, out_partial,
                             num_queries, num_heads, L_q, c_len, n_rep, scale, alpha_k, alpha_v, rope_base, start_pos,
-                            num_splits, 0, 0, true, stream);
+                            num_splits, 0, 0, true, nullptr, stream);
 }
 
 // launch_khq_attn_fp16 over a slice that holds every G-th `pos_chunk`-token chunk of a longer context
@@ -1130,7 +1131,7 @@ extern "C" int launch_khq_attn_strided_fp16(const void* q, const void* k_payload
     return attn_launch_impl(q, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
                             centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, out_attn, out_partial,
                             num_queries, num_heads, L_q, c_len, n_rep, scale, alpha_k, alpha_v, rope_base, start_pos,
-                            num_splits, pos_chunk, pos_stride, true, stream);
+                            num_splits, pos_chunk, pos_stride, true, nullptr, stream);
 }
 
 // CTAs of the one cluster that runs a raw window: a warp takes four tokens at a time.
@@ -1174,7 +1175,7 @@ static int decode_step_impl(
     const void* k_norms, const void* k_r_norms, const void* v_norms, const void* v_r_norms, const void* centroids_k,
     const void* centroids_v, const void* vq_centroids, const void* k_rotor, const void* v_rotor, const void* d_vec_k,
     const void* d_vec_v, void* attn_c, void* attn_partial, void* out, int c_len, int win_start, int win_len, int ring_cap,
-    int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, cudaStream_t stream) {
+    int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, const void* image, cudaStream_t stream) {
     const void* al[] = {q_gate, k_roped, v_new, k_unroped, ring_k, ring_v, ring_u, out};
     for (const void* p : al)
         if (p && !aligned(p, 16)) return -104;
@@ -1184,7 +1185,7 @@ static int decode_step_impl(
     if (c_len > 0) {
         const int rc = attn_launch_impl(q_gate, k_payload, v_payload, v_shared_meta, k_mask, k_norms, k_r_norms, v_norms, v_r_norms,
                                         centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor, d_vec_k, d_vec_v, attn_c, attn_partial,
-                                        HQ, HQ, 1, c_len, NREP, scale, alpha_k, alpha_v, rope_base, 0, num_splits, 0, 0, !tail_merges, stream);
+                                        HQ, HQ, 1, c_len, NREP, scale, alpha_k, alpha_v, rope_base, 0, num_splits, 0, 0, !tail_merges, image, stream);
         if (rc != 0) return rc;
     }
     cudaError_t err = ensure_smem_attrs();
@@ -1210,7 +1211,7 @@ extern "C" int launch_khq_decode_step_fp16(
     return decode_step_impl(q_gate, k_roped, v_new, k_unroped, ring_k, ring_v, ring_u, k_payload, v_payload, v_shared_meta, k_mask,
                             k_norms, k_r_norms, v_norms, v_r_norms, centroids_k, centroids_v, vq_centroids, k_rotor, v_rotor,
                             d_vec_k, d_vec_v, attn_c, attn_partial, out, c_len, win_start, win_len, ring_cap, num_splits, scale,
-                            alpha_k, alpha_v, rope_base, stream);
+                            alpha_k, alpha_v, rope_base, nullptr, stream);
 }
 
 // One decode step of one layer from a context that keeps the layer's addresses: compression event if due, compressed-region
@@ -1220,10 +1221,11 @@ struct khq_layer_ctx {
     void *ring_k, *ring_v, *ring_u;
     void *k_mask, *k_payload, *k_norms, *k_r_norms, *v_payload, *v_norms, *v_r_norms, *v_shared_meta;
     void *attn_c, *attn_partial;
+    const void* prepared;
     float ts_k, alpha_k, ts_v, alpha_v, rope_base;
     int ring_cap;
 };
-static_assert(sizeof(khq_layer_ctx) == 20 * 8 + 24, "ABI");
+static_assert(sizeof(khq_layer_ctx) == 21 * 8 + 24, "ABI");
 extern "C" int launch_khq_compress_fp16(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
                                         void*, int, int, float, float, int, cudaStream_t);
 
@@ -1231,7 +1233,7 @@ extern "C" int launch_khq_layer_step(const khq_layer_ctx* L, const void* q_gate,
                                      const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits,
                                      float scale, cudaStream_t stream) {
     constexpr int CHUNK = 128;
-    if (!L || !q_gate || !out || win_len <= 0 || c_len < 0 || !L->attn_c || (k_roped == nullptr) != (v_new == nullptr)) return -100;
+    if (!L || !q_gate || !out || win_len <= 0 || c_len < 0 || !L->attn_c || !aligned(L->prepared, 128) || (k_roped == nullptr) != (v_new == nullptr)) return -100;
     if (L->ring_cap <= 0 || win_len > L->ring_cap) return -103;
     if (compress) {  // the 128 oldest raw tokens, contiguous in the ring; the step's own token is not among them
         const int s0 = c_len % L->ring_cap, row = c_len * HKV;
@@ -1255,7 +1257,7 @@ extern "C" int launch_khq_layer_step(const khq_layer_ctx* L, const void* q_gate,
     return decode_step_impl(q_gate, k_roped, v_new, k_unroped, L->ring_k, L->ring_v, L->ring_u, L->k_payload, L->v_payload,
                             L->v_shared_meta, L->k_mask, L->k_norms, L->k_r_norms, L->v_norms, L->v_r_norms, L->cents_k, L->cents_v,
                             L->vq, L->rotor_k, L->rotor_v, L->d_k, L->d_v, L->attn_c, L->attn_partial, out, c_len,
-                            c_len % L->ring_cap, win_len, L->ring_cap, num_splits, scale, L->alpha_k, L->alpha_v, L->rope_base, stream);
+                            c_len % L->ring_cap, win_len, L->ring_cap, num_splits, scale, L->alpha_k, L->alpha_v, L->rope_base, L->prepared, stream);
 }
 
 extern "C" int launch_khq_gather_q_fp16(const void* q_gate, void* q_out, int H_q, int d,
@@ -1465,7 +1467,7 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
 
 static int decode_batched_impl(const void* descs, const void* tables, const void* items, int n_desc, int n_items,
                                void* workspace, size_t workspace_bytes, int n_slots_total, float scale, float rope_base,
-                               int ring_cap, int codebook_in_smem, float* out_partials, cudaStream_t stream) {
+                               int ring_cap, int codebook_in_smem, float* out_partials, const void* images, cudaStream_t stream) {
     if (n_desc <= 0 || n_items <= 0 || !descs || !tables || !items || !workspace) return -100;
     if (workspace_bytes < khq_b200_decode_workspace_bytes(n_slots_total) || ring_cap <= 0) return -105;
     if (!aligned(workspace, 256)) return -104;
@@ -1490,7 +1492,8 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
     else if (mma)
         err = launch_pdl(khq_decode_batched_mma_kernel, (unsigned)grid, 0, (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS,
                          static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
-                         static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap);
+                         static_cast<const KhqWorkItem*>(items), n_items, counter, partials, scale, rope_base, ring_cap,
+                         static_cast<const unsigned char* const*>(images));
     else if (vqs)
         khq_decode_batched_kernel<true><<<grid, DEC_THREADS, SM_TOTAL_VQ, stream>>>(
             static_cast<const KhqSeqDesc*>(descs), static_cast<const KhqTablesDesc*>(tables),
@@ -1520,7 +1523,39 @@ extern "C" int launch_khq_decode_batched_fp16(const void* descs, const void* tab
                                               float rope_base, int ring_cap, int codebook_in_smem,
                                               cudaStream_t stream) {
     return decode_batched_impl(descs, tables, items, n_desc, n_items, workspace, workspace_bytes, n_slots_total, scale,
-                               rope_base, ring_cap, codebook_in_smem, nullptr, stream);
+                               rope_base, ring_cap, codebook_in_smem, nullptr, nullptr, stream);
+}
+
+// The same launch with the tables' images (device array of pointers by table_id, see launch_khq_prepare_tables).
+extern "C" int launch_khq_decode_batched_prepared_fp16(const void* descs, const void* tables, const void* images, const void* items,
+                                                       int n_desc, int n_items, void* workspace, size_t workspace_bytes,
+                                                       int n_slots_total, float scale, float rope_base, int ring_cap,
+                                                       int codebook_in_smem, cudaStream_t stream) {
+    return decode_batched_impl(descs, tables, items, n_desc, n_items, workspace, workspace_bytes, n_slots_total, scale,
+                               rope_base, ring_cap, codebook_in_smem, nullptr, images, stream);
+}
+
+extern "C" size_t khq_b200_prepared_bytes(void) { return (M2_IMG_BYTES + 127) / 128 * 128; }
+
+// A layer's tables in the form the decode kernels use them, once per layer: see include/khq_b200.h.
+extern "C" int launch_khq_prepare_tables(const void* tables_desc, float rope_base, void* image, cudaStream_t stream) {
+    if (!tables_desc || !image) return -100;
+    const KhqTablesDesc& t = *static_cast<const KhqTablesDesc*>(tables_desc);  // host memory
+    const void* ptrs[] = {t.cents_k, t.cents_v, t.vq, t.k_rotor, t.v_rotor, t.d_k, t.d_v};
+    for (const void* p : ptrs)
+        if (!p || !aligned(p, 16)) return p ? -104 : -100;
+    if (!aligned(image, 128)) return -104;
+    CompressedKV P = {};
+    P.cents_k = t.cents_k;
+    P.cents_v = t.cents_v;
+    P.vq = t.vq;
+    P.k_rotor = t.k_rotor;
+    P.d_k = t.d_k;
+    P.alpha_k = t.alpha_k;
+    P.alpha_v = t.alpha_v;
+    P.rope_base = rope_base;
+    khq_prepare_tables_kernel<<<1, M2_THREADS, 0, stream>>>(P, static_cast<unsigned char*>(image));
+    return static_cast<int>(cudaGetLastError());
 }
 
 // The same launch, ending in one unnormalised record (acc[256], max, sum) per (problem, head) in
@@ -1532,7 +1567,7 @@ extern "C" int launch_khq_decode_batched_partial_fp16(const void* descs, const v
                                                       int codebook_in_smem, void* out_partials, cudaStream_t stream) {
     if (!out_partials || !aligned(out_partials, 8)) return out_partials ? -104 : -100;
     return decode_batched_impl(descs, tables, items, n_desc, n_items, workspace, workspace_bytes, n_slots_total, scale,
-                               rope_base, ring_cap, codebook_in_smem, static_cast<float*>(out_partials), stream);
+                               rope_base, ring_cap, codebook_in_smem, static_cast<float*>(out_partials), nullptr, stream);
 }
 
 // Per-sequence state of a batch engine that changes every step and is the same for all layers

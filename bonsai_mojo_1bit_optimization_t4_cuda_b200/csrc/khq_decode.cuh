@@ -104,6 +104,7 @@ struct CompressedKV {  // device pointers of one sequence-layer's compressed reg
     int start_pos;  // absolute position of compressed token 0
     int c_len;      // valid tokens in the arrays
     int bulk_ok;    // all eight arrays 16-byte aligned
+    const unsigned char* image;  // the layer's tables laid out by launch_khq_prepare_tables, or null
     // Positions of a slice that holds every G-th chunk of a longer context (chunk-cyclic context
     // partition): token s of the arrays sits at start_pos + (s / pos_chunk) * pos_stride + s % pos_chunk.
     // pos_chunk == 0: consecutive positions.

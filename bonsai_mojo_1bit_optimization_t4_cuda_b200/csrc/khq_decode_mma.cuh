@@ -58,12 +58,20 @@ constexpr int M2_VQ_ROW = (NP / 2) * 12 + 4;                         // 388 byte
 constexpr int M2_SM_VQ = M2_SM_STAGES + M2_STAGES_BYTES;
 constexpr int M2_SM_ROPE = M2_SM_VQ + 256 * M2_VQ_ROW;               // per group two buffers of M2_BT tokens x 64 floats
 constexpr int M2_SM_RSC = M2_SM_ROPE + 2 * M2_TT * 64 * 4;           // 16 rows x 2 float4 per warp: scalars of a block's rows
-constexpr int M2_SM_FREQ = M2_SM_RSC + M2_THREADS / 32 * 16 * 32;
-constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats
-constexpr int M2_SM_BARS = M2_SM_DINV + 256;
-constexpr int M2_SM_C3 = M2_SM_BARS + 64;              // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
-constexpr int M2_SM_RSTEP = M2_SM_C3 + NP * 8;                          // 32 x float2: cos / sin of one tile's worth (32 positions) of each rotary pair
-constexpr int M2_SM_QR = M2_SM_RSTEP + 32 * 8;                             // raw rotary query fragments: 4 kv-heads x 4 k-steps x 32 lanes x 8 B
+// small tables of a layer, in the order of the prepared image
+constexpr int M2_SM_FREQ = M2_SM_RSC + M2_THREADS / 32 * 16 * 32;      // 32 floats: RoPE frequencies
+constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats: 1 / (256 d) of the rotary dims
+constexpr int M2_SM_C3 = M2_SM_DINV + 256;                           // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
+constexpr int M2_SM_RSTEP = M2_SM_C3 + NP * 8;                       // 32 x float2: cos / sin of M2_TT positions of each rotary pair
+constexpr int M2_SMALL_BYTES = 128 + 256 + NP * 8 + 32 * 8;
+constexpr int M2_SM_BARS = M2_SM_FREQ + M2_SMALL_BYTES;              // M2_WPK * M2_NSTAGE stages, then the image's small tables and codebook
+constexpr int M2_BAR_SMALL = M2_WPK * M2_NSTAGE, M2_BAR_VQ = M2_BAR_SMALL + 1, M2_NBARS = M2_BAR_VQ + 1;
+constexpr int M2_SM_TMSLOT = M2_SM_BARS + M2_NBARS * 8;
+constexpr int M2_SM_QR = (M2_SM_TMSLOT + 4 + 15) / 16 * 16;   // raw rotary query fragments: 4 kv-heads x 4 k-steps x 32 lanes x 8 B
+// Prepared image of a layer's tables (launch_khq_prepare_tables): the codebook's shared-memory rows, the small tables, the
+// rotor fragments (two uint4 per k-step and lane).
+constexpr int M2_IMG_VQ = 0, M2_IMG_SMALL = 256 * M2_VQ_ROW, M2_IMG_ROT = M2_IMG_SMALL + M2_SMALL_BYTES, M2_IMG_BYTES = M2_IMG_ROT + 16 * 32 * 32;
+static_assert(M2_IMG_SMALL % 16 == 0 && M2_IMG_ROT % 16 == 0 && M2_SM_FREQ % 16 == 0 && M2_SM_QR % 16 == 0 && M2_SM_BARS % 8 == 0, "alignment");
 constexpr int M2_SM_TOTAL = M2_SM_QR + HKV * 4 * 32 * 8;
 // Tensor memory as a second register file.  The B fragments of the K side are per-lane constants: the query
 // side (ternary part q1 and residual part q2, fp16 hi and lo, eight registers per k-step) for a whole work
@@ -259,26 +267,23 @@ __device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __ha
     }
 }
 
-// Per-layer constants in shared memory: RoPE frequencies, dinv of the 64 rotary dims, dim-3 centroids and the V codebook.
-// Must be followed by __syncthreads().
-__device__ __forceinline__ void m2_setup_tables(unsigned char* smem, const CompressedKV& P, int tid) {
-    float* freq_s = reinterpret_cast<float*>(smem + M2_SM_FREQ);
-    float* dinv_s = reinterpret_cast<float*>(smem + M2_SM_DINV);
-    if (tid < 32) freq_s[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
+// A layer's small tables to `dst` (the order of M2_SM_FREQ ..), one entry per thread.
+__device__ __forceinline__ void m2_small_tables(unsigned char* dst, const CompressedKV& P, int tid) {
+    constexpr int O_DINV = M2_SM_DINV - M2_SM_FREQ, O_C3 = M2_SM_C3 - M2_SM_FREQ, O_RSTEP = M2_SM_RSTEP - M2_SM_FREQ;
+    if (tid < 32) reinterpret_cast<float*>(dst)[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
     if (tid >= 128 && tid < 128 + NP) {
         const float c0 = __half2float(P.cents_v[0 * D + 4 * (tid - 128) + 3]), c1 = __half2float(P.cents_v[1 * D + 4 * (tid - 128) + 3]);
-        reinterpret_cast<float2*>(smem + M2_SM_C3)[tid - 128] = make_float2(c0 * P.alpha_v, (c1 - c0) * P.alpha_v);
+        reinterpret_cast<float2*>(dst + O_C3)[tid - 128] = make_float2(c0 * P.alpha_v, (c1 - c0) * P.alpha_v);
     }
-    if (tid < 64) dinv_s[tid] = (1.0f / 256.0f) / (__half2float(P.d_k[tid]) + 1e-8f);
+    if (tid < 64) reinterpret_cast<float*>(dst + O_DINV)[tid] = (1.0f / 256.0f) / (__half2float(P.d_k[tid]) + 1e-8f);
     if (tid >= 192 && tid < 224) {
         const int m = tid - 192;
         // half turns of M2_TT positions: reduced in double, so the fp32 sine and cosine get an exact small argument
         double th = (double)M2_TT * (double)powf(P.rope_base, -2.0f * (float)m / 64.0f) * 0.3183098861837907;
         th -= 2.0 * rint(0.5 * th);
-        float* o = reinterpret_cast<float*>(smem + M2_SM_RSTEP) + 4 * (m >> 1) + (m & 1);
+        float* o = reinterpret_cast<float*>(dst + O_RSTEP) + 4 * (m >> 1) + (m & 1);
         sincospif((float)th, &o[2], &o[0]);
     }
-    m2_stage_codebook(smem + M2_SM_VQ, P.vq, tid);
 }
 
 // Query-side operands of one (sequence, layer, kv-head): this warp's B fragments.
@@ -342,53 +347,111 @@ __device__ __forceinline__ void m2_tm_free(uint32_t tmem, int warp) {
     }
 }
 
-// The layer's rotor fragments (with and without the centroid factor) into the tensor memory of every lane quadrant; the
-// M2_WPK warps of a quadrant share the k-steps.  The readers pass a CTA barrier and a tcgen05 fence before their first load.
-// The three low index bits of the 64-point Hadamard transform are folded in: u[8j + n] is produced by step s = 2j + (n >> 2)
-// as rotor output c = n & 3, and H64 = H8 (bits 0..2, inside a tile) x H8 (bits 3..5, across tiles), so column n' of the
+// A lane's rotor fragments of k-step s: rotor x centroid (ternary operand) and rotor (residual operand), fp16 and what fp16
+// lost.  The three low index bits of the 64-point Hadamard transform are folded in: u[8j + n] is produced by step s = 2j + (n
+// >> 2) as rotor output c = n & 3, and H64 = H8 (bits 0..2, inside a tile) x H8 (bits 3..5, across tiles), so column n' of the
 // folded operand is sum_n H8[n][n'] * (column n of the plain one).
-__device__ __forceinline__ void m2_rotor_to_tmem(const CompressedKV& P, uint32_t tmem, int warp, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + M2_TM_ROT;
-#pragma unroll 2
-    for (int s = warp >> 2; s < 16; s += M2_WPK) {
-        const int patch = 16 * t + s;
-        __half hr[16], hc[4];
-        *reinterpret_cast<uint4*>(&hr[0]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16);
-        *reinterpret_cast<uint4*>(&hr[8]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16 + 8);
-        *reinterpret_cast<uint2*>(&hc[0]) = *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s);
-        const int kk[4] = {0, 2, 1, 3};  // dims 64t+4s + {0, 2, 1, 3}
-        float rc[4], r1[4];
+__device__ __forceinline__ void m2_rotor_fragment(const CompressedKV& P, int s, int lane, uint32_t (&r)[8]) {
+    const int g = lane >> 2, t = lane & 3, patch = 16 * t + s;
+    __half hr[16], hc[4];
+    *reinterpret_cast<uint4*>(&hr[0]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16);
+    *reinterpret_cast<uint4*>(&hr[8]) = *reinterpret_cast<const uint4*>(P.k_rotor + patch * 16 + 8);
+    *reinterpret_cast<uint2*>(&hc[0]) = *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s);
+    const int kk[4] = {0, 2, 1, 3};  // dims 64t+4s + {0, 2, 1, 3}
+    float rc[4], r1[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc = 0.0f;
+    for (int i = 0; i < 4; ++i) {
+        float acc = 0.0f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int n = 4 * (s & 1) + c;
-                const float v = __half2float(hr[c * 4 + kk[i]]);
-                acc += (__popc(n & g) & 1) ? -v : v;
-            }
-            r1[i] = acc;
-            rc[i] = acc * __half2float(hc[kk[i]]);
+        for (int c = 0; c < 4; ++c) {
+            const int n = 4 * (s & 1) + c;
+            const float v = __half2float(hr[c * 4 + kk[i]]);
+            acc += (__popc(n & g) & 1) ? -v : v;
         }
-        uint2 b1, b1l, b2, b2l;  // rotor * centroid (ternary operand), rotor (residual operand): fp16 and what fp16 lost
-        m2_pack_hilo(rc[0], rc[1], b1.x, b1l.x);
-        m2_pack_hilo(rc[2], rc[3], b1.y, b1l.y);
-        m2_pack_hilo(r1[0], r1[1], b2.x, b2l.x);
-        m2_pack_hilo(r1[2], r1[3], b2.y, b2l.y);
-        m2_tm_st8(dst + 8 * s, b1.x, b1.y, b2.x, b2.y, b1l.x, b1l.y, b2l.x, b2l.y);
+        r1[i] = acc;
+        rc[i] = acc * __half2float(hc[kk[i]]);
+    }
+    m2_pack_hilo(rc[0], rc[1], r[0], r[4]);
+    m2_pack_hilo(rc[2], rc[3], r[1], r[5]);
+    m2_pack_hilo(r1[0], r1[1], r[2], r[6]);
+    m2_pack_hilo(r1[2], r1[3], r[3], r[7]);
+}
+
+// The layer's tables into shared memory and its rotor fragments into the tensor memory of every lane quadrant (the M2_WPK
+// warps of a quadrant share the k-steps).  Without an image they are computed (a CTA barrier and a tcgen05 fence have to
+// follow); with one they are fetched: bulk copies that m2_wait_tables waits for (`loads` counts them), a third of the
+// instructions that a CTA with one or two blocks per warp executes.
+__device__ __forceinline__ void m2_load_tables(unsigned char* smem, const CompressedKV& P, uint32_t tmem, int tid, int warp, int lane) {
+    const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + M2_TM_ROT;
+    if (P.image != nullptr) {
+        uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
+        if (tid == 0) {
+            mbar_arrive_expect_tx(&bars[M2_BAR_SMALL], M2_SMALL_BYTES);
+            bulk_g2s(smem + M2_SM_FREQ, P.image + M2_IMG_SMALL, M2_SMALL_BYTES, &bars[M2_BAR_SMALL]);
+            mbar_arrive_expect_tx(&bars[M2_BAR_VQ], 256 * M2_VQ_ROW);
+            bulk_g2s(smem + M2_SM_VQ, P.image + M2_IMG_VQ, 256 * M2_VQ_ROW, &bars[M2_BAR_VQ]);
+        }
+        const uint4* src = reinterpret_cast<const uint4*>(P.image + M2_IMG_ROT) + 2 * lane;
+#pragma unroll 2
+        for (int s = warp >> 2; s < 16; s += M2_WPK) {
+            const uint4 a = __ldg(src + 64 * s), b = __ldg(src + 64 * s + 1);
+            m2_tm_st8(dst + 8 * s, a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w);
+        }
+    } else {
+        m2_small_tables(smem + M2_SM_FREQ, P, tid);
+        m2_stage_codebook(smem + M2_SM_VQ, P.vq, tid);
+#pragma unroll 2
+        for (int s = warp >> 2; s < 16; s += M2_WPK) {
+            uint32_t r[8];
+            m2_rotor_fragment(P, s, lane, r);
+            m2_tm_st8(dst + 8 * s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
+        }
     }
     m2_tm_st_wait();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+
+// grid = 1: the image of one layer.
+__global__ void __launch_bounds__(M2_THREADS) khq_prepare_tables_kernel(CompressedKV P, unsigned char* __restrict__ image) {
+    m2_small_tables(image + M2_IMG_SMALL, P, threadIdx.x);
+    m2_stage_codebook(image + M2_IMG_VQ, P.vq, threadIdx.x);
+    for (int c = threadIdx.x; c < 256; c += M2_THREADS) *reinterpret_cast<uint32_t*>(image + M2_IMG_VQ + c * M2_VQ_ROW + M2_VQ_ROW - 4) = 0u;
+    for (int e = threadIdx.x; e < 16 * 32; e += M2_THREADS) {
+        uint32_t r[8];
+        m2_rotor_fragment(P, e >> 5, e & 31, r);
+        uint4* o = reinterpret_cast<uint4*>(image + M2_IMG_ROT) + 2 * e;
+        o[0] = make_uint4(r[0], r[1], r[2], r[3]);
+        o[1] = make_uint4(r[4], r[5], r[6], r[7]);
+    }
 }
 
 // Where the query build's scratch keeps the four dims 4c .. 4c + 3 of head h: swizzled so that the eight lanes (two heads, four
 // 64-dim quarters) of a float4 phase read distinct banks.
 __device__ __forceinline__ int m2_q_chunk(int h, int c) { return 4 * (c ^ ((c >> 4) & 3) ^ ((h & 1) << 2)); }
 
-// q: (H_q, ..) with `q_head_stride` halfs between heads.  scratch: this warp's NREP*D floats.
+// What the query build takes from the layer's tables: 1 / d and the rotor of the lane's 8 dims, and the centroids of the dims
+// 64 t + 4 s + {0..3} of the warp's k-steps.
+constexpr int M2_SPW = (16 + M2_WPK - 1) / M2_WPK;  // k-steps per warp (the last warps may have one less)
+struct M2QueryTables {
+    uint4 rotor[4], d;
+    uint2 cents[M2_SPW];
+    __device__ __forceinline__ void load(const CompressedKV& P, int sub, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        const uint4* rp = reinterpret_cast<const uint4*>(P.k_rotor + lane * 32);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rotor[i] = rp[i];
+        d = *reinterpret_cast<const uint4*>(P.d_k + lane * 8);
+#pragma unroll
+        for (int i = 0; i < M2_SPW; ++i) {
+            const int s = sub + M2_WPK * i;
+            cents[i] = (g < NREP && s < 16) ? *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s) : make_uint2(0u, 0u);
+        }
+    }
+};
+
+// q: (H_q, ..) with `q_head_stride` halfs between heads.  scratch: this kv-head's NREP*D floats.
 __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restrict__ q, size_t q_head_stride,
-                                               const CompressedKV& P, int kvh, int sub, int lane, float* scratch,
+                                               const M2QueryTables& qt, int kvh, int sub, int lane, float* scratch,
                                                uint2* qr_s /* this kv-head's [4][32] raw rotary query fragments */) {
     // The M2_WPK warps of a kv-head share the work (it runs once per work item, on the critical path): warp `sub`
     // transforms query heads sub, sub + M2_WPK, ... into the kv-head's scratch, the warps meet at a named barrier,
@@ -402,15 +465,7 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
 #pragma unroll
     for (int i = 0; i < HPW; ++i)
         qraw[i] = *reinterpret_cast<const uint4*>(q + (size_t)(kvh * NREP + sub + M2_WPK * i) * q_head_stride + lane * 8);
-    // for the fragments built after the transforms: the centroids of dims 64 t + 4 s + {0..3} and the raw rotary query dims
-    constexpr int SPW = (16 + M2_WPK - 1) / M2_WPK;  // k-steps per warp (the last warps may have one less)
-    uint2 cck[SPW];
-    uint32_t qrw[4][2];
-#pragma unroll
-    for (int i = 0; i < SPW; ++i) {
-        const int s = sub + M2_WPK * i;
-        cck[i] = (g < NREP && s < 16) ? *reinterpret_cast<const uint2*>(P.cents_k + 2 * D + 64 * t + 4 * s) : make_uint2(0u, 0u);
-    }
+    uint32_t qrw[4][2];  // the raw rotary query dims
     if (sub == 0) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
@@ -420,17 +475,10 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
         }
     }
     {
-        const uint4 dr = *reinterpret_cast<const uint4*>(P.d_k + lane * 8);
-        const uint4* rp = reinterpret_cast<const uint4*>(P.k_rotor + lane * 32);
-        const uint4 r0 = rp[0], r1 = rp[1], r2 = rp[2], r3 = rp[3];
-        const __half* hd = reinterpret_cast<const __half*>(&dr);
+        const __half* hd = reinterpret_cast<const __half*>(&qt.d);
+        const __half* hr = reinterpret_cast<const __half*>(qt.rotor);
 #pragma unroll
         for (int j = 0; j < 8; ++j) dv[j] = (lane >= 8) ? __fdividef(1.0f / 256.0f, __half2float(hd[j]) + 1e-8f) : 0.0f;
-        __half hr[32];
-        *reinterpret_cast<uint4*>(&hr[0]) = r0;
-        *reinterpret_cast<uint4*>(&hr[8]) = r1;
-        *reinterpret_cast<uint4*>(&hr[16]) = r2;
-        *reinterpret_cast<uint4*>(&hr[24]) = r3;
 #pragma unroll
         for (int p = 0; p < 2; ++p)
 #pragma unroll
@@ -459,14 +507,14 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
     }
     asm volatile("bar.sync %0, %1;" ::"r"(2 + kvh), "n"(32 * M2_WPK) : "memory");  // the kv-head's warps: all six heads are in the scratch
 #pragma unroll
-    for (int i = 0; i < SPW; ++i) {
+    for (int i = 0; i < M2_SPW; ++i) {
         const int s = sub + M2_WPK * i;
         if (s < 16) {
             const int d0 = 64 * t + 4 * s;
             float v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if (g < NREP) {
                 const float4 qq = *reinterpret_cast<const float4*>(scratch + g * D + m2_q_chunk(g, d0 >> 2));
-                const __half* hc = reinterpret_cast<const __half*>(&cck[i]);
+                const __half* hc = reinterpret_cast<const __half*>(&qt.cents[i]);
                 v[0] = qq.x; v[1] = qq.z; v[2] = qq.y; v[3] = qq.w;  // dims d0 + {0, 2, 1, 3}
                 c[0] = __half2float(hc[0]); c[1] = __half2float(hc[2]); c[2] = __half2float(hc[1]); c[3] = __half2float(hc[3]);
             }
@@ -645,7 +693,7 @@ __device__ __noinline__ void m2_k_gemm_odd(const M2KRows& kr0, const M2Query& Q0
 __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, const unsigned char* __restrict__ smem,
                                          const float* __restrict__ rope, int kvh, int lane, int valid_lo, int valid_hi,
                                          const M2Query& Q, const CompressedKV& P, float scale,
-                                         M2State& st) {
+                                         M2State& st, bool& vq_ready, uint64_t* vq_bar, uint32_t vq_parity) {
     const int g = lane >> 2, t = lane & 3;
     const float* dinv_s = reinterpret_cast<const float*>(smem + M2_SM_DINV);
     const uint2* qr_s = reinterpret_cast<const uint2*>(smem + M2_SM_QR) + kvh * 4 * 32;
@@ -813,6 +861,10 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
         hb[i] = ((row[24 + (g >> 2)] >> (8 * (g & 3))) & 0xFFu) << 7;  // bit 7 + pl = high code bit of patch pl
     }
     const unsigned char* vq = smem + M2_SM_VQ + 48 * g;
+    if (!vq_ready) {
+        mbar_wait_bounded(vq_bar, vq_parity, &g_status);
+        vq_ready = true;
+    }
 #pragma unroll
     for (int pp = 0; pp < 4; ++pp) {
         float o[5][4];
@@ -880,11 +932,12 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
 
 // Attention of all 24 query heads over compressed tokens [my_lo, my_hi) of P; the CTA's 12 warps
 // are (kv-head = warp & 3) x (group = warp >> 2: every third 16-token block).  On return (behind a CTA barrier) the
-// stages hold one record per warp (store_record's layout, rotated V domain).  The set-up of the tables may still be
-// under way (the barrier after the query build covers it); all M2_THREADS threads call it.
+// stages hold one record per warp (store_record's layout, rotated V domain).  The tables (see m2_load_tables, `table_loads` of them so
+// far) may still be under way; all M2_THREADS threads call it.
 __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const __half* __restrict__ q,
                                                     size_t q_head_stride, const CompressedKV& P, int my_lo, int my_hi,
-                                                    float scale, unsigned& blocks_done, uint32_t tmem, VInverse& inv) {
+                                                    float scale, unsigned& blocks_done, uint32_t tmem, const M2QueryTables& qt,
+                                                    unsigned table_loads, VInverse& inv) {
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;  // uniform: tensor-memory addresses are
     const int kvh = warp & 3, sub = warp >> 2, g = lane >> 2, t = lane & 3;
     const float* freq_s = reinterpret_cast<const float*>(smem + M2_SM_FREQ);
@@ -901,11 +954,16 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
     M2Query Q;
     Q.tm = tmem + ((uint32_t)(32 * kvh) << 16);
     Q.rot = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ROT;
-    m2_build_query(Q, q, q_head_stride, P, kvh, sub, lane, reinterpret_cast<float*>(smem + M2_SM_ROPE) + kvh * NREP * D,
+    m2_build_query(Q, q, q_head_stride, qt, kvh, sub, lane, reinterpret_cast<float*>(smem + M2_SM_ROPE) + kvh * NREP * D,
                    reinterpret_cast<uint2*>(smem + M2_SM_QR) + kvh * 4 * 32);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();  // the query scratch aliases the RoPE buffers
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the query and rotor fragments other warps stored
+    // a layer's tables that come as an image: the small ones now, the codebook before the first V side
+    uint64_t* table_bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS) + M2_BAR_SMALL;
+    const uint32_t table_parity = (table_loads + 1u) & 1u;
+    if (P.image != nullptr) mbar_wait_bounded(&table_bars[0], table_parity, &g_status);
+    bool vq_ready = P.image == nullptr;
     if (nblk > 0) m2_fill_rope(rope_tab, freq_s, P, base, gtid);
     M2State st;
     st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + M2_TM_ACC_WARP * (uint32_t)sub;
@@ -928,10 +986,11 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
         mbar_wait_bounded(&bars[stg], (uint32_t)((gi / M2_NSTAGE) & 1), &g_status);
         const int blk0 = base + i * M2_TT;
         m2_block(stages + stg * M2_STAGE_BYTES, smem, rope_tab + (i & 1) * M2_BT * 64, kvh, lane, max(my_lo - blk0, 0), min(my_hi - blk0, M2_BT), Q,
-                 P, scale, st);
+                 P, scale, st, vq_ready, &table_bars[1], table_parity);
         m2_group_sync(sub);  // stage and rope buffer free for the block after next
     }
     blocks_done = t0 + (unsigned)nblk;
+    if (!vq_ready) mbar_wait_bounded(&table_bars[1], table_parity, &g_status);  // a group without blocks: no copy outlives its phase
     __syncthreads();  // the records alias the stages
     inv.load(P, lane);  // for the caller, in flight behind the records
 
@@ -996,15 +1055,17 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
 __global__ void __launch_bounds__(M2_THREADS, 1)
 khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesDesc* __restrict__ tables,
                               const KhqWorkItem* __restrict__ items, int n_items, int* __restrict__ counter,
-                              float* __restrict__ partials, float scale, float rope_base, int ring_cap) {
+                              float* __restrict__ partials, float scale, float rope_base, int ring_cap,
+                              const unsigned char* const* __restrict__ images) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_next;
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     const int kvh = warp & 3, sub = warp >> 2;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
-    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
+    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_TMSLOT);
     if (tid == 0) {
-        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], HKV);
+        for (int s = 0; s < M2_BAR_SMALL; ++s) mbar_init(&bars[s], HKV);
+        for (int s = M2_BAR_SMALL; s < M2_NBARS; ++s) mbar_init(&bars[s], 1);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
@@ -1014,7 +1075,7 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
     pdl_wait();
     pdl_trigger();
     int cur_table = -1;
-    unsigned blocks_done = 0;
+    unsigned blocks_done = 0, table_loads = 0;
     const float* rec = reinterpret_cast<const float*>(smem + M2_SM_STAGES);
 #pragma unroll 1
     for (int it = blockIdx.x; it < n_items;) {
@@ -1029,15 +1090,18 @@ khq_decode_batched_mma_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTab
         P.v_rotor = tb.v_rotor; P.d_k = tb.d_k; P.d_v = tb.d_v;
         P.alpha_k = tb.alpha_k; P.alpha_v = tb.alpha_v; P.rope_base = rope_base;
         P.start_pos = d.start_pos; P.c_len = d.c_len; P.bulk_ok = 1;
+        P.image = images != nullptr ? images[d.table_id] : nullptr;
         unpack_pos(d.pos_pack, P);
         VInverse inv;
         if (w.kind == 0) {
+            M2QueryTables qt;
+            qt.load(P, sub, lane);
             if (d.table_id != cur_table) {
-                m2_setup_tables(smem, P, tid);
+                m2_load_tables(smem, P, tmem, tid, warp, lane);
                 cur_table = d.table_id;
-                m2_rotor_to_tmem(P, tmem, warp, lane);
+                ++table_loads;
             }
-            m2_compressed_range(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, tmem, inv);
+            m2_compressed_range(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, blocks_done, tmem, qt, table_loads, inv);
         } else {
             WarpState ws;
             ws.init();
@@ -1086,39 +1150,58 @@ khq_attn_compressed_mma_kernel(const __half* __restrict__ q, CompressedKV P, flo
     const int chunk = (((len + csize - 1) / csize) + 1) & ~1;
     const int my_lo = min(s_lo + crank * chunk, s_hi);
     const int my_hi = min(my_lo + chunk, s_hi);
-    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_BARS + 56);
+    uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_TMSLOT);
     if (tid == 0) {
-        for (int s = 0; s < M2_WPK * M2_NSTAGE; ++s) mbar_init(&bars[s], HKV);
+        for (int s = 0; s < M2_BAR_SMALL; ++s) mbar_init(&bars[s], HKV);
+        for (int s = M2_BAR_SMALL; s < M2_NBARS; ++s) mbar_init(&bars[s], 1);
         fence_barrier_init();
     }
     m2_tm_alloc(tm_slot, warp);
-    pdl_wait();
-    pdl_trigger();
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tm_slot, 0);
-    m2_setup_tables(smem, P, tid);
-    m2_rotor_to_tmem(P, tmem, warp, lane);
+    // Prepared tables are constants of the model, written long before the kernel in front of this one: fetched while that one
+    // still runs.
+    M2QueryTables qt;
+    if (P.image == nullptr) pdl_wait();
+    m2_load_tables(smem, P, tmem, tid, warp, lane);
+    qt.load(P, warp >> 2, lane);
+    if (P.image != nullptr) pdl_wait();
+    pdl_trigger();
     unsigned blocks_done = 0;
     VInverse inv;
-    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, tmem, inv);
+    m2_compressed_range(smem, q + (size_t)l_idx * 2 * D, (size_t)L_q * 2 * D, P, my_lo, my_hi, scale, blocks_done, tmem, qt, 1u, inv);
     // the query fragments are not needed any more; everything below is ordinary memory
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    cluster.sync();
+    if (csize > 1) cluster.sync();
+    else __syncthreads();
     m2_tm_free(tmem, warp);
     const float* rec = reinterpret_cast<const float*>(smem + M2_SM_STAGES);
+    const auto out_of = [&](int h) {
+        const int total_id = h * L_q + l_idx;
+        return (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART : out_attn + (size_t)total_id * PART;
+    };
+    if (csize == 1) {  // two heads per warp, side by side
+        static_assert(HQ == 2 * (M2_THREADS / 32), "two heads per warp");
+        HeadAcc a[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int h = warp + k * (HQ / 2);
+            a[k] = merge_head<true, M2_WPK>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) inv.apply(a[k].a, lane);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) store_head(a[k], out_of(warp + k * (HQ / 2)), lane);
+        return;
+    }
 #pragma unroll 1
     for (int h = crank + csize * warp; h < HQ; h += csize * (M2_THREADS / 32)) {
-        HeadAcc a;
-        if (csize == 1)
-            a = merge_head<true, M2_WPK>(M2_WPK, lane, [&](int i) { return m2_head_of_record(rec + (h / NREP + HKV * i) * M2_REC_FLOATS, h % NREP); });
-        else
-            a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
-                return m2_head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * M2_REC_FLOATS, h % NREP);
-            });
+        HeadAcc a = merge_head<true>(M2_WPK * csize, lane, [&](int i) {
+            return m2_head_of_record(cluster.map_shared_rank(rec, i / M2_WPK) + (h / NREP + HKV * (i % M2_WPK)) * M2_REC_FLOATS, h % NREP);
+        });
         inv.apply(a.a, lane);
-        const int total_id = h * L_q + l_idx;
-        store_head(a, (num_splits > 1) ? out_partial + ((size_t)total_id * num_splits + split_id) * PART : out_attn + (size_t)total_id * PART, lane);
+        store_head(a, out_of(h), lane);
     }
     cluster.sync();  // peers must stay resident until their records have been read
 }

@@ -122,7 +122,7 @@ extern "C" int launch_khq_engine_step(khq_engine* e, const khq_engine_layer* lay
                                                       static_cast<const char*>(y.ring_v) - static_cast<const char*>(y.ring_u), stream);
                 if (rc != 0) return rc;
             }
-            rc = launch_khq_decode_batched_fp16(static_cast<const char*>(s->descs) + (size_t)l * B * sizeof(khq_seq_desc), s->tables, s->d_items, B,
+            rc = launch_khq_decode_batched_prepared_fp16(static_cast<const char*>(s->descs) + (size_t)l * B * sizeof(khq_seq_desc), s->tables, s->images, s->d_items, B,
                                                 s->n_items, s->workspace, s->workspace_bytes, s->n_items, s->scale, s->rope_theta, s->ring_cap,
                                                 s->codebook_in_smem, stream);
             if (rc != 0) return rc;

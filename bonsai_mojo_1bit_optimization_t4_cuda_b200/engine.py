@@ -30,7 +30,7 @@ import numpy as np
 import torch
 
 from . import lib as _lib
-from .batched import SEQ_DESC, TABLES_DESC, WORK_ITEM
+from .batched import SEQ_DESC, TABLES_DESC, WORK_ITEM, prepare_tables
 from .calib import KhqLayerTables
 from .lib import check, current_stream
 from .synth import H_KV, H_Q
@@ -90,6 +90,8 @@ class BatchEngine:
                 t[k][i] = tb[k].data_ptr()
             t["alpha_k"][i], t["alpha_v"][i] = tb["alpha_k"], tb["alpha_v"]
         self.d_tables = torch.from_numpy(t.view(np.uint8).reshape(-1).copy()).to(dev)
+        self._images = prepare_tables(t, self.rope_theta, dev)
+        self._d_images = torch.tensor([im.data_ptr() for im in self._images], dtype=torch.int64, device=dev)
         self.norm_w = None
         if norm_weights is not None:
             self.norm_w = [(torch.as_tensor(np.asarray(q, np.float32)).to(dev), torch.as_tensor(np.asarray(k, np.float32)).to(dev))
@@ -197,6 +199,7 @@ class BatchEngine:
             setattr(a, "d_" + f, base + self._at[f])
         a.descs, a.tables, a.workspace, a.workspace_bytes = (self.d_descs.data_ptr(), self.d_tables.data_ptr(), self.workspace.data_ptr(),
                                                              self.ws_bytes)
+        a.images = self._d_images.data_ptr()
         a.n_layers, a.n_seq, a.ring_cap, a.rotary_dim, a.codebook_in_smem = self.L, self.B, RING, ROTARY_DIM, int(codebook_in_smem)
         a.rope_theta, a.rms_eps = self.rope_theta, self.rms_eps
         # A copy of a few tens of KB takes as long as one of 256 KB (3-4 us): layers are copied in groups of about that
@@ -328,11 +331,11 @@ class BatchEngine:
     def attention_resident(self, layer: int, scale: float = 1.0 / 16.0) -> None:
         """The hot path alone: one batched attention launch for `layer` over the current state,
         inputs already in HBM."""
-        rc = self.lib.launch_khq_decode_batched_fp16(
-            self.d_descs.data_ptr() + layer * self.B * SEQ_DESC.itemsize, self.d_tables.data_ptr(), self.d_items.data_ptr(),
+        rc = self.lib.launch_khq_decode_batched_prepared_fp16(
+            self.d_descs.data_ptr() + layer * self.B * SEQ_DESC.itemsize, self.d_tables.data_ptr(), self._d_images.data_ptr(), self.d_items.data_ptr(),
             self.B, self.n_items, self.workspace.data_ptr(), self.ws_bytes, self.n_items, float(scale), self.rope_theta, RING,
             int(self.codebook_in_smem), current_stream())
-        check("launch_khq_decode_batched_fp16", rc)
+        check("launch_khq_decode_batched_prepared_fp16", rc)
 
     def decode_step(self, scale: float = 1.0 / 16.0) -> torch.Tensor:
         """End-to-end token step from HOST buffers.  ``h_q`` (L, B, 24*512: query and gate halves, the

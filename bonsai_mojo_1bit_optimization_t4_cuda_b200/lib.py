@@ -40,6 +40,10 @@ SIGNATURES = {
     "launch_khq_attn_static_fp16": (
         c_int, [_P] * 17 + [c_int] * 5 + [c_float, c_float, c_float, c_float, c_int, c_int, _P]),
     "launch_khq_merge_slots_gate_fp16": (c_int, [_P, c_int, _P, _P, c_int, c_int, _P]),
+    "khq_b200_prepared_bytes": (c_size_t, []),
+    "launch_khq_prepare_tables": (c_int, [_P, c_float, _P, _P]),
+    "launch_khq_decode_batched_prepared_fp16": (
+        c_int, [_P, _P, _P, _P, c_int, c_int, _P, c_size_t, c_int, c_float, c_float, c_int, c_int, _P]),
     "launch_khq_layer_step": (c_int, [_P] * 6 + [c_int] * 4 + [c_float, _P]),
     "khq_b200_engine_create": (c_int, [POINTER(c_void_p)]),
     "khq_b200_engine_destroy": (c_int, [_P]),
@@ -126,7 +130,7 @@ class LayerCtx(ctypes.Structure):
 
     _fields_ = [(n, c_void_p) for n in (
         "d_k", "cents_k", "rotor_k", "d_v", "cents_v", "rotor_v", "vq", "ring_k", "ring_v", "ring_u", "k_mask", "k_payload", "k_norms",
-        "k_r_norms", "v_payload", "v_norms", "v_r_norms", "v_shared_meta", "attn_c", "attn_partial")] + [
+        "k_r_norms", "v_payload", "v_norms", "v_r_norms", "v_shared_meta", "attn_c", "attn_partial", "prepared")] + [
         (n, c_float) for n in ("ts_k", "alpha_k", "ts_v", "alpha_v", "rope_base")] + [("ring_cap", c_int)]
 
 
@@ -144,7 +148,7 @@ class EngineStep(ctypes.Structure):
 
     _fields_ = [(n, c_void_p) for n in (
         "h_q", "h_k", "h_v", "h_control", "h_out", "d_q", "d_k", "d_v", "d_out", "d_control", "d_items", "d_dyn", "d_slots", "d_pos", "d_segs",
-        "descs", "tables", "workspace")] + [("control_bytes", c_size_t), ("workspace_bytes", c_size_t)] + [
+        "descs", "tables", "images", "workspace")] + [("control_bytes", c_size_t), ("workspace_bytes", c_size_t)] + [
         (n, c_int) for n in ("n_layers", "n_seq", "n_items", "n_events", "layers_per_chunk", "parity", "ring_cap", "rotary_dim",
                              "codebook_in_smem")] + [(n, c_float) for n in ("scale", "rope_theta", "rms_eps")]
 

@@ -9,7 +9,10 @@ from __future__ import annotations
 
 import ctypes
 
+import numpy as np
+
 from . import lib as _lib
+from .batched import TABLES_DESC, prepare_tables
 from .lib import check, current_stream, ptr
 
 
@@ -105,7 +108,14 @@ class CudaOps:
                             ("v_r_norms", "vrn"), ("v_shared_meta", "vsm"), ("attn_c", "ac"), ("attn_partial", "ap")):
             setattr(c, field, L.t[name].data_ptr())
         c.ts_k, c.alpha_k, c.ts_v, c.alpha_v, c.rope_base, c.ring_cap = L.ts_k, L.alpha_k, L.ts_v, L.alpha_v, rope_base, ring_cap
-        return c, ctypes.addressof(c)
+        t = np.zeros(1, TABLES_DESC)
+        for field, name in (("cents_k", "ck"), ("cents_v", "cv"), ("vq", "vq"), ("k_rotor", "rk"), ("v_rotor", "rv"), ("d_k", "dk"),
+                            ("d_v", "dv")):
+            t[field] = L.t[name].data_ptr()
+        t["alpha_k"], t["alpha_v"] = L.alpha_k, L.alpha_v
+        image = prepare_tables(t, rope_base, L.t["vq"].device)
+        c.prepared = image.data_ptr()
+        return c, ctypes.addressof(c), image
 
     def layer_step(self, ctx, q_gate, k_roped, v_new, k_unroped, out, c_len, win_len, compress, num_splits, scale):
         rc = self.lib.launch_khq_layer_step(ctx[1], ptr(q_gate), ptr(k_roped), ptr(v_new), ptr(k_unroped), ptr(out), c_len, win_len,

@@ -169,6 +169,7 @@ class KhqRuntime:
         L.t["aw"] = z(H_q * (d + 2), torch.float32)
         L.t["ap"] = z(H_q * KHQ_MAX_SPLITS * (d + 2), torch.float32)
         L.ready = True
+        self._native_ctx(L)
 
     # ------------------------------------------------------------------ split policy
     def _khq_split_count(self, c_len: int) -> int:
@@ -216,6 +217,14 @@ class KhqRuntime:
         return True
 
     # ------------------------------------------------------------------ native step
+    def _native_ctx(self, L):
+        """The layer's native context (addresses and prepared tables), None where the backend has none."""
+        make = getattr(self.ops, "layer_ctx", None)
+        if make is None or (L.H_q, L.H_kv, L.D) != (24, 4, 256):
+            return None
+        L.t.ctx = make(L, KHQ_RING, ROPE_BASE)
+        return L.t.ctx
+
     def _native_step(self, layer_idx: int, L, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, scale: float) -> bool:
         """The step of one layer (append, event if due, both regions, merge, gate) as one native call.
         False: a step that only the call-by-call sequence covers (another backend, profiling, debug
@@ -223,13 +232,9 @@ class KhqRuntime:
         window = L.write_pos + 1 - L.boundary
         if self.prof or self.debug or window > KHQ_RING or window <= 0:
             return False
-        T = L.t
-        ctx = T.ctx
+        ctx = L.t.ctx or self._native_ctx(L)
         if ctx is None:
-            make = getattr(self.ops, "layer_ctx", None)
-            if make is None or (L.H_q, L.H_kv, L.D) != (24, 4, 256):
-                return False
-            ctx = T.ctx = make(L, KHQ_RING, ROPE_BASE)
+            return False
         c_len = L.boundary
         event = window >= KHQ_WATERMARK and c_len + KHQ_CHUNK <= L.cap
         c_after = c_len + KHQ_CHUNK if event else c_len

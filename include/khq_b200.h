@@ -268,6 +268,19 @@ int launch_khq_decode_step_fp16(
     const void* d_vec_v, void* attn_c, void* attn_partial, void* out, int c_len, int win_start, int win_len, int ring_cap,
     int num_splits, float scale, float alpha_k, float alpha_v, float rope_base, khq_stream_t stream);
 
+/* A layer's calibration tables in the form the decode kernels use them (V codebook rows, rotor and Hadamard fragments, 1/d,
+ * RoPE frequencies for `rope_base`), laid out once per layer by a host that keeps its tables: khq_b200_prepared_bytes()
+ * bytes at `image` (device memory, 128-byte aligned).  `tables_desc` is a khq_tables_desc in HOST memory; the tables it
+ * points to must not change while the image is in use.  Without an image the kernels compute the same values per CTA.
+ * Returns -100, -104 or a cudaError_t. */
+size_t khq_b200_prepared_bytes(void);
+int launch_khq_prepare_tables(const void* tables_desc, float rope_base, void* image, khq_stream_t stream);
+/* launch_khq_decode_batched_fp16 with such images: `images` is a device array of image pointers indexed by table_id. */
+int launch_khq_decode_batched_prepared_fp16(const void* descs, const void* tables, const void* images, const void* items,
+                                            int n_desc, int n_items, void* workspace, size_t workspace_bytes,
+                                            int n_slots_total, float scale, float rope_base, int ring_cap,
+                                            int codebook_in_smem, khq_stream_t stream);
+
 /* The same step from a context that keeps a layer's addresses (a host that calls once per layer and token fills it once).
  * In order: when `compress` is nonzero the event of the reference's khq_step (src/khq/runtime.mojo:486-553): the 128 oldest
  * raw tokens, ring slots c_len % ring_cap .., are compressed to rows c_len * 4 .. and the regions move on by 128; then the
@@ -279,6 +292,7 @@ typedef struct khq_layer_ctx {
     void *ring_k, *ring_v, *ring_u;
     void *k_mask, *k_payload, *k_norms, *k_r_norms, *v_payload, *v_norms, *v_r_norms, *v_shared_meta;
     void *attn_c, *attn_partial;
+    const void* prepared; /* image of launch_khq_prepare_tables for these tables and rope_base, or NULL */
     float ts_k, alpha_k, ts_v, alpha_v, rope_base;
     int32_t ring_cap;
 } khq_layer_ctx;
@@ -309,7 +323,7 @@ typedef struct khq_engine_step {
     void *d_q, *d_k, *d_v, *d_out, *d_control;
     const void *d_items, *d_dyn, *d_slots, *d_pos, *d_segs;
     void *descs;
-    const void *tables;
+    const void *tables, *images; /* images: device array of pointers by table_id (launch_khq_prepare_tables), or NULL */
     void *workspace;
     size_t control_bytes, workspace_bytes;
     int32_t n_layers, n_seq, n_items, n_events, layers_per_chunk, parity, ring_cap, rotary_dim, codebook_in_smem;
