@@ -19,10 +19,14 @@ namespace khq {
 
 constexpr int CMP_WARPS = 4;  // warps per block, each on its own row or group of rows
 constexpr int CMP_KROWS = 2;  // rows of a K group (large launches); four would halve the blocks per SM
-constexpr int CMP_VROWS = 4;  // rows a warp carries through the V code search together (large launches)
-// Below this a launch keeps one row per warp: groups of rows would leave SMs without work
-// (148 SMs x 8 blocks x 4 warps x 4 rows = 18 944 rows fill the GPU once).
-constexpr long long CMP_VROWS_MIN_N = 24576;
+constexpr int CMP_VROWS = 4;  // V rows of a CTA whose warps share the code search
+// Below this a K launch keeps one row per warp: groups of rows would leave SMs without work.
+constexpr long long CMP_KROWS_MIN_N = 24576;
+// V launches.  Up to two CTAs of four rows per SM (148 x 2 x 4 rows) the length of one CTA is what counts: 16 warps (512 rows:
+// 9.2 us, 11.1 with 8 warps).  Above, 8 warps overlap more of the unshared work (8192 rows: 59 us, 66 with 16).  The filtered
+// search takes 128 rows per SM and 50 us a time, so it wins once several of those fill the GPU (24 576 rows: 156 against
+// 163 us, 65 536: 338 against 430).
+constexpr int CMP_V16_MAX_N = 1184, CMP_VMMA_MIN_N = 24576;
 
 // One run of rows of a batched launch: source rows (fp16, D per row, contiguous) and the first
 // output row in the launch's output arrays (mirrored in include/khq_b200.h).
@@ -44,12 +48,11 @@ struct CompressScratchK {
     unsigned char os[64];   // outlier sign flags, by outlier ordinal
 };
 
-template <int R>
 struct CompressScratchV {
-    float p[R][D + 4];           // x as float, then the rotated projection, per row of the group
-    float a[R][NP + 4];          // per-patch true energies
-    float b[R][NP + 4];          // per-patch codebook energies
-    unsigned short code[R][NP];  // chosen code per (row, patch)
+    float p[CMP_VROWS][D + 4];           // x as float, then the rotated projection
+    float a[CMP_VROWS][NP + 4];          // per-patch true energies
+    float b[CMP_VROWS][NP + 4];          // per-patch codebook energies
+    unsigned short code[CMP_VROWS][NP];  // chosen code per (row, patch)
 };
 
 // One launch over one contiguous run of rows (segs == nullptr: input row = output row), or over
@@ -330,6 +333,11 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
     unsigned long long r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -340,6 +348,21 @@ __device__ __forceinline__ float f_min3(float a, float b, float c) {
     float d;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
+}
+
+// The 8 codes of a patch that a lane scans, as fp32 (exact), paired by neighbouring codes: cc[k][i] = (code 2i, code 2i+1) of
+// dim k.
+__device__ __forceinline__ void v_load_codes(const __half* __restrict__ vq, int p, int lane, unsigned long long (&cc)[3][4]) {
+    const uint4* cbp = reinterpret_cast<const uint4*>(vq + ((size_t)p * 256 + lane * 8) * 3);
+    __half hcb[24];
+    *reinterpret_cast<uint4*>(&hcb[0]) = __ldg(cbp);
+    *reinterpret_cast<uint4*>(&hcb[8]) = __ldg(cbp + 1);
+    *reinterpret_cast<uint4*>(&hcb[16]) = __ldg(cbp + 2);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            cc[k][i] = f2_pack(__half2float(hcb[6 * i + k]), __half2float(hcb[6 * i + 3 + k]));
 }
 
 // Code search of one (row, patch): every lane scans its 8 consecutive codes in ascending order, then
@@ -380,11 +403,78 @@ __device__ __forceinline__ void v_search_row(const float* __restrict__ proj_row,
     if (lane == 0) code_row[p] = (unsigned short)bi;
 }
 
-// ============ V rows: a warp takes R rows through the code search on one codebook load ============
-// The search dominates a V row (64 patches x 256 codes); the codebook slice a lane scans (8 codes
-// of the patch) is loaded and converted once per patch and used for the R rows of the group.
-template <int R>
-__global__ void __launch_bounds__(CMP_WARPS * 32, 8)
+// What follows the code search of a V row: energies of its 64 patches (to a_row / b_row, for the in-order sums), dim-3
+// centroid choice, residual, packing.  `codes`: the lane's two codes.
+__device__ __forceinline__ void v_row_store(const float (&proj)[8], unsigned codes, long long row, const __half* __restrict__ vq,
+                                            const __half* __restrict__ cents, float alpha, unsigned char* __restrict__ out_payload,
+                                            unsigned char* __restrict__ out_shared_meta, float* a_row, float* b_row, int lane) {
+    unsigned code[2];
+    code[0] = codes & 0xFFFFu;
+    code[1] = codes >> 16;
+    // per-patch energies, dim-3 centroid choice and residual (in the owning lane)
+    float e_true[2], e_vq[2], pres[2];
+    unsigned sel[2];
+    float max_res = 0.0f;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const int pid = lane * 2 + p;
+        const float v0 = proj[p * 4 + 0], v1 = proj[p * 4 + 1], v2 = proj[p * 4 + 2];
+        const __half* cbp = vq + ((size_t)pid * 256 + code[p]) * 3;
+        const float b0 = __half2float(cbp[0]) * alpha;
+        const float b1 = __half2float(cbp[1]) * alpha;
+        const float b2 = __half2float(cbp[2]) * alpha;
+        e_true[p] = __fmaf_rn(v2, v2, __fmaf_rn(v0, v0, v1 * v1));
+        e_vq[p] = __fmaf_rn(b2, b2, __fmaf_rn(b0, b0, b1 * b1));
+        const float v3 = proj[p * 4 + 3];
+        const float c0 = __half2float(cents[0 * D + pid * 4 + 3]);
+        const float c1 = __half2float(cents[1 * D + pid * 4 + 3]);
+        const float dist0 = fabsf(__fmaf_rn(-c0, alpha, v3));
+        const float dist1 = fabsf(__fmaf_rn(-c1, alpha, v3));
+        // ascending scan from min=1e20 with strict '<': index 1 only when strictly closer
+        unsigned s = 0;
+        float bd = 1e20f;
+        if (dist0 < bd) { bd = dist0; s = 0; }
+        if (dist1 < bd) { bd = dist1; s = 1; }
+        sel[p] = s;
+        const float cbest = s ? c1 : c0;
+        pres[p] = __fmaf_rn(-cbest, alpha, v3);
+        max_res = fmaxf(max_res, fabsf(pres[p]));
+        a_row[pid] = e_true[p];
+        b_row[pid] = e_vq[p];
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1)
+        max_res = fmaxf(max_res, __shfl_xor_sync(0xFFFFFFFFu, max_res, m));
+    if (lane == 0) *reinterpret_cast<float*>(out_shared_meta + row * 4) = max_res;
+    const float rs = fmaxf(max_res, 1e-4f);
+    unsigned f24 = 0, hb = 0;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const float scaled = __fmaf_rn(__fdiv_rn(pres[p], rs), 7.0f, 8.0f);
+        const unsigned dump = (unsigned)fmaxf(0.0f, fminf(15.0f, roundf(scaled)));
+        const unsigned f = (code[p] & 0x7Fu) | ((sel[p] & 1u) << 7) | ((dump & 0xFu) << 8);
+        f24 |= f << (12 * p);
+        hb |= ((code[p] >> 7) & 1u) << p;
+    }
+    // 8 patches = 4 lanes = 96 bits = 3 words; lane k of the quad holds bits [24k, 24k+24)
+    const unsigned nxt = __shfl_down_sync(0xFFFFFFFFu, f24, 1);
+    unsigned int* prow = reinterpret_cast<unsigned int*>(out_payload + row * V_PAY);
+    const int k4 = lane & 3, g = lane >> 2;
+    if (k4 == 0) prow[g * 3 + 0] = f24 | (nxt << 24);
+    else if (k4 == 1) prow[g * 3 + 1] = (f24 >> 8) | (nxt << 16);
+    else if (k4 == 2) prow[g * 3 + 2] = (f24 >> 16) | (nxt << 8);
+    const unsigned hv = hb << (2 * (lane & 15));
+    const unsigned lo = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? hv : 0u);
+    const unsigned hi = __reduce_or_sync(0xFFFFFFFFu, lane >= 16 ? hv : 0u);
+    if (lane == 0) { prow[24] = lo; prow[25] = hi; }
+}
+
+// ============ V rows: the W warps of a CTA share the code search of 4 rows ============
+// The search dominates a V row (64 patches x 256 codes).  Small launches are bound by its length, not by throughput, so the 64
+// patches of four rows go to all warps of a CTA; a codebook slice is loaded once for the four rows, the first one while the
+// first four warps prepare the rows.  512 rows: 23.5 us with a warp per row, 9.2 us; 8192 rows: 72 and 59 us.
+template <int W>
+__global__ void __launch_bounds__(W * 32, 32 / W)
 khq_compress_v_kernel(const __half* __restrict__ x, const __half* __restrict__ d_vec,
                       const __half* __restrict__ rotor, const __half* __restrict__ cents,
                       const __half* __restrict__ vq, __half* __restrict__ out_norms,
@@ -392,177 +482,374 @@ khq_compress_v_kernel(const __half* __restrict__ x, const __half* __restrict__ d
                       unsigned char* __restrict__ out_shared_meta, int d_val, int n, float alpha,
                       const KhqCompressSeg* __restrict__ segs, int rows_per_seg,
                       long long x_byte_offset) {
-    __shared__ __align__(16) CompressScratchV<R> scratch[CMP_WARPS];
+    __shared__ __align__(16) CompressScratchV S;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    CompressScratchV<R>& S = scratch[warp];
     const float f_s = rsqrtf((float)d_val);
-    const long long n_groups = ((long long)n + R - 1) / R;
-
-    for (long long grp = (long long)blockIdx.x * CMP_WARPS + warp; grp < n_groups;
-         grp += (long long)gridDim.x * CMP_WARPS) {
-        const long long l0 = grp * R;
-        const int nr = (n - l0 < R) ? (int)(n - l0) : R;
-        // ---- front of every row of the group; the projection stays in shared memory ------------
-#pragma unroll 1
-        for (int r = 0; r < nr; ++r) {
-            long long row;
-            const __half* xrow = compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
-            const uint4 raw = *reinterpret_cast<const uint4*>(xrow + lane * 8);
-            const __half2* hx = reinterpret_cast<const __half2*>(&raw);
-            const float2 x0 = __half22float2(hx[0]), x1 = __half22float2(hx[1]), x2 = __half22float2(hx[2]),
-                         x3 = __half22float2(hx[3]);
-            *reinterpret_cast<float4*>(&S.p[r][lane * 8]) = make_float4(x0.x, x0.y, x1.x, x1.y);
-            *reinterpret_cast<float4*>(&S.p[r][lane * 8 + 4]) = make_float4(x2.x, x2.y, x3.x, x3.y);
+    const long long l0 = (long long)blockIdx.x * CMP_VROWS;
+    const int nr = (n - l0 < CMP_VROWS) ? (int)(n - l0) : CMP_VROWS;
+    unsigned long long cc[3][4];
+    v_load_codes(vq, warp, lane, cc);
+    long long row = 0;
+    if (warp < nr) {
+        const __half* xrow = compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + warp, row);
+        const uint4 raw = *reinterpret_cast<const uint4*>(xrow + lane * 8);
+        const __half2* hx = reinterpret_cast<const __half2*>(&raw);
+        float xv[8], proj[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(hx[j]);
+            xv[2 * j] = f.x;
+            xv[2 * j + 1] = f.y;
         }
+        float* pr = S.p[warp];
+        *reinterpret_cast<float4*>(&pr[lane * 8]) = make_float4(xv[0], xv[1], xv[2], xv[3]);
+        *reinterpret_cast<float4*>(&pr[lane * 8 + 4]) = make_float4(xv[4], xv[5], xv[6], xv[7]);
         __syncwarp();
-        // sums of squares strictly in dim order, the R rows at once: lane l follows row l % R
-        const int cr = lane & (R - 1);
+        // sum of squares strictly in dim order
         float sum_sq = 0.0f;
 #pragma unroll 8
         for (int i = 0; i < D; i += 4) {
-            const float4 t = *reinterpret_cast<const float4*>(&S.p[cr][i]);
+            const float4 t = *reinterpret_cast<const float4*>(&pr[i]);
             sum_sq = __fmaf_rn(t.x, t.x, sum_sq);
             sum_sq = __fmaf_rn(t.y, t.y, sum_sq);
             sum_sq = __fmaf_rn(t.z, t.z, sum_sq);
             sum_sq = __fmaf_rn(t.w, t.w, sum_sq);
         }
         __syncwarp();
+        const float norm = sqrtf(sum_sq + 1e-8f);
+        if (lane == 0) out_norms[row] = __float2half(norm);
+        compress_rotate(xv, norm, d_vec, rotor, f_s, lane, proj);
+        *reinterpret_cast<float4*>(&pr[lane * 8]) = make_float4(proj[0], proj[1], proj[2], proj[3]);
+        *reinterpret_cast<float4*>(&pr[lane * 8 + 4]) = make_float4(proj[4], proj[5], proj[6], proj[7]);
+    }
+    __syncthreads();
+    const unsigned long long nalpha2 = f2_pack(-alpha, -alpha);
 #pragma unroll 1
-        for (int r = 0; r < nr; ++r) {
-            long long row;
-            (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
-            const float norm = sqrtf(__shfl_sync(0xFFFFFFFFu, sum_sq, r) + 1e-8f);
-            if (lane == 0) out_norms[row] = __float2half(norm);
-            float xv[8], proj[8];
-            *reinterpret_cast<float4*>(&xv[0]) = *reinterpret_cast<const float4*>(&S.p[r][lane * 8]);
-            *reinterpret_cast<float4*>(&xv[4]) = *reinterpret_cast<const float4*>(&S.p[r][lane * 8 + 4]);
-            compress_rotate(xv, norm, d_vec, rotor, f_s, lane, proj);
-            *reinterpret_cast<float4*>(&S.p[r][lane * 8]) = make_float4(proj[0], proj[1], proj[2], proj[3]);
-            *reinterpret_cast<float4*>(&S.p[r][lane * 8 + 4]) = make_float4(proj[4], proj[5], proj[6], proj[7]);
+    for (int p = warp; p < NP; p += W) {
+        if (p != warp) v_load_codes(vq, p, lane, cc);
+        if (nr == CMP_VROWS) {
+#pragma unroll
+            for (int r = 0; r < CMP_VROWS; ++r) v_search_row(S.p[r], S.code[r], p, cc, nalpha2, lane);
+        } else {
+            for (int r = 0; r < nr; ++r) v_search_row(S.p[r], S.code[r], p, cc, nalpha2, lane);
         }
-        __syncwarp();
-        // ---- code search: for each patch every lane scans 8 consecutive codes in ascending
-        // order, then the warp takes the lexicographic (distance, index) minimum -----------------
-        const unsigned long long nalpha2 = f2_pack(-alpha, -alpha);
-#pragma unroll 1
-        for (int p = 0; p < NP; ++p) {
-            const uint4* cbp = reinterpret_cast<const uint4*>(vq + ((size_t)p * 256 + lane * 8) * 3);
-            __half hcb[24];
-            *reinterpret_cast<uint4*>(&hcb[0]) = __ldg(cbp);
-            *reinterpret_cast<uint4*>(&hcb[8]) = __ldg(cbp + 1);
-            *reinterpret_cast<uint4*>(&hcb[16]) = __ldg(cbp + 2);
-            // the lane's 8 codes x 3 dims as fp32 (exact), paired by neighbouring codes:
-            // cc[k][i] = (code 2i, code 2i+1) of dim k
-            unsigned long long cc[3][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    cc[k][i] = f2_pack(__half2float(hcb[6 * i + k]), __half2float(hcb[6 * i + 3 + k]));
-            if (nr == R) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    v_search_row(S.p[r], S.code[r], p, cc, nalpha2, lane);
-            } else {
-                for (int r = 0; r < nr; ++r) v_search_row(S.p[r], S.code[r], p, cc, nalpha2, lane);
-            }
-        }
-        __syncwarp();
-        // ---- per row: energies, dim-3 centroid choice, residual, packing ------------------------
-#pragma unroll 1
-        for (int r = 0; r < nr; ++r) {
-            long long row;
-            (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
-            float proj[8];
-            *reinterpret_cast<float4*>(&proj[0]) = *reinterpret_cast<const float4*>(&S.p[r][lane * 8]);
-            *reinterpret_cast<float4*>(&proj[4]) = *reinterpret_cast<const float4*>(&S.p[r][lane * 8 + 4]);
-            unsigned code[2];
-            {
-                const unsigned pr = *reinterpret_cast<const unsigned*>(&S.code[r][lane * 2]);
-                code[0] = pr & 0xFFFFu;
-                code[1] = pr >> 16;
-            }
-            // per-patch energies, dim-3 centroid choice and residual (in the owning lane)
-            float e_true[2], e_vq[2], pres[2];
-            unsigned sel[2];
-            float max_res = 0.0f;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const int pid = lane * 2 + p;
-                const float v0 = proj[p * 4 + 0], v1 = proj[p * 4 + 1], v2 = proj[p * 4 + 2];
-                const __half* cbp = vq + ((size_t)pid * 256 + code[p]) * 3;
-                const float b0 = __half2float(cbp[0]) * alpha;
-                const float b1 = __half2float(cbp[1]) * alpha;
-                const float b2 = __half2float(cbp[2]) * alpha;
-                e_true[p] = __fmaf_rn(v2, v2, __fmaf_rn(v0, v0, v1 * v1));
-                e_vq[p] = __fmaf_rn(b2, b2, __fmaf_rn(b0, b0, b1 * b1));
-                const float v3 = proj[p * 4 + 3];
-                const float c0 = __half2float(cents[0 * D + pid * 4 + 3]);
-                const float c1 = __half2float(cents[1 * D + pid * 4 + 3]);
-                const float dist0 = fabsf(__fmaf_rn(-c0, alpha, v3));
-                const float dist1 = fabsf(__fmaf_rn(-c1, alpha, v3));
-                // ascending scan from min=1e20 with strict '<': index 1 only when strictly closer
-                unsigned s = 0;
-                float bd = 1e20f;
-                if (dist0 < bd) { bd = dist0; s = 0; }
-                if (dist1 < bd) { bd = dist1; s = 1; }
-                sel[p] = s;
-                const float cbest = s ? c1 : c0;
-                pres[p] = __fmaf_rn(-cbest, alpha, v3);
-                max_res = fmaxf(max_res, fabsf(pres[p]));
-                S.a[r][pid] = e_true[p];
-                S.b[r][pid] = e_vq[p];
-            }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1)
-                max_res = fmaxf(max_res, __shfl_xor_sync(0xFFFFFFFFu, max_res, m));
-            if (lane == 0) *reinterpret_cast<float*>(out_shared_meta + row * 4) = max_res;
-            const float rs = fmaxf(max_res, 1e-4f);
-            unsigned f24 = 0, hb = 0;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const float scaled = __fmaf_rn(__fdiv_rn(pres[p], rs), 7.0f, 8.0f);
-                const unsigned dump = (unsigned)fmaxf(0.0f, fminf(15.0f, roundf(scaled)));
-                const unsigned f = (code[p] & 0x7Fu) | ((sel[p] & 1u) << 7) | ((dump & 0xFu) << 8);
-                f24 |= f << (12 * p);
-                hb |= ((code[p] >> 7) & 1u) << p;
-            }
-            // 8 patches = 4 lanes = 96 bits = 3 words; lane k of the quad holds bits [24k, 24k+24)
-            const unsigned nxt = __shfl_down_sync(0xFFFFFFFFu, f24, 1);
-            unsigned int* prow = reinterpret_cast<unsigned int*>(out_payload + row * V_PAY);
-            const int k4 = lane & 3, g = lane >> 2;
-            if (k4 == 0) prow[g * 3 + 0] = f24 | (nxt << 24);
-            else if (k4 == 1) prow[g * 3 + 1] = (f24 >> 8) | (nxt << 16);
-            else if (k4 == 2) prow[g * 3 + 2] = (f24 >> 16) | (nxt << 8);
-            const unsigned hv = hb << (2 * (lane & 15));
-            const unsigned lo = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? hv : 0u);
-            const unsigned hi = __reduce_or_sync(0xFFFFFFFFu, lane >= 16 ? hv : 0u);
-            if (lane == 0) { prow[24] = lo; prow[25] = hi; }
-        }
-        __syncwarp();
-        // the two energy sums strictly in patch order, the R rows at once
-        float st = 0.0f, sv = 0.0f;
+    }
+    __syncthreads();
+    if (warp >= nr) return;
+    // ---- per row: energies, dim-3 centroid choice, residual, packing ------------------------
+    float proj[8];
+    *reinterpret_cast<float4*>(&proj[0]) = *reinterpret_cast<const float4*>(&S.p[warp][lane * 8]);
+    *reinterpret_cast<float4*>(&proj[4]) = *reinterpret_cast<const float4*>(&S.p[warp][lane * 8 + 4]);
+    v_row_store(proj, *reinterpret_cast<const unsigned*>(&S.code[warp][lane * 2]), row, vq, cents, alpha, out_payload,
+                out_shared_meta, S.a[warp], S.b[warp], lane);
+    __syncwarp();
+    // the two energy sums strictly in patch order
+    float st = 0.0f, sv = 0.0f;
 #pragma unroll 4
-        for (int i = 0; i < NP; i += 4) {
-            const float4 ta = *reinterpret_cast<const float4*>(&S.a[cr][i]);
-            const float4 tb = *reinterpret_cast<const float4*>(&S.b[cr][i]);
-            st += ta.x; sv += tb.x;
-            st += ta.y; sv += tb.y;
-            st += ta.z; sv += tb.z;
-            st += ta.w; sv += tb.w;
+    for (int i = 0; i < NP; i += 4) {
+        const float4 ta = *reinterpret_cast<const float4*>(&S.a[warp][i]);
+        const float4 tb = *reinterpret_cast<const float4*>(&S.b[warp][i]);
+        st += ta.x; sv += tb.x;
+        st += ta.y; sv += tb.y;
+        st += ta.z; sv += tb.z;
+        st += ta.w; sv += tb.w;
+    }
+    if (lane == 0) out_r_norms[row] = __float2half(sqrtf(__fdiv_rn(st, sv + 1e-8f)));
+}
+
+// ============ V rows, large launches: the code search filtered on the tensor cores ============
+// Of the 256 exact distances per (row, patch) only the smallest matters, and it is almost always smaller than the others by
+// far more than an approximation is off.  The approximation is one m16n8k16 product per 16 rows x 8 codes:
+//     64 (|a c|^2 - 2 a v.c)  =  (64 v, 64) . (-2 a c, |a c|^2)
+// with v and a c as fp16 pieces that carry 22 bits (v = vh + vl, -2 a c = ch + cl, the norm in three pieces):
+//     k   0..2 vh ch   3: 64 n1   4..6 vl ch   7: 64 n2   8..10 vh cl   11: 64 n3   12..15: 0.
+// Each omitted or rounded term is below 2^-22 of its factors and the fp32 accumulation of twelve terms below 2^-19 of their
+// magnitude B = V^2 + 2 V cm + 3 cm^2 (V = |v0| + |v1| + |v2|, cm = largest |a c_k| of the patch), which also bounds what the
+// reference's own fp32 evaluation is off (3 x 2^-24 of a distance <= B).  If exactly one code lies within 2^-16 B of the
+// smallest approximation it is the reference's choice; every other (row, patch) goes through the exact search
+// (v_search_row).  So the code words stay bit-identical.
+//
+// CTA = four groups of two warps; a group owns 16 rows (one M tile), its warps search patches 0..31 and 32..63 and share the
+// rows in front and behind.  The B fragments of a patch (8 KB) are built once per CTA and step by all threads, double
+// buffered.  A thread holds 2 rows x 32 codes of a half patch: minimum by three-input min, then the sign bits of (value -
+// minimum - margin) shifted into a mask.  44 warp instructions per (row, patch) against 85 of the exact search, about two per
+// cycle; 0.9 % of the pairs are redone.  129 024 rows: 800 -> 657 us.
+constexpr int VM_ROWS = 16;  // rows per group
+constexpr int VM_GROUPS = 4;   // per CTA; eight halve the building of fragments but not the time (694 us)
+struct CompressScratchVM {
+    float p[VM_GROUPS * VM_ROWS][D + 4];   // x as float, then the projection, then (per row) the patch energies
+    uint4 b[2][2][256 * 2];                // [buffer][half][code]: k pairs of lanes t = 0..3 (b0, b1 each)
+    float cm[2][2][8];                     // largest |a c_k| per warp's share of a patch
+    unsigned short code[VM_GROUPS * VM_ROWS][NP];
+};
+
+__device__ __forceinline__ uint32_t vm_pack(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// B fragments of one code (c: its three halfs).
+__device__ __forceinline__ void vm_build(const __half (&c)[3], float alpha, uint4* dst, float& cmax) {
+    float a[3], q[3], n = 0.0f;
+    cmax = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a[k] = __half2float(c[k]) * alpha;
+        cmax = fmaxf(cmax, fabsf(a[k]));
+        n = fmaf(a[k], a[k], n);
+        q[k] = -2.0f * a[k];
+    }
+    const float h0 = __half2float(__float2half(q[0])), h1 = __half2float(__float2half(q[1])), h2 = __half2float(__float2half(q[2]));
+    const float n1 = __half2float(__float2half(n)), n2 = __half2float(__float2half(n - n1));
+    const uint32_t p01 = vm_pack(h0, h1);
+    dst[0] = make_uint4(p01, vm_pack(q[0] - h0, q[1] - h1), vm_pack(h2, n1), vm_pack(q[2] - h2, (n - n1) - n2));
+    dst[1] = make_uint4(p01, 0u, vm_pack(h2, n2), 0u);
+}
+
+__global__ void __launch_bounds__(VM_GROUPS * 64, 2)
+khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict__ d_vec,
+                          const __half* __restrict__ rotor, const __half* __restrict__ cents,
+                          const __half* __restrict__ vq, __half* __restrict__ out_norms,
+                          __half* __restrict__ out_r_norms, unsigned char* __restrict__ out_payload,
+                          unsigned char* __restrict__ out_shared_meta, int d_val, int n, float alpha,
+                          const KhqCompressSeg* __restrict__ segs, int rows_per_seg,
+                          long long x_byte_offset) {
+    extern __shared__ __align__(16) unsigned char vm_smem[];
+    CompressScratchVM& S = *reinterpret_cast<CompressScratchVM*>(vm_smem);
+    constexpr int RW = VM_ROWS / 2;  // rows per warp in front and behind
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = warp >> 1, half = warp & 1;
+    const int g = lane >> 2, t = lane & 3;
+    const float f_s = rsqrtf((float)d_val);
+    const int r_first = grp * VM_ROWS + half * RW;  // this warp's rows of the CTA
+    const long long l0 = (long long)blockIdx.x * (VM_GROUPS * VM_ROWS) + r_first;
+    const int nr = n - l0 >= RW ? RW : (n > l0 ? (int)(n - l0) : 0);
+
+    // the codes a thread prepares for a step: code `tid` of patches step and step + 32
+    static_assert(VM_GROUPS * 64 == 256, "a thread per code");
+    __half cn[2][3];
+    const auto fetch = [&](int step) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const __half* c = vq + ((size_t)(step + 32 * u) * 256 + tid) * 3;
+            cn[u][0] = c[0];
+            cn[u][1] = c[1];
+            cn[u][2] = c[2];
         }
-        if (lane < nr) {
+    };
+    const auto build = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            float m;
+            vm_build(cn[u], alpha, &S.b[buf][u][2 * tid], m);
+            const unsigned mb = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m));
+            if (lane == 0) S.cm[buf][u][warp] = __uint_as_float(mb);
+        }
+    };
+    fetch(0);
+    // ---- front: rows as fp32, in-order sums of squares, projections ----------------------------
+#pragma unroll 1
+    for (int r = 0; r < RW; ++r) {
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        if (r < nr) {
             long long row;
-            (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + lane, row);
-            out_r_norms[row] = __float2half(sqrtf(__fdiv_rn(st, sv + 1e-8f)));
+            const __half* xrow = compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
+            const uint4 raw = *reinterpret_cast<const uint4*>(xrow + lane * 8);
+            const __half2* hx = reinterpret_cast<const __half2*>(&raw);
+            const float2 x0 = __half22float2(hx[0]), x1 = __half22float2(hx[1]), x2 = __half22float2(hx[2]), x3 = __half22float2(hx[3]);
+            lo = make_float4(x0.x, x0.y, x1.x, x1.y);
+            hi = make_float4(x2.x, x2.y, x3.x, x3.y);
         }
-        __syncwarp();
+        *reinterpret_cast<float4*>(&S.p[r_first + r][lane * 8]) = lo;
+        *reinterpret_cast<float4*>(&S.p[r_first + r][lane * 8 + 4]) = hi;
+    }
+    __syncwarp();
+    const int cr = lane & (RW - 1);
+    float sum_sq = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < D; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&S.p[r_first + cr][i]);
+        sum_sq = __fmaf_rn(v.x, v.x, sum_sq);
+        sum_sq = __fmaf_rn(v.y, v.y, sum_sq);
+        sum_sq = __fmaf_rn(v.z, v.z, sum_sq);
+        sum_sq = __fmaf_rn(v.w, v.w, sum_sq);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int r = 0; r < nr; ++r) {
+        long long row;
+        (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
+        const float norm = sqrtf(__shfl_sync(0xFFFFFFFFu, sum_sq, r) + 1e-8f);
+        if (lane == 0) out_norms[row] = __float2half(norm);
+        float* pr = S.p[r_first + r];
+        float xv[8], proj[8];
+        *reinterpret_cast<float4*>(&xv[0]) = *reinterpret_cast<const float4*>(&pr[lane * 8]);
+        *reinterpret_cast<float4*>(&xv[4]) = *reinterpret_cast<const float4*>(&pr[lane * 8 + 4]);
+        compress_rotate(xv, norm, d_vec, rotor, f_s, lane, proj);
+        *reinterpret_cast<float4*>(&pr[lane * 8]) = make_float4(proj[0], proj[1], proj[2], proj[3]);
+        *reinterpret_cast<float4*>(&pr[lane * 8 + 4]) = make_float4(proj[4], proj[5], proj[6], proj[7]);
+    }
+    build(0);
+    __syncthreads();
+    // ---- code search ---------------------------------------------------------------------------
+    const int m_row = grp * VM_ROWS;
+#pragma unroll 1
+    for (int step = 0; step < NP / 2; ++step) {
+        const int buf = step & 1, patch = step + 32 * half;
+        if (step + 1 < NP / 2) fetch(step + 1);
+        float cm = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) {
+            const float4 c = *reinterpret_cast<const float4*>(&S.cm[buf][half][k]);
+            cm = fmaxf(cm, fmaxf(fmaxf(c.x, c.y), fmaxf(c.z, c.w)));
+        }
+        uint32_t a[4];
+        float thr[2];
+        bool safe[2];
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            const float4 v = *reinterpret_cast<const float4*>(&S.p[m_row + g + 8 * y][patch * 4]);
+            const float V = fabsf(v.x) + fabsf(v.y) + fabsf(v.z);
+            thr[y] = fmaf(V, fmaf(2.0f, cm, V), 3.0f * cm * cm) * 0.0009765625f;  // 64 x 2^-16 x B
+            safe[y] = V < 500.0f && cm < 200.0f;  // nothing overflows fp16; false for NaN
+            const float e0 = 64.0f * ((t & 1) ? v.z : v.x), e1 = (t & 1) ? 64.0f : 64.0f * v.y;
+            const uint32_t hi = vm_pack(e0, e1);
+            const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+            const uint32_t lo = vm_pack(e0 - hf.x, t == 3 ? 64.0f : e1 - hf.y);
+            a[y] = t < 2 ? hi : lo;
+            a[2 + y] = t < 2 ? hi : 0u;
+        }
+        const uint4* bp = S.b[buf][half];
+        float best[2];
+        uint32_t mask[2], chunk[2];
+        bool tie[2];
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+            float acc[16][4];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const uint2 b = reinterpret_cast<const uint2*>(bp)[(ch * 16 + j) * 32 + lane];
+                asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                    : "=f"(acc[j][0]), "=f"(acc[j][1]), "=f"(acc[j][2]), "=f"(acc[j][3])
+                    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "f"(0.0f));
+            }
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                float m4[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {  // eight values each
+                    m4[k] = f_min3(acc[4 * k][2 * y], acc[4 * k][2 * y + 1], acc[4 * k + 1][2 * y]);
+                    m4[k] = f_min3(m4[k], acc[4 * k + 1][2 * y + 1], acc[4 * k + 2][2 * y]);
+                    m4[k] = f_min3(m4[k], acc[4 * k + 2][2 * y + 1], acc[4 * k + 3][2 * y]);
+                    m4[k] = fminf(m4[k], acc[4 * k + 3][2 * y + 1]);
+                }
+                const float m = f_min3(fminf(m4[0], m4[1]), m4[2], m4[3]);
+                const float nlim = -(m + thr[y]);
+                uint32_t w[2] = {0u, 0u};  // sign bits of the values of tiles 0..7 and 8..15, first value on top
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float d0, d1;
+                    f2_unpack(f2_add(f2_pack(acc[j][2 * y], acc[j][2 * y + 1]), f2_pack(nlim, nlim)), d0, d1);
+                    w[j >> 3] = __funnelshift_l(__float_as_uint(d0), w[j >> 3], 1);
+                    w[j >> 3] = __funnelshift_l(__float_as_uint(d1), w[j >> 3], 1);
+                }
+                const uint32_t mk = (w[0] << 16) | w[1];
+                if (ch == 0) {
+                    best[y] = m;
+                    mask[y] = mk;
+                    chunk[y] = 0;
+                    tie[y] = false;
+                } else {
+                    tie[y] = !(fabsf(m - best[y]) > thr[y]);
+                    if (m < best[y]) {
+                        best[y] = m;
+                        mask[y] = mk;
+                        chunk[y] = 128;
+                    }
+                }
+            }
+        }
+        unsigned redo = 0;  // rows of the tile that need the exact search
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+            float m = fminf(best[y], __shfl_xor_sync(0xFFFFFFFFu, best[y], 1));
+            m = fminf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+            const int i = __clz((int)mask[y]);  // position of the first candidate among the lane's 32 values
+            uint32_t mine = (tie[y] ? 2u : (uint32_t)__popc(mask[y])) << 16;
+            mine |= chunk[y] + 8u * (uint32_t)(i >> 1) + 2u * (uint32_t)t + (uint32_t)(i & 1);
+            if (!(best[y] <= m + thr[y])) mine = 0u;
+            mine += __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
+            mine += __shfl_xor_sync(0xFFFFFFFFu, mine, 2);
+            const bool one = safe[y] && (mine >> 16) == 1u;
+            if (t == 0 && one) S.code[m_row + g + 8 * y][patch] = (unsigned short)(mine & 0xFFFFu);
+            redo |= __ballot_sync(0xFFFFFFFFu, t == 0 && !one) << y;  // bit 4 g + y: row g + 8 y
+        }
+        if (redo) {
+            const unsigned long long nalpha2 = f2_pack(-alpha, -alpha);
+            unsigned long long cc[3][4];
+            v_load_codes(vq, patch, lane, cc);
+#pragma unroll 1
+            while (redo) {
+                const int k = __ffs((int)redo) - 1, r = m_row + (k >> 2) + 8 * (k & 3);
+                redo &= redo - 1;
+                v_search_row(S.p[r], S.code[r], patch, cc, nalpha2, lane);
+            }
+        }
+        if (step + 1 < NP / 2) build(buf ^ 1);
+        __syncthreads();
+    }
+    // ---- per row: energies, dim-3 centroid choice, residual, packing ------------------------------
+#pragma unroll 1
+    for (int r = 0; r < nr; ++r) {
+        long long row;
+        (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + r, row);
+        float* pr = S.p[r_first + r];
+        float proj[8];
+        *reinterpret_cast<float4*>(&proj[0]) = *reinterpret_cast<const float4*>(&pr[lane * 8]);
+        *reinterpret_cast<float4*>(&proj[4]) = *reinterpret_cast<const float4*>(&pr[lane * 8 + 4]);
+        __syncwarp();  // the energies take the row's place
+        v_row_store(proj, *reinterpret_cast<const unsigned*>(&S.code[r_first + r][lane * 2]), row, vq, cents, alpha, out_payload,
+                    out_shared_meta, pr, pr + NP, lane);
+    }
+    __syncwarp();
+    // the two energy sums strictly in patch order, the warp's rows at once
+    float st = 0.0f, sv = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < NP; i += 4) {
+        const float4 ta = *reinterpret_cast<const float4*>(&S.p[r_first + cr][i]);
+        const float4 tb = *reinterpret_cast<const float4*>(&S.p[r_first + cr][NP + i]);
+        st += ta.x; sv += tb.x;
+        st += ta.y; sv += tb.y;
+        st += ta.z; sv += tb.z;
+        st += ta.w; sv += tb.w;
+    }
+    if (lane < nr) {
+        long long row;
+        (void)compress_map_row(x, segs, rows_per_seg, x_byte_offset, l0 + lane, row);
+        out_r_norms[row] = __float2half(sqrtf(__fdiv_rn(st, sv + 1e-8f)));
     }
 }
 
 }  // namespace khq
 
 namespace {
+int launch_v_mma(const __half* x, const __half* dv, const __half* ro, const __half* ce, const void* vq, __half* on, __half* orn,
+                 unsigned char* op, unsigned char* om, int d, int n, float alpha, const khq::KhqCompressSeg* segs, int rows_per_seg,
+                 long long x_byte_offset, cudaStream_t stream) {
+    using namespace khq;
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return static_cast<int>(err);
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        err = cudaFuncSetAttribute(khq_compress_v_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CompressScratchVM));
+        if (err != cudaSuccess) return static_cast<int>(err);
+        if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+    khq_compress_v_mma_kernel<<<(unsigned)((n + VM_GROUPS * VM_ROWS - 1) / (VM_GROUPS * VM_ROWS)), VM_GROUPS * 64, sizeof(CompressScratchVM), stream>>>(
+        x, dv, ro, ce, static_cast<const __half*>(vq), on, orn, op, om, d, n, alpha, segs, rows_per_seg, x_byte_offset);
+    return 0;
+}
+
 int compress_launch(const __half* x, const void* d_vec, const void* rotor, const void* centroids,
                     const void* vq_centroids, void* out_mask, void* out_norms, void* out_r_norms,
                     void* out_payload, void* out_shared_meta, int d, int n, float threshold_scale, float alpha,
@@ -581,7 +868,7 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
     __half* orn = static_cast<__half*>(out_r_norms);
     unsigned char* op = static_cast<unsigned char*>(out_payload);
     unsigned char* om = static_cast<unsigned char*>(out_shared_meta);
-    if (!is_v && n >= CMP_VROWS_MIN_N) {
+    if (!is_v && n >= CMP_KROWS_MIN_N) {
         khq_compress_k_kernel<CMP_KROWS><<<grid(((long long)n + CMP_KROWS - 1) / CMP_KROWS), CMP_WARPS * 32, 0,
                                            stream>>>(x, dv, ro, ce, static_cast<unsigned int*>(out_mask), on, orn, op,
                                                      om, d, n, threshold_scale, segs, rows_per_seg, x_byte_offset);
@@ -589,14 +876,14 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
         khq_compress_k_kernel<1><<<grid(n), CMP_WARPS * 32, 0, stream>>>(
             x, dv, ro, ce, static_cast<unsigned int*>(out_mask), on, orn, op, om, d, n, threshold_scale, segs,
             rows_per_seg, x_byte_offset);
-    } else if (n >= CMP_VROWS_MIN_N) {
-        khq_compress_v_kernel<CMP_VROWS><<<grid(((long long)n + CMP_VROWS - 1) / CMP_VROWS), CMP_WARPS * 32, 0,
-                                           stream>>>(x, dv, ro, ce, static_cast<const __half*>(vq_centroids), on, orn,
-                                                     op, om, d, n, alpha, segs, rows_per_seg, x_byte_offset);
+    } else if (n >= CMP_VMMA_MIN_N) {
+        const int rc = launch_v_mma(x, dv, ro, ce, vq_centroids, on, orn, op, om, d, n, alpha, segs, rows_per_seg, x_byte_offset, stream);
+        if (rc != 0) return rc;
     } else {
-        khq_compress_v_kernel<1><<<grid(n), CMP_WARPS * 32, 0, stream>>>(
-            x, dv, ro, ce, static_cast<const __half*>(vq_centroids), on, orn, op, om, d, n, alpha, segs,
-            rows_per_seg, x_byte_offset);
+        const unsigned blocks = (unsigned)((n + CMP_VROWS - 1) / CMP_VROWS);
+        const auto kernel = n <= CMP_V16_MAX_N ? khq_compress_v_kernel<16> : khq_compress_v_kernel<8>;
+        kernel<<<blocks, n <= CMP_V16_MAX_N ? 512 : 256, 0, stream>>>(x, dv, ro, ce, static_cast<const __half*>(vq_centroids), on, orn, op,
+                                                                      om, d, n, alpha, segs, rows_per_seg, x_byte_offset);
     }
     const cudaError_t err = cudaGetLastError();
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
