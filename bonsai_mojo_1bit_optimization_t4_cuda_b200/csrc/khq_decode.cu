@@ -1260,6 +1260,61 @@ extern "C" int launch_khq_layer_step(const khq_layer_ctx* L, const void* q_gate,
                             c_len % L->ring_cap, win_len, L->ring_cap, num_splits, scale, L->alpha_k, L->alpha_v, L->rope_base, L->prepared, stream);
 }
 
+// The newest rows of a prompt into the three rings, row by row at slot = token % ring_cap.  Grid (16-byte vectors, 3 rings).  One
+// launch instead of up to six copies: short prompts are bound by launches (a 2 KB row per token and ring, 1.5 us).
+__global__ void __launch_bounds__(256)
+khq_ring_fill_kernel(const uint4* __restrict__ k_roped, const uint4* __restrict__ v, const uint4* __restrict__ k_unroped,
+                     uint4* __restrict__ ring_k, uint4* __restrict__ ring_v, uint4* __restrict__ ring_u, int first, int tokens,
+                     int ring_cap) {
+    constexpr int ROW = HKV * D / 8;
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= tokens * ROW) return;
+    const int token = first + i / ROW;
+    const uint4* src = blockIdx.y == 0 ? k_roped : blockIdx.y == 1 ? v : k_unroped;
+    uint4* dst = blockIdx.y == 0 ? ring_k : blockIdx.y == 1 ? ring_v : ring_u;
+    dst[(size_t)(token % ring_cap) * ROW + i % ROW] = src[(size_t)token * ROW + i % ROW];
+}
+
+extern "C" int launch_khq_gqa_prefill_fp16(const void*, const void*, const void*, void*, int, int, int, int, int, float, long long,
+                                           long long, long long, cudaStream_t);
+
+extern "C" int launch_khq_layer_prefill(const khq_layer_ctx* L, const void* q_gate, const void* k_unroped, const void* k_roped,
+                                        const void* v, void* out, int T, int n_chunks, float scale, cudaStream_t stream) {
+    constexpr int CHUNK = 128;
+    if (!L || !q_gate || !k_unroped || !k_roped || !v || !out || T <= 0 || n_chunks < 0 || n_chunks > T / CHUNK) return -100;
+    if (L->ring_cap <= 0) return -103;
+    if (!aligned(k_unroped, 16) || !aligned(L->ring_k, 16) || !aligned(L->ring_v, 16) || !aligned(L->ring_u, 16)) return -104;
+    int rc = launch_khq_gqa_prefill_fp16(q_gate, k_roped, v, out, 1, T, HQ, HKV, D, scale, (long long)T * HQ * 2 * D,
+                                         (long long)T * HKV * D, (long long)T * HQ * D, stream);
+    if (rc != 0) return rc;
+    if (n_chunks > 0) {  // K first: it zeroes the shared meta rows that the V launch then fills
+        const int rows = n_chunks * CHUNK * HKV;
+        rc = launch_khq_compress_fp16(k_unroped, L->d_k, L->rotor_k, L->cents_k, L->cents_k, L->k_mask, L->k_norms, L->k_r_norms,
+                                      L->k_payload, L->v_shared_meta, rows, D, L->ts_k, L->alpha_k, 0, stream);
+        if (rc != 0) return rc;
+        rc = launch_khq_compress_fp16(v, L->d_v, L->rotor_v, L->cents_v, L->vq, L->k_mask, L->v_norms, L->v_r_norms, L->v_payload,
+                                      L->v_shared_meta, rows, D, L->ts_v, L->alpha_v, 1, stream);
+        if (rc != 0) return rc;
+    }
+    const int tokens = T < L->ring_cap ? T : L->ring_cap;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((tokens * (HKV * D / 8) + 255) / 256), 3, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, khq_ring_fill_kernel, static_cast<const uint4*>(k_roped), static_cast<const uint4*>(v),
+                                               static_cast<const uint4*>(k_unroped), static_cast<uint4*>(L->ring_k),
+                                               static_cast<uint4*>(L->ring_v), static_cast<uint4*>(L->ring_u), T - tokens, tokens,
+                                               L->ring_cap);
+    return (err == cudaSuccess) ? 0 : static_cast<int>(err);
+}
+
 extern "C" int launch_khq_gather_q_fp16(const void* q_gate, void* q_out, int H_q, int d,
                                         cudaStream_t stream) {
     if (H_q <= 0 || d <= 0) return -100;

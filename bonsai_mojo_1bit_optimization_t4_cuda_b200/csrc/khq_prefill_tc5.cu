@@ -50,6 +50,7 @@
 #include <stdlib.h>
 
 #include "khq_common.cuh"
+#include "khq_launch.cuh"
 
 namespace khq_prefill5 {
 
@@ -323,6 +324,9 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         for (int q = 0; q < 4; ++q) khq::mbar_init(&bars[B_XCHG + q], 2);  // the two warps of a lane quarter
         khq::fence_barrier_init();
     }
+    // Everything above overlaps the kernel before; tensor memory is only taken once that kernel has finished (it may still have
+    // to allocate its own on this SM).
+    khq::pdl_wait();
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "n"(TM_COLS)
@@ -742,8 +746,8 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     __half* op = static_cast<__half*>(out);
     const float sl2 = scale * 1.4426950408889634f;
 #define KHQ_TC5_LAUNCH(PERSIST, BF16)                                                                                  \
-    khq_gqa_prefill_tc5_kernel<PERSIST, BF16><<<grid, NTHREADS, SMEM_BYTES, stream>>>(                                  \
-        mq, mk, mv, qp, op, T, H_q, H_kv, batch, group_major, sl2, q_batch_stride, out_batch_stride)
+    err = khq::launch_pdl(khq_gqa_prefill_tc5_kernel<PERSIST, BF16>, grid, 0, SMEM_BYTES, stream, (unsigned)NTHREADS, mq, mk, mv, qp, op, \
+                          T, H_q, H_kv, batch, group_major, sl2, q_batch_stride, out_batch_stride)
     if (ctas == items) {
         if (bf16) KHQ_TC5_LAUNCH(false, true);
         else KHQ_TC5_LAUNCH(false, false);
@@ -752,7 +756,6 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
         else KHQ_TC5_LAUNCH(true, false);
     }
 #undef KHQ_TC5_LAUNCH
-    err = cudaGetLastError();
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 }  // namespace

@@ -123,6 +123,12 @@ class CudaOps:
         if rc != 0:
             check("launch_khq_layer_step", rc)
 
+    def layer_prefill(self, ctx, q_gate, k_unroped, k_roped, v, out, T, n_chunks, scale):
+        rc = self.lib.launch_khq_layer_prefill(ctx[1], ptr(q_gate), ptr(k_unroped), ptr(k_roped), ptr(v), ptr(out), T, n_chunks, scale,
+                                               current_stream())
+        if rc != 0:
+            check("launch_khq_layer_prefill", rc)
+
     # -- peer-memory exchange of context-parallel partials ----------------------------------------
     def publish_partials(self, src, n_records, peer_slots, peer_flags, world, rank, first_slot, parity_offset_records, epoch):
         rc = self.lib.launch_khq_publish_partials_fp32(ptr(src), int(n_records), ptr(peer_slots), ptr(peer_flags), int(world),

@@ -393,11 +393,14 @@ class KhqRuntime:
                 "v": v_dev.numel(), "out": out_dev.numel()}
         if T <= 0 or any(have[k] != want[k] for k in want):
             raise ValueError(f"khq_prefill: tensors do not hold T={T} rows of (H_q={H_q}, H_kv={H_kv}, d={d}): {have} vs {want}")
-        ops.gqa_prefill(q_gate_dev, k_roped_dev, v_dev, out_dev, 1, T, H_q, H_kv, d, scale)
         # the per-token path compresses chunk c when write_pos reaches 128*(c+2), capped by `cap`
         n_chunks = 0
         while (n_chunks + 2) * KHQ_CHUNK <= T and (n_chunks + 1) * KHQ_CHUNK <= L.cap:
             n_chunks += 1
+        if self._native_prefill(L, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T, n_chunks, scale):
+            self._prefill_done(layer_idx, L, T, n_chunks)
+            return True
+        ops.gqa_prefill(q_gate_dev, k_roped_dev, v_dev, out_dev, 1, T, H_q, H_kv, d, scale)
         if n_chunks > 0:
             rows = n_chunks * KHQ_CHUNK * H_kv
             ku = k_unroped_dev.reshape(-1)
@@ -406,8 +409,6 @@ class KhqRuntime:
                          Tn["vsm"], rows, d, L.ts_k, L.alpha_k, False)
             ops.compress(vv, Tn["dv"], Tn["rv"], Tn["cv"], Tn["vq"], Tn["kmask"], Tn["vnorm"], Tn["vrn"], Tn["vpay"],
                          Tn["vsm"], rows, d, L.ts_v, L.alpha_v, True)
-        L.boundary = n_chunks * KHQ_CHUNK
-        L.write_pos = T
         # newest min(T, 256) tokens into the rings at slot = token % 256
         first = max(0, T - KHQ_RING)
         for name, src in (("ring_k", k_roped_dev), ("ring_v", v_dev), ("ring_u", k_unroped_dev)):
@@ -419,8 +420,25 @@ class KhqRuntime:
             ring[a:a + head].copy_(s2[first:first + head])
             if n > head:
                 ring[0:n - head].copy_(s2[first + head:T])
+        self._prefill_done(layer_idx, L, T, n_chunks)
+        return True
+
+    def _prefill_done(self, layer_idx: int, L, T: int, n_chunks: int) -> None:
+        L.boundary = n_chunks * KHQ_CHUNK
+        L.write_pos = T
         for c in range(n_chunks):
             self.events.append(KhqCompressEvent(layer_idx, c + 1, (c + 1) * KHQ_CHUNK, (c + 2) * KHQ_CHUNK, KHQ_CHUNK))
+
+    def _native_prefill(self, L, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T: int, n_chunks: int, scale: float) -> bool:
+        """The whole prompt of one layer as one native call.  False: another backend or shape, other types than fp16, or rows that
+        need a copy first (not contiguous, or not on 16 bytes)."""
+        ctx = L.t.ctx or self._native_ctx(L)
+        if ctx is None:
+            return False
+        for t in (q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev):
+            if t.dtype is not torch.float16 or not t.is_contiguous() or t.data_ptr() & 15:
+                return False
+        self.ops.layer_prefill(ctx, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T, n_chunks, float(scale))
         return True
 
     # ------------------------------------------------------------------ khq_prof_report

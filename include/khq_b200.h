@@ -299,6 +299,11 @@ typedef struct khq_layer_ctx {
 int launch_khq_layer_step(const khq_layer_ctx* ctx, const void* q_gate, const void* k_roped, const void* v_new,
                           const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits, float scale,
                           khq_stream_t stream);
+/* A whole prompt of T rows of a fresh layer: launch_khq_gqa_prefill_fp16, compression of the first n_chunks * 128 tokens, and
+ * the newest min(T, ring_cap) rows of K RoPE'd, V and K un-RoPE'd into the rings at slot = token % ring_cap.  q_gate (T, 24, 512),
+ * k_unroped / k_roped / v (T, 4, 256), out (T, 24, 256), fp16, all 16-byte aligned (-104). */
+int launch_khq_layer_prefill(const khq_layer_ctx* ctx, const void* q_gate, const void* k_unroped, const void* k_roped,
+                             const void* v, void* out, int T, int n_chunks, float scale, khq_stream_t stream);
 
 /* ---- A batch engine's token step in one call (no counterpart in the reference) -----------------
  * What a host would issue per layer for n_seq sequences: inputs from pinned host memory (copies on the engine's own
