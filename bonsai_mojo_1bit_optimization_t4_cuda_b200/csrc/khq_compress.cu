@@ -18,10 +18,12 @@
 namespace khq {
 
 constexpr int CMP_WARPS = 4;  // warps per block, each on its own row or group of rows
-constexpr int CMP_KROWS = 2;  // rows of a K group (large launches); four would halve the blocks per SM
+constexpr int CMP_KROWS = 4;  // K rows that a warp takes together (large launches)
 constexpr int CMP_VROWS = 4;  // V rows of a CTA whose warps share the code search
-// Below this a K launch keeps one row per warp: groups of rows would leave SMs without work.
-constexpr long long CMP_KROWS_MIN_N = 24576;
+// Below this a K launch keeps one row per warp: groups of four give each of 16 warps per SM one group (148 x 16 x 4 rows), and
+// fewer rows than that leave warps without work (8192 rows: 26.4 us either way, 4096: 15.5 against 20.8, 16 384: 47.1 against
+// 38.8).  Eight rows a warp cost more in occupancy than their shared sums save (129 024 rows: 259 against 227 us).
+constexpr long long CMP_KROWS_MIN_N = 9472;
 // V launches.  Up to two CTAs of four rows per SM (148 x 2 x 4 rows) the length of one CTA is what counts: 16 warps (512 rows:
 // 9.2 us, 11.1 with 8 warps).  Above, 8 warps overlap more of the unshared work (8192 rows: 59 us, 66 with 16).  The filtered
 // search takes 128 rows per SM and 50 us a time, so it wins once several of those fill the GPU (24 576 rows: 156 against
@@ -40,10 +42,9 @@ static_assert(sizeof(KhqCompressSeg) == 16, "ABI");
 // follows row l % R), and the odd multiple of 16 bytes keeps those 16-byte reads on different banks.
 template <int R>
 struct CompressScratchK {
-    float a[R][D + 4];      // x as float, then per-dim |proj| contributions
-    float b[R][D + 4];      // per-dim centroid contributions
-    float q[R][D];          // the rotated projection
-    int incl[R][32];        // per lane: outlier candidates up to and including the lane's dims
+    float q[R][D + 4];      // x as float, then the rotated projection
+    unsigned char in[R][32 + (R > 1 ? 4 : 0)];  // per lane: which of its dims belong to the two conditional sums
+    short incl[R][32];      // per lane: outlier candidates up to and including the lane's dims
     unsigned char oc[64];   // outlier 4-bit codes, by outlier ordinal
     unsigned char os[64];   // outlier sign flags, by outlier ordinal
 };
@@ -106,7 +107,9 @@ __device__ __forceinline__ void compress_rotate(const float (&xv)[8], float norm
 // The three order-sensitive sums of a K row (256 squares, then the two conditional 256-term sums
 // behind the base multiplier) are dependent chains that every lane of the warp would compute
 // alike; with R rows per warp lane l follows row l % R, so one pass over shared memory serves R
-// rows.  Between the passes a row's projection and outlier ordinals wait in shared memory.
+// rows.  Between the passes a row's projection, which of its dims are in the sums (a bit each) and
+// its outlier ordinals wait in shared memory: 1.2 KB a row, so that four rows a warp still leave
+// 32 warps on an SM.  129 024 rows: 251 us with two rows a warp and the terms stored, 227 so.
 template <int R>
 __global__ void __launch_bounds__(CMP_WARPS * 32, 8)
 khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d_vec,
@@ -117,6 +120,7 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
                       const KhqCompressSeg* __restrict__ segs, int rows_per_seg,
                       long long x_byte_offset) {
     __shared__ __align__(16) CompressScratchK<R> scratch[CMP_WARPS];
+    __shared__ __align__(16) float cents2[D];  // the centroid row the base multiplier is fitted to
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     CompressScratchK<R>& S = scratch[warp];
     // The reference computes this factor at run time from the dimension argument.
@@ -130,6 +134,11 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
         const __half* hc = reinterpret_cast<const __half*>(&craw);
 #pragma unroll
         for (int j = 0; j < 8; ++j) cb[j] = __half2float(hc[j]);
+        if (warp == 0) {
+            *reinterpret_cast<float4*>(&cents2[lane * 8]) = make_float4(cb[0], cb[1], cb[2], cb[3]);
+            *reinterpret_cast<float4*>(&cents2[lane * 8 + 4]) = make_float4(cb[4], cb[5], cb[6], cb[7]);
+        }
+        __syncthreads();
     }
 
     for (long long grp = (long long)blockIdx.x * CMP_WARPS + warp; grp < n_groups;
@@ -145,14 +154,14 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
             const __half2* hx = reinterpret_cast<const __half2*>(&raw);
             const float2 x0 = __half22float2(hx[0]), x1 = __half22float2(hx[1]), x2 = __half22float2(hx[2]),
                          x3 = __half22float2(hx[3]);
-            *reinterpret_cast<float4*>(&S.a[r][lane * 8]) = make_float4(x0.x, x0.y, x1.x, x1.y);
-            *reinterpret_cast<float4*>(&S.a[r][lane * 8 + 4]) = make_float4(x2.x, x2.y, x3.x, x3.y);
+            *reinterpret_cast<float4*>(&S.q[r][lane * 8]) = make_float4(x0.x, x0.y, x1.x, x1.y);
+            *reinterpret_cast<float4*>(&S.q[r][lane * 8 + 4]) = make_float4(x2.x, x2.y, x3.x, x3.y);
         }
         __syncwarp();
         float sum_sq = 0.0f;
 #pragma unroll 8
         for (int i = 0; i < D; i += 4) {
-            const float4 t = *reinterpret_cast<const float4*>(&S.a[cr][i]);
+            const float4 t = *reinterpret_cast<const float4*>(&S.q[cr][i]);
             sum_sq = __fmaf_rn(t.x, t.x, sum_sq);
             sum_sq = __fmaf_rn(t.y, t.y, sum_sq);
             sum_sq = __fmaf_rn(t.z, t.z, sum_sq);
@@ -167,8 +176,8 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
             const float norm = sqrtf(__shfl_sync(0xFFFFFFFFu, sum_sq, r) + 1e-8f);
             if (lane == 0) out_norms[row] = __float2half(norm);
             float xv[8], proj[8];
-            *reinterpret_cast<float4*>(&xv[0]) = *reinterpret_cast<const float4*>(&S.a[r][lane * 8]);
-            *reinterpret_cast<float4*>(&xv[4]) = *reinterpret_cast<const float4*>(&S.a[r][lane * 8 + 4]);
+            *reinterpret_cast<float4*>(&xv[0]) = *reinterpret_cast<const float4*>(&S.q[r][lane * 8]);
+            *reinterpret_cast<float4*>(&xv[4]) = *reinterpret_cast<const float4*>(&S.q[r][lane * 8 + 4]);
             compress_rotate(xv, norm, d_vec, rotor, f_s, lane, proj);
             *reinterpret_cast<float4*>(&S.q[r][lane * 8]) = make_float4(proj[0], proj[1], proj[2], proj[3]);
             *reinterpret_cast<float4*>(&S.q[r][lane * 8 + 4]) = make_float4(proj[4], proj[5], proj[6], proj[7]);
@@ -185,17 +194,15 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
                 const int t = __shfl_up_sync(0xFFFFFFFFu, incl, dlt);
                 if (lane >= dlt) incl += t;
             }
-            S.incl[r][lane] = incl;
+            S.incl[r][lane] = (short)incl;
             int ord = incl - cnt;
 
             unsigned sym16 = 0;
-            float cn[8], cc[8];
+            unsigned in = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float pj = proj[j];
                 unsigned sym;
-                cn[j] = 0.0f;
-                cc[j] = 0.0f;
                 if (cand & (1u << j)) {
                     // kept outlier, or overflow outlier (not part of the sums)
                     sym = (ord < MAX_OUT) ? 3u : ((pj > 0.0f) ? 2u : 1u);
@@ -204,15 +211,11 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
                     if (pj > th_lo) sym = 2;
                     else if (pj < -th_lo) sym = 1;
                     else sym = 0;
-                    if (sym != 0) { cn[j] = fabsf(pj); cc[j] = cb[j]; }
+                    if (sym != 0) in |= 1u << j;
                 }
                 sym16 |= sym << (2 * j);
             }
-            // adding +0.0f leaves a non-negative fp32 sum unchanged
-            *reinterpret_cast<float4*>(&S.a[r][lane * 8]) = make_float4(cn[0], cn[1], cn[2], cn[3]);
-            *reinterpret_cast<float4*>(&S.a[r][lane * 8 + 4]) = make_float4(cn[4], cn[5], cn[6], cn[7]);
-            *reinterpret_cast<float4*>(&S.b[r][lane * 8]) = make_float4(cc[0], cc[1], cc[2], cc[3]);
-            *reinterpret_cast<float4*>(&S.b[r][lane * 8 + 4]) = make_float4(cc[4], cc[5], cc[6], cc[7]);
+            S.in[r][lane] = (unsigned char)in;
             // mask word w = dims 16w..16w+15 = lanes 2w (low half) and 2w+1 (high half)
             const unsigned hi16 = __shfl_down_sync(0xFFFFFFFFu, sym16, 1);
             if ((lane & 1) == 0) out_mask[row * 16 + (lane >> 1)] = sym16 | (hi16 << 16);
@@ -220,14 +223,19 @@ khq_compress_k_kernel(const __half* __restrict__ x, const __half* __restrict__ d
         __syncwarp();
         // ---- the two conditional sums in dim order, R rows side by side ------------------------
         float sum_n = 0.0f, sum_c = 0.0f;
-#pragma unroll 8
-        for (int i = 0; i < D; i += 4) {
-            const float4 ta = *reinterpret_cast<const float4*>(&S.a[cr][i]);
-            const float4 tb = *reinterpret_cast<const float4*>(&S.b[cr][i]);
-            sum_n += ta.x; sum_c += tb.x;
-            sum_n += ta.y; sum_c += tb.y;
-            sum_n += ta.z; sum_c += tb.z;
-            sum_n += ta.w; sum_c += tb.w;
+        // (a dim that is not in the sums adds nothing)
+#pragma unroll (R == 1 ? 2 : 1)
+        for (int w = 0; w < 8; ++w) {
+            const unsigned in = *reinterpret_cast<const unsigned*>(&S.in[cr][w * 4]);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(&S.q[cr][w * 32 + i]);
+                const float4 c = *reinterpret_cast<const float4*>(&cents2[w * 32 + i]);
+                if (in & (1u << i)) { sum_n += fabsf(t.x); sum_c += c.x; }
+                if (in & (2u << i)) { sum_n += fabsf(t.y); sum_c += c.y; }
+                if (in & (4u << i)) { sum_n += fabsf(t.z); sum_c += c.z; }
+                if (in & (8u << i)) { sum_n += fabsf(t.w); sum_c += c.w; }
+            }
         }
         float mult_own = (sum_c > 1e-5f) ? __fdiv_rn(sum_n, sum_c) : 1.0f;
         if (mult_own < 0.1f || mult_own > 10.0f || isnan(mult_own)) mult_own = 1.0f;

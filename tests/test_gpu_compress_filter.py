@@ -46,3 +46,29 @@ def test_v_codes_vs_oracle(cuda_ops, oracle, rows, kind):
         w = np.resize(w, (rows, w.shape[1]))
         bad = np.nonzero((g != w).any(axis=1) & finite)[0]
         assert len(bad) == 0, f"{kind}: {name} differs in rows {bad[:8]} ({len(bad)} rows)"
+
+
+@pytest.mark.parametrize("rows", [9471, 9472, 9473, 9475])
+def test_k_rows_vs_oracle(cuda_ops, oracle, rows):
+    """K launches on either side of the line where a warp takes four rows, and with a last group of one to three rows."""
+    import torch
+
+    rng = np.random.default_rng(rows)
+    base = 1201
+    k, v = synth.make_kv(rng, (base + 3) // 4)
+    tb = synth.make_tables(rng, 3, k.reshape(-1, D), v.reshape(-1, D)).as_f16()
+    x = k.reshape(-1, D)[:base].copy()
+    x[17] = 0
+    want = oracle.compress(x, tb["d_k"], tb["rotor_k"], tb["cents_k"], tb["cents_k"].reshape(-1), base, 1.95, 1.0, False)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    out = dict(mask=torch.zeros(rows * 16, dtype=torch.int32, device="cuda"), norms=torch.zeros(rows, dtype=torch.float16, device="cuda"),
+               r_norms=torch.zeros(rows, dtype=torch.float16, device="cuda"), payload=torch.zeros(rows * 40, dtype=torch.uint8, device="cuda"))
+    meta = torch.ones(rows * 4, dtype=torch.uint8, device="cuda")
+    cuda_ops.compress(dev(np.resize(x, (rows, D))), dev(tb["d_k"]), dev(tb["rotor_k"]), dev(tb["cents_k"]), dev(tb["cents_k"]), out["mask"],
+                      out["norms"], out["r_norms"], out["payload"], meta, rows, D, 1.95, 1.0, False)
+    assert not meta.any()
+    for name, got in out.items():
+        g = got.cpu().numpy().view(np.uint8).reshape(rows, -1)
+        w = np.ascontiguousarray(want[name]).view(np.uint8).reshape(base, -1)
+        bad = np.nonzero((g != np.resize(w, (rows, w.shape[1]))).any(axis=1))[0]
+        assert len(bad) == 0, f"{name} differs in rows {bad[:8]} ({len(bad)} rows)"
