@@ -8,14 +8,18 @@
 // A work item = 128 query rows of one query head; key tiles of 128.  A CTA works through one item
 // (long prompts: one CTA per item, left to the hardware scheduler) or through several (short
 // prompts: one persistent CTA per SM; the producers and the MMA thread then run ahead into the
-// next item while the softmax warps finish the epilogue of the current one).  Eleven warps:
+// next item while the softmax warps finish the epilogue of the current one).  Twelve warps:
 //   warps 0-7  softmax, two threads per query row (warp w and warp w+4 share the tensor-memory
 //              lane quarter w%4 and a scheduler): a row's S and O live in tensor-memory lane i,
 //              so there are no shuffles; the two threads of a row take 64 keys of a tile each
 //              and swap their half maxima (and, at the end, half sums) through shared memory.
 //              Per tile a thread reads 64 S columns with tcgen05.ld and writes P (fp16 pairs, 32
 //              columns) back over the S buffer with tcgen05.st; O is rescaled lazily (only when
-//              the running max grew by more than 2^8); the epilogue normalises, gates, stores.
+//              the running max grew by more than 2^8); the epilogue normalises and gates.
+//   warp 11    brings the gates into shared memory in pieces and stores the outputs that take their
+//              place (a softmax thread owns a row: its own global accesses would cost a line each,
+//              16 000 of the 45 000 cycles of an item of 11 tiles; 9 x 1531 rows 386 -> 373 us,
+//              32 x 512: 290 -> 263).
 //   warps 8,10 producers: one thread each issues the TMA loads of Q and the K tiles (warp 8, a
 //              K tile in two halves of 128 head dims, each released as soon as the Q K^T steps
 //              that read it have completed) and of the V tiles (warp 10, two halves of 64 keys,
@@ -60,24 +64,31 @@ constexpr int D = 256;
 constexpr int BR = 128;     // query rows per CTA
 constexpr int BC = 128;     // keys per tile
 constexpr int NSOFT = 256;  // softmax threads: two per query row, 64 of a tile's 128 keys each
-constexpr int NTHREADS = NSOFT + 96;
+constexpr int NTHREADS = NSOFT + 128;
 constexpr int Q_BYTES = BR * D * 2;        // 64 KB
 constexpr int KHALF_BYTES = BC * 128 * 2;  // 32 KB: 128 keys x 128 head dims (two 64-dim groups)
 constexpr int VHALF_BYTES = 64 * D * 2;    // 32 KB: 64 keys x 256 head dims (four 64-dim groups)
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
 constexpr int OFF_V = OFF_K + 2 * KHALF_BYTES;
-constexpr int OFF_XCHG = OFF_V + 2 * VHALF_BYTES;  // float [2 parities][2 halves][128 rows]
+constexpr int STG_BYTES = BR * 64 * 2;     // gate / output piece: 128 rows x 64 columns
+constexpr int OFF_STG = OFF_V + 2 * VHALF_BYTES;
+constexpr int OFF_XCHG = OFF_STG + 2 * STG_BYTES;  // float [2 parities][2 halves][128 rows]
 constexpr int OFF_BARS = OFF_XCHG + 2 * 2 * 128 * 4;
 constexpr int SMEM_BYTES = OFF_BARS + 256;
 constexpr uint32_t TM_COLS = 512, TM_O = 0, TM_S = 256;
+// Up to half a row tile the epilogue reads gates and writes outputs straight from and to global memory: its lines (one per thread)
+// are few then, and the pieces through shared memory one after the other take longer (one prompt of 57 rows: 10.3 us against
+// 11.2; of 128 rows 12.8 against 11.4).
+constexpr int DIRECT_MAX_T = BR / 2;
 constexpr float RESCALE_LOG2 = 8.0f;
 
 enum Bar {
     B_KFULL = 0, B_VFULL = 2, B_KEMPTY = 4, B_VEMPTY = 6, B_SFULL = 8, B_QFULL = 10, B_PREADY = 11, B_PVDONE = 12,
-    B_XCHG = 14, B_QEMPTY = 18, B_OFREE = 19, B_PREADY2 = 20, B_COUNT = 21
+    B_XCHG = 14, B_QEMPTY = 18, B_OFREE = 19, B_PREADY2 = 20, B_GFULL = 21, B_OUT = 23,
+    B_COUNT = 25
 };
-static_assert(B_COUNT * 8 <= 192, "barriers overlap the tensor-memory slot");
+static_assert(B_COUNT * 8 <= 240, "barriers overlap the tensor-memory slot");
 
 __device__ int g_prefill_status = 0;
 
@@ -178,6 +189,13 @@ __device__ __forceinline__ float ex2_approx(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// 1 / (1 + e^-x): four instructions, two of them approximations of 2^-22 relative error; subnormal terms are below the sum's rounding
+// (and below 2^-126 of the result).
+__device__ __forceinline__ float sigmoid(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.0f + ex2_approx(x * -1.4426950408889634f)));
+    return y;
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -191,6 +209,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// A piece of the gates to L2; a piece of the outputs from shared memory.
+__device__ __forceinline__ void tma_prefetch_5d(const CUtensorMap* map, int c1, int c2, int c3, int c4) {
+    asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global.tile [%0, {%1, %2, %3, %4, %5}];" ::"l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* map, uint32_t src, int c1, int c2, int c3, int c4) {
+    asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(src), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 
 // One 5-D tiled TMA load of a single CTA; coordinate 0 is always 0, so the 16-byte rule holds.
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c1, int c2,
@@ -238,6 +270,19 @@ __device__ __forceinline__ bool mbar_wait_all_bounded(uint64_t* const (&bar)[N],
     }
     atomicExch(status, 1);
     return false;
+}
+
+// Eight columns: O normalised, times the sigmoids of the gates g, as 16-bit values.
+template <bool BF16>
+__device__ __forceinline__ uint4 gated(const uint32_t* o, float inv, const uint4& g) {
+    const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+    uint32_t ow[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 gf = unpack2<BF16>(gw[e]);
+        ow[e] = pack2<BF16>(__uint_as_float(o[2 * e]) * inv * sigmoid(gf.x), __uint_as_float(o[2 * e + 1]) * inv * sigmoid(gf.y));
+    }
+    return make_uint4(ow[0], ow[1], ow[2], ow[3]);
 }
 
 // ---- the kernel ----------------------------------------------------------------------------------
@@ -288,12 +333,14 @@ __device__ __forceinline__ bool get_item(int ordinal, int T, int H_q, int H_kv, 
 template <bool PERSIST, bool BF16>
 __global__ void __launch_bounds__(NTHREADS, 1)
 khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                           const __grid_constant__ CUtensorMap tm_v, const __half* __restrict__ q_gate,
-                           __half* __restrict__ out, int T, int H_q, int H_kv, int batch, int group_major,
-                           float scale_log2e, long long q_bs, long long o_bs) {
+                           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
+                           const __grid_constant__ CUtensorMap tm_o, const __half* __restrict__ q_gate,
+                           __half* __restrict__ out, long long q_bs, long long o_bs, int T, int H_q, int H_kv, int batch, int group_major,
+                           float scale_log2e) {
+    const bool direct = !PERSIST && T <= DIRECT_MAX_T;  // gates and outputs without shared memory
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BARS + 192);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BARS + 240);
     float* xchg = reinterpret_cast<float*>(smem + OFF_XCHG);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int* status = &g_prefill_status;
@@ -321,6 +368,10 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         khq::mbar_init(&bars[B_PREADY], NSOFT / 32);
         khq::mbar_init(&bars[B_PREADY2], NSOFT / 32);
         khq::mbar_init(&bars[B_OFREE], NSOFT / 32);
+        for (int q = 0; q < 2; ++q) {
+            khq::mbar_init(&bars[B_GFULL + q], 1);
+            khq::mbar_init(&bars[B_OUT + q], NSOFT / 32);
+        }
         for (int q = 0; q < 4; ++q) khq::mbar_init(&bars[B_XCHG + q], 2);  // the two warps of a lane quarter
         khq::fence_barrier_init();
     }
@@ -471,22 +522,55 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 have = have_nx;
             }
         }
+    } else if (warp == 11) {
+        // ================================ gates in, outputs out =====================================
+        // Four pieces of 64 columns per item through two buffers: the gates of a piece come in, the softmax warps overwrite them
+        // with the outputs, the piece is stored and the buffer takes the piece after the next (of the next item, too).
+        if (lane == 0 && !direct) {
+            Item in, st;
+            int i_in = 0, c_in = 0, loads = 0, n = 0;
+            bool more = get_item<PERSIST>(0, T, H_q, H_kv, batch, group_major, in), ok = true;
+            const auto load_next = [&]() {
+                if (!more) return;
+                const int b = loads & 1;
+                khq::mbar_arrive_expect_tx(&bars[B_GFULL + b], STG_BYTES);
+                tma_load_5d(sbase + OFF_STG + b * STG_BYTES, &tm_g, &bars[B_GFULL + b], in.q0, c_in, in.h, in.b);
+                if (c_in < 2) tma_prefetch_5d(&tm_g, in.q0, c_in + 2, in.h, in.b);
+                ++loads;
+                if (++c_in == 4) {
+                    c_in = 0;
+                    more = get_item<PERSIST>(++i_in, T, H_q, H_kv, batch, group_major, in);
+                }
+            };
+            load_next();
+            load_next();
+            for (int i = 0; ok && get_item<PERSIST>(i, T, H_q, H_kv, batch, group_major, st); ++i) {
+                for (int c = 0; c < 4; ++c, ++n) {
+                    ok = khq::mbar_wait_bounded(&bars[B_OUT + (n & 1)], (uint32_t)((n >> 1) & 1), status);
+                    if (!ok) break;
+                    tma_store_5d(&tm_o, sbase + OFF_STG + (n & 1) * STG_BYTES, st.q0, c, st.h, st.b);
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    load_next();
+                }
+            }
+            // nothing this thread started may still be in flight when the CTA leaves
+            for (int k = max(0, loads - 2); k < loads; ++k)
+                khq::mbar_wait_bounded(&bars[B_GFULL + (k & 1)], (uint32_t)((k >> 1) & 1), status);
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
     } else {
         // ================================ softmax + epilogue ======================================
         // Two threads per query row: half 0 (warps 0-3) takes keys 0-63 of a tile and columns 0-127
         // of O, half 1 (warps 4-7) keys 64-127 and columns 128-255.  Both warps of a row sit on the
         // same tensor-memory lane quarter (warp % 4) and on the same scheduler.
         const int half = warp >> 2, r = tid & 127;
-        const long long q_row = (long long)H_q * 2 * D, o_row = (long long)H_q * D;
         const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         uint64_t* xbar = &bars[B_XCHG + (warp & 3)];
-        int g = 0, x = 0;  // running tile index; running phase of the exchange barrier
+        int g = 0, x = 0, n = 0;  // running tile index; running phase of the exchange barrier; running epilogue piece
         bool ok = true;
         Item it;
         for (int i = 0; ok && get_item<PERSIST>(i, T, H_q, H_kv, batch, group_major, it); ++i) {
             const int q0 = it.q0, row = q0 + r;
-            const bool live = row < T;
-            const __half* qrow = q_gate + it.b * q_bs + (long long)(live ? row : 0) * q_row + (long long)it.h * 2 * D;
             float m_used = -1e30f, l_run = 0.0f;
             for (int j = 0; j < it.n_tiles; ++j, ++g, ++x) {
                 ok = __all_sync(0xFFFFFFFFu, khq::mbar_wait_bounded(&bars[B_SFULL + (g & 1)], (uint32_t)((g >> 1) & 1), status));
@@ -567,12 +651,13 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             }
             if (!ok) break;
             // ---- epilogue of the item -------------------------------------------------------------
-            // this thread's 128 gate values: all sixteen 16-byte loads go out together, ahead of the
-            // final waits (issued one per use they cost a full memory latency each)
-            const __half* gate = qrow + D + half * 128;
-            uint4 g4[16];
+            const bool live = row < T;
+            uint4 g4[PERSIST ? 1 : 16];  // direct: this thread's 128 gate values, all loads ahead of the final waits
+            if (!PERSIST && direct && live) {
+                const __half* gate = q_gate + it.b * q_bs + (long long)row * H_q * 2 * D + (long long)it.h * 2 * D + D + half * 128;
 #pragma unroll
-            for (int q = 0; q < 16; ++q) g4[q] = live ? __ldg(reinterpret_cast<const uint4*>(gate) + q) : make_uint4(0u, 0u, 0u, 0u);
+                for (int q = 0; q < (PERSIST ? 1 : 16); ++q) g4[q] = __ldg(reinterpret_cast<const uint4*>(gate) + q);
+            }
             // row sum over both halves (one more phase of the exchange barrier)
             xchg[((x & 1) * 2 + half) * 128 + r] = l_run;
             __syncwarp();
@@ -585,34 +670,47 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             if (!ok) break;
             tc_fence_after();
             const float inv = 1.0f / (l_run + 1e-9f);
-            __half* op = out + it.b * o_bs + (long long)(live ? row : 0) * o_row + (long long)it.h * D + half * 128;
+            if constexpr (!PERSIST) {
+                if (direct) {
+                    __half* op = out + it.b * o_bs + (long long)(live ? row : 0) * H_q * D + (long long)it.h * D + half * 128;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t orr[32];
+                        tmem_ld32(lane_base + TM_O + half * 128 + c * 32, orr);
+                        tmem_ld_wait();
+                        if (live) {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                *reinterpret_cast<uint4*>(op + c * 32 + q * 8) = gated<BF16>(orr + 8 * q, inv, g4[c * 4 + q]);
+                        }
+                    }
+                    break;
+                }
+            }
+            // Pieces of 64 columns, 32 per thread.  Gates and outputs pass through shared memory (128-byte swizzle, free of bank
+            // conflicts) and TMA: a thread owns a row, so its own global accesses would take a line each (16 400 cycles per
+            // item for 64 KB in and 64 KB out).
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c, ++n) {
                 uint32_t orr[32];
-                tmem_ld32(lane_base + TM_O + half * 128 + c * 32, orr);
+                tmem_ld32(lane_base + TM_O + c * 64 + half * 32, orr);
+                ok = __all_sync(0xFFFFFFFFu, khq::mbar_wait_bounded(&bars[B_GFULL + (n & 1)], (uint32_t)((n >> 1) & 1), status));
                 tmem_ld_wait();
+                if (!ok) break;
                 if (PERSIST && c == 3) {  // O has been read: the next item's first P V may overwrite it
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) khq::mbar_arrive(&bars[B_OFREE]);
                 }
-                if (live) {
+                unsigned char* const prow = smem + OFF_STG + (n & 1) * STG_BYTES + r * 128;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint4 gq = g4[c * 4 + q];
-                        const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-                        uint32_t ow[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 gf = unpack2<BF16>(gw[e]);
-                            const float g0 = gf.x, g1 = gf.y;
-                            const float x0 = __uint_as_float(orr[q * 8 + 2 * e]) * inv * __fdividef(1.0f, 1.0f + __expf(-g0));
-                            const float x1 = __uint_as_float(orr[q * 8 + 2 * e + 1]) * inv * __fdividef(1.0f, 1.0f + __expf(-g1));
-                            ow[e] = pack2<BF16>(x0, x1);
-                        }
-                        *reinterpret_cast<uint4*>(op + c * 32 + q * 8) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-                    }
+                for (int q = 0; q < 4; ++q) {
+                    uint4* const at = reinterpret_cast<uint4*>(prow + (((half * 4 + q) ^ (r & 7)) << 4));
+                    *at = gated<BF16>(orr + 8 * q, inv, *at);
                 }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) khq::mbar_arrive(&bars[B_OUT + (n & 1)]);
             }
         }
     }
@@ -691,10 +789,12 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     for (const void* p : ptrs)
         if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return -104;
     if (batch > 1 && ((q_batch_stride | kv_batch_stride | out_batch_stride) & 7) != 0) return -104;
-    CUtensorMap mq, mk, mv;
+    CUtensorMap mq, mk, mv, mg, mo;
     int rc = make_map(&mq, q_gate, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 4, bf16);
     if (rc == 0) rc = make_map(&mk, k, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, BC, 2, bf16);
     if (rc == 0) rc = make_map(&mv, v, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, 64, 4, bf16);
+    if (rc == 0) rc = make_map(&mg, static_cast<const __half*>(q_gate) + D, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 1, bf16);
+    if (rc == 0) rc = make_map(&mo, out, T, H_q, batch, (long long)H_q * D, D, out_batch_stride, BR, 1, bf16);
     if (rc != 0) return rc;
     static bool attr_done[64] = {};
     static int sm_count[64] = {};
@@ -746,8 +846,8 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     __half* op = static_cast<__half*>(out);
     const float sl2 = scale * 1.4426950408889634f;
 #define KHQ_TC5_LAUNCH(PERSIST, BF16)                                                                                  \
-    err = khq::launch_pdl(khq_gqa_prefill_tc5_kernel<PERSIST, BF16>, grid, 0, SMEM_BYTES, stream, (unsigned)NTHREADS, mq, mk, mv, qp, op, \
-                          T, H_q, H_kv, batch, group_major, sl2, q_batch_stride, out_batch_stride)
+    err = khq::launch_pdl(khq_gqa_prefill_tc5_kernel<PERSIST, BF16>, grid, 0, SMEM_BYTES, stream, (unsigned)NTHREADS, mq, mk, mv, mg, mo, qp, op, \
+                          q_batch_stride, out_batch_stride, T, H_q, H_kv, batch, group_major, sl2)
     if (ctas == items) {
         if (bf16) KHQ_TC5_LAUNCH(false, true);
         else KHQ_TC5_LAUNCH(false, false);
