@@ -1347,22 +1347,34 @@ static int plan_sm_count() {
 
 // ---- host planner -----------------------------------------------------------------------------
 // The CTAs of the persistent kernels pull items off one counter in array order, so a plan is judged
-// by the makespan of list scheduling on `sms` workers.  Costs are in compressed-token units: one
-// per compressed token, PLAN_WINDOW_COST per raw-window token (4 KB of fp16 against 880 B),
-// PLAN_ITEM_COST per item (query set-up, partial record).
+// by the makespan of list scheduling on `sms` workers, in units of 61 ns (half a compressed token).  Measured on
+// launches of 148 equal items: 6.1 us per round of 48 tokens (each of the three groups one block of 16), 3.7 us for a last round
+// of one block and 4.9 of two, 9.2 us per item (query set-up, records, their merge); a raw window takes 0.18 us a
+// token and 12 us an item when its rows come from HBM.
 #include <algorithm>
 #include <functional>
 #include <queue>
 #include <vector>
 
 namespace {
-constexpr int PLAN_WINDOW_COST = 3, PLAN_ITEM_COST = 56;  // measured: 0.25 us per compressed token, 0.75 us per window token, 14 us per item
+constexpr int PLAN_ROUND = 48;        // compressed tokens
+constexpr int PLAN_WINDOW_TOKENS = 3;  // a window is cut so that its pieces stay below a third of a compressed piece, in tokens
+long long plan_cost(int kind, int n) {
+    if (kind) return 200 + 3LL * n;
+    const int r = n % PLAN_ROUND;
+    return 150 + 2LL * (n - r) + (r ? 60 + r * 36 / PLAN_ROUND : 0);
+}
+
+struct PlanPiece {
+    int problem, lo, hi;
+};
 
 struct PlanRule {
-    int kind;   // 0: guided self-scheduling (cap, floor), windows whole; 1: piece counts per problem (pieces, win_pieces)
+    int kind;   // 0: guided self-scheduling (cap, floor), windows whole; 1: piece counts per problem (pieces, win_pieces); 2: a list
     int cap, floor_;
     const std::vector<int>* pieces;
     const std::vector<int>* win_pieces;
+    const std::vector<PlanPiece>* list = nullptr;
 };
 
 // Walks the items of a plan in launch order: fn(problem, kind, lo, hi).
@@ -1374,9 +1386,13 @@ void plan_walk(const PlanRule& rule, const int* c_len, const int* win_len, int n
     for (int i = 0; i < n_desc; ++i) {
         const int wl = win_len[i];
         if (wl <= 0) continue;
-        const int wp = rule.kind == 1 ? (*rule.win_pieces)[i] : 1;
+        const int wp = rule.win_pieces ? (*rule.win_pieces)[i] : 1;
         const int per = (wl + wp - 1) / wp;
         for (int lo = 0; lo < wl; lo += per) fn(i, 1, lo, lo + per < wl ? lo + per : wl);
+    }
+    if (rule.kind == 2) {
+        for (const PlanPiece& p : *rule.list) fn(p.problem, 0, p.lo, p.hi);
+        return;
     }
     for (int i = 0; i < n_desc; ++i) {
         const int cl = c_len[i] > 0 ? c_len[i] : 0;
@@ -1407,7 +1423,7 @@ long long plan_makespan(const PlanRule& rule, const int* c_len, const int* win_l
     for (int w = 0; w < sms; ++w) free_at.push(0);
     long long end = 0;
     plan_walk(rule, c_len, win_len, n_desc, sms, [&](int, int kind, int lo, int hi) {
-        const long long t = free_at.top() + (long long)(hi - lo) * (kind ? PLAN_WINDOW_COST : 1) + PLAN_ITEM_COST;
+        const long long t = free_at.top() + plan_cost(kind, hi - lo);
         free_at.pop();
         free_at.push(t);
         if (t > end) end = t;
@@ -1437,11 +1453,41 @@ bool plan_even_pieces(const int* c_len, int n_desc, int total, int max_piece, st
     }
     return largest.top().first <= (double)max_piece;
 }
+
+// Pieces that fill every worker up to `limit`: the worker that is free first takes as many whole rounds of the problem at hand as fit
+// (it is the one the kernel's counter serves next), the rest of the problem goes to the next worker, and a worker that a
+// problem's end left with time takes the first piece of a later one.  False: the tokens do not fit.
+bool plan_fill(const int* c_len, const int* win_len, const std::vector<int>& win_pieces, int n_desc, int sms, int max_piece, long long limit,
+               std::vector<PlanPiece>& list) {
+    list.clear();
+    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
+    for (int w = 0; w < sms; ++w) free_at.push(0);
+    const PlanRule windows = {2, 0, 0, nullptr, &win_pieces, &list};  // (the list is empty)
+    plan_walk(windows, c_len, win_len, n_desc, sms, [&](int, int kind, int lo, int hi) {
+        const long long t = free_at.top() + plan_cost(kind, hi - lo);
+        free_at.pop();
+        free_at.push(t);
+    });
+    for (int i = 0; i < n_desc; ++i)
+        for (int lo = 0, left = c_len[i]; left > 0;) {
+            const long long t = free_at.top();
+            long long size = (limit - t - plan_cost(0, 0)) / 2 / PLAN_ROUND * PLAN_ROUND;
+            if (size > max_piece) size = max_piece / PLAN_ROUND * PLAN_ROUND;
+            if (left <= size + PLAN_ROUND / 2) size = left;  // a short rest joins the piece
+            else if (size < 2 * PLAN_ROUND) return false;    // not worth an item
+            list.push_back({i, lo, lo + (int)size});
+            free_at.pop();
+            free_at.push(t + plan_cost(0, (int)size));
+            lo += (int)size;
+            left -= (int)size;
+        }
+    return true;
+}
 }  // namespace
 
-// Cuts every problem into one item for its raw window and items of its compressed region.  Candidates: guided self-scheduling with a 96- or a 48-token floor, and one, two or three
+// Cuts every problem into one item for its raw window and items of its compressed region.  Candidates: guided self-scheduling with a 96- or a 48-token floor, one, two or three
 // waves of equal pieces (a launch small enough that every CTA gets one to three pieces is balanced
-// best by exactly that); the one with the shortest simulated makespan is written out.
+// best by exactly that), and pieces that fill every worker; the one with the shortest simulated makespan is written out.
 extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_desc, int tokens_per_item,
                                     void* items_out, int max_items, int* first_slot, int* n_slots) {
     if (n_desc < 0 || !c_len || !win_len) return -100;
@@ -1458,6 +1504,7 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
     tokens_per_item = ((tokens_per_item + 95) / 96) * 96;  // a multiple of every generation's staging tile (24, 32 tokens)
 
     std::vector<int> pieces[3], win_pieces[3];
+    std::vector<PlanPiece> filled;
     PlanRule best = {0, tokens_per_item, 96, nullptr, nullptr};
     // A launch of many waves is planned by the guided rule as it stands (its tail is a fraction of a percent);
     // smaller ones compare the candidates.
@@ -1474,7 +1521,7 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
         // an explicit tokens_per_item stays an upper bound on every piece
         const int max_piece = auto_size ? 8256 : tokens_per_item;
         long long work = total;
-        for (int i = 0; i < n_desc; ++i) work += (long long)PLAN_WINDOW_COST * (win_len[i] > 0 ? win_len[i] : 0);
+        for (int i = 0; i < n_desc; ++i) work += (long long)PLAN_WINDOW_TOKENS * (win_len[i] > 0 ? win_len[i] : 0);
         for (int k = 1; k <= 3; ++k) {
             // k items per SM of about work / (k x SMs) each: a raw window that costs more than that is cut too
             const long long target = std::max<long long>(work / ((long long)k * sms), 48);
@@ -1483,13 +1530,28 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
             int n_win = 0;
             for (int i = 0; i < n_desc; ++i)
                 if (win_len[i] > 0) {
-                    long long c = ((long long)PLAN_WINDOW_COST * win_len[i] + target / 2) / target;
+                    long long c = ((long long)PLAN_WINDOW_TOKENS * win_len[i] + target / 2) / target;
                     c = std::min<long long>(std::max<long long>(c, 1), std::max(win_len[i] / 16, 1));
                     wp[i] = (int)c;
                     n_win += (int)c;
                 }
             if (plan_even_pieces(c_len, n_desc, k * sms - n_win, max_piece, pieces[k - 1]))
                 consider(PlanRule{1, 0, 0, &pieces[k - 1], &wp});
+        }
+        // Filled workers: some 1.2 items per SM instead of the guided rule's six, or of equal pieces of which the workers that took the
+        // windows have one less.  Not for launches whose guided items are at the cap (2 x 8192 tokens per SM, 2 ms): their
+        // small last items also even out what the SMs differ by, and cost little there.
+        if (total < 2LL * sms * 8192) {
+            long long cost = 0;
+            plan_walk(PlanRule{2, 0, 0, nullptr, &win_pieces[0], &filled}, c_len, win_len, n_desc, sms,
+                      [&](int, int kind, int lo, int hi) { cost += plan_cost(kind, hi - lo); });
+            for (int i = 0; i < n_desc; ++i) cost += c_len[i] > 0 ? plan_cost(0, c_len[i]) : 0;
+            const long long least = cost / sms + plan_cost(0, 0);
+            for (int step = 0; step < 8; ++step)  // 1.5 % more each time
+                if (plan_fill(c_len, win_len, win_pieces[0], n_desc, sms, max_piece, least + least * step * 3 / 200, filled)) {
+                    consider(PlanRule{2, 0, 0, nullptr, &win_pieces[0], &filled});
+                    break;
+                }
         }
     }
 
@@ -1520,6 +1582,14 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
     return n;  // > max_items means the items buffer was too small
 }
 
+// The item counter of a persistent launch.  A kernel, because a memset between two kernels keeps the launch of the second one from
+// overlapping the end of the first.
+__global__ void khq_zero_counter_kernel(int* counter) {
+    pdl_wait();
+    pdl_trigger();
+    if (threadIdx.x == 0) *counter = 0;
+}
+
 static int decode_batched_impl(const void* descs, const void* tables, const void* items, int n_desc, int n_items,
                                void* workspace, size_t workspace_bytes, int n_slots_total, float scale, float rope_base,
                                int ring_cap, int codebook_in_smem, float* out_partials, const void* images, cudaStream_t stream) {
@@ -1533,7 +1603,7 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
     const int grid = n_items < sm_count() ? n_items : sm_count();
     const bool vqs = codebook_in_smem != 0, mma = codebook_in_smem == 2 || codebook_in_smem < 0;
     if (!mma || n_items > grid) {  // the default kernel takes its first item without the counter
-        err = cudaMemsetAsync(workspace, 0, 256, stream);
+        err = launch_pdl(khq_zero_counter_kernel, 1, 0, 0, stream, 32u, counter);
         if (err != cudaSuccess) return static_cast<int>(err);
     }
     if (codebook_in_smem == 4)

@@ -94,3 +94,23 @@ def test_small_launch_cuts_the_raw_window_too():
     win = items[items["kind"] == 1]
     comp = items[items["kind"] == 0]
     assert len(win) >= 3 and (win["hi"] - win["lo"]).max() * 3 <= (comp["hi"] - comp["lo"]).max() + 24
+
+
+@pytest.mark.parametrize("n,lo,hi", [(2, 3000, 9000), (32, 1024, 16384), (96, 128, 4000), (148, 1000, 16000)])
+def test_launches_of_a_few_items_per_sm_fill_every_sm(n, lo, hi):
+    rng = np.random.default_rng(n)
+    ctx = rng.integers(lo, hi, size=n)
+    c_len = np.maximum((ctx - 128) // 128 * 128, 0).astype(np.int32)
+    win_len = (ctx - c_len).astype(np.int32)
+    items, first, cnt = batched.plan(c_len, win_len, 0)
+    _check_cover(items, first, cnt, c_len, win_len)
+
+    def cost(it):  # microseconds, see the planner
+        n = int(it["hi"] - it["lo"])
+        return 12.2 + 0.183 * n if it["kind"] else 9.2 + 0.122 * n
+
+    free = [0.0] * 148
+    for it in items:
+        heapq.heappush(free, heapq.heappop(free) + cost(it))
+    least = (0.122 * c_len.sum() + (12.2 + 0.183 * win_len).sum()) / 148 + 9.2
+    assert max(free) <= 1.1 * least + 12.0
