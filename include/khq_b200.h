@@ -177,8 +177,8 @@ size_t khq_b200_decode_workspace_bytes(int n_slots_total);
  * codebook staged in shared memory / gathered from global memory, 2 = warp-level tensor-core kernel
  * (mma.sync), 3 = tcgen05 kernel (tensor-memory accumulators, code words decoded one payload row
  * per thread), 4 = the same formulation run by 32 light warps (two mask words or two patches per
- * thread, CTA-wide step barriers), -1 let the library choose.  Allocates nothing; the only non-kernel call is a 256-byte
- * cudaMemsetAsync on `stream`.  Returns -100 (empty/NULL arguments), -104 (alignment), -105
+ * thread, CTA-wide step barriers), -1 let the library choose.  Allocates nothing, makes no call
+ * but kernel launches on `stream`.  Returns -100 (empty/NULL arguments), -104 (alignment), -105
  * (workspace too small). */
 int launch_khq_decode_batched_fp16(const void* descs, const void* tables, const void* items, int n_desc,
                                    int n_items, void* workspace, size_t workspace_bytes,
