@@ -25,10 +25,14 @@ constexpr int CMP_VROWS = 4;  // V rows of a CTA whose warps share the code sear
 // 38.8).  Eight rows a warp cost more in occupancy than their shared sums save (129 024 rows: 259 against 227 us).
 constexpr long long CMP_KROWS_MIN_N = 9472;
 // V launches.  Up to two CTAs of four rows per SM (148 x 2 x 4 rows) the length of one CTA is what counts: 16 warps (512 rows:
-// 9.2 us, 11.1 with 8 warps).  Above, 8 warps overlap more of the unshared work (8192 rows: 59 us, 66 with 16).  The filtered
-// search takes 128 rows per SM and 50 us a time, so it wins once several of those fill the GPU (24 576 rows: 156 against
-// 163 us, 65 536: 338 against 430).
-constexpr int CMP_V16_MAX_N = 1184, CMP_VMMA_MIN_N = 24576;
+// 9.2 us, 11.1 with 8 warps).  Above, 8 warps overlap more of the unshared work (8192 rows: 59 us, 66 with 16), 6.6 us per 1000
+// rows.  The filtered search takes 64 rows per CTA, two CTAs per SM, and 50 us for each time that 148 x 64 rows are begun (61 the
+// first time), so it wins where that is less: from 8485 rows, except just behind a multiple of 9472 up to 29 500 rows.
+constexpr int CMP_V16_MAX_N = 1184;
+inline bool compress_v_filtered(long long n) {
+    const long long waves = (n + 148 * 64 - 1) / (148 * 64);
+    return (waves > 1 ? 50000 * waves : 61000) < 5000 + 33 * n / 5;  // ns
+}
 
 // One run of rows of a batched launch: source rows (fp16, D per row, contiguous) and the first
 // output row in the launch's output arrays (mirrored in include/khq_b200.h).
@@ -573,15 +577,15 @@ khq_compress_v_kernel(const __half* __restrict__ x, const __half* __restrict__ d
 //     k   0..2 vh ch   3: 64 n1   4..6 vl ch   7: 64 n2   8..10 vh cl   11: 64 n3   12..15: 0.
 // Each omitted or rounded term is below 2^-22 of its factors and the fp32 accumulation of twelve terms below 2^-19 of their
 // magnitude B = V^2 + 2 V cm + 3 cm^2 (V = |v0| + |v1| + |v2|, cm = largest |a c_k| of the patch), which also bounds what the
-// reference's own fp32 evaluation is off (3 x 2^-24 of a distance <= B).  If exactly one code lies within 2^-16 B of the
-// smallest approximation it is the reference's choice; every other (row, patch) goes through the exact search
-// (v_search_row).  So the code words stay bit-identical.
+// reference's own fp32 evaluation is off (3 x 2^-24 of a distance <= B).  Two values are so off by less than 2^-17 B against
+// each other; if exactly one code lies within that of the smallest approximation it is the reference's choice, and every other
+// (row, patch) goes through the exact search (v_search_row) behind the steps.  So the code words stay bit-identical.
 //
 // CTA = four groups of two warps; a group owns 16 rows (one M tile), its warps search patches 0..31 and 32..63 and share the
 // rows in front and behind.  The B fragments of a patch (8 KB) are built once per CTA and step by all threads, double
 // buffered.  A thread holds 2 rows x 32 codes of a half patch: minimum by three-input min, then the sign bits of (value -
 // minimum - margin) shifted into a mask.  44 warp instructions per (row, patch) against 85 of the exact search, about two per
-// cycle; 0.9 % of the pairs are redone.  129 024 rows: 800 -> 657 us.
+// cycle; 0.5 % of the pairs are redone.  129 024 rows: 800 -> 636 us.
 constexpr int VM_ROWS = 16;  // rows per group
 constexpr int VM_GROUPS = 4;   // per CTA; eight halve the building of fragments but not the time (694 us)
 struct CompressScratchVM {
@@ -589,7 +593,9 @@ struct CompressScratchVM {
     uint4 b[2][2][256 * 2];                // [buffer][half][code]: k pairs of lanes t = 0..3 (b0, b1 each)
     float cm[2][2][8];                     // largest |a c_k| per warp's share of a patch
     unsigned short code[VM_GROUPS * VM_ROWS][NP];
+    alignas(16) unsigned undecided[NP][VM_GROUPS];  // rows of a group that need the exact search, bit 4 g + y: row g + 8 y
 };
+static_assert(2 * (sizeof(CompressScratchVM) + 1024) <= 228 * 1024, "two CTAs per SM");
 
 __device__ __forceinline__ uint32_t vm_pack(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
@@ -717,7 +723,7 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
         for (int y = 0; y < 2; ++y) {
             const float4 v = *reinterpret_cast<const float4*>(&S.p[m_row + g + 8 * y][patch * 4]);
             const float V = fabsf(v.x) + fabsf(v.y) + fabsf(v.z);
-            thr[y] = fmaf(V, fmaf(2.0f, cm, V), 3.0f * cm * cm) * 0.0009765625f;  // 64 x 2^-16 x B
+            thr[y] = fmaf(V, fmaf(2.0f, cm, V), 3.0f * cm * cm) * 0.00048828125f;  // 64 x 2^-17 x B
             safe[y] = V < 500.0f && cm < 200.0f;  // nothing overflows fp16; false for NaN
             const float e0 = 64.0f * ((t & 1) ? v.z : v.x), e1 = (t & 1) ? 64.0f : 64.0f * v.y;
             const uint32_t hi = vm_pack(e0, e1);
@@ -791,20 +797,29 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
             if (t == 0 && one) S.code[m_row + g + 8 * y][patch] = (unsigned short)(mine & 0xFFFFu);
             redo |= __ballot_sync(0xFFFFFFFFu, t == 0 && !one) << y;  // bit 4 g + y: row g + 8 y
         }
-        if (redo) {
-            const unsigned long long nalpha2 = f2_pack(-alpha, -alpha);
-            unsigned long long cc[3][4];
-            v_load_codes(vq, patch, lane, cc);
-#pragma unroll 1
-            while (redo) {
-                const int k = __ffs((int)redo) - 1, r = m_row + (k >> 2) + 8 * (k & 3);
-                redo &= redo - 1;
-                v_search_row(S.p[r], S.code[r], patch, cc, nalpha2, lane);
-            }
-        }
+        if (lane == 0) S.undecided[patch][grp] = redo;
         if (step + 1 < NP / 2) build(buf ^ 1);
         __syncthreads();
     }
+    // ---- exact search of the undecided pairs, a patch per warp: within the steps it held up the other seven warps -----------
+#pragma unroll 1
+    for (int p = warp; p < NP; p += VM_GROUPS * 2) {
+        const uint4 u = *reinterpret_cast<const uint4*>(S.undecided[p]);
+        if ((u.x | u.y | u.z | u.w) == 0u) continue;
+        const unsigned long long nalpha2 = f2_pack(-alpha, -alpha);
+        unsigned long long cc[3][4];
+        v_load_codes(vq, p, lane, cc);
+#pragma unroll 1
+        for (int gr = 0; gr < VM_GROUPS; ++gr) {
+            unsigned redo = S.undecided[p][gr];
+            while (redo) {
+                const int k = __ffs((int)redo) - 1, r = gr * VM_ROWS + (k >> 2) + 8 * (k & 3);
+                redo &= redo - 1;
+                v_search_row(S.p[r], S.code[r], p, cc, nalpha2, lane);
+            }
+        }
+    }
+    __syncthreads();
     // ---- per row: energies, dim-3 centroid choice, residual, packing ------------------------------
 #pragma unroll 1
     for (int r = 0; r < nr; ++r) {
@@ -884,7 +899,7 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
         khq_compress_k_kernel<1><<<grid(n), CMP_WARPS * 32, 0, stream>>>(
             x, dv, ro, ce, static_cast<unsigned int*>(out_mask), on, orn, op, om, d, n, threshold_scale, segs,
             rows_per_seg, x_byte_offset);
-    } else if (n >= CMP_VMMA_MIN_N) {
+    } else if (compress_v_filtered(n)) {
         const int rc = launch_v_mma(x, dv, ro, ce, vq_centroids, on, orn, op, om, d, n, alpha, segs, rows_per_seg, x_byte_offset, stream);
         if (rc != 0) return rc;
     } else {

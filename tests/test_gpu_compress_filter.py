@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 D = 256
 
 
-@pytest.mark.parametrize("rows,kind", [(3, "plain"), (1184, "near"), (1185, "ties"), (24575, "plain"), (24576, "plain"), (24577, "ties"),
-                                       (24639, "near"), (24641, "wide"), (25000, "odd_rows")])
+@pytest.mark.parametrize("rows,kind", [(3, "plain"), (1184, "near"), (1185, "ties"), (8484, "plain"), (8485, "plain"), (9472, "ties"),
+                                       (9473, "near"), (24641, "wide"), (25000, "odd_rows"), (28417, "ties")])
 def test_v_codes_vs_oracle(cuda_ops, oracle, rows, kind):
     import torch
 
