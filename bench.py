@@ -1118,14 +1118,14 @@ def main():
                     "covers": "per sequence and layer: pinned-host copies of q_gate/K/V, batched pre-step (norm, K capture, RoPE, "
                               "ring appends), batched compression of the sequences whose window reached 256 (%d events in the "
                               "timed steps), re-planned batched attention, copy of the gated output to pinned host memory" % n_events},
-            "gpu_launches": 2 * len(launch_ms),
-            "gpu_launches_e2e_per_step": "per layer: 1 pre-step + 2 compress (steps with events) + 2 attention; + 1 descriptor update",
+            "gpu_launches": 3 * len(launch_ms),
+            "gpu_launches_e2e_per_step": "per layer: 1 pre-step + 2 compress (steps with events) + 3 attention; + 1 descriptor update",
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s",
                          "frac": achieved / peak_gbs, "traffic": NCU_TRAFFIC_RATIO * bytes_layer,
                          "traffic_source": "ncu dram__bytes_read+write of an 8-sequence x 1-layer launch (117.0 MB for "
                                            "116.6 MB algorithmic), scaled by payload rows: nothing is re-read",
                          "peak_source": peak_src,
-                         "kernel": "%s (+ its merge kernel and a 256 B memset, inside the same events)" % kname,
+                         "kernel": "%s (+ its merge kernel and the one that zeroes the item counter, inside the same events)" % kname,
                          "algorithmic_bytes_per_launch": bytes_layer, "avg_launch_ms": avg_launch_ms},
             "payload_gb_per_layer_launch": bytes_layer / 1e9, "work_items_per_launch": n_items,
             "us_per_layer_step_per_sequence": 1e3 * avg_launch_ms / args.seqs,
