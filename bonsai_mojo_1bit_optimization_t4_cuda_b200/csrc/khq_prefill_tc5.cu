@@ -814,12 +814,12 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
         attr_done[dev] = true;
     }
     const long long items = (long long)((T + BR - 1) / BR) * H_q * batch;
-    // Short prompts (up to 24 row blocks): a persistent grid of one CTA per SM, each working through
-    // its items and overlapping one item's epilogue with the next one's first tiles (32 x 512:
-    // 0.26 ms against 0.31 ms; 8 x 2048: 0.49 against 0.53).  Longer prompts: one CTA per item, one
-    // (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
-    // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation
-    // of the kernel (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99).
+    // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
+    // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
+    // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
+    // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
+    // 24 row blocks (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99), and above 16 where a CTA has few
+    // items to even out its share (1 x 2500: 89 against 92 us, 1 x 3000: 116 against 122, 4 x 3000: 473 against 550).
     // khq_b200_prefill_tc5_items_per_cta(n) or KHQ_PREFILL_ITEMS_PER_CTA (read once) force a mode:
     // 1 = one item per CTA, larger = that many items per CTA (the setter wins; 0 = automatic).
     static int env_forced = -1;
@@ -832,7 +832,7 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     const int nqb = (T + BR - 1) / BR;
     long long ctas;
     int group_major = 0;
-    if (forced == 1 || (forced == 0 && nqb > 24)) {
+    if (forced == 1 || (forced == 0 && (nqb > 24 || (nqb > 16 && items <= 16LL * sm_count[dev])))) {
         ctas = items;
         group_major = 1;
     } else if (forced > 1) {

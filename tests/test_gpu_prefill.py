@@ -180,3 +180,13 @@ def test_prefill_honours_batch_strides(cuda_ops, oracle, entry):
         ref = oracle.gqa_prefill(qg[b, :T].cpu().numpy(), k[b, :T].cpu().numpy(), v[b, :T].cpu().numpy(), T, H_Q, H_KV, D, SCALE)
         ok, mx, exc = cases.attention_close(got[b], ref)
         assert ok, f"{entry} batch {b}: max abs {mx:.3e}, excess {exc:.3e}"
+
+
+@pytest.mark.parametrize("B,T", [(1, 2048), (1, 2049), (1, 3073)])
+def test_prefill_either_side_of_the_grid_rule(cuda_ops, B, T):
+    """The automatic choice between a persistent grid and one CTA per item does not show in the results."""
+    rng = np.random.default_rng(T)
+    qg = rng.standard_normal((B, T, H_Q, 2 * D)).astype(np.float16)
+    k, v = (rng.standard_normal((B, T, H_KV, D)) * 0.25).astype(np.float16), rng.standard_normal((B, T, H_KV, D)).astype(np.float16)
+    auto, one, many = (_run(cuda_ops, qg, k, v, B, T, kernel=m) for m in ("tc5", "tc5-one-item-per-cta", "tc5-persistent"))
+    assert np.array_equal(auto, one) and np.array_equal(auto, many)
