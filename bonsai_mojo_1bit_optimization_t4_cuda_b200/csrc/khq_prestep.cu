@@ -37,13 +37,18 @@ __device__ __forceinline__ void norm_head(__half* x, const float* w, int dim, fl
     __syncwarp();
 }
 
-__device__ __forceinline__ void rope_head(__half* x, int rotary_dim, int pos, float theta, int lane) {
+// cosine and sine of the lane's rotary pair
+__device__ __forceinline__ float2 rope_turn(int rotary_dim, int pos, float theta, int lane) {
+    const float ex = -(float)(2 * lane) / (float)rotary_dim;
+    const float freq = expf(logf(theta) * ex);
+    const float ang = (float)pos * freq;
+    return make_float2(cosf(ang), sinf(ang));
+}
+
+__device__ __forceinline__ void rope_head(__half* x, int rotary_dim, float2 turn, int lane) {
     const int half_r = rotary_dim / 2;
     if (lane < half_r) {
-        const float ex = -(float)(2 * lane) / (float)rotary_dim;
-        const float freq = expf(logf(theta) * ex);
-        const float ang = (float)pos * freq;
-        const float c = cosf(ang), s = sinf(ang);
+        const float c = turn.x, s = turn.y;
         const float x0 = __half2float(x[lane]), x1 = __half2float(x[lane + half_r]);
         x[lane] = __float2half(x0 * c - x1 * s);
         x[lane + half_r] = __float2half(x0 * s + x1 * c);
@@ -56,29 +61,76 @@ __device__ __forceinline__ void copy_head(__half* dst, const __half* src, int di
         *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(src + d);
 }
 
-// grid = H_q + H_kv warps (one block of 32 threads each).
+// d = 256 with 64 rotary dims: a head stays in registers (lane l holds dims l + 32 i, so both halves of its rotary pair), one load
+// and one store instead of three passes over global memory that depend on each other.  turn(): cosine and sine, evaluated
+// while the loads are in flight.  ring_u takes the head before the rotation, ring_r (K) behind it, ring_v copies v.
+template <class Turn>
+__device__ __forceinline__ void head_256(__half* x, const float* w, float eps, int lane, Turn turn, __half* ring_u, __half* ring_r,
+                                         __half* ring_v, const __half* v) {
+    __half h[8];
+    float wv[8];
+    uint4 vv = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = x[lane + 32 * i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wv[i] = w ? w[lane + 32 * i] : 1.0f;
+    if (ring_v) vv = *reinterpret_cast<const uint4*>(v + lane * 8);
+    const float2 cs = turn();
+    float sum_sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float f = __half2float(h[i]);
+        sum_sq += f * f;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum_sq += __shfl_down_sync(0xFFFFFFFFu, sum_sq, off);
+    float rms = 0.0f;
+    if (lane == 0) rms = 1.0f / sqrtf(sum_sq / 256.0f + eps);
+    rms = __shfl_sync(0xFFFFFFFFu, rms, 0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        h[i] = __float2half(__half2float(h[i]) * rms * wv[i]);
+        if (ring_u) ring_u[lane + 32 * i] = h[i];
+    }
+    const float x0 = __half2float(h[0]), x1 = __half2float(h[1]);
+    h[0] = __float2half(x0 * cs.x - x1 * cs.y);
+    h[1] = __float2half(x0 * cs.y + x1 * cs.x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        x[lane + 32 * i] = h[i];
+        if (ring_r) ring_r[lane + 32 * i] = h[i];
+    }
+    if (ring_v) *reinterpret_cast<uint4*>(ring_v + lane * 8) = vv;
+}
+
+// grid = H_q + H_kv warps (one block of 32 threads each).  Latency-bound, and in the chain of every step: 3.7 us behind the kernel
+// before it when cosine and sine were evaluated there and the head went through global memory between the passes, 1.9 so.
 __global__ void __launch_bounds__(32)
 khq_prestep_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, const __half* __restrict__ v,
                    const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, __half* __restrict__ ring_k,
                    __half* __restrict__ ring_v, __half* __restrict__ ring_u, int H_q, int d, int rotary_dim, int pos,
                    float theta, float eps, int has_norms) {
     const int h = blockIdx.x, lane = threadIdx.x;
+    const float2 cs = rope_turn(rotary_dim, pos, theta, lane);
     khq::pdl_wait();
     khq::pdl_trigger();
-    if (h < H_q) {
-        __half* x = q_gate + (size_t)h * 2 * d;
-        norm_head(x, has_norms ? q_norm_w : nullptr, d, eps, lane);
-        rope_head(x, rotary_dim, pos, theta, lane);
-    } else {
-        const int g = h - H_q;
-        __half* x = k + (size_t)g * d;
-        norm_head(x, has_norms ? k_norm_w : nullptr, d, eps, lane);
-        if (ring_u) copy_head(ring_u + (size_t)g * d, x, d, lane);
-        __syncwarp();
-        rope_head(x, rotary_dim, pos, theta, lane);
-        if (ring_k) copy_head(ring_k + (size_t)g * d, x, d, lane);
-        if (ring_v) copy_head(ring_v + (size_t)g * d, v + (size_t)g * d, d, lane);
+    const bool is_q = h < H_q;
+    const size_t off = (size_t)(is_q ? h : h - H_q) * d;
+    __half* x = is_q ? q_gate + 2 * off : k + off;
+    const float* w = !has_norms ? nullptr : is_q ? q_norm_w : k_norm_w;
+    __half* u = !is_q && ring_u ? ring_u + off : nullptr;
+    __half* rk = !is_q && ring_k ? ring_k + off : nullptr;
+    __half* rv = !is_q && ring_v ? ring_v + off : nullptr;
+    if (d == 256 && rotary_dim == 64) {
+        head_256(x, w, eps, lane, [&] { return cs; }, u, rk, rv, v + off);
+        return;
     }
+    norm_head(x, w, d, eps, lane);
+    if (u) copy_head(u, x, d, lane);
+    __syncwarp();
+    rope_head(x, rotary_dim, cs, lane);
+    if (rk) copy_head(rk, x, d, lane);
+    if (rv) copy_head(rv, v + off, d, lane);
 }
 
 // The same work for B sequences in one launch: grid = B * (H_q + H_kv) warps.  Sequence b reads
@@ -94,22 +146,24 @@ khq_prestep_batched_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, 
     const int b = blockIdx.x / per, h = blockIdx.x % per, lane = threadIdx.x;
     khq::pdl_wait();
     khq::pdl_trigger();
-    const int pos = positions[b];
-    if (h < H_q) {
-        __half* x = q_gate + ((size_t)b * H_q + h) * 2 * d;
-        norm_head(x, has_norms ? q_norm_w : nullptr, d, eps, lane);
-        rope_head(x, rotary_dim, pos, theta, lane);
-    } else {
-        const int g = h - H_q;
-        __half* x = k + ((size_t)b * H_kv + g) * d;
-        const size_t slot_off = (size_t)b * ring_seq_stride + ((size_t)slots[b] * H_kv + g) * d;
-        norm_head(x, has_norms ? k_norm_w : nullptr, d, eps, lane);
-        if (ring_u) copy_head(ring_u + slot_off, x, d, lane);
-        __syncwarp();
-        rope_head(x, rotary_dim, pos, theta, lane);
-        if (ring_k) copy_head(ring_k + slot_off, x, d, lane);
-        if (ring_v) copy_head(ring_v + slot_off, v + ((size_t)b * H_kv + g) * d, d, lane);
+    const bool is_q = h < H_q;
+    const size_t in = is_q ? 0 : ((size_t)b * H_kv + (h - H_q)) * d;
+    const size_t slot_off = is_q ? 0 : (size_t)b * ring_seq_stride + ((size_t)slots[b] * H_kv + (h - H_q)) * d;
+    __half* x = is_q ? q_gate + ((size_t)b * H_q + h) * 2 * d : k + in;
+    const float* w = !has_norms ? nullptr : is_q ? q_norm_w : k_norm_w;
+    __half* u = !is_q && ring_u ? ring_u + slot_off : nullptr;
+    __half* rk = !is_q && ring_k ? ring_k + slot_off : nullptr;
+    __half* rv = !is_q && ring_v ? ring_v + slot_off : nullptr;
+    if (d == 256 && rotary_dim == 64) {
+        head_256(x, w, eps, lane, [&] { return rope_turn(64, positions[b], theta, lane); }, u, rk, rv, v + in);
+        return;
     }
+    norm_head(x, w, d, eps, lane);
+    if (u) copy_head(u, x, d, lane);
+    __syncwarp();
+    rope_head(x, rotary_dim, rope_turn(rotary_dim, positions[b], theta, lane), lane);
+    if (rk) copy_head(rk, x, d, lane);
+    if (rv) copy_head(rv, v + in, d, lane);
 }
 
 }  // namespace khq_prestep
