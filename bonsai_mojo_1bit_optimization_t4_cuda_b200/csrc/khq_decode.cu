@@ -1585,8 +1585,8 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
 // The item counter of a persistent launch.  A kernel, because a memset between two kernels keeps the launch of the second one from
 // overlapping the end of the first.
 __global__ void khq_zero_counter_kernel(int* counter) {
-    pdl_wait();
     pdl_trigger();
+    pdl_wait();
     if (threadIdx.x == 0) *counter = 0;
 }
 

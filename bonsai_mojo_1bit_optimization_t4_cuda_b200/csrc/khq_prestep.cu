@@ -111,9 +111,9 @@ khq_prestep_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, const __
                    __half* __restrict__ ring_v, __half* __restrict__ ring_u, int H_q, int d, int rotary_dim, int pos,
                    float theta, float eps, int has_norms) {
     const int h = blockIdx.x, lane = threadIdx.x;
+    khq::pdl_trigger();  // the kernel behind reads nothing but constants before its own wait
     const float2 cs = rope_turn(rotary_dim, pos, theta, lane);
     khq::pdl_wait();
-    khq::pdl_trigger();
     const bool is_q = h < H_q;
     const size_t off = (size_t)(is_q ? h : h - H_q) * d;
     __half* x = is_q ? q_gate + 2 * off : k + off;
@@ -144,8 +144,8 @@ khq_prestep_batched_kernel(__half* __restrict__ q_gate, __half* __restrict__ k, 
                            int H_q, int H_kv, int d, int rotary_dim, float theta, float eps, int has_norms) {
     const int per = H_q + H_kv;
     const int b = blockIdx.x / per, h = blockIdx.x % per, lane = threadIdx.x;
-    khq::pdl_wait();
     khq::pdl_trigger();
+    khq::pdl_wait();
     const bool is_q = h < H_q;
     const size_t in = is_q ? 0 : ((size_t)b * H_kv + (h - H_q)) * d;
     const size_t slot_off = is_q ? 0 : (size_t)b * ring_seq_stride + ((size_t)slots[b] * H_kv + (h - H_q)) * d;
