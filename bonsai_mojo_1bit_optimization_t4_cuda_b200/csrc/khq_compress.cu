@@ -575,23 +575,30 @@ khq_compress_v_kernel(const __half* __restrict__ x, const __half* __restrict__ d
 //     64 (|a c|^2 - 2 a v.c)  =  (64 v, 64) . (-2 a c, |a c|^2)
 // with v and a c as fp16 pieces that carry 22 bits (v = vh + vl, -2 a c = ch + cl, the norm in three pieces):
 //     k   0..2 vh ch   3: 64 n1   4..6 vl ch   7: 64 n2   8..10 vh cl   11: 64 n3   12..15: 0.
-// Each omitted or rounded term is below 2^-22 of its factors and the fp32 accumulation of twelve terms below 2^-19 of their
-// magnitude B = V^2 + 2 V cm + 3 cm^2 (V = |v0| + |v1| + |v2|, cm = largest |a c_k| of the patch), which also bounds what the
-// reference's own fp32 evaluation is off (3 x 2^-24 of a distance <= B).  Two values are so off by less than 2^-17 B against
-// each other; if exactly one code lies within that of the smallest approximation it is the reference's choice, and every other
-// (row, patch) goes through the exact search (v_search_row) behind the steps.  So the code words stay bit-identical.
+// Both factors are first brought to a fixed range: per patch, v and a c are multiplied by the power of two that puts cm, the
+// largest |a c_k| of the patch, into [8, 16).  That changes neither the order of the distances nor a rounding, and it keeps the
+// pieces away from the ends of fp16: |2 a c| < 32, |a c|^2 < 768, 64 v < 32 000 (V < 500 is asked for below, V = |v0| + |v1| +
+// |v2|).  A second piece is then off by at most 2^-22 of its factor, or by 2^-25 where it is subnormal, which against
+// 64 B >= 64 x 3 x 8^2 is below 2^-28 even after the multiplication by the other factor; without the scaling the subnormal
+// pieces of a codebook with |a c| of some hundredths lost whole distances.  So each omitted or rounded term is below 2^-21 of
+// 64 B, B = V^2 + 2 V cm + 3 cm^2, and the fp32 accumulation of twelve terms below 2^-19; B also bounds what the reference's own
+// fp32 evaluation is off (3 x 2^-24 of a distance <= B).  Two values are so off by less than 2^-17 B against each other; if
+// exactly one code lies within that of the smallest approximation it is the reference's choice, and every other (row, patch)
+// goes through the exact search (v_search_row) behind the steps, as do all pairs of a patch with cm outside [2^-40, 2^21).
+// So the code words stay bit-identical.
 //
 // CTA = four groups of two warps; a group owns 16 rows (one M tile), its warps search patches 0..31 and 32..63 and share the
-// rows in front and behind.  The B fragments of a patch (8 KB) are built once per CTA and step by all threads, double
-// buffered.  A thread holds 2 rows x 32 codes of a half patch: minimum by three-input min, then the sign bits of (value -
-// minimum - margin) shifted into a mask.  44 warp instructions per (row, patch) against 85 of the exact search, about two per
-// cycle; 0.5 % of the pairs are redone.  129 024 rows: 800 -> 636 us.
+// rows in front and behind.  The scales of all patches come first (a patch per warp at a time, 1 % of the CTA's instructions).
+// The B fragments of a patch (8 KB) are built once per CTA and step by all threads, double buffered.  A thread holds 2 rows x 32
+// codes of a half patch: minimum by three-input min, then the sign bits of (value - minimum - margin) shifted into a mask.  44 warp
+// instructions per (row, patch) against 85 of the exact search, about two per cycle; 0.5 % of the pairs are redone.  129 024
+// rows: 800 us with the exact search alone, 646 filtered without the scaling, 664 with it.
 constexpr int VM_ROWS = 16;  // rows per group
 constexpr int VM_GROUPS = 4;   // per CTA; eight halve the building of fragments but not the time (694 us)
 struct CompressScratchVM {
     float p[VM_GROUPS * VM_ROWS][D + 4];   // x as float, then the projection, then (per row) the patch energies
     uint4 b[2][2][256 * 2];                // [buffer][half][code]: k pairs of lanes t = 0..3 (b0, b1 each)
-    float cm[2][2][8];                     // largest |a c_k| per warp's share of a patch
+    float2 scale[NP];                      // per patch: its power of two, cm times that (NaN: not for the filter)
     unsigned short code[VM_GROUPS * VM_ROWS][NP];
     alignas(16) unsigned undecided[NP][VM_GROUPS];  // rows of a group that need the exact search, bit 4 g + y: row g + 8 y
 };
@@ -602,16 +609,21 @@ __device__ __forceinline__ uint32_t vm_pack(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// B fragments of one code (c: its three halfs).
-__device__ __forceinline__ void vm_build(const __half (&c)[3], float alpha, uint4* dst, float& cmax) {
-    float a[3], q[3], n = 0.0f;
-    cmax = 0.0f;
+// The power of two that puts cm into [8, 16), and cm times that; NaN for a patch that the filter does not take.
+__device__ __forceinline__ float2 vm_scale(float cm) {
+    const unsigned e = __float_as_uint(cm) >> 23, in = min(max(e, 127u - 40u), 127u + 20u);
+    const float s = __uint_as_float((2u * 127u + 3u - in) << 23);
+    return make_float2(s, e == in ? cm * s : __int_as_float(0x7FFFFFFF));
+}
+
+// B fragments of one code (c: its three halfs); alpha: with the patch's power of two.
+__device__ __forceinline__ void vm_build(const __half (&c)[3], float alpha, uint4* dst) {
+    float q[3], n = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        a[k] = __half2float(c[k]) * alpha;
-        cmax = fmaxf(cmax, fabsf(a[k]));
-        n = fmaf(a[k], a[k], n);
-        q[k] = -2.0f * a[k];
+        const float a = __half2float(c[k]) * alpha;
+        n = fmaf(a, a, n);
+        q[k] = -2.0f * a;
     }
     const float h0 = __half2float(__float2half(q[0])), h1 = __half2float(__float2half(q[1])), h2 = __half2float(__float2half(q[2]));
     const float n1 = __half2float(__float2half(n)), n2 = __half2float(__float2half(n - n1));
@@ -650,16 +662,23 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
             cn[u][2] = c[2];
         }
     };
-    const auto build = [&](int buf) {
+    const auto build = [&](int step) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            float m;
-            vm_build(cn[u], alpha, &S.b[buf][u][2 * tid], m);
-            const unsigned mb = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m));
-            if (lane == 0) S.cm[buf][u][warp] = __uint_as_float(mb);
-        }
+        for (int u = 0; u < 2; ++u) vm_build(cn[u], alpha * S.scale[step + 32 * u].x, &S.b[step & 1][u][2 * tid]);
     };
     fetch(0);
+#pragma unroll 2
+    for (int p = warp; p < NP; p += VM_GROUPS * 2) {
+        const uint4* cbp = reinterpret_cast<const uint4*>(vq + ((size_t)p * 256 + lane * 8) * 3);
+        const uint4 c[3] = {__ldg(cbp), __ldg(cbp + 1), __ldg(cbp + 2)};
+        __half2 m = __float2half2_rn(0.0f);
+#pragma unroll
+        for (int i = 0; i < 12; ++i) m = __hmax2(m, __habs2(reinterpret_cast<const __half2*>(c)[i]));
+        // the largest product is the product of the largest: rounding keeps the order
+        const float cm = fabsf(__half2float(__hmax(__low2half(m), __high2half(m))) * alpha);
+        const unsigned all = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(cm));
+        if (lane == 0) S.scale[p] = vm_scale(__uint_as_float(all));
+    }
     // ---- front: rows as fp32, in-order sums of squares, projections ----------------------------
 #pragma unroll 1
     for (int r = 0; r < RW; ++r) {
@@ -702,6 +721,7 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
         *reinterpret_cast<float4*>(&pr[lane * 8]) = make_float4(proj[0], proj[1], proj[2], proj[3]);
         *reinterpret_cast<float4*>(&pr[lane * 8 + 4]) = make_float4(proj[4], proj[5], proj[6], proj[7]);
     }
+    __syncthreads();
     build(0);
     __syncthreads();
     // ---- code search ---------------------------------------------------------------------------
@@ -710,22 +730,18 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
     for (int step = 0; step < NP / 2; ++step) {
         const int buf = step & 1, patch = step + 32 * half;
         if (step + 1 < NP / 2) fetch(step + 1);
-        float cm = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; k += 4) {
-            const float4 c = *reinterpret_cast<const float4*>(&S.cm[buf][half][k]);
-            cm = fmaxf(cm, fmaxf(fmaxf(c.x, c.y), fmaxf(c.z, c.w)));
-        }
+        const float vs = S.scale[patch].x, cm = S.scale[patch].y;
         uint32_t a[4];
         float thr[2];
         bool safe[2];
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
             const float4 v = *reinterpret_cast<const float4*>(&S.p[m_row + g + 8 * y][patch * 4]);
-            const float V = fabsf(v.x) + fabsf(v.y) + fabsf(v.z);
+            const float V = vs * (fabsf(v.x) + fabsf(v.y) + fabsf(v.z));
             thr[y] = fmaf(V, fmaf(2.0f, cm, V), 3.0f * cm * cm) * 0.00048828125f;  // 64 x 2^-17 x B
-            safe[y] = V < 500.0f && cm < 200.0f;  // nothing overflows fp16; false for NaN
-            const float e0 = 64.0f * ((t & 1) ? v.z : v.x), e1 = (t & 1) ? 64.0f : 64.0f * v.y;
+            safe[y] = V < 500.0f && cm < 16.0f;  // nothing overflows fp16; false for NaN
+            const float v64 = 64.0f * vs;
+            const float e0 = v64 * ((t & 1) ? v.z : v.x), e1 = (t & 1) ? 64.0f : v64 * v.y;
             const uint32_t hi = vm_pack(e0, e1);
             const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
             const uint32_t lo = vm_pack(e0 - hf.x, t == 3 ? 64.0f : e1 - hf.y);
@@ -798,7 +814,7 @@ khq_compress_v_mma_kernel(const __half* __restrict__ x, const __half* __restrict
             redo |= __ballot_sync(0xFFFFFFFFu, t == 0 && !one) << y;  // bit 4 g + y: row g + 8 y
         }
         if (lane == 0) S.undecided[patch][grp] = redo;
-        if (step + 1 < NP / 2) build(buf ^ 1);
+        if (step + 1 < NP / 2) build(step + 1);
         __syncthreads();
     }
     // ---- exact search of the undecided pairs, a patch per warp: within the steps it held up the other seven warps -----------
