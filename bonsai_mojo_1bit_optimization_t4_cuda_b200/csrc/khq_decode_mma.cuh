@@ -61,7 +61,7 @@ constexpr int M2_SM_RSC = M2_SM_ROPE + 2 * M2_TT * 64 * 4;           // 16 rows 
 // small tables of a layer, in the order of the prepared image
 constexpr int M2_SM_FREQ = M2_SM_RSC + M2_THREADS / 32 * 16 * 32;      // 32 floats: RoPE frequencies
 constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats: 1 / (256 d) of the rotary dims
-constexpr int M2_SM_C3 = M2_SM_DINV + 256;                           // 64 patches x float2: alpha_v x (centroid 0, centroid 1 - centroid 0) of dim 3
+constexpr int M2_SM_C3 = M2_SM_DINV + 256;                           // 64 patches x float2: alpha_v x (mean, half the difference 0 - 1) of the two dim-3 centroids
 constexpr int M2_SM_RSTEP = M2_SM_C3 + NP * 8;                       // 32 x float2: cos / sin of M2_TT positions of each rotary pair
 constexpr int M2_SMALL_BYTES = 128 + 256 + NP * 8 + 32 * 8;
 constexpr int M2_SM_BARS = M2_SM_FREQ + M2_SMALL_BYTES;              // M2_WPK * M2_NSTAGE stages, then the image's small tables and codebook
@@ -273,7 +273,7 @@ __device__ __forceinline__ void m2_small_tables(unsigned char* dst, const Compre
     if (tid < 32) reinterpret_cast<float*>(dst)[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
     if (tid >= 128 && tid < 128 + NP) {
         const float c0 = __half2float(P.cents_v[0 * D + 4 * (tid - 128) + 3]), c1 = __half2float(P.cents_v[1 * D + 4 * (tid - 128) + 3]);
-        reinterpret_cast<float2*>(dst + O_C3)[tid - 128] = make_float2(c0 * P.alpha_v, (c1 - c0) * P.alpha_v);
+        reinterpret_cast<float2*>(dst + O_C3)[tid - 128] = make_float2(0.5f * (c0 + c1) * P.alpha_v, 0.5f * (c0 - c1) * P.alpha_v);
     }
     if (tid < 64) reinterpret_cast<float*>(dst + O_DINV)[tid] = (1.0f / 256.0f) / (__half2float(P.d_k[tid]) + 1e-8f);
     if (tid >= 192 && tid < 224) {
@@ -539,14 +539,18 @@ __device__ __forceinline__ void m2_build_query(M2Query& Q, const __half* __restr
 //
 // O^T lives in tensor memory, twenty columns per pair of patches (2pp, 2pp + 1) of the thread's patch group g: three
 // accumulator tiles of the dims 0..2 (rows idx = 2 jj + r of the pair's six (patch, dim) rows), one of the dim-3 residual
-// fields, one of the dim-3 centroid bits.  Dim 3 of a patch is centroid[bit] * alpha_v * s2 + (field - 8) * s3 per token
-// with per-token scales s2, s3; both sums over tokens are taken over the raw bit fields as they lie in the payload,
-//     sum p s2 bit  and  sum p s3 field   (exact fp16 operands: a bit field is a subnormal fp16 number),
-// and the centroids, their difference and the -8 enter once per item, with sum p s2 and sum p s3 kept per head.
+// fields, one of the dim-3 centroid signs.  Dim 3 of a patch is centroid[bit] * alpha_v * s2 + (field - 8) * s3 per token
+// with per-token scales s2, s3; the sums over tokens are
+//     sum p s2 (1 - 2 bit)  and  sum p s3 (field - 8)   (exact fp16 operands made from the payload's bits),
+// and half the centroids' difference and, with sum p s2, their mean enter once per item.  Both operands are signed, so that
+// what an accumulator holds cancels as it goes, like the dims 0..2: sums of the raw non-negative fields with the -8 taken off at the
+// end grow with the number of tokens while the wanted sum grows with its root, and the tensor core's additions lose on one side.
+// Error of dim 3 relative to the spread of the sums, 131 072 tokens of equal weight through one split: 8.5e-3 with the raw
+// fields, 4e-6 so (dims 0..2: 1.2e-5); an item of 8192 tokens: 8.6e-4 and 2e-6.  Time: 0.5 % of a full batch's step.
 struct M2State {
     uint32_t tm_o;
-    float m[2], l[2], p2[2], p3[2];  // reference of the weights, sum of weights, sums of p s2 and p s3 (per lane)
-    float top[2];                    // largest score (per lane)
+    float m[2], l[2], p2[2];  // reference of the weights, sum of weights, sum of p s2 (per lane)
+    float top[2];             // largest score (per lane)
     __device__ __forceinline__ void init() {  // whole warp
         float z[16];
 #pragma unroll
@@ -556,15 +560,23 @@ struct M2State {
         m2_tm_st_wait();
         m[0] = m[1] = top[0] = top[1] = NEG_BIG;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) l[e] = p2[e] = p3[e] = 0.0f;
+        for (int e = 0; e < 2; ++e) l[e] = p2[e] = 0.0f;
     }
 };
 constexpr float M2_SLACK = 2.0f;
-// What a unit of the two dim-3 accumulators of patch parity u stands for: the fields sit at bits 0..3 (even patch) or
-// 4..7 (odd), the centroid bit at 7 or 3, of a subnormal fp16 number (units of 2^-24).
-__device__ __forceinline__ constexpr float m2_field_unit(int u) { return u ? 1048576.0f : 16777216.0f; }
-__device__ __forceinline__ constexpr float m2_bit_unit(int u) { return u ? 2097152.0f : 131072.0f; }
-
+// Two tokens' dim-3 operands.  field - 8: a field in bits 0..3 under the bits of 1024 (unit 1), or in bits 4..7 under those of
+// 64 (unit 1/16), minus the offset in one packed subtraction, exact.  1 - 2 bit: the bit as the sign of 1.
+__device__ __forceinline__ uint32_t m2_field_lo(uint32_t w) {
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"((w & 0x000F000Fu) | 0x64006400u), "r"(0x64086408u));
+    return r;
+}
+__device__ __forceinline__ uint32_t m2_field_hi(uint32_t w) {
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"((w & 0x00F000F0u) | 0x54005400u), "r"(0x54805480u));
+    return r;
+}
+__device__ __forceinline__ uint32_t m2_sign(uint32_t w) { return (w & 0x80008000u) | 0x3C003C00u; }
 
 // The two rows of a lane (g and g + 8 of the block), its 64-dim quarter of each.
 struct M2KRows {
@@ -809,7 +821,6 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             st.m[e] = mn;
             st.l[e] *= corr[e];
             st.p2[e] *= corr[e];
-            st.p3[e] *= corr[e];
         }
     }
 #pragma unroll
@@ -830,10 +841,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
             s3[x] = v.z;  // dim 3: residual field
         }
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            st.p2[e] = fmaf(pw[1][e], s2[1], fmaf(pw[0][e], s2[0], st.p2[e]));
-            st.p3[e] = fmaf(pw[1][e], s3[1], fmaf(pw[0][e], s3[0], st.p3[e]));
-        }
+        for (int e = 0; e < 2; ++e) st.p2[e] = fmaf(pw[1][e], s2[1], fmaf(pw[0][e], s2[0], st.p2[e]));
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             uint32_t hi, lo;
@@ -900,10 +908,9 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
         // the odd patch the centroid bit too; the even patch's centroid bit is the top bit of byte 0.  The masks leave
         // nothing of the neighbouring bits.
         const uint32_t b01l = __byte_perm(f24[0], f24[1], 0x5410), b01h = __byte_perm(f24[2], f24[3], 0x5410);
-        const uint32_t b1l = b01l >> 8, b1h = b01h >> 8;
         const uint32_t b2l = __byte_perm(f24[0], f24[1], 0x7632), b2h = __byte_perm(f24[2], f24[3], 0x7632);
-        const uint32_t da[4] = {b1l & 0x000F000Fu, b2l & 0x00F000F0u, b1h & 0x000F000Fu, b2h & 0x00F000F0u};
-        const uint32_t ca[4] = {b01l & 0x00800080u, b2l & 0x00080008u, b01h & 0x00800080u, b2h & 0x00080008u};
+        const uint32_t da[4] = {m2_field_lo(b01l >> 8), m2_field_hi(b2l), m2_field_lo(b01h >> 8), m2_field_hi(b2h)};
+        const uint32_t ca[4] = {m2_sign(b01l << 8), m2_sign(b2l << 12), m2_sign(b01h << 8), m2_sign(b2h << 12)};
         m2_tm_ld_wait();
         if (rescale) {
 #pragma unroll
@@ -1001,7 +1008,6 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
         for (int m = 4; m <= 16; m <<= 1) {
             st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], m);
             st.p2[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p2[e], m);
-            st.p3[e] += __shfl_xor_sync(0xFFFFFFFFu, st.p3[e], m);
         }
     // the record is relative to the largest score itself
     float fin[2];
@@ -1031,8 +1037,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const float2 c = c3s[2 * pp + u];
-                    v[4 * u + 3] = fin[e] * (fmaf(c.x, st.p2[e], c.y * (m2_bit_unit(u) * o[4][2 * u + e])) +
-                                             fmaf(-8.0f, st.p3[e], m2_field_unit(u) * o[3][2 * u + e]));
+                    v[4 * u + 3] = fin[e] * fmaf(c.x, st.p2[e], fmaf(c.y, o[4][2 * u + e], o[3][2 * u + e]));
                 }
                 *reinterpret_cast<float4*>(rp) = make_float4(v[0], v[1], v[2], v[3]);
                 *reinterpret_cast<float4*>(rp + 4) = make_float4(v[4], v[5], v[6], v[7]);
