@@ -20,6 +20,7 @@ import numpy as np
 import torch
 
 from .calib import KhqLayerTables, read_calib
+from .lib import ptr
 
 KHQ_MAX_LAYERS = 64
 KHQ_RING = 256
@@ -52,6 +53,17 @@ class _Tensors(dict):
     def __setitem__(self, name, value):
         self.ctx = None
         dict.__setitem__(self, name, value)
+
+
+def _row_address(row, kv: int, device: int) -> int:
+    """Address of a token's row that a kernel can read as it is: kv contiguous fp16 values on the device, on 16 bytes.  0 for any
+    other, which ``ops.ring_write`` copies and converts.  (An int is an address already.)"""
+    if row.__class__ is int:
+        return row
+    if row.dtype is not torch.float16 or row.numel() != kv or row.get_device() != device or not row.is_contiguous():
+        return 0
+    at = row.data_ptr()
+    return 0 if at & 15 else at
 
 
 class KhqLayer:
@@ -228,12 +240,24 @@ class KhqRuntime:
     def _native_step(self, layer_idx: int, L, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, scale: float) -> bool:
         """The step of one layer (append, event if due, both regions, merge, gate) as one native call.
         False: a step that only the call-by-call sequence covers (another backend, profiling, debug
-        output, a window beyond the ring)."""
+        output, a window beyond the ring, rows that have to be copied or converted, an output off 16 bytes)."""
         window = L.write_pos + 1 - L.boundary
         if self.prof or self.debug or window > KHQ_RING or window <= 0:
             return False
         ctx = L.t.ctx or self._native_ctx(L)
         if ctx is None:
+            return False
+        kv, device = L.H_kv * L.D, L.t["ring_k"].get_device()
+        if k_roped_dev is not None:
+            k_roped_dev, v_dev = _row_address(k_roped_dev, kv, device), _row_address(v_dev, kv, device)
+            if not k_roped_dev or not v_dev:
+                return False
+        if k_unroped_dev is not None:
+            k_unroped_dev = _row_address(k_unroped_dev, kv, device)
+            if not k_unroped_dev:
+                return False
+        out_dev = ptr(out_dev)
+        if out_dev & 15:
             return False
         c_len = L.boundary
         event = window >= KHQ_WATERMARK and c_len + KHQ_CHUNK <= L.cap
@@ -351,7 +375,8 @@ class KhqRuntime:
         the compression event if it is due, the three ring appends, both attention regions, the merge and
         the gate in one host call and two launches (four with an event) instead of seven.  A step whose window
         would exceed the ring takes the classic sequence (compressed capacity exhausted: the reference keeps
-        stepping with window > 256, ``README.md:259``, and so does ``khq_step``).  The state afterwards
+        stepping with window > 256, ``README.md:259``, and so does ``khq_step``), and so does one whose rows are
+        not contiguous fp16 on 16 bytes.  The state afterwards
         is the one the classic calls leave."""
         if not self.active or not self.ready or layer_idx < 0 or layer_idx >= KHQ_MAX_LAYERS:
             return False

@@ -292,3 +292,52 @@ def test_decode_step_error_codes(cuda_ops):
     b = list(a)
     b[1] = 8
     assert fn(*b, 0, 0, 1, 256, 1, 0.0625, 1.0, 1.0, 1e7, 0) == -104          # misaligned token
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("at", [200, 255])  # a plain step, and one with a compression event
+def test_rows_in_other_forms(cuda_ops, at, fused):
+    """Rows that are slices of a fused projection, fp32, in host memory or off 16 bytes, and an output off 16 bytes, give the step that
+    contiguous fp16 rows give: rings bit by bit, outputs within the attention bar."""
+    import torch
+
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.runtime import KhqRuntime
+
+    case = cases.make_case(cases.synth.seed_for(1, 23), at + 1, "calib", layer_id=3)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    ku, kr, v, q = dev(case["k_unroped"]), dev(case["k_roped"]), dev(case["v"]), dev(case["q_gate"])
+
+    def strided(x):
+        wide = torch.full((H_KV, 3, D), float("nan"), dtype=torch.float16, device="cuda")
+        wide[:, 1] = x
+        return wide[:, 1]
+
+    def unaligned(x):
+        buf = torch.zeros(H_KV * D + 1, dtype=torch.float16, device="cuda")
+        buf[1:] = x.reshape(-1)
+        return buf[1:]
+
+    forms = dict(plain=lambda x: x, strided=strided, fp32=lambda x: x.float(), host=lambda x: x.cpu(), unaligned=unaligned, out=lambda x: x)
+    got = {}
+    for name, form in forms.items():
+        rt = KhqRuntime(cuda_ops, device="cuda")
+        assert rt.khq_activate([case["tables"]], max_seq=512)
+        rt.khq_init_layer(3, H_Q, H_KV, D)
+        L = rt.layers[3]
+        for ring, rows in (("ring_u", ku), ("ring_k", kr), ("ring_v", v)):
+            L.t[ring].view(256, -1)[:at] = rows[:at].reshape(at, -1)
+        L.write_pos = at
+        out = torch.zeros(H_Q * D + 1, dtype=torch.float16, device="cuda")
+        out = out[1:] if name == "out" else out[:-1]
+        if fused:
+            assert rt.khq_step_fused(3, q, form(ku[at]), form(kr[at]), form(v[at]), out, SCALE)
+        else:
+            rt.khq_capture_unroped(3, form(ku[at]))
+            assert rt.khq_step(3, q, form(kr[at]), form(v[at]), out, SCALE)
+        got[name] = (out.float().cpu().numpy(), {n: L.t[n].clone() for n in ("ring_k", "ring_v", "ring_u", "kpay", "vpay")})
+        assert (L.write_pos, L.boundary) == (at + 1, 128 * (at == 255))
+    for name, (out, state) in got.items():
+        ok, mx, exc = cases.attention_close(out, got["plain"][0])
+        assert ok, f"{name}: max abs {mx:.3e}, excess {exc:.3e}"
+        for n, t in state.items():
+            assert torch.equal(t, got["plain"][1][n]), (name, n)
