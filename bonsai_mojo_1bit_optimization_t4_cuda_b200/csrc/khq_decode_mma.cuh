@@ -563,7 +563,9 @@ struct M2State {
         for (int e = 0; e < 2; ++e) l[e] = p2[e] = 0.0f;
     }
 };
-constexpr float M2_SLACK = 2.0f;
+// How far a score may lie above the reference maximum before that follows: the weights stay below e^2.  Times a row's V
+// scales they are fp16 operands, so a block with a scale from 8192 on (8192 e^2 < 65 504) allows none.
+constexpr float M2_SLACK = 2.0f, M2_SLACK_SCALES = 8192.0f;
 // Two tokens' dim-3 operands.  field - 8: a field in bits 0..3 under the bits of 1024 (unit 1), or in bits 4..7 under those of
 // 64 (unit 1/16), minus the offset in one packed subtraction, exact.  1 - 2 bit: the bit as the sign of 1.
 __device__ __forceinline__ uint32_t m2_field_lo(uint32_t w) {
@@ -714,6 +716,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     // ---- the block's row scalars, one row per lane ---------------------------------------------
     // {score scale of the ternary part, of the residual part, residual / ternary scale of the rotor sums, -} and the three
     // V scales {dims 0..2, dim-3 centroid bit, dim-3 residual field, -}; the residual operand is in units of 2^-24
+    bool large = false;
     if (lane < 16) {
         const int row = lane * HKV + kvh;
         float mult = (float)*reinterpret_cast<const uint32_t*>(S + M2_OFF_KPAY + row * K_PAY) / 1000.0f;
@@ -724,8 +727,10 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
         const float en = hbits2f(reinterpret_cast<const uint16_t*>(S + M2_OFF_VRN)[row]);
         const float sm = reinterpret_cast<const float*>(S + M2_OFF_VSM)[row];
         const bool in = lane >= valid_lo && lane < valid_hi;
+        const float s1 = P.alpha_v * vn * en, s3 = sm * vn * (1.0f / 7.0f);
+        large = in && !(fmaxf(fmaxf(fabsf(s1), fabsf(s3)), vn) < M2_SLACK_SCALES);
         rsc[2 * lane] = make_float4(kn * mult, kn * rs, rs / mult, 0.0f);
-        rsc[2 * lane + 1] = in ? make_float4(P.alpha_v * vn * en, vn, sm * vn * (1.0f / 7.0f), 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        rsc[2 * lane + 1] = in ? make_float4(s1, vn, s3, 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     // ================================ K side: scores ==========================================
     M2KRows kr;
@@ -794,6 +799,7 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     float sc[2][2], pw[2][2];  // [row x: g, g+8][head e: 2t, 2t+1]
     bool valid[2];
     bool raise = false;
+    const float slack = __any_sync(0xFFFFFFFFu, large) ? 0.0f : M2_SLACK;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         valid[x] = (g + 8 * x) >= valid_lo && (g + 8 * x) < valid_hi;
@@ -802,11 +808,11 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
         for (int e = 0; e < 2; ++e) {
             sc[x][e] = valid[x] ? fmaf(sp.x, cs[2 * x + e] + cr[2 * x + e], sp.y * cs2[2 * x + e]) : -1e30f;
             st.top[e] = fmaxf(st.top[e], sc[x][e]);
-            raise = raise || sc[x][e] > st.m[e] + M2_SLACK;
+            raise = raise || sc[x][e] > st.m[e] + slack;
         }
     }
-    // The reference the weights are taken against follows the maximum only when a score is M2_SLACK above it: the weights
-    // stay below e^2, and most blocks need no reduction over the warp and no pass over the accumulators.
+    // The reference the weights are taken against follows the maximum only when a score is more than the slack above it: most
+    // blocks need no reduction over the warp and no pass over the accumulators.
     float corr[2] = {1.0f, 1.0f};
     const bool rescale = __any_sync(0xFFFFFFFFu, raise);
     if (rescale) {

@@ -132,3 +132,30 @@ def test_long_items(cuda_ops, context):
     for w in items:
         r = recs[w["slot"]]
         _check(r[:, :D], np.exp(r[:, D:D + 1].astype(np.float64)), sums(int(w["lo"]), int(w["hi"])), f, 8192 / 48, f"item at {w['lo']}")
+
+
+@pytest.mark.parametrize("norm", [7000, 20000, 50000])
+def test_large_v_rows(cuda_ops, oracle, norm):
+    """V rows whose norms approach the end of fp16: the weights' products with them are fp16 operands, whatever the order in which
+    the scores come."""
+    import torch
+
+    import cases
+
+    c_len = 1200
+    case = cases.make_case(31 + norm, c_len, "calib")
+    v = case["v"].astype(np.float32)
+    v *= norm / np.sqrt((v ** 2).sum(-1, keepdims=True))
+    case["v"] = v.astype(np.float16)
+    kv = cases.compress_with(oracle.compress, case, c_len)
+    tb, f = case["tables"], case["f16"]
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    t, tab = {k: dev(a) for k, a in kv.items() if k != "near_ties"}, {k: dev(a) for k, a in f.items()}
+    out = torch.zeros(HQ, D + 2, dtype=torch.float32, device="cuda")
+    cuda_ops.attn(dev(case["q_gate"]), t["k_payload"], t["v_payload"], t["v_shared_meta"], t["k_mask"], t["k_norms"], t["k_r_norms"], t["v_norms"],
+                  t["v_r_norms"], tab["cents_k"], tab["cents_v"], tab["vq"], tab["rotor_k"], tab["rotor_v"], tab["d_k"], tab["d_v"], out, None, HQ, HQ,
+                  1, c_len, c_len, 6, 1 / 16, tb.alpha_k, tb.alpha_v, 1e7, 0, 1)
+    want = oracle.attn_partial(case["q_gate"], kv, cases.tables_dict(f), HQ, 6, 1 / 16, tb.alpha_k, tb.alpha_v, 1e7, 0, 0, c_len)
+    got, want = cases.normalised(out.cpu().numpy()) / norm, cases.normalised(want) / norm
+    ok, mx, exc = cases.attention_close(got * 16, want * 16)  # as for rows of norm 16
+    assert ok, f"max abs {mx:.3e} excess {exc:.3e}"
