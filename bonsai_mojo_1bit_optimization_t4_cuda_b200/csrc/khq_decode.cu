@@ -1662,6 +1662,12 @@ extern "C" int launch_khq_decode_batched_prepared_fp16(const void* descs, const 
 
 extern "C" size_t khq_b200_prepared_bytes(void) { return (M2_IMG_BYTES + 127) / 128 * 128; }
 
+// Orders an image before everything behind it in the stream.  A step's kernels are launched with the programmatic attribute: one
+// of them may start before what is in front of its predecessor has completed, and khq_attn_compressed_mma_kernel reads the image
+// before its wait.  This kernel starts when the image is complete and visible (an ordinary launch), and as it has no trigger, a
+// kernel behind it starts when it has ended, and what is behind that one later still.
+__global__ void khq_after_prepare_kernel() {}
+
 // A layer's tables in the form the decode kernels use them, once per layer: see include/khq_b200.h.
 extern "C" int launch_khq_prepare_tables(const void* tables_desc, float rope_base, void* image, cudaStream_t stream) {
     if (!tables_desc || !image) return -100;
@@ -1680,6 +1686,7 @@ extern "C" int launch_khq_prepare_tables(const void* tables_desc, float rope_bas
     P.alpha_v = t.alpha_v;
     P.rope_base = rope_base;
     khq_prepare_tables_kernel<<<1, M2_THREADS, 0, stream>>>(P, static_cast<unsigned char*>(image));
+    khq_after_prepare_kernel<<<1, 1, 0, stream>>>();
     return static_cast<int>(cudaGetLastError());
 }
 

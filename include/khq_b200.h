@@ -272,7 +272,9 @@ int launch_khq_decode_step_fp16(
  * RoPE frequencies for `rope_base`), laid out once per layer by a host that keeps its tables: khq_b200_prepared_bytes()
  * bytes at `image` (device memory, 128-byte aligned).  `tables_desc` is a khq_tables_desc in HOST memory; the tables it
  * points to must not change while the image is in use.  Without an image the kernels compute the same values per CTA.
- * Returns -100, -104 or a cudaError_t. */
+ * Ordered like any launch: steps behind it on `stream` see the image, other streams need an event or a synchronisation in
+ * between.  Steps read the image and the K tables before they wait for the launch in front of them, so whoever writes
+ * into either by other means than this call has to synchronise before the next step.  Returns -100, -104 or a cudaError_t. */
 size_t khq_b200_prepared_bytes(void);
 int launch_khq_prepare_tables(const void* tables_desc, float rope_base, void* image, khq_stream_t stream);
 /* launch_khq_decode_batched_fp16 with such images: `images` is a device array of image pointers indexed by table_id. */

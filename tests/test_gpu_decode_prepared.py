@@ -54,3 +54,53 @@ def test_prepared_tables_vs_oracle(cuda_ops, oracle, variant, c_len, win_len, de
     assert torch.equal(p["out"], plain)  # the same values, wherever the tables come from
     ok, mx, exc = cases.attention_close(plain.float().cpu().numpy().reshape(H_Q, D), ref.astype(np.float32))
     assert ok, f"max abs {mx:.3e} excess {exc:.3e}"
+
+
+def test_step_right_behind_prepare(cuda_ops):
+    """launch_khq_prepare_tables and a step of the layer on one stream, with nothing in between but the pre-step (which lets the attention
+    start early): every step sees the image of its own tables."""
+    import torch
+
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.batched import TABLES_DESC
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.lib import check, current_stream
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.runtime import ROPE_BASE, KhqRuntime
+
+    n = 300
+    case = cases.make_case(612, n, "calib", layer_id=3)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    rt = KhqRuntime(cuda_ops, device="cuda")
+    assert rt.khq_activate([case["tables"]], max_seq=512)
+    rt.khq_init_layer(3, H_Q, cases.H_KV, D)
+    L = rt.layers[3]
+    rows = [dev(case[a]) for a in ("k_unroped", "k_roped", "v")]
+    q = dev(case["q_gate"]).reshape(-1)
+    out = torch.zeros(H_Q * D, dtype=torch.float16, device="cuda")
+    for t in range(n - 1):
+        assert rt.khq_step_fused(3, q, *(x[t] for x in rows), out, SCALE)
+    descs = []
+    for alpha_v in (1.0, 0.5):  # two sets of tables that share all but one scalar
+        t = np.zeros(1, TABLES_DESC)
+        for field, name in (("cents_k", "ck"), ("cents_v", "cv"), ("vq", "vq"), ("k_rotor", "rk"), ("v_rotor", "rv"), ("d_k", "dk"), ("d_v", "dv")):
+            t[field] = L.t[name].data_ptr()
+        t["alpha_k"], t["alpha_v"] = L.alpha_k, alpha_v
+        descs.append(t)
+    image, (boundary, write_pos) = L.t.ctx[2], (L.boundary, L.write_pos)
+    assert boundary == 128
+
+    def step(desc, wait):
+        L.boundary, L.write_pos = boundary, write_pos
+        qn, o = q.clone(), torch.zeros_like(out)
+        k = rows[0][n - 1].reshape(-1).clone()
+        check("launch_khq_prepare_tables", cuda_ops.lib.launch_khq_prepare_tables(desc.ctypes.data, ROPE_BASE, image.data_ptr(), current_stream()))
+        if wait:
+            torch.cuda.synchronize()
+        assert rt.khq_prestep(3, qn, k, rows[2][n - 1], n - 1)
+        assert rt.khq_step(3, qn, k, rows[2][n - 1], o, SCALE, rings_written=True)
+        return o
+
+    want = [step(d, True) for d in descs]
+    assert not torch.equal(want[0], want[1])
+    got = [step(descs[i % 2], False) for i in range(20)]
+    torch.cuda.synchronize()
+    for i, o in enumerate(got):
+        assert torch.equal(o, want[i % 2]), f"step {i}"
