@@ -59,7 +59,8 @@ class BatchEngine:
         """``c_len`` / ``win_len``: compressed and raw tokens each sequence starts with (``c_len`` a
         multiple of 128, as the state machine leaves it).  ``grow_tokens``: compressed capacity kept
         free behind every sequence's initial prefix.  ``norm_weights``: per layer ``(q_w, k_w)`` fp32
-        (256,) arrays for the head RMS norms, or None for the unweighted norm."""
+        (256,) arrays for the head RMS norms, or None for the unweighted norm.  The tables (``self.tables``) are laid out
+        for the kernels here: whoever changes one of them later calls ``refresh_tables``."""
         self.lib = _lib.load()
         self.device = torch.device(device)
         self.L = len(tables)
@@ -84,11 +85,7 @@ class BatchEngine:
                 v_rotor=torch.from_numpy(f["rotor_v"]).to(dev), d_k=torch.from_numpy(f["d_k"]).to(dev),
                 d_v=torch.from_numpy(f["d_v"]).to(dev), alpha_k=tb.alpha_k, alpha_v=tb.alpha_v,
                 ts_k=tb.ts_k, ts_v=tb.ts_v))
-        t = np.zeros(self.L, TABLES_DESC)
-        for i, tb in enumerate(self.tables):
-            for k in ("cents_k", "cents_v", "vq", "k_rotor", "v_rotor", "d_k", "d_v"):
-                t[k][i] = tb[k].data_ptr()
-            t["alpha_k"][i], t["alpha_v"][i] = tb["alpha_k"], tb["alpha_v"]
+        t = self._tables_desc()
         self.d_tables = torch.from_numpy(t.view(np.uint8).reshape(-1).copy()).to(dev)
         self._images = prepare_tables(t, self.rope_theta, dev)
         self._d_images = torch.tensor([im.data_ptr() for im in self._images], dtype=torch.int64, device=dev)
@@ -179,16 +176,13 @@ class BatchEngine:
                 check("khq_b200_engine_create", self.lib.khq_b200_engine_create(ctypes.byref(self._native)))
         self._layers = (_lib.EngineLayer * self.L)()
         for l in range(self.L):
-            y, tb = self._layers[l], self.tables[l]
-            for f, src in (("d_k", "d_k"), ("cents_k", "cents_k"), ("rotor_k", "k_rotor"), ("d_v", "d_v"), ("cents_v", "cents_v"),
-                           ("rotor_v", "v_rotor"), ("vq", "vq")):
-                setattr(y, f, tb[src].data_ptr())
+            y = self._layers[l]
             for f, src in self.pay[l].items():
                 setattr(y, f, src.data_ptr())
             y.ring_k, y.ring_v, y.ring_u = self.ring_k[l].data_ptr(), self.ring_v[l].data_ptr(), self.ring_u[l].data_ptr()
             if self.norm_w is not None:
                 y.q_norm, y.k_norm = self.norm_w[l][0].data_ptr(), self.norm_w[l][1].data_ptr()
-            y.ts_k, y.alpha_k, y.ts_v, y.alpha_v = tb["ts_k"], tb["alpha_k"], tb["ts_v"], tb["alpha_v"]
+        self._fill_layer_tables()
         self._ring_u_at = np.array([r.data_ptr() for r in self.ring_u], np.uint64)
         a = self._args = _lib.EngineStep()
         a.h_q, a.h_k, a.h_v, a.h_out = self.h_q.data_ptr(), self.h_k.data_ptr(), self.h_v.data_ptr(), self.h_out.data_ptr()
@@ -220,6 +214,33 @@ class BatchEngine:
         if native:
             self.lib.khq_b200_engine_destroy(native)
             self._native = None
+
+    # ---------------------------------------------------------------------------------- tables
+    def _tables_desc(self) -> np.ndarray:
+        t = np.zeros(self.L, TABLES_DESC)
+        for i, tb in enumerate(self.tables):
+            for k in ("cents_k", "cents_v", "vq", "k_rotor", "v_rotor", "d_k", "d_v"):
+                t[k][i] = tb[k].data_ptr()
+            t["alpha_k"][i], t["alpha_v"][i] = tb["alpha_k"], tb["alpha_v"]
+        return t
+
+    def _fill_layer_tables(self) -> None:
+        for y, tb in zip(self._layers, self.tables):
+            for f, src in (("d_k", "d_k"), ("cents_k", "cents_k"), ("rotor_k", "k_rotor"), ("d_v", "d_v"), ("cents_v", "cents_v"),
+                           ("rotor_v", "v_rotor"), ("vq", "vq")):
+                setattr(y, f, tb[src].data_ptr())
+            y.ts_k, y.alpha_k, y.ts_v, y.alpha_v = tb["ts_k"], tb["alpha_k"], tb["ts_v"], tb["alpha_v"]
+
+    def refresh_tables(self) -> None:
+        """Entries of ``self.tables`` have been replaced or written into: the steps behind this call use the new values.  Waits for
+        the device."""
+        with torch.cuda.device(self.device):
+            torch.cuda.synchronize()  # steps in flight read the old tables; writes into the new ones have to be complete
+            t = self._tables_desc()
+            self.d_tables.copy_(torch.from_numpy(t.view(np.uint8).reshape(-1).copy()))
+            self._images.copy_(prepare_tables(t, self.rope_theta, self.device))
+            self._fill_layer_tables()
+            torch.cuda.synchronize()
 
     # ---------------------------------------------------------------------------------- sizes
     @property

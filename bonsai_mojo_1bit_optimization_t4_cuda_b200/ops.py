@@ -185,6 +185,12 @@ class CudaOps:
     def ring_write(self, dst_row, src):
         dst_row.copy_(src.reshape(dst_row.shape), non_blocking=True)
 
+    def finish_device(self):
+        """Waits for all streams of the current device."""
+        import torch
+
+        torch.cuda.synchronize()
+
     def synchronize(self):
         import torch
 

@@ -46,13 +46,55 @@ def _env_int(name: str, fallback: int) -> int:
 
 
 class _Tensors(dict):
-    """A layer's tensors by name.  ``ctx`` is the native context that keeps their addresses; replacing a tensor drops it."""
+    """A layer's tensors by name.  ``ctx`` is the native context made from them (their addresses, and the tables as the decode
+    kernels use them); every change of the dict drops it.  Dropped ones wait in ``old``: steps may still be running from them."""
 
     ctx = None
+    old = ()
 
-    def __setitem__(self, name, value):
-        self.ctx = None
-        dict.__setitem__(self, name, value)
+    def drop(self):
+        if self.ctx is not None:
+            self.old += (self.ctx,)
+            self.ctx = None
+
+    def _dropping(name):
+        change = getattr(dict, name)
+
+        def method(self, *args, **kwargs):
+            self.drop()
+            return change(self, *args, **kwargs)
+
+        method.__name__ = name
+        return method
+
+    for _name in ("__setitem__", "__delitem__", "__ior__", "update", "setdefault", "pop", "popitem", "clear"):
+        locals()[_name] = _dropping(_name)
+    del _dropping, _name
+
+
+# the tables that a native context holds in another form
+KHQ_TABLES = ("dk", "ck", "rk", "dv", "cv", "rv", "vq")
+
+
+def _version(tables) -> int:
+    """Grows with every write that torch makes into one of the tables."""
+    n = 0
+    for t in tables:
+        n += t._version
+    return n
+
+
+def _constant(name):
+    """A scalar of a layer that its native context holds a copy of: assigning it drops the context."""
+
+    def get(self):
+        return self.__dict__[name]
+
+    def put(self, value):
+        self.__dict__[name] = value
+        self.t.drop()
+
+    return property(get, put)
 
 
 def _row_address(row, kv: int, device: int) -> int:
@@ -67,9 +109,18 @@ def _row_address(row, kv: int, device: int) -> int:
 
 
 class KhqLayer:
-    """KHQ state of one attention layer (all tensors live on the runtime's device)."""
+    """KHQ state of one attention layer (all tensors live on the runtime's device).
+
+    The scalars and the tables may be replaced or, by torch operations on the runtime's stream, written into; the next step uses the
+    new values.  After a write that torch does not count (another library's kernel, ``.data``, tensors made in inference mode)
+    call ``KhqRuntime.khq_refresh_tables``."""
+
+    ts_k, alpha_k, ts_v, alpha_v = (_constant(n) for n in ("ts_k", "alpha_k", "ts_v", "alpha_v"))
 
     def __init__(self):
+        # tables: h_dk h_ck h_rk h_dv h_cv h_rv h_vq; rings: h_ring_k h_ring_v h_ring_u;
+        # payload: h_kmask h_kpay h_knorm h_krn h_vpay h_vnorm h_vrn h_vsm; scratch: h_ac h_aw h_ap
+        self.t: Dict[str, torch.Tensor] = {}
         self.ready = False
         self.has_tables = False
         self.ts_k, self.alpha_k, self.ts_v, self.alpha_v = 1.0, 1.0, 1.95, 1.0
@@ -78,12 +129,21 @@ class KhqLayer:
         self.cap = 0
         self.boundary = 0
         self.write_pos = 0
-        # tables: h_dk h_ck h_rk h_dv h_cv h_rv h_vq; rings: h_ring_k h_ring_v h_ring_u;
-        # payload: h_kmask h_kpay h_knorm h_krn h_vpay h_vnorm h_vrn h_vsm; scratch: h_ac h_aw h_ap
-        self.t: Dict[str, torch.Tensor] = _Tensors()
+
+    @property
+    def t(self) -> Dict[str, torch.Tensor]:
+        return self._t
+
+    @t.setter
+    def t(self, tensors) -> None:
+        old = self.__dict__.get("_t")
+        self._t = _Tensors(tensors)
+        if old is not None:
+            old.drop()
+            self._t.old = old.old
 
     def __getattr__(self, name):  # h_xxx accessors, as the reference's fields are named
-        t = self.__dict__.get("t")
+        t = self.__dict__.get("_t")
         if t is not None and name.startswith("h_") and name[2:] in t:
             return t[name[2:]]
         raise AttributeError(name)
@@ -230,12 +290,28 @@ class KhqRuntime:
 
     # ------------------------------------------------------------------ native step
     def _native_ctx(self, L):
-        """The layer's native context (addresses and prepared tables), None where the backend has none."""
+        """The layer's native context (addresses, and tables in the kernels' form), None where the backend has none."""
+        T = L.t
+        if T.ctx is not None and _version(T.counted) == T.version:
+            return T.ctx
         make = getattr(self.ops, "layer_ctx", None)
         if make is None or (L.H_q, L.H_kv, L.D) != (24, 4, 256):
             return None
-        L.t.ctx = make(L, KHQ_RING, ROPE_BASE)
-        return L.t.ctx
+        if self.device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+            return None  # tables laid out in a graph would be there only once it has run
+        T.drop()
+        if T.old:
+            self.ops.finish_device()
+            T.old = ()
+        T.counted = [T[n] for n in KHQ_TABLES if not T[n].is_inference()]
+        T.version = _version(T.counted)
+        T.ctx = make(L, KHQ_RING, ROPE_BASE)
+        return T.ctx
+
+    def khq_refresh_tables(self, layer_idx: int) -> None:
+        """The layer's tables have been written into in a way that torch does not count: the next step reads them anew.  The writes
+        have to be complete, or queued on the stream of that step."""
+        self.layers[layer_idx].t.drop()
 
     def _native_step(self, layer_idx: int, L, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, scale: float) -> bool:
         """The step of one layer (append, event if due, both regions, merge, gate) as one native call.
@@ -244,7 +320,7 @@ class KhqRuntime:
         window = L.write_pos + 1 - L.boundary
         if self.prof or self.debug or window > KHQ_RING or window <= 0:
             return False
-        ctx = L.t.ctx or self._native_ctx(L)
+        ctx = self._native_ctx(L)
         if ctx is None:
             return False
         kv, device = L.H_kv * L.D, L.t["ring_k"].get_device()
@@ -457,7 +533,7 @@ class KhqRuntime:
     def _native_prefill(self, L, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T: int, n_chunks: int, scale: float) -> bool:
         """The whole prompt of one layer as one native call.  False: another backend or shape, other types than fp16, or rows that
         need a copy first (not contiguous, or not on 16 bytes)."""
-        ctx = L.t.ctx or self._native_ctx(L)
+        ctx = self._native_ctx(L)
         if ctx is None:
             return False
         for t in (q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev):

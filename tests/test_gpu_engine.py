@@ -106,3 +106,41 @@ def test_engine_decodes_like_independent_runtimes(cuda_ops, generation):
             for ring, rkey in ((eng.ring_k, "ring_k"), (eng.ring_v, "ring_v"), (eng.ring_u, "ring_u")):
                 assert torch.equal(ring[l][s].reshape(-1), Lr.t[rkey].reshape(-1)), f"sequence {s} layer {l}: {rkey} differs"
     print(f"engine vs independent runtimes, generation {generation}: {eng.events_fired} events, worst output |err| {worst:.2e}")
+
+
+def _small_engine(layers, seqs=2, alpha_v=1.0):
+    """An engine with the same tables in every layer, on synthetic state and inputs."""
+    import torch
+
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.engine import BatchEngine
+
+    rng = np.random.default_rng(4)
+    k, v = cases.synth.make_kv(rng, 64)
+    tb = cases.synth.make_tables(rng, 3, k.reshape(-1, D), v.reshape(-1, D), vq_scale=1.0 / 16.0)
+    tb.alpha_v = alpha_v
+    eng = BatchEngine([tb] * layers, [256, 128][:seqs], [150, 140][:seqs], grow_tokens=128)
+    eng.fill_synthetic(7)
+    g = torch.Generator().manual_seed(9)
+    for h in (eng.h_q, eng.h_k, eng.h_v):
+        h.copy_(torch.randn(h.shape, generator=g).half())
+    return eng
+
+
+def test_refreshed_tables(cuda_ops):
+    """Tables changed behind the constructor take effect with refresh_tables."""
+    import torch
+
+    want, eng = _small_engine(2, alpha_v=0.5), _small_engine(2)
+    for l in range(2):  # the same code words and raw tokens
+        for n, t in eng.pay[l].items():
+            want.pay[l][n].copy_(t)
+        for a, b in ((want.ring_k, eng.ring_k), (want.ring_v, eng.ring_v), (want.ring_u, eng.ring_u)):
+            a[l].copy_(b[l])
+        want.tables[l]["vq"].mul_(0.75)
+    want.refresh_tables()
+    for tb in eng.tables:
+        tb["vq"], tb["alpha_v"] = tb["vq"] * 0.75, 0.5
+    eng.refresh_tables()
+    a, b = want.decode_step(SCALE), eng.decode_step(SCALE)
+    torch.cuda.synchronize()
+    assert a.any() and torch.equal(a, b)

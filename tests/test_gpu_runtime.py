@@ -341,3 +341,42 @@ def test_rows_in_other_forms(cuda_ops, at, fused):
         assert ok, f"{name}: max abs {mx:.3e}, excess {exc:.3e}"
         for n, t in state.items():
             assert torch.equal(t, got["plain"][1][n]), (name, n)
+
+
+@pytest.mark.parametrize("change", ["alpha_v", "ts_k", "vq in place", "dk replaced"])
+def test_changed_tables_take_effect(cuda_ops, change):
+    """A scalar or a table that changes between two steps: the native steps behind it agree with the call-by-call sequence (which
+    profiling takes), also on the compression event that follows."""
+    import torch
+
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.runtime import KhqRuntime
+
+    n = 390  # events at 256 and 384, the change at 300
+    case = cases.make_case(cases.synth.seed_for(1, 25), n, "calib", layer_id=3)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    ku, kr, v, q = dev(case["k_unroped"]), dev(case["k_roped"]), dev(case["v"]), dev(case["q_gate"])
+    got = []
+    for prof in (False, True):
+        rt = KhqRuntime(cuda_ops, device="cuda")
+        assert rt.khq_activate([case["tables"]], max_seq=512)
+        rt.khq_init_layer(3, H_Q, H_KV, D)
+        rt.prof = prof
+        L, outs = rt.layers[3], []
+        for t in range(n):
+            if t == 300:
+                if change == "vq in place":
+                    L.t["vq"].mul_(0.5)
+                elif change == "dk replaced":
+                    L.t["dk"] = -L.t["dk"]
+                else:
+                    setattr(L, change, 0.5 * getattr(L, change))
+            out = torch.zeros(H_Q * D, dtype=torch.float16, device="cuda")
+            assert rt.khq_step_fused(3, q, ku[t], kr[t], v[t], out, SCALE)
+            if t in (299, 300, 389):
+                outs.append(out.float().cpu().numpy())
+        got.append((outs, {a: L.t[a].clone() for a in ("kmask", "kpay", "krn", "vpay", "vrn")}))
+    for i in range(3):
+        ok, mx, exc = cases.attention_close(got[0][0][i], got[1][0][i])
+        assert ok, f"max abs {mx:.3e}, excess {exc:.3e}"
+    for a, t in got[0][1].items():
+        assert torch.equal(t, got[1][1][a]), a
