@@ -28,6 +28,15 @@ extern "C" int khq_b200_engine_destroy(khq_engine* e) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != e->device) cudaSetDevice(e->device);
+    // The caller frees the step's buffers behind this call, and no allocator knows of the copies: wait for them.  The output copies
+    // follow the step's kernels.  (Relaxed: waiting for these streams does not concern a capture on another one.)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    for (int i = 0; i < 2; ++i)
+        if (e->control_used[i]) cudaEventSynchronize(e->control[i]);
+    if (e->in) cudaStreamSynchronize(e->in);
+    if (e->out) cudaStreamSynchronize(e->out);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     for (int i = 0; i < MAX_LAYERS; ++i) {
         if (e->ready[i]) cudaEventDestroy(e->ready[i]);
         if (e->done[i]) cudaEventDestroy(e->done[i]);

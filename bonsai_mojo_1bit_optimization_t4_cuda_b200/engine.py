@@ -209,7 +209,7 @@ class BatchEngine:
             check("launch_khq_update_descs", self.lib.launch_khq_update_descs(self.d_descs.data_ptr(), self.d_dyn.data_ptr(), self.B,
                                                                               self.L, current_stream()))
 
-    def __del__(self):
+    def __del__(self):  # the buffers go after this, which waits for the copies of a step in flight
         native = getattr(self, "_native", None)
         if native:
             self.lib.khq_b200_engine_destroy(native)
@@ -366,7 +366,8 @@ class BatchEngine:
         synchronised)."""
         parity = self._step & 1
         ctl, a, lib = self._ctl[parity], self._args, self.lib
-        lib.khq_b200_engine_wait_control(self._native, parity)  # the copy that last read this parity's host block has finished
+        # the copy that last read this parity's host block has finished
+        check("khq_b200_engine_wait_control", lib.khq_b200_engine_wait_control(self._native, parity))
         # ---- host state machine (src/khq/runtime.mojo:486-553, for every sequence) -----------------
         window = self.write_pos + 1 - self.boundary
         due = (window >= WATERMARK) & (self.boundary + CHUNK <= self.cap)

@@ -315,7 +315,8 @@ int launch_khq_layer_prefill(const khq_layer_ctx* ctx, const void* q_gate, const
  * launch_khq_update_descs.  d_items, d_dyn, d_slots, d_pos and d_segs lie inside the device control block.  h_q (n_layers,
  * n_seq, 24 * 512), h_k / h_v (n_layers, n_seq, 4 * 256), h_out (n_layers, n_seq, 24 * 256) fp16 and the device buffers of
  * the same shapes.  The caller's stream waits for the output copies.  Calls on one engine come from one thread at a time;
- * parity (0 or 1) says which of two control blocks is used, khq_b200_engine_wait_control returns when it may be rewritten. */
+ * parity (0 or 1) says which of two control blocks is used, khq_b200_engine_wait_control returns when it may be rewritten.
+ * khq_b200_engine_destroy returns when the engine's copies have ended, so the buffers may be freed behind it. */
 typedef struct khq_engine khq_engine;
 typedef struct khq_engine_layer {
     const void *d_k, *cents_k, *rotor_k, *d_v, *cents_v, *rotor_v, *vq;

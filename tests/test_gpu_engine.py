@@ -144,3 +144,25 @@ def test_refreshed_tables(cuda_ops):
     a, b = want.decode_step(SCALE), eng.decode_step(SCALE)
     torch.cuda.synchronize()
     assert a.any() and torch.equal(a, b)
+
+
+def test_engine_dropped_with_a_step_in_flight(cuda_ops):
+    """An engine that goes away while its step is still queued waits for it: the outputs are complete behind that."""
+    import gc
+
+    import torch
+
+    eng = _small_engine(3)
+    want = eng.decode_step(SCALE)
+    torch.cuda.synchronize()
+    want = want.clone()
+    del eng
+    eng = _small_engine(3)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about a tenth of a second in front of the step
+    got = eng.decode_step(SCALE)
+    assert not torch.cuda.current_stream().query()
+    del eng
+    gc.collect()
+    assert want.any() and torch.equal(got, want)
+    torch.cuda.synchronize()
