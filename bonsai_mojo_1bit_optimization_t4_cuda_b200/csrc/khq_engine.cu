@@ -11,14 +11,17 @@
 
 namespace {
 constexpr int HKV = 4, HQ = 24, D = 256, KV = HKV * D, QG = HQ * 2 * D, CHUNK_ROWS = 128 * HKV;
-constexpr int MAX_LAYERS = 64;
 }  // namespace
 
 // Streams and events of one engine: nothing of it is shared with another engine.
 struct khq_engine {
     int device;
     cudaStream_t in, out;                       // host -> device and device -> host copies, beside the kernels
-    cudaEvent_t ready[MAX_LAYERS], done[MAX_LAYERS];  // a chunk of layers: inputs landed, outputs computed
+    struct Chunk {
+        cudaEvent_t ready, done;                // a chunk of layers: inputs landed, outputs computed
+    };
+    Chunk* chunks;
+    int n_chunks;
     cudaEvent_t begin, end, control[2];
     bool control_used[2];
 };
@@ -37,10 +40,11 @@ extern "C" int khq_b200_engine_destroy(khq_engine* e) {
     if (e->in) cudaStreamSynchronize(e->in);
     if (e->out) cudaStreamSynchronize(e->out);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    for (int i = 0; i < MAX_LAYERS; ++i) {
-        if (e->ready[i]) cudaEventDestroy(e->ready[i]);
-        if (e->done[i]) cudaEventDestroy(e->done[i]);
+    for (int i = 0; i < e->n_chunks; ++i) {
+        cudaEventDestroy(e->chunks[i].ready);
+        cudaEventDestroy(e->chunks[i].done);
     }
+    delete[] e->chunks;
     cudaEvent_t more[] = {e->begin, e->end, e->control[0], e->control[1]};
     for (cudaEvent_t v : more)
         if (v) cudaEventDestroy(v);
@@ -61,10 +65,6 @@ extern "C" int khq_b200_engine_create(khq_engine** out) {
     };
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->in, cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->out, cudaStreamNonBlocking);
-    for (int i = 0; i < MAX_LAYERS; ++i) {
-        event(&e->ready[i]);
-        event(&e->done[i]);
-    }
     event(&e->begin);
     event(&e->end);
     event(&e->control[0]);
@@ -77,15 +77,39 @@ extern "C" int khq_b200_engine_create(khq_engine** out) {
     return 0;
 }
 
+// Events for at least n chunks: created by the first step, as many as its chunks of layers.
+static cudaError_t have_chunks(khq_engine* e, int n) {
+    if (n <= e->n_chunks) return cudaSuccess;
+    khq_engine::Chunk* more = new (std::nothrow) khq_engine::Chunk[n];
+    if (!more) return cudaErrorMemoryAllocation;
+    for (int i = 0; i < e->n_chunks; ++i) more[i] = e->chunks[i];
+    delete[] e->chunks;
+    e->chunks = more;
+    while (e->n_chunks < n) {
+        khq_engine::Chunk c = {};
+        cudaError_t err = cudaEventCreateWithFlags(&c.ready, cudaEventDisableTiming);
+        if (err != cudaSuccess) return err;
+        err = cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming);
+        if (err != cudaSuccess) {
+            cudaEventDestroy(c.ready);
+            return err;
+        }
+        more[e->n_chunks++] = c;
+    }
+    return cudaSuccess;
+}
+
 extern "C" int khq_b200_engine_wait_control(khq_engine* e, int parity) {
     if (!e || parity < 0 || parity > 1) return -100;
     return e->control_used[parity] ? static_cast<int>(cudaEventSynchronize(e->control[parity])) : 0;
 }
 
 extern "C" int launch_khq_engine_step(khq_engine* e, const khq_engine_layer* layers, const khq_engine_step* s, khq_stream_t stream) {
-    if (!e || !layers || !s || s->n_layers <= 0 || s->n_layers > MAX_LAYERS || s->n_seq <= 0) return -100;
-    const int L = s->n_layers, B = s->n_seq, per = s->layers_per_chunk > 0 ? s->layers_per_chunk : 1;
-    cudaError_t err = cudaSuccess;
+    if (!e || !layers || !s || s->n_layers <= 0 || s->n_seq <= 0) return -100;
+    const int L = s->n_layers, B = s->n_seq;
+    const int per = s->layers_per_chunk <= 0 ? 1 : s->layers_per_chunk < L ? s->layers_per_chunk : L, chunks = (L + per - 1) / per;
+    cudaError_t err = have_chunks(e, chunks);
+    if (err != cudaSuccess) return static_cast<int>(err);
     const auto ok = [&](cudaError_t r) {
         if (err == cudaSuccess) err = r;
         return err == cudaSuccess;
@@ -99,20 +123,19 @@ extern "C" int launch_khq_engine_step(khq_engine* e, const khq_engine_layer* lay
     ok(cudaStreamWaitEvent(e->in, e->begin, 0));
     if (err != cudaSuccess) return static_cast<int>(err);
     const size_t q_row = (size_t)B * QG * 2, kv_row = (size_t)B * KV * 2, o_row = (size_t)B * HQ * D * 2;
-    const int chunks = (L + per - 1) / per;
     const auto stage = [&](int c) {  // inputs of chunk c: three copies, whatever the number of its layers
         const size_t l0 = (size_t)c * per, n = l0 + per <= (size_t)L ? per : L - l0;
         ok(cudaMemcpyAsync(static_cast<char*>(s->d_q) + l0 * q_row, static_cast<const char*>(s->h_q) + l0 * q_row, n * q_row, cudaMemcpyHostToDevice, e->in));
         ok(cudaMemcpyAsync(static_cast<char*>(s->d_k) + l0 * kv_row, static_cast<const char*>(s->h_k) + l0 * kv_row, n * kv_row, cudaMemcpyHostToDevice, e->in));
         ok(cudaMemcpyAsync(static_cast<char*>(s->d_v) + l0 * kv_row, static_cast<const char*>(s->h_v) + l0 * kv_row, n * kv_row, cudaMemcpyHostToDevice, e->in));
-        ok(cudaEventRecord(e->ready[c], e->in));
+        ok(cudaEventRecord(e->chunks[c].ready, e->in));
     };
     stage(0);
     int rc = launch_khq_update_descs(s->descs, s->d_dyn, B, L, stream);
     if (rc != 0) return rc;
     for (int c = 0; c < chunks; ++c) {
         if (c + 1 < chunks) stage(c + 1);
-        if (!ok(cudaStreamWaitEvent(stream, e->ready[c], 0))) return static_cast<int>(err);
+        if (!ok(cudaStreamWaitEvent(stream, e->chunks[c].ready, 0))) return static_cast<int>(err);
         const int hi = (c + 1) * per < L ? (c + 1) * per : L;
         for (int l = c * per; l < hi; ++l) {
             const khq_engine_layer& y = layers[l];
@@ -136,8 +159,8 @@ extern "C" int launch_khq_engine_step(khq_engine* e, const khq_engine_layer* lay
                                                 s->codebook_in_smem, stream);
             if (rc != 0) return rc;
         }
-        ok(cudaEventRecord(e->done[c], stream));
-        ok(cudaStreamWaitEvent(e->out, e->done[c], 0));
+        ok(cudaEventRecord(e->chunks[c].done, stream));
+        ok(cudaStreamWaitEvent(e->out, e->chunks[c].done, 0));
         const size_t l0 = (size_t)c * per;
         ok(cudaMemcpyAsync(static_cast<char*>(s->h_out) + l0 * o_row, static_cast<const char*>(s->d_out) + l0 * o_row, (hi - l0) * o_row,
                            cudaMemcpyDeviceToHost, e->out));

@@ -166,3 +166,24 @@ def test_engine_dropped_with_a_step_in_flight(cuda_ops):
     gc.collect()
     assert want.any() and torch.equal(got, want)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("layers,per_chunk", [(65, 1), (66, 0)])  # 0: as the constructor chooses
+def test_more_than_64_layers(cuda_ops, layers, per_chunk):
+    """The number of layers, and of the groups that are copied together, has no limit: the outputs of every layer are those that the
+    attention alone gives over the state behind the step."""
+    import torch
+
+    eng = _small_engine(layers)
+    if per_chunk:
+        eng._args.layers_per_chunk = per_chunk
+    got = eng.decode_step(SCALE)
+    torch.cuda.synchronize()
+    got = got.clone()
+    for l in range(layers):
+        eng.out[l].zero_()
+        eng.attention_resident(l, SCALE)
+    torch.cuda.synchronize()
+    assert got.any(-1).all() and torch.equal(got, eng._out.cpu())
+    assert eng.decode_step(SCALE) is eng.h_out
+    torch.cuda.synchronize()
