@@ -23,6 +23,7 @@ slice sized for its capacity and starting on a 128-row boundary.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 from typing import Optional, Sequence
 
@@ -59,8 +60,8 @@ class BatchEngine:
         """``c_len`` / ``win_len``: compressed and raw tokens each sequence starts with (``c_len`` a
         multiple of 128, as the state machine leaves it).  ``grow_tokens``: compressed capacity kept
         free behind every sequence's initial prefix.  ``norm_weights``: per layer ``(q_w, k_w)`` fp32
-        (256,) arrays for the head RMS norms, or None for the unweighted norm.  The tables (``self.tables``) are laid out
-        for the kernels here: whoever changes one of them later calls ``refresh_tables``."""
+        (256,) arrays for the head RMS norms, or None for the unweighted norm.  The tables (``self.tables``) and norms
+        (``self.norm_w``) are laid out for the kernels here: whoever changes one of them later calls ``refresh_tables``."""
         self.lib = _lib.load()
         self.device = torch.device(device)
         self.L = len(tables)
@@ -161,6 +162,8 @@ class BatchEngine:
         self.h_k = pin(self.L, self.B, KV)
         self.h_v = pin(self.L, self.B, KV)
         self.h_out = pin(self.L, self.B, H_Q * D)
+        self._staging = dict(q=self.h_q, k=self.h_k, v=self.h_v, out=self.h_out)
+        self._in_flight = collections.deque(maxlen=4)  # host buffers of the last steps (at most two are not complete)
         self._ctl = []
         for _ in range(2):
             block = pin(n, dt=torch.uint8)
@@ -180,12 +183,9 @@ class BatchEngine:
             for f, src in self.pay[l].items():
                 setattr(y, f, src.data_ptr())
             y.ring_k, y.ring_v, y.ring_u = self.ring_k[l].data_ptr(), self.ring_v[l].data_ptr(), self.ring_u[l].data_ptr()
-            if self.norm_w is not None:
-                y.q_norm, y.k_norm = self.norm_w[l][0].data_ptr(), self.norm_w[l][1].data_ptr()
         self._fill_layer_tables()
         self._ring_u_at = np.array([r.data_ptr() for r in self.ring_u], np.uint64)
         a = self._args = _lib.EngineStep()
-        a.h_q, a.h_k, a.h_v, a.h_out = self.h_q.data_ptr(), self.h_k.data_ptr(), self.h_v.data_ptr(), self.h_out.data_ptr()
         a.d_q, a.d_k, a.d_v, a.d_out = self._q.data_ptr(), self._k.data_ptr(), self._v.data_ptr(), self._out.data_ptr()
         base = self.d_control.data_ptr()
         a.d_control = base
@@ -194,8 +194,8 @@ class BatchEngine:
         a.descs, a.tables, a.workspace, a.workspace_bytes = (self.d_descs.data_ptr(), self.d_tables.data_ptr(), self.workspace.data_ptr(),
                                                              self.ws_bytes)
         a.images = self._d_images.data_ptr()
-        a.n_layers, a.n_seq, a.ring_cap, a.rotary_dim, a.codebook_in_smem = self.L, self.B, RING, ROTARY_DIM, int(codebook_in_smem)
-        a.rope_theta, a.rms_eps = self.rope_theta, self.rms_eps
+        a.n_layers, a.n_seq, a.ring_cap, a.rotary_dim = self.L, self.B, RING, ROTARY_DIM
+        self._laid_out_theta = a.rope_theta = self.rope_theta
         # A copy of a few tens of KB takes as long as one of 256 KB (3-4 us): layers are copied in groups of about that
         # much, at most half of them at once so that copies and kernels still overlap.
         a.layers_per_chunk = int(min(max(COPY_BYTES // (self.B * (H_Q * 2 * D + 2 * KV) * 2), 1), max(self.L // 2, 1)))
@@ -225,21 +225,24 @@ class BatchEngine:
         return t
 
     def _fill_layer_tables(self) -> None:
-        for y, tb in zip(self._layers, self.tables):
+        for l, (y, tb) in enumerate(zip(self._layers, self.tables)):
+            if self.norm_w is not None:
+                y.q_norm, y.k_norm = self.norm_w[l][0].data_ptr(), self.norm_w[l][1].data_ptr()
             for f, src in (("d_k", "d_k"), ("cents_k", "cents_k"), ("rotor_k", "k_rotor"), ("d_v", "d_v"), ("cents_v", "cents_v"),
                            ("rotor_v", "v_rotor"), ("vq", "vq")):
                 setattr(y, f, tb[src].data_ptr())
             y.ts_k, y.alpha_k, y.ts_v, y.alpha_v = tb["ts_k"], tb["alpha_k"], tb["ts_v"], tb["alpha_v"]
 
     def refresh_tables(self) -> None:
-        """Entries of ``self.tables`` have been replaced or written into: the steps behind this call use the new values.  Waits for
-        the device."""
+        """Entries of ``self.tables`` have been replaced or written into, or ones of ``self.norm_w`` replaced: the steps behind this
+        call use the new values.  Waits for the device."""
         with torch.cuda.device(self.device):
             torch.cuda.synchronize()  # steps in flight read the old tables; writes into the new ones have to be complete
             t = self._tables_desc()
             self.d_tables.copy_(torch.from_numpy(t.view(np.uint8).reshape(-1).copy()))
             self._images.copy_(prepare_tables(t, self.rope_theta, self.device))
             self._fill_layer_tables()
+            self._laid_out_theta = self._args.rope_theta = self.rope_theta
             torch.cuda.synchronize()
 
     # ---------------------------------------------------------------------------------- sizes
@@ -358,12 +361,19 @@ class BatchEngine:
             int(self.codebook_in_smem), current_stream())
         check("launch_khq_decode_batched_prepared_fp16", rc)
 
+    def _host_buffer(self, t, name: str):
+        """``t`` if the native step can copy from or to it as it is, else the engine's own buffer of that name."""
+        own = self._staging[name]
+        plain = isinstance(t, torch.Tensor) and t.is_cpu and t.dtype is torch.float16 and t.numel() == own.numel() and t.is_contiguous()
+        return t if plain else own
+
     def decode_step(self, scale: float = 1.0 / 16.0) -> torch.Tensor:
         """End-to-end token step from HOST buffers.  ``h_q`` (L, B, 24*512: query and gate halves, the
         query not yet normed or rotated), ``h_k`` and ``h_v`` (L, B, 4*256) hold this step's projections
         in pinned host memory.  Every sequence advances by one token: append, compression event if
         due, attention.  The gated outputs land in ``h_out`` (returned; valid once the stream has
-        synchronised)."""
+        synchronised).  Any of the four may be replaced by another tensor between steps; what is not contiguous
+        fp16 in host memory costs a wait and a copy."""
         parity = self._step & 1
         ctl, a, lib = self._ctl[parity], self._args, self.lib
         # the copy that last read this parity's host block has finished
@@ -389,5 +399,21 @@ class BatchEngine:
         self._plan(ctl)
         a.h_control, a.control_bytes, a.parity = ctl["block"].data_ptr(), self._control_bytes(n_ev), parity
         a.n_items, a.n_events, a.scale = self.n_items, n_ev, float(scale)
+        a.codebook_in_smem, a.rms_eps = int(self.codebook_in_smem), self.rms_eps
+        if self.rope_theta != self._laid_out_theta:
+            self.refresh_tables()
+        given = dict(q=self.h_q, k=self.h_k, v=self.h_v, out=self.h_out)
+        host = {n: self._host_buffer(t, n) for n, t in given.items()}
+        for n in ("q", "k", "v"):
+            if host[n] is not given[n]:
+                torch.cuda.current_stream().synchronize()  # the step before has copied from the engine's buffer
+                for l in range(self.L):
+                    host[n][l].copy_(given[n][l])
+        a.h_q, a.h_k, a.h_v, a.h_out = host["q"].data_ptr(), host["k"].data_ptr(), host["v"].data_ptr(), host["out"].data_ptr()
+        self._in_flight.append(host)
         check("launch_khq_engine_step", lib.launch_khq_engine_step(self._native, self._layers, ctypes.addressof(a), current_stream()))
+        if host["out"] is not given["out"]:
+            torch.cuda.current_stream().synchronize()
+            for l in range(self.L):
+                given["out"][l].copy_(host["out"][l])
         return self.h_out

@@ -187,3 +187,40 @@ def test_more_than_64_layers(cuda_ops, layers, per_chunk):
     assert got.any(-1).all() and torch.equal(got, eng._out.cpu())
     assert eng.decode_step(SCALE) is eng.h_out
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("form", ["pinned", "pageable", "fp32", "strided", "device", "list"])
+def test_replaced_host_buffers(cuda_ops, form):
+    """The host buffers are the attributes' at every step: other tensors of the same values give the same outputs."""
+    import torch
+
+    eng = _small_engine(3)
+    start = eng.boundary.copy(), eng.write_pos.copy()
+
+    def step():
+        eng.boundary[:], eng.write_pos[:] = start
+        return eng.decode_step(SCALE)
+
+    first = step()
+    torch.cuda.synchronize()
+    first = first.clone()
+    g = torch.Generator().manual_seed(19)
+    other = [torch.randn(h.shape, generator=g).half() for h in (eng.h_q, eng.h_k, eng.h_v)]
+    own = eng.h_q, eng.h_k, eng.h_v, eng.h_out
+    for h, x in zip(own, other):
+        h.copy_(x)
+    want = step()
+    torch.cuda.synchronize()
+    want = want.clone()
+    assert not torch.equal(want, first)
+    for h in own:
+        h.fill_(float("nan"))  # nothing may be read from here any more
+    make = dict(pinned=lambda x: x.pin_memory(), pageable=lambda x: x.clone(), fp32=lambda x: x.float(), device=lambda x: x.cuda(),
+                strided=lambda x: torch.stack([x, x], -1)[..., 0], list=lambda x: [r.clone() for r in x])[form]
+    eng.h_q, eng.h_k, eng.h_v = (make(x) for x in other)
+    eng.h_out = make(torch.zeros_like(want))
+    got = step()
+    assert got is eng.h_out
+    torch.cuda.synchronize()
+    got = torch.stack(list(got)) if form == "list" else got
+    assert torch.equal(got.cpu().half(), want)
