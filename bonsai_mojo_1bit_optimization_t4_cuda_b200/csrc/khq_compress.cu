@@ -14,24 +14,27 @@
 // Arithmetic that feeds a threshold or a rounding is written with explicit __fmaf_rn where the
 // reference's build (default -fmad=true) fuses a multiply into the following add/subtract.
 #include "khq_common.cuh"
+#include "khq_launch.cuh"
 
 namespace khq {
 
 constexpr int CMP_WARPS = 4;  // warps per block, each on its own row or group of rows
 constexpr int CMP_KROWS = 4;  // K rows that a warp takes together (large launches)
 constexpr int CMP_VROWS = 4;  // V rows of a CTA whose warps share the code search
-// Below this a K launch keeps one row per warp: groups of four give each of 16 warps per SM one group (148 x 16 x 4 rows), and
+// The rules count rows per SM; the figures are of 148 SMs.
+// Below 64 rows an SM a K launch keeps one row per warp: groups of four give each of 16 warps per SM one group (9472 rows), and
 // fewer rows than that leave warps without work (8192 rows: 26.4 us either way, 4096: 15.5 against 20.8, 16 384: 47.1 against
 // 38.8).  Eight rows a warp cost more in occupancy than their shared sums save (129 024 rows: 259 against 227 us).
-constexpr long long CMP_KROWS_MIN_N = 9472;
-// V launches.  Up to two CTAs of four rows per SM (148 x 2 x 4 rows) the length of one CTA is what counts: 16 warps (512 rows:
+constexpr long long CMP_KROWS_MIN_PER_SM = 16 * CMP_KROWS;
+// V launches.  Up to two CTAs of four rows per SM (1184 rows) the length of one CTA is what counts: 16 warps (512 rows:
 // 9.2 us, 11.1 with 8 warps).  Above, 8 warps overlap more of the unshared work (8192 rows: 59 us, 66 with 16), 6.6 us per 1000
-// rows.  The filtered search takes 64 rows per CTA, two CTAs per SM, and 50 us for each time that 148 x 64 rows are begun (61 the
-// first time), so it wins where that is less: from 8485 rows, except just behind a multiple of 9472 up to 29 500 rows.
-constexpr int CMP_V16_MAX_N = 1184;
-inline bool compress_v_filtered(long long n) {
-    const long long waves = (n + 148 * 64 - 1) / (148 * 64);
-    return (waves > 1 ? 50000 * waves : 61000) < 5000 + 33 * n / 5;  // ns
+// rows (977 ns per row an SM).  The filtered search takes 64 rows per CTA, two CTAs per SM, and 50 us for each time that 64 rows
+// an SM are begun (61 the first time), so it wins where that is less: from 8485 rows, except just behind a multiple of 9472 up
+// to 29 500 rows.
+constexpr long long CMP_V16_MAX_PER_SM = 2 * CMP_VROWS;
+inline bool compress_v_filtered(long long n, long long sms) {
+    const long long waves = (n + sms * 64 - 1) / (sms * 64);
+    return (waves > 1 ? 50000 * waves : 61000) < 5000 + 4884 * n / (5 * sms);  // ns
 }
 
 // One run of rows of a batched launch: source rows (fp16, D per row, contiguous) and the first
@@ -895,7 +898,7 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
                     int is_v, const khq::KhqCompressSeg* segs, int rows_per_seg, long long x_byte_offset,
                     cudaStream_t stream) {
     using namespace khq;
-    const long long cap = 148LL * 64;  // grid-stride beyond this
+    const long long sms = sm_count(), cap = sms * 64;  // grid-stride beyond this
     const auto grid = [&](long long units) {
         long long blocks = (units + CMP_WARPS - 1) / CMP_WARPS;
         return (unsigned)(blocks > cap ? cap : blocks);
@@ -907,7 +910,7 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
     __half* orn = static_cast<__half*>(out_r_norms);
     unsigned char* op = static_cast<unsigned char*>(out_payload);
     unsigned char* om = static_cast<unsigned char*>(out_shared_meta);
-    if (!is_v && n >= CMP_KROWS_MIN_N) {
+    if (!is_v && n >= CMP_KROWS_MIN_PER_SM * sms) {
         khq_compress_k_kernel<CMP_KROWS><<<grid(((long long)n + CMP_KROWS - 1) / CMP_KROWS), CMP_WARPS * 32, 0,
                                            stream>>>(x, dv, ro, ce, static_cast<unsigned int*>(out_mask), on, orn, op,
                                                      om, d, n, threshold_scale, segs, rows_per_seg, x_byte_offset);
@@ -915,13 +918,14 @@ int compress_launch(const __half* x, const void* d_vec, const void* rotor, const
         khq_compress_k_kernel<1><<<grid(n), CMP_WARPS * 32, 0, stream>>>(
             x, dv, ro, ce, static_cast<unsigned int*>(out_mask), on, orn, op, om, d, n, threshold_scale, segs,
             rows_per_seg, x_byte_offset);
-    } else if (compress_v_filtered(n)) {
+    } else if (compress_v_filtered(n, sms)) {
         const int rc = launch_v_mma(x, dv, ro, ce, vq_centroids, on, orn, op, om, d, n, alpha, segs, rows_per_seg, x_byte_offset, stream);
         if (rc != 0) return rc;
     } else {
         const unsigned blocks = (unsigned)((n + CMP_VROWS - 1) / CMP_VROWS);
-        const auto kernel = n <= CMP_V16_MAX_N ? khq_compress_v_kernel<16> : khq_compress_v_kernel<8>;
-        kernel<<<blocks, n <= CMP_V16_MAX_N ? 512 : 256, 0, stream>>>(x, dv, ro, ce, static_cast<const __half*>(vq_centroids), on, orn, op,
+        const bool wide = n <= CMP_V16_MAX_PER_SM * sms;
+        const auto kernel = wide ? khq_compress_v_kernel<16> : khq_compress_v_kernel<8>;
+        kernel<<<blocks, wide ? 512 : 256, 0, stream>>>(x, dv, ro, ce, static_cast<const __half*>(vq_centroids), on, orn, op,
                                                                       om, d, n, alpha, segs, rows_per_seg, x_byte_offset);
     }
     const cudaError_t err = cudaGetLastError();

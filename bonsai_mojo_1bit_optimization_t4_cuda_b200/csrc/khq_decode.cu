@@ -964,18 +964,6 @@ static cudaError_t ensure_smem_attrs() {
     return cudaSuccess;
 }
 
-static int sm_count() {
-    static int n[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (n[dev] == 0) {
-        int v = 0;
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-        n[dev] = v;
-    }
-    return n[dev];
-}
-
 // How many clusters of `c` CTAs of the compressed-attention kernel fit on the device at once.
 static int max_clusters(int c) {
     static int cache[64][9] = {};

@@ -4,6 +4,19 @@
 
 namespace khq {
 
+// SMs of the current device (148 where the query fails).
+static inline int sm_count() {
+    static int n[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (n[dev] == 0) {
+        int v = 0;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+        n[dev] = v;
+    }
+    return n[dev];
+}
+
 // cluster == 0: no cluster attribute.  All kernels launched through here begin with pdl_wait() (or know what they may do
 // before it), so they carry the programmatic-serialisation attribute: their launch latency and prologue overlap the end of
 // the kernel before them.
