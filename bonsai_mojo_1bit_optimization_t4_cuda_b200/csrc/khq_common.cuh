@@ -80,7 +80,6 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- small math helpers ---------------------------------------------------------------------
-__device__ __forceinline__ float h2f(__half h) { return __half2float(h); }
 __device__ __forceinline__ float hbits2f(uint16_t b) { return __half2float(__ushort_as_half(b)); }
 
 // Packed pairs of fp32 (one instruction; each half is rounded like the scalar operation).
@@ -120,10 +119,5 @@ __device__ __forceinline__ void fwht256_lane8(float (&v)[8], int lane) {
         }
     }
 }
-
-// Online-softmax state of one query head held redundantly by every lane of a warp.
-struct Softmax {
-    float m, l;
-};
 
 }  // namespace khq

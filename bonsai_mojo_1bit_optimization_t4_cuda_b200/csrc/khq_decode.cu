@@ -317,9 +317,8 @@ __device__ __forceinline__ void compressed_range(unsigned char* smem, const __ha
     tiles_done = t0 + (unsigned)ntiles;
 }
 
-// Inverse V rotor + FWHT + /16/(d_v+1e-8) of the merged state of head h, stored as one
+// Inverse V rotor + FWHT + /16/(d_v+1e-8) of the merged state of the kv-head's heads, each stored as one
 // (acc[256], max, sum_exp) record.  Called by one warp per kv-head.
-template <int H0 = 0, int H1 = NREP>  // heads [H0, H1) of the kv-head: several warps may share the six
 __device__ __forceinline__ void v_epilogue_store(const WarpState& st, const CompressedKV& P, int lane,
                                                  float* const (&ob)[NREP]) {
     float dvi[8];
@@ -344,7 +343,7 @@ __device__ __forceinline__ void v_epilogue_store(const WarpState& st, const Comp
             for (int i = 0; i < 16; ++i) rv[p][i] = __half2float(hr[p * 16 + i]);
     }
 #pragma unroll
-    for (int h = H0; h < H1; ++h) {
+    for (int h = 0; h < NREP; ++h) {
         float z[8];
 #pragma unroll
         for (int p = 0; p < 2; ++p)
@@ -632,12 +631,12 @@ khq_decode_batched_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesD
                 cur_table = d.table_id;
             }
             compressed_range<VQS>(smem, d.q_gate, (size_t)2 * D, P, w.lo, w.hi, scale, st, tiles_done);
-            merge_cta_and_cluster(st, reinterpret_cast<float*>(smem + SM_MERGE_A), kvh, sub, lane);
+            merge_cta(st, reinterpret_cast<float*>(smem + SM_MERGE), kvh, sub, lane);
             if (sub == 0) v_epilogue_store(st, P, lane, ob);
         } else {
             window_range<4>(d.q_gate, d.ring_k, d.ring_v, d.win_start, w.lo + sub, DEC_WPK, w.hi, ring_cap, scale, kvh,
                             lane, st);
-            merge_cta_and_cluster(st, reinterpret_cast<float*>(smem + SM_MERGE_A), kvh, sub, lane);
+            merge_cta(st, reinterpret_cast<float*>(smem + SM_MERGE), kvh, sub, lane);
             if (sub == 0) raw_store(st, lane, ob);
         }
     }

@@ -48,9 +48,8 @@ constexpr int SM_TOTAL_VQ = SM_VQ + 256 * NP * 8;
 static_assert(SM_VQ % 16 == 0 && SM_TOTAL_VQ <= 227 * 1024, "shared memory budget");
 // Per-kv-head merge record: acc[NREP][D], m[NREP], l[NREP]  (+pad to 16 B)
 constexpr int MERGE_FLOATS = NREP * D + 2 * NREP + 4;       // 1552
-constexpr int SM_MERGE_A = 0;                               // aliases the stages after the loop
-constexpr int SM_MERGE_E = SM_MERGE_A + HKV * MERGE_FLOATS * 4;
-static_assert(SM_MERGE_E + HKV * MERGE_FLOATS * 4 <= NSTAGE * STAGE_BYTES, "merge areas alias the stages");
+constexpr int SM_MERGE = 0;                                 // aliases the stages after the loop
+static_assert(SM_MERGE + HKV * MERGE_FLOATS * 4 <= NSTAGE * STAGE_BYTES, "the merge area aliases the stages");
 
 // ---- batched decode: device-resident descriptor tables (mirrored in include/khq_b200.h) -------
 struct KhqSeqDesc {  // one (sequence, layer) decode problem
@@ -206,8 +205,7 @@ __device__ __forceinline__ void accumulate_v(WarpState& st, const float (&p)[NRE
         for (int j = 0; j < 8; ++j) st.acc[h][j] = fmaf(p[h], v[j], st.acc[h][j]);
 }
 
-// st <- LSE-merge(st, record in memory).  rec may point to this CTA's or a peer CTA's shared
-// memory (distributed shared memory of the cluster).
+// st <- LSE-merge(st, record in shared memory).
 __device__ __forceinline__ void merge_from(WarpState& st, const float* rec, int lane) {
 #pragma unroll
     for (int h = 0; h < NREP; ++h) {
@@ -324,35 +322,17 @@ __device__ __forceinline__ void store_head(const HeadAcc& h, float* o, int lane)
     }
 }
 
-// Merge the DEC_WPK warps of each kv-head inside the CTA, then the CTAs of the cluster.  On
-// return the sub==0 warps of cluster rank 0 hold the merged state.  `area` is shared memory no
-// longer used for anything else (>= 2*HKV*MERGE_FLOATS floats).  Must be called by all threads
-// of all CTAs of the cluster.
-__device__ __forceinline__ void merge_cta_and_cluster(WarpState& st, float* area, int kvh, int sub,
-                                                      int lane) {
-    cg::cluster_group cluster = cg::this_cluster();
-    float* recA = area + kvh * MERGE_FLOATS;
-    float* recE = area + (HKV + kvh) * MERGE_FLOATS;
+// Merge the DEC_WPK warps of each kv-head.  On return the sub == 0 warps hold the merged state.  `area` is shared memory no
+// longer used for anything else (HKV * MERGE_FLOATS floats).  Must be called by all threads of the CTA.
+__device__ __forceinline__ void merge_cta(WarpState& st, float* area, int kvh, int sub, int lane) {
+    float* rec = area + kvh * MERGE_FLOATS;
     __syncthreads();
 #pragma unroll
     for (int src = 1; src < DEC_WPK; ++src) {
-        if (sub == src) store_record(st, recA, lane);
+        if (sub == src) store_record(st, rec, lane);
         __syncthreads();
-        if (sub == 0) merge_from(st, recA, lane);
+        if (sub == 0) merge_from(st, rec, lane);
         __syncthreads();
-    }
-    const unsigned nblk = cluster.num_blocks();
-    if (nblk > 1) {
-        if (sub == 0) store_record(st, recE, lane);
-        cluster.sync();
-        if (cluster.block_rank() == 0 && sub == 0) {
-#pragma unroll 1
-            for (unsigned r = 1; r < nblk; ++r) {
-                const float* remote = cluster.map_shared_rank(recE, r);
-                merge_from(st, remote, lane);
-            }
-        }
-        cluster.sync();  // peers must stay resident until rank 0 has read their records
     }
 }
 
