@@ -74,8 +74,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 
 // ---- programmatic dependent launch ------------------------------------------------------------
 // A kernel launched with the attribute may start while the one before it in the stream still runs; wait() returns when
-// that one has completed and its writes are visible.  trigger() lets the next kernel start; it comes after this kernel's
-// own wait(), so that a kernel that has started knows everything before its predecessor to be complete.
+// that one has completed and its writes are visible.  trigger() lets the next kernel start.
+//   * Late trigger, behind the kernel's own wait(): what starts then knows everything before its predecessor to be complete.  All
+//     kernels but those of the next point.
+//   * Early trigger, before the own wait(): the two pre-steps, the counter kernel, and the step's tail with a compressed region.  What
+//     starts behind one of them may run beside the kernel before that one too.
+// So before its own wait() a kernel reads nothing but constants of the model (tables, their image: launch_khq_prepare_tables and
+// the runtime order their writes) and writes nothing.  One exception: khq_window_step_kernel with a compressed region reads the step's
+// inputs and rings and appends to the rings first.  decode_step_impl launches it directly behind the attention or its
+// reduction, which trigger late, read no ring and write none of that.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -732,8 +732,9 @@ khq_batched_merge_partial_kernel(const KhqSeqDesc* __restrict__ descs, const flo
 // the raw-window attention over win_len tokens (the new one is the last), then the cluster's warps
 // merge the heads they are dealt: the window records, the n_c <= 32 records per head of the compressed region
 // (head-major, PART floats each), /(den + 1e-8), sigmoid gate, fp16 store.
-// With n_c > 0 the launch before it in the stream is the compressed-region kernel of the same step, which starts only when
-// everything before it is complete and writes nothing but those records: the window part runs beside it.
+// With n_c > 0 the launch before it in the stream has to be the compressed-region kernel of the same step (or its reduction), which
+// lets it start only when everything before that is complete, reads no ring and writes nothing but those records: the appends and the
+// window part run beside it.
 __global__ void __launch_bounds__(DEC_THREADS, 1)
 khq_window_step_kernel(const __half* __restrict__ q, __half* __restrict__ ring_k, __half* __restrict__ ring_v,
                        __half* __restrict__ ring_u, const __half* __restrict__ new_k, const __half* __restrict__ new_v,
@@ -1178,6 +1179,7 @@ static int decode_step_impl(
     cudaError_t err = ensure_smem_attrs();
     if (err != cudaSuccess) return static_cast<int>(err);
     const float* part_c = static_cast<const float*>(tail_merges ? attn_partial : attn_c);
+    // Nothing may be launched between the attention above and this: see the kernel.
     err = launch_pdl(khq_window_step_kernel, window_cluster(win_len), window_cluster(win_len), (size_t)WIN_SMEM,
                      stream, (unsigned)DEC_THREADS, static_cast<const __half*>(q_gate), static_cast<__half*>(ring_k),
                      static_cast<__half*>(ring_v), static_cast<__half*>(ring_u), static_cast<const __half*>(k_roped),

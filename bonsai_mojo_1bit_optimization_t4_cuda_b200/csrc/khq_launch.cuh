@@ -17,9 +17,8 @@ static inline int sm_count() {
     return n[dev];
 }
 
-// cluster == 0: no cluster attribute.  All kernels launched through here begin with pdl_wait() (or know what they may do
-// before it), so they carry the programmatic-serialisation attribute: their launch latency and prologue overlap the end of
-// the kernel before them.
+// cluster == 0: no cluster attribute.  All kernels launched through here call pdl_wait() and keep to the rules beside it, so they
+// carry the programmatic-serialisation attribute: their launch latency and prologue overlap the end of the kernel before them.
 template <typename Kernel, typename... Args>
 static cudaError_t launch_pdl(Kernel kernel, unsigned grid, unsigned cluster, size_t smem_bytes,
                               cudaStream_t stream, unsigned threads, Args... args) {
