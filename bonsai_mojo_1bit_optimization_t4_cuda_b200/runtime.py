@@ -76,12 +76,16 @@ class _Tensors(dict):
 KHQ_TABLES = ("dk", "ck", "rk", "dv", "cv", "rv", "vq")
 
 
-def _version(tables) -> int:
-    """Grows with every write that torch makes into one of the tables."""
-    n = 0
-    for t in tables:
-        n += t._version
-    return n
+class _Writes:
+    """Counts the writes that torch makes into any of some tensors, under the name by which a tensor counts its own."""
+
+    def __init__(self, tensors):
+        bases = (t if t._base is None else t._base for t in tensors if not t.is_inference())
+        self.tensors = list({id(t): t for t in bases}.values())  # views of one buffer count together
+
+    @property
+    def _version(self) -> int:
+        return sum(t._version for t in self.tensors)
 
 
 def _constant(name):
@@ -191,9 +195,12 @@ class KhqRuntime:
             L = self.layers[tb.layer_id]
             L.ts_k, L.alpha_k, L.ts_v, L.alpha_v = tb.ts_k, tb.alpha_k, tb.ts_v, tb.alpha_v
             f16 = tb.as_f16()
-            for key, name in (("d_k", "dk"), ("cents_k", "ck"), ("rotor_k", "rk"), ("d_v", "dv"),
-                              ("cents_v", "cv"), ("rotor_v", "rv"), ("vq", "vq")):
-                L.t[name] = torch.from_numpy(f16[key]).to(self.device)
+            # one buffer: its views share a version counter, so a step looks at one and not at seven
+            parts = [f16[key].reshape(-1) for key in ("d_k", "cents_k", "rotor_k", "d_v", "cents_v", "rotor_v", "vq")]
+            buf, at = torch.from_numpy(np.concatenate(parts)).to(self.device), 0
+            for name, part in zip(KHQ_TABLES, parts):
+                L.t[name] = buf[at:at + part.size]
+                at += part.size
             L.cap = max_seq
             L.ready = False
             L.has_tables = True
@@ -278,7 +285,7 @@ class KhqRuntime:
             return False
         kv = L.H_kv * L.D
         slot = L.write_pos % KHQ_RING
-        T = L.t
+        T = L._t
         if hasattr(self.ops, "layer_ctx"):  # addresses will do: no views of the rings
             off = slot * kv * 2
             rings = [T[r].data_ptr() + off for r in ("ring_k", "ring_v", "ring_u")]
@@ -291,8 +298,8 @@ class KhqRuntime:
     # ------------------------------------------------------------------ native step
     def _native_ctx(self, L):
         """The layer's native context (addresses, and tables in the kernels' form), None where the backend has none."""
-        T = L.t
-        if T.ctx is not None and _version(T.counted) == T.version:
+        T = L._t
+        if T.ctx is not None and T.writes._version == T.version:
             return T.ctx
         make = getattr(self.ops, "layer_ctx", None)
         if make is None or (L.H_q, L.H_kv, L.D) != (24, 4, 256):
@@ -303,8 +310,11 @@ class KhqRuntime:
         if T.old:
             self.ops.finish_device()
             T.old = ()
-        T.counted = [T[n] for n in KHQ_TABLES if not T[n].is_inference()]
-        T.version = _version(T.counted)
+        T.writes = _Writes(T[n] for n in KHQ_TABLES)
+        if len(T.writes.tensors) == 1:
+            T.writes = T.writes.tensors[0]
+        T.version = T.writes._version
+        T.device = T["ring_k"].get_device()
         T.ctx = make(L, KHQ_RING, ROPE_BASE)
         return T.ctx
 
@@ -320,10 +330,13 @@ class KhqRuntime:
         window = L.write_pos + 1 - L.boundary
         if self.prof or self.debug or window > KHQ_RING or window <= 0:
             return False
-        ctx = self._native_ctx(L)
-        if ctx is None:
-            return False
-        kv, device = L.H_kv * L.D, L.t["ring_k"].get_device()
+        T = L._t
+        ctx = T.ctx
+        if ctx is None or T.writes._version != T.version:
+            ctx = self._native_ctx(L)
+            if ctx is None:
+                return False
+        kv, device = L.H_kv * L.D, T.device
         if k_roped_dev is not None:
             k_roped_dev, v_dev = _row_address(k_roped_dev, kv, device), _row_address(v_dev, kv, device)
             if not k_roped_dev or not v_dev:
@@ -483,7 +496,7 @@ class KhqRuntime:
         L = self.layers[layer_idx]
         if not L.ready or L.write_pos != 0:
             return False
-        ops, Tn = self.ops, L.t
+        ops, Tn = self.ops, L._t
         H_q, H_kv, d = L.H_q, L.H_kv, L.D
         kv = H_kv * d
         T = int(k_roped_dev.shape[0])
@@ -533,9 +546,12 @@ class KhqRuntime:
     def _native_prefill(self, L, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T: int, n_chunks: int, scale: float) -> bool:
         """The whole prompt of one layer as one native call.  False: another backend or shape, other types than fp16, or rows that
         need a copy first (not contiguous, or not on 16 bytes)."""
-        ctx = self._native_ctx(L)
-        if ctx is None:
-            return False
+        Tn = L._t
+        ctx = Tn.ctx
+        if ctx is None or Tn.writes._version != Tn.version:
+            ctx = self._native_ctx(L)
+            if ctx is None:
+                return False
         for t in (q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev):
             if t.dtype is not torch.float16 or not t.is_contiguous() or t.data_ptr() & 15:
                 return False

@@ -62,7 +62,12 @@ def _view(L):
     L.t["ck"].view(4, D)[2].mul_(3.0)
 
 
-CHANGES = [_set, _update, _union, _pop, _delete, _dict, _in_place, _view, *SCALARS]
+def _replaced_then_in_place(L):
+    L.t["vq"] = L.t["vq"].clone()  # no longer a part of the layer's own buffer
+    L.t["vq"].mul_(0.5)
+
+
+CHANGES = [_set, _update, _union, _pop, _delete, _dict, _in_place, _view, _replaced_then_in_place, *SCALARS]
 
 
 @pytest.mark.parametrize("change", CHANGES, ids=lambda c: c if isinstance(c, str) else c.__name__.strip("_"))
@@ -80,6 +85,10 @@ def test_next_step_uses_the_new_values(change):
         change(L)
     assert step() and step()
     assert rt.ops.made == 2 and rt.ops.finished == 1  # one new context; the device had finished with the old one
+    for n in KHQ_TABLES:  # and it counts the writes into each of the tables that are there now
+        made = rt.ops.made
+        L.t[n].add_(1)
+        assert step() and step() and rt.ops.made == made + 1, n
     tables, scalars, at = rt.ops.used
     for n in KHQ_TABLES:
         assert torch.equal(tables[n], L.t[n]), n
