@@ -19,7 +19,7 @@
 //   warp 11    brings the gates into shared memory in pieces and stores the outputs that take their
 //              place (a softmax thread owns a row: its own global accesses would cost a line each,
 //              16 000 of the 45 000 cycles of an item of 11 tiles; 9 x 1531 rows 386 -> 373 us,
-//              32 x 512: 290 -> 263).
+//              32 x 512: 290 -> 270).
 //   warps 8,10 producers: one thread each issues the TMA loads of Q and the K tiles (warp 8, a
 //              K tile in two halves of 128 head dims, each released as soon as the Q K^T steps
 //              that read it have completed) and of the V tiles (warp 10, two halves of 64 keys,
