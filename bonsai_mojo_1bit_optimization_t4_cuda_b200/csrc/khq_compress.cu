@@ -591,11 +591,12 @@ khq_compress_v_kernel(const __half* __restrict__ x, const __half* __restrict__ d
 // So the code words stay bit-identical.
 //
 // CTA = four groups of two warps; a group owns 16 rows (one M tile), its warps search patches 0..31 and 32..63 and share the
-// rows in front and behind.  The scales of all patches come first (a patch per warp at a time, 1 % of the CTA's instructions).
+// rows in front and behind.  The scales of all patches come first (a patch per warp at a time).
 // The B fragments of a patch (8 KB) are built once per CTA and step by all threads, double buffered.  A thread holds 2 rows x 32
 // codes of a half patch: minimum by three-input min, then the sign bits of (value - minimum - margin) shifted into a mask.  46 warp
 // instructions per (row, patch) against 85 of the exact search, about two per cycle; 0.5 % of the pairs are redone.  129 024
-// rows: 800 us with the exact search alone, 646 filtered without the scaling (44 instructions), 664 with it.
+// rows: 800 us with the exact search alone, 646 filtered without the scaling, 664 with it (the latency of the scan;
+// 0.5 % more instructions).
 constexpr int VM_ROWS = 16;  // rows per group
 constexpr int VM_GROUPS = 4;   // per CTA; eight halve the building of fragments but not the time (694 us)
 struct CompressScratchVM {
