@@ -646,6 +646,7 @@ khq_decode_batched_kernel(const KhqSeqDesc* __restrict__ descs, const KhqTablesD
 #include "khq_decode_mma.cuh"
 #include "khq_decode_tc5.cuh"
 #include "khq_decode_tc5w.cuh"
+#include "khq_step.cuh"
 namespace khq {
 
 // Per problem and query head: LSE merge of the problem's partial slots, /(den+1e-8), sigmoid
@@ -960,6 +961,8 @@ static cudaError_t ensure_smem_attrs() {
     if ((e = cudaFuncSetAttribute(m3::khq_decode_batched_tc5w_kernel, attr, m3::SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_window_attn_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_window_step_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_kernel, attr, ST_SM_TOTAL)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_wide_kernel, attr, M2_SM_TOTAL)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev] = true;
     return cudaSuccess;
 }
@@ -1218,35 +1221,139 @@ static_assert(sizeof(khq_layer_ctx) == 21 * 8 + 24, "ABI");
 extern "C" int launch_khq_compress_fp16(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
                                         void*, int, int, float, float, int, cudaStream_t);
 
+// Shape of a step: csize 0, khq_step_kernel, else khq_step_wide_kernel with clusters of csize CTAs; n_comp clusters (per kv-head) on the
+// compressed region and blocks of 16 tokens per CTA.  Measured on 148 SMs, a layer of a chain of steps, us:
+//     compressed tokens          384   1024   1536   2176   3072   4096   8192  16384  32768  131072
+//     one block per CTA          12.0   15.8   18.1   21.4   27.9   29.5   44.0   67.2    114     370
+//     wide, 14 clusters of 8     18.9   20.9   21.0   21.6   23.0   23.4   29.3   40.3   59.4     177
+//     wide, 31 clusters of 4     19.6   22.1   23.3   22.9   25.1   25.3   31.5   39.5   57.9     165
+//     two kernels (before)       20.4   23.4          25.8          29.9   37.5   48.4            209
+// The first as long as every CTA has one block and not all of the device is taken: at 2176 tokens (136 blocks, 576 CTAs, four on an SM) it
+// is as fast in this chain, but leaves a pre-step between two layers no room to start (30.3 us a layer, 24.3 with the wide
+// one; 1792 tokens: 21.3 and 23.9).  Clusters live inside a GPC, so fewer fit on the
+// device than SMs / size (measured 15 of 8 and 33 of 4, the occupancy query does not know); one is the window's.
+static void step_shape(int c_len, int& csize, int& n_comp, int& per_cta) {
+    const int blocks = (c_len + M2_BT - 1) / M2_BT, sms = sm_count();
+    const auto at_least = [](int n) { return n < 1 ? 1 : n > ST_MAX_RECORDS - 1 ? ST_MAX_RECORDS - 1 : n; };
+    int most = at_least(4 * sms / (HKV * ST_CLUSTER) - 4);
+    csize = 0;
+    if (blocks > most * ST_CLUSTER) {
+        csize = 8;
+        most = at_least(sms / 8 - 4);
+        if (blocks > 1024) {
+            csize = 4;
+            most = at_least(sms / 4 - 5);
+        }
+    }
+    const int ctas = csize ? csize : ST_CLUSTER;
+    per_cta = (blocks + most * ctas - 1) / (most * ctas);
+    n_comp = blocks > 0 ? (blocks + per_cta * ctas - 1) / (per_cta * ctas) : 0;
+}
+
+// The compression event of a step, if due: moves the regions on by 128 tokens.
+static int layer_event(const khq_layer_ctx* L, int& c_len, int& win_len, int compress, cudaStream_t stream) {
+    constexpr int CHUNK = 128;
+    if (!compress) return 0;
+    // the 128 oldest raw tokens, contiguous in the ring; the step's own token is not among them
+    const int s0 = c_len % L->ring_cap, row = c_len * HKV;
+    if (win_len <= CHUNK || s0 + CHUNK > L->ring_cap) return -103;
+    const auto at = [](void* p, size_t bytes) { return static_cast<void*>(static_cast<char*>(p) + bytes); };
+    const size_t src = (size_t)s0 * HKV * D * sizeof(__half);
+    // K first: it zeroes the shared meta rows that the V launch then fills
+    int rc = launch_khq_compress_fp16(at(L->ring_u, src), L->d_k, L->rotor_k, L->cents_k, L->cents_k, at(L->k_mask, (size_t)row * 64),
+                                      at(L->k_norms, (size_t)row * 2), at(L->k_r_norms, (size_t)row * 2),
+                                      at(L->k_payload, (size_t)row * K_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
+                                      L->ts_k, L->alpha_k, 0, stream);
+    if (rc != 0) return rc;
+    rc = launch_khq_compress_fp16(at(L->ring_v, src), L->d_v, L->rotor_v, L->cents_v, L->vq, at(L->k_mask, (size_t)row * 64),
+                                  at(L->v_norms, (size_t)row * 2), at(L->v_r_norms, (size_t)row * 2),
+                                  at(L->v_payload, (size_t)row * V_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
+                                  L->ts_v, L->alpha_v, 1, stream);
+    if (rc != 0) return rc;
+    c_len += CHUNK;
+    win_len -= CHUNK;
+    return 0;
+}
+
 extern "C" int launch_khq_layer_step(const khq_layer_ctx* L, const void* q_gate, const void* k_roped, const void* v_new,
                                      const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits,
                                      float scale, cudaStream_t stream) {
-    constexpr int CHUNK = 128;
     if (!L || !q_gate || !out || win_len <= 0 || c_len < 0 || !L->attn_c || !aligned(L->prepared, 128) || (k_roped == nullptr) != (v_new == nullptr)) return -100;
     if (L->ring_cap <= 0 || win_len > L->ring_cap) return -103;
-    if (compress) {  // the 128 oldest raw tokens, contiguous in the ring; the step's own token is not among them
-        const int s0 = c_len % L->ring_cap, row = c_len * HKV;
-        if (win_len <= CHUNK || s0 + CHUNK > L->ring_cap) return -103;
-        const auto at = [](void* p, size_t bytes) { return static_cast<void*>(static_cast<char*>(p) + bytes); };
-        const size_t src = (size_t)s0 * HKV * D * sizeof(__half);
-        // K first: it zeroes the shared meta rows that the V launch then fills
-        int rc = launch_khq_compress_fp16(at(L->ring_u, src), L->d_k, L->rotor_k, L->cents_k, L->cents_k, at(L->k_mask, (size_t)row * 64),
-                                          at(L->k_norms, (size_t)row * 2), at(L->k_r_norms, (size_t)row * 2),
-                                          at(L->k_payload, (size_t)row * K_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
-                                          L->ts_k, L->alpha_k, 0, stream);
-        if (rc != 0) return rc;
-        rc = launch_khq_compress_fp16(at(L->ring_v, src), L->d_v, L->rotor_v, L->cents_v, L->vq, at(L->k_mask, (size_t)row * 64),
-                                      at(L->v_norms, (size_t)row * 2), at(L->v_r_norms, (size_t)row * 2),
-                                      at(L->v_payload, (size_t)row * V_PAY), at(L->v_shared_meta, (size_t)row * 4), CHUNK * HKV, D,
-                                      L->ts_v, L->alpha_v, 1, stream);
-        if (rc != 0) return rc;
-        c_len += CHUNK;
-        win_len -= CHUNK;
-    }
+    const int rc = layer_event(L, c_len, win_len, compress, stream);
+    if (rc != 0) return rc;
     return decode_step_impl(q_gate, k_roped, v_new, k_unroped, L->ring_k, L->ring_v, L->ring_u, L->k_payload, L->v_payload,
                             L->v_shared_meta, L->k_mask, L->k_norms, L->k_r_norms, L->v_norms, L->v_r_norms, L->cents_k, L->cents_v,
                             L->vq, L->rotor_k, L->rotor_v, L->d_k, L->d_v, L->attn_c, L->attn_partial, out, c_len,
                             c_len % L->ring_cap, win_len, L->ring_cap, num_splits, scale, L->alpha_k, L->alpha_v, L->rope_base, L->prepared, stream);
+}
+
+extern "C" int launch_khq_layer_token(const khq_layer_ctx* L, void* counters, const void* q_gate, const void* k_roped, const void* v_new,
+                                      const void* k_unroped, void* out, int c_len, int win_len, int compress, float scale,
+                                      cudaStream_t stream) {
+    if (!L || !counters || !q_gate || !out || win_len <= 0 || c_len < 0 || !L->prepared || !L->attn_partial ||
+        (k_roped == nullptr) != (v_new == nullptr))
+        return -100;
+    if (L->ring_cap <= 0 || win_len > L->ring_cap) return -103;
+    const void* al[] = {q_gate, k_roped, v_new, k_unroped, out, L->ring_k, L->ring_v, L->ring_u, L->attn_partial, L->cents_k, L->rotor_k, L->rotor_v, L->d_k, L->d_v};
+    for (const void* p : al)
+        if (!aligned(p, 16)) return -104;
+    if (!aligned(L->prepared, 128) || !aligned(counters, 4)) return -104;
+    const void* arrays[] = {L->k_payload, L->v_payload, L->v_shared_meta, L->k_mask, L->k_norms, L->k_r_norms, L->v_norms, L->v_r_norms};
+    for (const void* a : arrays)
+        if (!aligned(a, 4)) return -104;
+    const int rc = layer_event(L, c_len, win_len, compress, stream);
+    if (rc != 0) return rc;
+    cudaError_t err = ensure_smem_attrs();
+    if (err != cudaSuccess) return static_cast<int>(err);
+    StepArgs A = {};
+    CompressedKV& P = A.kv;
+    P.k_payload = static_cast<const unsigned char*>(L->k_payload);
+    P.v_payload = static_cast<const unsigned char*>(L->v_payload);
+    P.v_shared_meta = static_cast<const unsigned char*>(L->v_shared_meta);
+    P.k_mask = static_cast<const unsigned int*>(L->k_mask);
+    P.k_norms = static_cast<const __half*>(L->k_norms);
+    P.k_r_norms = static_cast<const __half*>(L->k_r_norms);
+    P.v_norms = static_cast<const __half*>(L->v_norms);
+    P.v_r_norms = static_cast<const __half*>(L->v_r_norms);
+    P.cents_k = static_cast<const __half*>(L->cents_k);
+    P.k_rotor = static_cast<const __half*>(L->rotor_k);
+    P.v_rotor = static_cast<const __half*>(L->rotor_v);
+    P.d_k = static_cast<const __half*>(L->d_k);
+    P.d_v = static_cast<const __half*>(L->d_v);
+    P.alpha_k = L->alpha_k;
+    P.alpha_v = L->alpha_v;
+    P.rope_base = L->rope_base;
+    P.c_len = c_len;
+    P.image = static_cast<const unsigned char*>(L->prepared);
+    A.q = static_cast<const __half*>(q_gate);
+    A.ring_k = static_cast<__half*>(L->ring_k);
+    A.ring_v = static_cast<__half*>(L->ring_v);
+    A.ring_u = static_cast<__half*>(L->ring_u);
+    A.new_k = static_cast<const __half*>(k_roped);
+    A.new_v = static_cast<const __half*>(v_new);
+    A.new_u = static_cast<const __half*>(k_unroped);
+    A.out = static_cast<__half*>(out);
+    A.records = static_cast<float*>(L->attn_partial);
+    A.counters = static_cast<int*>(counters);
+    A.win_start = c_len % L->ring_cap;
+    A.win_len = win_len;
+    A.ring_cap = L->ring_cap;
+    A.scale = scale;
+    P.cents_v = static_cast<const __half*>(L->cents_v);
+    P.vq = static_cast<const __half*>(L->vq);
+    bool bulk_ok = true;
+    for (const void* a : arrays) bulk_ok = bulk_ok && aligned(a, 16);
+    P.bulk_ok = bulk_ok ? 1 : 0;
+    A.wide = aligned(L->k_mask, 16) && aligned(L->k_payload, 8) && aligned(L->v_payload, 8);
+    int csize;
+    step_shape(c_len, csize, A.n_comp, A.blocks_per_cta);
+    if (csize == 0)
+        err = launch_pdl(khq_step_kernel, (unsigned)((A.n_comp + 1) * HKV * ST_CLUSTER), (unsigned)ST_CLUSTER, (size_t)ST_SM_TOTAL, stream,
+                         (unsigned)ST_THREADS, A);
+    else
+        err = launch_pdl(khq_step_wide_kernel, (unsigned)((A.n_comp + 1) * csize), (unsigned)csize, (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS, A);
+    return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
 // The newest rows of a prompt into the three rings, row by row at slot = token % ring_cap.  Grid (16-byte vectors, 3 rings).  One

@@ -69,9 +69,11 @@ constexpr int M2_BAR_SMALL = M2_WPK * M2_NSTAGE, M2_BAR_VQ = M2_BAR_SMALL + 1, M
 constexpr int M2_SM_TMSLOT = M2_SM_BARS + M2_NBARS * 8;
 constexpr int M2_SM_QR = (M2_SM_TMSLOT + 4 + 15) / 16 * 16;   // raw rotary query fragments: 4 kv-heads x 4 k-steps x 32 lanes x 8 B
 // Prepared image of a layer's tables (launch_khq_prepare_tables): the codebook's shared-memory rows, the small tables, the
-// rotor fragments (two uint4 per k-step and lane).
-constexpr int M2_IMG_VQ = 0, M2_IMG_SMALL = 256 * M2_VQ_ROW, M2_IMG_ROT = M2_IMG_SMALL + M2_SMALL_BYTES, M2_IMG_BYTES = M2_IMG_ROT + 16 * 32 * 32;
-static_assert(M2_IMG_SMALL % 16 == 0 && M2_IMG_ROT % 16 == 0 && M2_SM_FREQ % 16 == 0 && M2_SM_QR % 16 == 0 && M2_SM_BARS % 8 == 0, "alignment");
+// rotor fragments (two uint4 per k-step and lane), and the codebook once more as [code][patch] of 8 bytes (one load per look-up
+// for kernels that leave it in L2).
+constexpr int M2_IMG_VQ = 0, M2_IMG_SMALL = 256 * M2_VQ_ROW, M2_IMG_ROT = M2_IMG_SMALL + M2_SMALL_BYTES, M2_IMG_VQ8 = M2_IMG_ROT + 16 * 32 * 32,
+              M2_IMG_BYTES = M2_IMG_VQ8 + 256 * NP * 8;
+static_assert(M2_IMG_VQ8 % 16 == 0 && M2_IMG_SMALL % 16 == 0 && M2_IMG_ROT % 16 == 0 && M2_SM_FREQ % 16 == 0 && M2_SM_QR % 16 == 0 && M2_SM_BARS % 8 == 0, "alignment");
 constexpr int M2_SM_TOTAL = M2_SM_QR + HKV * 4 * 32 * 8;
 // Tensor memory as a second register file.  The B fragments of the K side are per-lane constants: the query
 // side (ternary part q1 and residual part q2, fp16 hi and lo, eight registers per k-step) for a whole work
@@ -416,6 +418,11 @@ __global__ void __launch_bounds__(M2_THREADS) khq_prepare_tables_kernel(Compress
     m2_small_tables(image + M2_IMG_SMALL, P, threadIdx.x);
     m2_stage_codebook(image + M2_IMG_VQ, P.vq, threadIdx.x);
     for (int c = threadIdx.x; c < 256; c += M2_THREADS) *reinterpret_cast<uint32_t*>(image + M2_IMG_VQ + c * M2_VQ_ROW + M2_VQ_ROW - 4) = 0u;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < 256 * NP; e += M2_THREADS) {  // e = patch * 256 + code
+        const unsigned short* c = reinterpret_cast<const unsigned short*>(P.vq) + 3 * e;
+        reinterpret_cast<uint2*>(image + M2_IMG_VQ8)[(e & 255) * NP + (e >> 8)] = make_uint2(c[0] | ((uint32_t)c[1] << 16), c[2]);
+    }
     for (int e = threadIdx.x; e < 16 * 32; e += M2_THREADS) {
         uint32_t r[8];
         m2_rotor_fragment(P, e >> 5, e & 31, r);

@@ -107,6 +107,12 @@ class CudaOps:
                             ("k_payload", "kpay"), ("k_norms", "knorm"), ("k_r_norms", "krn"), ("v_payload", "vpay"), ("v_norms", "vnorm"),
                             ("v_r_norms", "vrn"), ("v_shared_meta", "vsm"), ("attn_c", "ac"), ("attn_partial", "ap")):
             setattr(c, field, L.t[name].data_ptr())
+        import torch
+
+        scratch = L.t["ap"]  # 32 records per head, on 16 bytes
+        if scratch.numel() * scratch.element_size() < 24 * 32 * 258 * 4 or scratch.data_ptr() & 15:
+            scratch = torch.empty(24 * 32 * 258, dtype=torch.float32, device=L.t["vq"].device)
+            c.attn_partial = scratch.data_ptr()
         c.ts_k, c.alpha_k, c.ts_v, c.alpha_v, c.rope_base, c.ring_cap = L.ts_k, L.alpha_k, L.ts_v, L.alpha_v, rope_base, ring_cap
         t = np.zeros(1, TABLES_DESC)
         for field, name in (("cents_k", "ck"), ("cents_v", "cv"), ("vq", "vq"), ("k_rotor", "rk"), ("v_rotor", "rv"), ("d_k", "dk"),
@@ -115,13 +121,15 @@ class CudaOps:
         t["alpha_k"], t["alpha_v"] = L.alpha_k, L.alpha_v
         image = prepare_tables(t, rope_base, L.t["vq"].device)
         c.prepared = image.data_ptr()
-        return c, ctypes.addressof(c), image
+        counters = torch.zeros(32, dtype=torch.int32, device=L.t["vq"].device)
+        return c, ctypes.addressof(c), image, counters, counters.data_ptr(), scratch
 
     def layer_step(self, ctx, q_gate, k_roped, v_new, k_unroped, out, c_len, win_len, compress, num_splits, scale):
-        rc = self.lib.launch_khq_layer_step(ctx[1], ptr(q_gate), ptr(k_roped), ptr(v_new), ptr(k_unroped), ptr(out), c_len, win_len,
-                                            compress, num_splits, scale, current_stream())
+        """``num_splits`` is not used: the launch cuts the compressed region by its own rule."""
+        rc = self.lib.launch_khq_layer_token(ctx[1], ctx[4], ptr(q_gate), ptr(k_roped), ptr(v_new), ptr(k_unroped), ptr(out), c_len, win_len,
+                                             compress, scale, current_stream())
         if rc != 0:
-            check("launch_khq_layer_step", rc)
+            check("launch_khq_layer_token", rc)
 
     def layer_prefill(self, ctx, q_gate, k_unroped, k_roped, v, out, T, n_chunks, scale):
         rc = self.lib.launch_khq_layer_prefill(ctx[1], ptr(q_gate), ptr(k_unroped), ptr(k_roped), ptr(v), ptr(out), T, n_chunks, scale,

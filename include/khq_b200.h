@@ -301,6 +301,12 @@ typedef struct khq_layer_ctx {
 int launch_khq_layer_step(const khq_layer_ctx* ctx, const void* q_gate, const void* k_roped, const void* v_new,
                           const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits, float scale,
                           khq_stream_t stream);
+/* The same step as ONE kernel beside the event's two: the library cuts the regions by its own rule.  Needs ctx->prepared;
+ * ctx->attn_partial holds (24, 32, 258) fp32 on 16 bytes; `counters`: 24 int32 on the device, zero before the first step that is
+ * given them (each step leaves them zero) and, like attn_partial, not shared by steps that may run at the same time.  Returns as
+ * launch_khq_layer_step. */
+int launch_khq_layer_token(const khq_layer_ctx* ctx, void* counters, const void* q_gate, const void* k_roped, const void* v_new,
+                           const void* k_unroped, void* out, int c_len, int win_len, int compress, float scale, khq_stream_t stream);
 /* A whole prompt of T rows of a fresh layer: launch_khq_gqa_prefill_fp16, compression of the first n_chunks * 128 tokens, and
  * the newest min(T, ring_cap) rows of K RoPE'd, V and K un-RoPE'd into the rings at slot = token % ring_cap.  q_gate (T, 24, 512),
  * k_unroped / k_roped / v (T, 4, 256), out (T, 24, 256), fp16, all 16-byte aligned (-104). */
