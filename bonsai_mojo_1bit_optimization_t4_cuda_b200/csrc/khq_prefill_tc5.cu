@@ -24,16 +24,16 @@
 //              K tile in two halves of 128 head dims, each released as soon as the Q K^T steps
 //              that read it have completed) and of the V tiles (warp 10, two halves of 64 keys,
 //              each released when the P V steps that read it have completed).
-//   warp 9     MMA: one thread issues S = Q K^T (M128 N128 K256, A = Q from shared memory) for
+//   warp 9     MMA: one lane issues S = Q K^T (M128 N128 K256, A = Q from shared memory) for
 //              tile j+1, then O += P V (M128 N256 K128, A = P from tensor memory) for tile j;
 //              tcgen05.commit signals the mbarriers.
 // Tensor memory columns: O [0,256), S/P ping [256,384), S/P pong [384,512).  An A operand in
 // tensor memory is row = lane, 16 consecutive K elements = 8 columns of fp16 pairs.
-// Why these shapes: one tcgen05.mma of M 128 costs the tensor pipe at least ~93 cycles whatever
-// its N (measured: N 64 and N 128 both 93, N 256 138 with A in tensor memory; 107 / 171 for
-// N 128 / 256 with A in shared memory), so 64-key tiles (N 64, ideal 32 cycles) run Q K^T at a
-// third of the pipe's rate; tensor memory (512 columns) holds O plus two 128-key S buffers, which
+// Why these shapes: back to back the pipe takes 64 cycles for a Q K^T step (N 128) and 128 for a P V step (N 256); 64-key tiles
+// would issue twice the instructions for the same work.  Tensor memory (512 columns) holds O plus two 128-key S buffers, which
 // leaves no room for Q, so Q stays in shared memory.
+// Prompts of many row blocks go to CTA pairs instead (khq_prefill_pair.cuh); this kernel has the short ones, where a row's two
+// threads shorten the chain of the few tiles of an item, and odd numbers of query heads per kv head.
 //
 // Shared-memory operand layout: the 128-byte-swizzle canonical layouts.  A 5-D tensor map
 // {64 halfs, row, 64-column group, head, batch} with 128-byte swizzle makes TMA write a
@@ -96,11 +96,11 @@ __device__ int g_prefill_status = 0;
 // Shared-memory matrix descriptor (64 bits): start address, leading and stride byte offsets (all in
 // 16-byte units; bits 0-13, 16-29, 32-45), descriptor version 1 in bits 46-47, layout type 2
 // (128-byte swizzle) in bits 61-63.  It is assembled from a low and a high word, see desc_lo/desc_hi.
-// Instruction descriptor for kind::f16: fp32 accumulate, fp16 A and B, A K-major, M = 128.
+// Instruction descriptor for kind::f16: fp32 accumulate, fp16 A and B, A K-major, M = 128 (256: a CTA pair).
 // (A/B format field: 0 = fp16, 1 = bf16, bits 7-9 and 10-12.)
-__host__ __device__ constexpr uint32_t instr_desc(int n, bool b_mn_major, bool bf16) {
+__host__ __device__ constexpr uint32_t instr_desc(int m, int n, bool b_mn_major, bool bf16) {
     return (1u << 4) | (bf16 ? ((1u << 7) | (1u << 10)) : 0u) | (b_mn_major ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(128 >> 4) << 24);
+           ((uint32_t)(m >> 4) << 24);
 }
 // Two floats -> one 32-bit word of the 16-bit storage type (round to nearest even), and back.
 template <bool BF16>
@@ -119,7 +119,7 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
 }
 
 // ---- tcgen05 / TMA wrappers ----------------------------------------------------------------------
-// The issuing thread is on the critical path: the 64-bit descriptors are assembled from a
+// The issuing warp is on the critical path: the 64-bit descriptors are assembled from a
 // precomputed low word (start address and leading offset; the caller adds the K-step offset, which
 // never carries out of the 14-bit address field) and a constant high word.  umma_ss: A and B from
 // shared memory; umma_ts: A from tensor memory (row = lane, fp16 pairs, 8 columns per K step of 16).
@@ -129,30 +129,39 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) {
 __host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo) {
     return ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);  // version 1 (bit 46), 128-byte swizzle (bits 61-63)
 }
+// All lanes of the MMA warp call these and one of them issues (`one`): the operands are then values of the whole warp, which the
+// compiler keeps and steps in uniform registers (see khq_prefill_pair.cuh).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+    return r;
+}
 template <int ACC>
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+__device__ __forceinline__ void umma_ss(uint32_t one, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                         uint32_t idesc) {
     asm volatile(
-        "{\n\t.reg .b64 da, db;\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .b64 da, db;\n\t.reg .pred p, q;\n\t"
         "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-        "setp.ne.u32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
+        "setp.ne.u32 p, %6, 0;\n\tsetp.ne.u32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC), "r"(one)
         : "memory");
 }
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+__device__ __forceinline__ void umma_ts(uint32_t one, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                         uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .b64 db;\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .b64 db;\n\t.reg .pred p, q;\n\t"
         "mov.b64 db, {%2, %3};\n\t"
-        "setp.ne.u32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        "setp.ne.u32 p, %5, 0;\n\tsetp.ne.u32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(one)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t one, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(one)
+        : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -220,7 +229,7 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 }
 
 // Bounded wait on up to three barriers at once.  A satisfied mbarrier wait still costs a ~250-cycle
-// round trip, so the MMA thread polls the barriers of a step together (the polls overlap) instead
+// round trip, so the MMA warp polls the barriers of a step together (the polls overlap) instead
 // of one after the other; a barrier found complete stays "done" (its next phase cannot complete
 // before this thread moves on).
 __device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
@@ -234,6 +243,13 @@ __device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok;
 }
+// Waits of a whole warp: all lanes go on together.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* status) {
+    for (uint32_t it = 0; it < (1u << 22); ++it)
+        if (__any_sync(0xFFFFFFFFu, khq::mbar_try_wait(bar, parity))) return true;
+    atomicExch(status, 1);
+    return false;
+}
 template <int N>
 __device__ __forceinline__ bool mbar_wait_all_bounded(uint64_t* const (&bar)[N], const uint32_t (&parity)[N], int* status) {
     uint32_t done = 0;
@@ -242,13 +258,13 @@ __device__ __forceinline__ bool mbar_wait_all_bounded(uint64_t* const (&bar)[N],
 #pragma unroll
         for (int i = 0; i < N; ++i) got[i] = mbar_test(bar[i], parity[i]);
 #pragma unroll
-        for (int i = 0; i < N; ++i) done |= got[i] << i;
+        for (int i = 0; i < N; ++i) done |= (uint32_t)__any_sync(0xFFFFFFFFu, got[i]) << i;
         if (done == (1u << N) - 1u) return true;
         bool parked = false;  // park (a blocking try_wait) on the first barrier that is still open
 #pragma unroll
         for (int i = 0; i < N; ++i)
             if (!parked && !((done >> i) & 1u)) {
-                if (khq::mbar_try_wait(bar[i], parity[i])) done |= 1u << i;
+                if (__any_sync(0xFFFFFFFFu, khq::mbar_try_wait(bar[i], parity[i]))) done |= 1u << i;
                 parked = true;
             }
         if (done == (1u << N) - 1u) return true;
@@ -327,7 +343,7 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BARS + 240);
     float* xchg = reinterpret_cast<float*>(smem + OFF_XCHG);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     int* status = &g_prefill_status;
     if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
         if (tid == 0) atomicExch(status, 2);
@@ -372,7 +388,7 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
     const uint32_t sbase = smem_u32(smem);
 
     if (warp == 8) {
@@ -432,9 +448,10 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         }
     } else if (warp == 9) {
         // ================================ MMA issuer ==============================================
-        if (lane == 0) {
-            constexpr uint32_t IDESC_S = instr_desc(BC, false, BF16);
-            constexpr uint32_t IDESC_O = instr_desc(D, true, BF16);
+        {
+            const uint32_t one = elect_one();
+            constexpr uint32_t IDESC_S = instr_desc(BR, BC, false, BF16);
+            constexpr uint32_t IDESC_O = instr_desc(BR, D, true, BF16);
             constexpr uint32_t HI_K = desc_hi(1024);  // Q, K (K-major) and V (MN-major): 1024 bytes between 8-row groups
             const uint32_t q_lo = desc_lo(sbase + OFF_Q, 16), k_lo = desc_lo(sbase + OFF_K, 16);
             const uint32_t v_lo = desc_lo(sbase + OFF_V, 64 * 128);  // leading offset: the next 64-column group
@@ -454,20 +471,20 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                         // byte offsets / 16: next 64-dim group = rows*128 bytes, next K step = 32 bytes
                         const uint32_t oa = (uint32_t)((ks >> 2) * (BR * 128) + (ks & 3) * 32) >> 4;
                         const uint32_t ob = (uint32_t)(hf * KHALF_BYTES + (kk >> 2) * (BC * 128) + (kk & 3) * 32) >> 4;
-                        if (ks == 0) umma_ss<0>(s_tmem, q_lo + oa, HI_K, k_lo + ob, HI_K, IDESC_S);
-                        else umma_ss<1>(s_tmem, q_lo + oa, HI_K, k_lo + ob, HI_K, IDESC_S);
+                        if (ks == 0) umma_ss<0>(one, s_tmem, q_lo + oa, HI_K, k_lo + ob, HI_K, IDESC_S);
+                        else umma_ss<1>(one, s_tmem, q_lo + oa, HI_K, k_lo + ob, HI_K, IDESC_S);
                     }
-                    umma_commit(&bars[B_KEMPTY + hf]);
+                    umma_commit(one, &bars[B_KEMPTY + hf]);
                 }
-                umma_commit(&bars[B_SFULL + (g & 1)]);
+                umma_commit(one, &bars[B_SFULL + (g & 1)]);
             };
             Item it, nx;
             bool have = get_item<PERSIST>(0, T, H_q, H_kv, batch, group_major, it);
             int g = 0;
             if (have) {
-                ok = khq::mbar_wait_bounded(&bars[B_QFULL], 0u, status);
+                ok = warp_wait(&bars[B_QFULL], 0u, status);
                 if (ok) issue_qk(0);
-                if (PERSIST && ok && it.n_tiles == 1) umma_commit(&bars[B_QEMPTY]);
+                if (PERSIST && ok && it.n_tiles == 1) umma_commit(one, &bars[B_QEMPTY]);
             }
             for (int i = 0; have && ok; ++i) {
                 const bool have_nx = get_item<PERSIST>(i + 1, T, H_q, H_kv, batch, group_major, nx);
@@ -475,11 +492,11 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                     // run ahead: Q K^T of the next tile, which may be the first tile of the next item
                     const bool same_item = j + 1 < it.n_tiles;
                     if (same_item || have_nx) {
-                        if (!same_item) ok = khq::mbar_wait_bounded(&bars[B_QFULL], (uint32_t)((i + 1) & 1), status);
+                        if (!same_item) ok = warp_wait(&bars[B_QFULL], (uint32_t)((i + 1) & 1), status);
                         if (ok) issue_qk(g + 1);
                         // once the last Q K^T of an item is out, its Q buffer may be reloaded
                         const bool last_qk = same_item ? (j + 2 == it.n_tiles) : (nx.n_tiles == 1);
-                        if (PERSIST && ok && last_qk) umma_commit(&bars[B_QEMPTY]);
+                        if (PERSIST && ok && last_qk) umma_commit(one, &bars[B_QEMPTY]);
                     }
                     if (!ok) break;
                     uint64_t* const pb[3] = {&bars[(g & 1) ? B_PREADY2 : B_PREADY], &bars[B_VFULL], &bars[B_VFULL + 1]};
@@ -487,7 +504,7 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                     ok = mbar_wait_all_bounded(pb, pp, status);
                     // the first P V of an item overwrites O: the previous item's epilogue must have read it
                     if (PERSIST && ok && j == 0 && i > 0)
-                        ok = khq::mbar_wait_bounded(&bars[B_OFREE], (uint32_t)((i - 1) & 1), status);
+                        ok = warp_wait(&bars[B_OFREE], (uint32_t)((i - 1) & 1), status);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t p_tmem = tmem + TM_S + (uint32_t)(g & 1) * BC;
@@ -496,11 +513,11 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
                             const uint32_t ob = (uint32_t)(hf * VHALF_BYTES + kk * 2048) >> 4;  // 16 keys = 2048 bytes
-                            umma_ts(tmem + TM_O, p_tmem + (hf * 4 + kk) * 8, v_lo + ob, HI_K, IDESC_O,
+                            umma_ts(one, tmem + TM_O, p_tmem + (hf * 4 + kk) * 8, v_lo + ob, HI_K, IDESC_O,
                                     (hf > 0 || kk > 0) ? 1u : (uint32_t)(j > 0));
                         }
-                        if (hf == 1) umma_commit(&bars[B_PVDONE + (g & 1)]);
-                        umma_commit(&bars[B_VEMPTY + hf]);
+                        if (hf == 1) umma_commit(one, &bars[B_PVDONE + (g & 1)]);
+                        umma_commit(one, &bars[B_VEMPTY + hf]);
                     }
                 }
                 it = nx;
@@ -709,6 +726,7 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 }
 
 }  // namespace khq_prefill5
+#include "khq_prefill_pair.cuh"
 
 // ---- host side -----------------------------------------------------------------------------------
 namespace {
@@ -753,7 +771,14 @@ int make_map(CUtensorMap* map, const void* base, int T, int heads, int batch, lo
 
 }  // namespace
 
-static int g_tc5_items_per_cta = 0;
+static int g_tc5_items_per_cta = 0, g_tc5_pairs = 0;
+
+// 0 = CTA pairs by the size of the prompts, 1 = wherever the heads allow it, 2 = never.
+extern "C" int khq_b200_prefill_pairs(int mode) {
+    if (mode < 0 || mode > 2) return -100;
+    g_tc5_pairs = mode;
+    return 0;
+}
 
 // 0 = choose by prompt length, 1 = one item per CTA, n > 1 = n items per CTA (a large n gives
 // the fully persistent grid).  Returns -100 for a negative value.
@@ -764,6 +789,16 @@ extern "C" int khq_b200_prefill_tc5_items_per_cta(int n) {
 }
 
 namespace {
+// Whether CTA pairs take the items of two neighbouring heads of a kv head together.  From nine row blocks on, below that the chain of an
+// item's few tiles counts (T = 1000: 16 prompts 353 us either way, 4 prompts 92.8 against 91.7), and from 2.25 items per SM on, so that
+// the epilogue of one item runs beside the tiles of others (T = 1531: one prompt 41.5 us against 39.1, two 85.0 against 85.8, nine
+// 355 against 373; one of 2000: 58 against 62; 8 x 2048: 492 against 533; 4 x 8192 in a row, both at the power limit: 2.45 to 2.84 ms
+// against 2.65 to 2.97).
+bool use_pair(int row_blocks, long long items, int n_rep, int sms) {
+    if (n_rep % 2 != 0 || g_tc5_pairs == 2) return false;
+    return g_tc5_pairs == 1 || (row_blocks > 8 && 4 * items > 9LL * sms);
+}
+
 int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int batch, int T, int H_q, int H_kv, int d,
                float scale, long long q_batch_stride, long long kv_batch_stride, long long out_batch_stride,
                cudaStream_t stream, bool bf16) {
@@ -774,13 +809,6 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     for (const void* p : ptrs)
         if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return -104;
     if (batch > 1 && ((q_batch_stride | kv_batch_stride | out_batch_stride) & 7) != 0) return -104;
-    CUtensorMap mq, mk, mv, mg, mo;
-    int rc = make_map(&mq, q_gate, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 4, bf16);
-    if (rc == 0) rc = make_map(&mk, k, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, BC, 2, bf16);
-    if (rc == 0) rc = make_map(&mv, v, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, 64, 4, bf16);
-    if (rc == 0) rc = make_map(&mg, static_cast<const __half*>(q_gate) + D, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 1, bf16);
-    if (rc == 0) rc = make_map(&mo, out, T, H_q, batch, (long long)H_q * D, D, out_batch_stride, BR, 1, bf16);
-    if (rc != 0) return rc;
     static bool attr_done[64] = {};
     static int sm_count[64] = {};
     int dev = 0;
@@ -794,18 +822,17 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
             err = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
             if (err != cudaSuccess) return static_cast<int>(err);
         }
+        for (const void* kf : {(const void*)pair::khq_gqa_prefill_pair_kernel<false>, (const void*)pair::khq_gqa_prefill_pair_kernel<true>}) {
+            err = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM);
+            if (err != cudaSuccess) return static_cast<int>(err);
+        }
         err = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess) return static_cast<int>(err);
         attr_done[dev] = true;
     }
-    const long long items = (long long)((T + BR - 1) / BR) * H_q * batch;
-    // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
-    // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
-    // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
-    // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
-    // 24 row blocks (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99), and above 16 where a CTA has few
-    // items to even out its share (1 x 2500: 89 against 92 us, 1 x 3000: 116 against 122, 4 x 3000: 473 against 550).
-    // khq_b200_prefill_tc5_items_per_cta(n) or KHQ_PREFILL_ITEMS_PER_CTA (read once) force a mode:
+    const int nqb = (T + BR - 1) / BR;
+    const long long items = (long long)nqb * H_q * batch;
+    // khq_b200_prefill_tc5_items_per_cta(n) or KHQ_PREFILL_ITEMS_PER_CTA (read once) force a mode of the kernel without pairs, for prompts that pairs do not take:
     // 1 = one item per CTA, larger = that many items per CTA (the setter wins; 0 = automatic).
     static int env_forced = -1;
     if (env_forced < 0) {
@@ -814,7 +841,26 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
         if (env_forced < 0) env_forced = 0;
     }
     const int forced = g_tc5_items_per_cta > 0 ? g_tc5_items_per_cta : env_forced;
-    const int nqb = (T + BR - 1) / BR;
+    const bool pairs = use_pair(nqb, items, H_q / H_kv, sm_count[dev]);
+    CUtensorMap mq, mk, mv, mg, mo;
+    int rc = make_map(&mq, q_gate, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 4, bf16);
+    if (rc == 0) rc = make_map(&mk, k, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? 64 : BC, pairs ? 4 : 2, bf16);
+    if (rc == 0) rc = make_map(&mv, v, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? BC : 64, pairs ? 2 : 4, bf16);
+    if (rc == 0) rc = make_map(&mg, static_cast<const __half*>(q_gate) + D, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 1, bf16);
+    if (rc == 0) rc = make_map(&mo, out, T, H_q, batch, (long long)H_q * D, D, out_batch_stride, BR, 1, bf16);
+    if (rc != 0) return rc;
+    const float sl2 = scale * 1.4426950408889634f;
+    if (pairs) {
+        err = khq::launch_pdl(bf16 ? pair::khq_gqa_prefill_pair_kernel<true> : pair::khq_gqa_prefill_pair_kernel<false>, (unsigned)items, 2u, (size_t)pair::SMEM,
+                              stream, (unsigned)NTHREADS, mq, mk, mv, mg, mo, T, H_q, H_kv, sl2);
+        return (err == cudaSuccess) ? 0 : static_cast<int>(err);
+    }
+    // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
+    // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
+    // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
+    // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
+    // 24 row blocks (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99), and above 16 where a CTA has few
+    // items to even out its share (1 x 2500: 89 against 92 us, 1 x 3000: 116 against 122, 4 x 3000: 473 against 550).
     long long ctas;
     int group_major = 0;
     if (forced == 1 || (forced == 0 && (nqb > 24 || (nqb > 16 && items <= 16LL * sm_count[dev])))) {
@@ -829,7 +875,6 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     const unsigned grid = (unsigned)ctas;
     const __half* qp = static_cast<const __half*>(q_gate);  // 16-bit storage; the kernel converts per its type flag
     __half* op = static_cast<__half*>(out);
-    const float sl2 = scale * 1.4426950408889634f;
 #define KHQ_TC5_LAUNCH(PERSIST, BF16)                                                                                  \
     err = khq::launch_pdl(khq_gqa_prefill_tc5_kernel<PERSIST, BF16>, grid, 0, SMEM_BYTES, stream, (unsigned)NTHREADS, mq, mk, mv, mg, mo, qp, op, \
                           q_batch_stride, out_batch_stride, T, H_q, H_kv, batch, group_major, sl2)

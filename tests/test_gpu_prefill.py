@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 # tcgen05 / tensor-memory kernel (the default; also forced into each of its two work distributions)
 # and the warp-level mma.sync kernel
-KERNELS = ["tc5", "mma", "tc5-one-item-per-cta", "tc5-persistent"]
+KERNELS = ["tc5", "mma", "tc5-one-item-per-cta", "tc5-persistent", "tc5-pairs"]
 
 
 def _run(cuda_ops, qg, k, v, B, T, H_q=H_Q, H_kv=H_KV, kernel="tc5"):
@@ -19,6 +19,7 @@ def _run(cuda_ops, qg, k, v, B, T, H_q=H_Q, H_kv=H_KV, kernel="tc5"):
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     out = torch.full((B, T, H_q, D), float("nan"), dtype=torch.float16, device="cuda")
     assert cuda_ops.lib.khq_b200_prefill_select(1 if kernel == "mma" else 0) == 0
+    assert cuda_ops.lib.khq_b200_prefill_pairs(1 if kernel == "tc5-pairs" else 0) == 0
     assert cuda_ops.lib.khq_b200_prefill_tc5_items_per_cta({"tc5-one-item-per-cta": 1, "tc5-persistent": 1 << 20}.get(kernel, 0)) == 0
     try:
         cuda_ops.gqa_prefill(dev(qg), dev(k), dev(v), out, B, T, H_q, H_kv, D, SCALE)
@@ -26,6 +27,7 @@ def _run(cuda_ops, qg, k, v, B, T, H_q=H_Q, H_kv=H_KV, kernel="tc5"):
     finally:
         cuda_ops.lib.khq_b200_prefill_select(0)
         cuda_ops.lib.khq_b200_prefill_tc5_items_per_cta(0)
+        cuda_ops.lib.khq_b200_prefill_pairs(0)
     assert cuda_ops.lib.khq_b200_prefill_status() == 0
     return out.float().cpu().numpy()
 
@@ -190,3 +192,29 @@ def test_prefill_either_side_of_the_grid_rule(cuda_ops, B, T):
     k, v = (rng.standard_normal((B, T, H_KV, D)) * 0.25).astype(np.float16), rng.standard_normal((B, T, H_KV, D)).astype(np.float16)
     auto, one, many = (_run(cuda_ops, qg, k, v, B, T, kernel=m) for m in ("tc5", "tc5-one-item-per-cta", "tc5-persistent"))
     assert np.array_equal(auto, one) and np.array_equal(auto, many)
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("B,T", [(4, 1153), (4, 1280), (3, 1531), (1, 2100)])
+def test_prompts_of_many_row_blocks_pair_against_single(cuda_ops, B, T, dtype):
+    """The rule's own choice (CTA pairs from nine row blocks and 2.25 items per SM on) against the kernel without pairs: the same
+    products, sums in another order, and weights against another reference; then one rounding to 16 bits on each side."""
+    import torch
+
+    dt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dt)
+    q, k, v = rnd(B, T, H_Q, 2 * D), rnd(B, T, H_KV, D), rnd(B, T, H_KV, D)
+    k[:, ::7] *= 3.0  # scores that move the reference
+    outs = []
+    for mode in (0, 2):
+        assert cuda_ops.lib.khq_b200_prefill_pairs(mode) == 0
+        out = torch.full((B, T, H_Q, D), float("nan"), dtype=dt, device="cuda")
+        cuda_ops.gqa_prefill(q, k, v, out, B, T, H_Q, H_KV, D, SCALE)
+        outs.append(out.float())
+    cuda_ops.lib.khq_b200_prefill_pairs(0)
+    assert cuda_ops.lib.khq_b200_prefill_status() == 0
+    eps = 2.0 ** (-10 if dtype == "float16" else -7)  # one unit in the last place
+    # the weights are 16-bit operands too: half a unit each, relative to the row's largest terms
+    assert bool(((outs[0] - outs[1]).abs() <= eps * outs[1].abs() + 2 * eps * outs[1].abs().amax(-1, keepdim=True)).all())
+    assert cuda_ops.lib.khq_b200_prefill_pairs(3) == -100
