@@ -961,8 +961,10 @@ static cudaError_t ensure_smem_attrs() {
     if ((e = cudaFuncSetAttribute(m3::khq_decode_batched_tc5w_kernel, attr, m3::SM_TOTAL)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_window_attn_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(khq_window_step_kernel, attr, WIN_SMEM)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(khq_step_kernel, attr, ST_SM_TOTAL)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(khq_step_wide_kernel, attr, M2_SM_TOTAL)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_kernel<false>, attr, ST_SM_TOTAL)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_kernel<true>, attr, ST_SM_TOTAL)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_wide_kernel<false>, attr, SW_TOTAL)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(khq_step_wide_kernel<true>, attr, SW_TOTAL)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev] = true;
     return cudaSuccess;
 }
@@ -1334,7 +1336,8 @@ extern "C" int launch_khq_layer_token(const khq_layer_ctx* L, void* counters, co
     A.new_v = static_cast<const __half*>(v_new);
     A.new_u = static_cast<const __half*>(k_unroped);
     A.out = static_cast<__half*>(out);
-    A.records = static_cast<float*>(L->attn_partial);
+    A.sums = static_cast<float*>(L->attn_partial);
+    A.ml = reinterpret_cast<float2*>(A.sums + ST_MAX_RECORDS * HQ * D);
     A.counters = static_cast<int*>(counters);
     A.win_start = c_len % L->ring_cap;
     A.win_len = win_len;
@@ -1346,13 +1349,15 @@ extern "C" int launch_khq_layer_token(const khq_layer_ctx* L, void* counters, co
     for (const void* a : arrays) bulk_ok = bulk_ok && aligned(a, 16);
     P.bulk_ok = bulk_ok ? 1 : 0;
     A.wide = aligned(L->k_mask, 16) && aligned(L->k_payload, 8) && aligned(L->v_payload, 8);
-    int csize;
-    step_shape(c_len, csize, A.n_comp, A.blocks_per_cta);
+    int csize, n_comp;
+    step_shape(c_len, csize, n_comp, A.blocks_per_cta);
+    A.n_records = n_comp + 1;
     if (csize == 0)
-        err = launch_pdl(khq_step_kernel, (unsigned)((A.n_comp + 1) * HKV * ST_CLUSTER), (unsigned)ST_CLUSTER, (size_t)ST_SM_TOTAL, stream,
-                         (unsigned)ST_THREADS, A);
+        err = launch_pdl(khq_step_kernel<false>, (unsigned)(A.n_records * HKV * ST_CLUSTER), (unsigned)ST_CLUSTER, (size_t)ST_SM_TOTAL, stream,
+                         (unsigned)ST_THREADS, A, StepBatch{});
     else
-        err = launch_pdl(khq_step_wide_kernel, (unsigned)((A.n_comp + 1) * csize), (unsigned)csize, (size_t)M2_SM_TOTAL, stream, (unsigned)M2_THREADS, A);
+        err = launch_pdl(khq_step_wide_kernel<false>, (unsigned)(A.n_records * csize), (unsigned)csize, (size_t)SW_TOTAL, stream, (unsigned)M2_THREADS, A,
+                         StepBatch{});
     return (err == cudaSuccess) ? 0 : static_cast<int>(err);
 }
 
@@ -1428,6 +1433,7 @@ extern "C" size_t khq_b200_decode_workspace_bytes(int n_slots_total) {
     if (n_slots_total < 0) n_slots_total = 0;
     return 256 + (size_t)n_slots_total * HQ * PART * sizeof(float);
 }
+
 
 // SM count for the planner's default item size.  The planner itself makes no CUDA call that can
 // fail the plan: when no device is current or the query fails it plans for 148 SMs.
@@ -1680,6 +1686,51 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
 
 // The item counter of a persistent launch.  A kernel, because a memset between two kernels keeps the launch of the second one from
 // overlapping the end of the first.
+static size_t step_counter_bytes(int n_desc) { return ((size_t)n_desc * HQ * sizeof(int) + 255) / 256 * 256; }
+
+// A small batch as clusters of the step kernels (khq_step.cuh), mirrored in include/khq_b200.h: where every CTA has one block
+// (khq_step_kernel), else where the clusters that fit on the device take the compressed regions in one or two rounds of 48 tokens per
+// CTA, three for a single sequence; beyond, the persistent kernel's finer items and 148 CTAs win.  Measured per layer of a serving
+// chain with its pre-step, us, persistent kernel and merge / this: sequences of compressed tokens 1 x 0: 18.5 / 10.7, 1 x 768: 28.3 /
+// 18.4, 2 x 128: 26.6 / 16.7, 12 x ~20: 46.4 / 24.2 (one block); 1 x 2304: 33.4 / 28.7, 3 of 128 to 1536: 33.8 / 29.5, 6 x ~256: 38.4 /
+// 32.0 (a round); 6 x ~790: 44.1 / 40.4, 1 x 7680: 42.3 / 38.2 (two); 1 x 15872: 50.5 / 44.5, but 2 x 4736: 41.4 / 43.9 and 4 x ~2500:
+// 42.3 / 44.2 (three).  Returns the kernel (5: khq_step_kernel, 6:
+// khq_step_wide_kernel) and the number of items, or 0 for a batch that is better off with the items of khq_b200_plan_decode.
+extern "C" int khq_b200_plan_steps(const int* c_len, const int* win_len, int n_desc, void* items, int max_items, int* n_items, int* first_slot,
+                                   int* n_slots) {
+    if (!c_len || !win_len || n_desc <= 0 || !items || !n_items || !first_slot || !n_slots) return -100;
+    const int most = plan_sm_count() / 8 - 3;  // clusters of eight CTAs that run side by side; as many sets of four clusters of khq_step_kernel
+    int total = 0;
+    for (int i = 0; i < n_desc; ++i) {
+        if (c_len[i] < 0 || win_len[i] <= 0) return 0;
+        total += (c_len[i] + M2_BT - 1) / M2_BT;
+    }
+    int mode = 0, per = 0;
+    const auto clusters = [&](int p) {
+        int n = 0;
+        for (int i = 0; i < n_desc; ++i) {
+            const int k = ((c_len[i] + M2_BT - 1) / M2_BT + p * ST_CLUSTER - 1) / (p * ST_CLUSTER);
+            if (k + 1 > ST_MAX_RECORDS) return max_items + most + 1;
+            n += k + 1;
+        }
+        return n;
+    };
+    if (clusters(1) <= most) mode = 5, per = 1;
+    for (int p = 3; mode == 0 && p <= (n_desc == 1 ? 9 : 6); p += 3)
+        if (clusters(p) <= most) mode = 6, per = p;
+    if (mode == 0 || clusters(per) > max_items) return 0;
+    KhqWorkItem* w = static_cast<KhqWorkItem*>(items);
+    int n = 0;
+    for (int i = 0; i < n_desc; ++i) {
+        const int blocks = (c_len[i] + M2_BT - 1) / M2_BT, k = (blocks + per * ST_CLUSTER - 1) / (per * ST_CLUSTER);
+        first_slot[i] = n;
+        n_slots[i] = k + 1;
+        for (int j = 0; j <= k; ++j, ++n) w[n] = KhqWorkItem{i, j < k ? 0 : 1, j * per * ST_CLUSTER, per, n, first_slot[i], k + 1, 0};
+    }
+    *n_items = n;
+    return mode;
+}
+
 __global__ void khq_zero_counter_kernel(int* counter) {
     pdl_trigger();
     pdl_wait();
@@ -1696,6 +1747,29 @@ static int decode_batched_impl(const void* descs, const void* tables, const void
     if (err != cudaSuccess) return static_cast<int>(err);
     int* counter = static_cast<int*>(workspace);
     float* partials = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
+    if (codebook_in_smem == 5 || codebook_in_smem == 6) {  // items of khq_b200_plan_steps
+        if (!images || out_partials) return -103;
+        const size_t counters = step_counter_bytes(n_desc);
+        if (workspace_bytes % 256 != 0 || workspace_bytes < khq_b200_decode_workspace_bytes(n_slots_total) + counters) return -105;
+        StepBatch B;
+        B.descs = static_cast<const KhqSeqDesc*>(descs);
+        B.tables = static_cast<const KhqTablesDesc*>(tables);
+        B.images = static_cast<const unsigned char* const*>(images);
+        B.items = static_cast<const KhqWorkItem*>(items);
+        B.sums = partials;
+        B.ml = reinterpret_cast<float2*>(partials + (size_t)n_slots_total * HQ * D);
+        B.counters = reinterpret_cast<int*>(static_cast<unsigned char*>(workspace) + workspace_bytes - counters);
+        B.scale = scale;
+        B.rope_base = rope_base;
+        B.ring_cap = ring_cap;
+        if (codebook_in_smem == 5)
+            err = launch_pdl(khq_step_kernel<true>, (unsigned)(n_items * HKV * ST_CLUSTER), (unsigned)ST_CLUSTER, (size_t)ST_SM_TOTAL, stream,
+                             (unsigned)ST_THREADS, StepArgs{}, B);
+        else
+            err = launch_pdl(khq_step_wide_kernel<true>, (unsigned)(n_items * ST_CLUSTER), (unsigned)ST_CLUSTER, (size_t)SW_TOTAL, stream,
+                             (unsigned)M2_THREADS, StepArgs{}, B);
+        return (err == cudaSuccess) ? 0 : static_cast<int>(err);
+    }
     const int grid = n_items < sm_count() ? n_items : sm_count();
     const bool vqs = codebook_in_smem != 0, mma = codebook_in_smem == 2 || codebook_in_smem < 0;
     if (!mma || n_items > grid) {  // the default kernel takes its first item without the counter

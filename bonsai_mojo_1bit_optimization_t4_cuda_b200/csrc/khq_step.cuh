@@ -28,10 +28,6 @@ constexpr int ST_CLUSTER = 8;                   // CTAs that split the tokens of
 constexpr int ST_MAX_RECORDS = 32;              // records per head
 constexpr int ST_REC = D + 28;                  // a head's sums, four floats of padding after every 32 (bank conflicts)
 constexpr int ST_RECV = ST_REC + 8;             // ... its maximum and sum of weights, and padding
-// Scratch in global memory, (24, 32, 258) floats of the caller: the sums of all records (record, head, 256), then their (maximum, sum
-// of weights) pairs.
-constexpr int ST_ML = ST_MAX_RECORDS * HQ * D;
-static_assert(ST_ML + ST_MAX_RECORDS * HQ * 2 == HQ * ST_MAX_RECORDS * PART, "the caller's split records are the scratch");
 
 // Shared memory of khq_step_kernel.  A staged block: mask words, K payload and V payload of 16 rows.
 constexpr int ST_KPAY = M2_BT * 64, ST_VPAY = ST_KPAY + M2_BT * K_PAY;
@@ -44,7 +40,8 @@ constexpr int ST_SM_RSC = ST_SM_ROT + 16 * 32 * 32;           // per parity of t
 constexpr int ST_SM_RSTEP = ST_SM_RSC + 2 * 16 * 32;          // cos / sin of 16 positions of each rotary pair
 constexpr int ST_SM_RECV = ST_SM_RSTEP + 256;                 // the owned head's records of the cluster's CTAs
 constexpr int ST_SM_BAR = ST_SM_RECV + ST_CLUSTER * ST_RECV * 4;
-constexpr int ST_SM_TOTAL = ST_SM_BAR + 16;
+constexpr int ST_SM_ARGS = ST_SM_BAR + 16;  // of a batch
+constexpr int ST_SM_TOTAL = ST_SM_ARGS + 320;
 constexpr int ST_SM_SEND = 0;                                 // the CTA's records, behind the last block
 static_assert(ST_X_BYTES == NREP * D * 4, "the query build's scratch aliases the exchange buffers");
 static_assert(NREP * ST_RECV * 4 <= ST_SM_SMALL, "the records alias the stages and exchange buffers");
@@ -57,14 +54,72 @@ struct StepArgs {
     __half *ring_k, *ring_v, *ring_u;
     const __half *new_k, *new_v, *new_u;  // the step's token; new_k == nullptr: it is in the rings already
     __half* out;
-    float* records;   // (records, 24, ST_OUT)
+    float* sums;      // (records, 24, 256)
+    float2* ml;       // (records, 24): maximum, sum of weights
     int* counters;    // 24, zero before and after a launch
     int win_start, win_len, ring_cap;
-    int n_comp;       // clusters per kv-head on the compressed region; one more is on the window
+    int n_records;    // clusters (of khq_step_kernel: per kv-head)
+    int rec;          // a batch: this cluster's record; otherwise record 0 .. n_records - 2 are the compressed region's clusters
+    int comp;         // a batch: whether that is the compressed region's
+    int block0;       // a batch: the cluster's first block of 16 tokens
     int blocks_per_cta;
     int wide;         // masks on 16 bytes, payloads on 8
     float scale;
 };
+constexpr int ST_ARGS_BYTES = 320;
+static_assert(sizeof(StepArgs) <= ST_ARGS_BYTES && sizeof(StepArgs) % 8 == 0, "shared memory of a batch");
+// A batch (khq_b200_plan_steps): item i is cluster i (of khq_step_kernel: clusters 4i .. 4i + 3, one per kv-head).
+struct StepBatch {
+    const KhqSeqDesc* descs;  // all with the same tables
+    const KhqTablesDesc* tables;
+    const unsigned char* const* images;
+    const KhqWorkItem* items;  // kind 0 / 1, lo: first block, hi: blocks per CTA, slot: record, r0: the problem's first one, r1: its number
+    float* sums;
+    float2* ml;
+    int* counters;  // (problems, 24)
+    float scale, rope_base;
+    int ring_cap;
+};
+// The layer's constants, which may be read ahead of the kernel's wait, and the item.
+__device__ __forceinline__ void st_fill_constants(StepArgs& A, const StepBatch& B) {
+    const int id = B.descs[0].table_id;
+    const KhqTablesDesc& t = B.tables[id];
+    A.kv.cents_k = t.cents_k; A.kv.cents_v = t.cents_v; A.kv.vq = t.vq; A.kv.k_rotor = t.k_rotor;
+    A.kv.v_rotor = t.v_rotor; A.kv.d_k = t.d_k; A.kv.d_v = t.d_v;
+    A.kv.alpha_k = t.alpha_k; A.kv.alpha_v = t.alpha_v; A.kv.rope_base = B.rope_base;
+    A.kv.image = B.images[id];
+}
+__device__ __forceinline__ void st_fill_item(StepArgs& A, const StepBatch& B, int item) {
+    const KhqWorkItem w = B.items[item];
+    const KhqSeqDesc& d = B.descs[w.desc];
+    A.kv.k_payload = d.k_payload; A.kv.v_payload = d.v_payload; A.kv.v_shared_meta = d.v_shared_meta;
+    A.kv.k_mask = d.k_mask; A.kv.k_norms = d.k_norms; A.kv.k_r_norms = d.k_r_norms;
+    A.kv.v_norms = d.v_norms; A.kv.v_r_norms = d.v_r_norms;
+    A.kv.start_pos = d.start_pos; A.kv.c_len = d.c_len;
+    const auto off = [](const void* p) { return (uint32_t)reinterpret_cast<uintptr_t>(p); };
+    A.kv.bulk_ok = ((off(d.k_payload) | off(d.v_payload) | off(d.v_shared_meta) | off(d.k_mask) | off(d.k_norms) | off(d.k_r_norms) |
+                     off(d.v_norms) | off(d.v_r_norms)) & 15u) == 0u;
+    A.wide = (off(d.k_mask) & 15u) == 0u && ((off(d.k_payload) | off(d.v_payload)) & 7u) == 0u;
+    unpack_pos(d.pos_pack, A.kv);
+    A.q = d.q_gate;
+    A.ring_k = const_cast<__half*>(d.ring_k);
+    A.ring_v = const_cast<__half*>(d.ring_v);
+    A.ring_u = nullptr;
+    A.new_k = A.new_v = A.new_u = nullptr;
+    A.out = d.out;
+    A.sums = B.sums + (size_t)w.r0 * HQ * D;
+    A.ml = B.ml + (size_t)w.r0 * HQ;
+    A.counters = B.counters + w.desc * HQ;
+    A.win_start = d.win_start;
+    A.win_len = d.win_len;
+    A.ring_cap = B.ring_cap;
+    A.n_records = w.r1;
+    A.rec = w.slot - w.r0;
+    A.comp = w.kind == 0;
+    A.block0 = w.lo;
+    A.blocks_per_cta = w.hi;
+    A.scale = B.scale;
+}
 
 __device__ __forceinline__ void st_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -686,12 +741,12 @@ __device__ __forceinline__ void st_window(unsigned char* smem, const StepArgs& A
 // The warp's share of head h, record `rec` of n: with several records the warp that arrives last merges them all; then the division
 // and the gate.
 __device__ __forceinline__ void st_finish_head(const StepArgs& A, int h, int rec, int lane, HeadAcc& a, const uint4& gate) {
-    const int n = A.n_comp + 1;
+    const int n = A.n_records;
     if (n > 1) {
-        float* r = A.records + ((size_t)rec * HQ + h) * D + lane * 8;
+        float* r = A.sums + ((size_t)rec * HQ + h) * D + lane * 8;
         __stcg(reinterpret_cast<float4*>(r), make_float4(a.a[0], a.a[1], a.a[2], a.a[3]));
         __stcg(reinterpret_cast<float4*>(r + 4), make_float4(a.a[4], a.a[5], a.a[6], a.a[7]));
-        float2* ml_of = reinterpret_cast<float2*>(A.records + ST_ML) + h;
+        float2* ml_of = A.ml + h;
         if (lane == 0) __stcg(ml_of + rec * HQ, make_float2(a.m, a.l));
         __syncwarp();
         int order = 0;
@@ -703,7 +758,7 @@ __device__ __forceinline__ void st_finish_head(const StepArgs& A, int h, int rec
         if (__shfl_sync(0xFFFFFFFFu, order, 0) != n - 1) return;
         if (lane == 0) A.counters[h] = 0;
         constexpr int AHEAD = 6;  // records whose sums are on their way beside the maxima
-        const float* base = A.records + (size_t)h * D + lane * 8;
+        const float* base = A.sums + (size_t)h * D + lane * 8;
         float2 ml = make_float2(NEG_BIG, 0.0f);
         if (lane < n) ml = __ldcg(ml_of + lane * HQ);
         float4 v[AHEAD][2];
@@ -748,26 +803,27 @@ __device__ __forceinline__ void st_finish_head(const StepArgs& A, int h, int rec
     *reinterpret_cast<uint4*>(A.out + (size_t)h * D + lane * 8) = o;
 }
 
-// grid = 4 kv-heads x (n_comp + 1) clusters; the last four serve the window.
-__global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_constant__ StepArgs A) {
+// grid = 4 kv-heads x n_records clusters, the last four serve the window; or four clusters per item of a batch.
+template <bool BATCH>
+__global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_constant__ StepArgs one, const __grid_constant__ StepBatch batch) {
     extern __shared__ __align__(128) unsigned char smem[];
+    StepArgs& filled = *reinterpret_cast<StepArgs*>(smem + ST_SM_ARGS);
+    const StepArgs& A = BATCH ? filled : one;
     const int tid = threadIdx.x, part = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
-    const int rank = (int)blockIdx.x % ST_CLUSTER, cl = (int)blockIdx.x / ST_CLUSTER, kvh = cl % HKV, rec = cl / HKV;
-    const bool comp = rec < A.n_comp;
+    const int rank = (int)blockIdx.x % ST_CLUSTER, cl = (int)blockIdx.x / ST_CLUSTER, kvh = cl % HKV;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + ST_SM_BAR);
     float* recv = reinterpret_cast<float*>(smem + ST_SM_RECV);
     if (tid == 0) {
         mbar_init(bar, 1);
         fence_barrier_init();
         mbar_arrive_expect_tx(bar, ST_CLUSTER * ST_RECV * 4);
+        if (BATCH) st_fill_constants(filled, batch);
     }
     __syncthreads();
     st_cluster_arrive();  // waited for before the first push: the peers' barriers are there
-    const int block0 = (rec * ST_CLUSTER + rank) * A.blocks_per_cta;
-    const int nblk = comp ? min(max((A.kv.c_len + M2_BT - 1) / M2_BT - block0, 0), A.blocks_per_cta) : 0;
     StepQueryTables qt;
     float4 rope[2];
-    if (comp) {  // constants of the model: fetched while the kernel in front still runs
+    if (BATCH || cl / HKV < A.n_records - 1) {  // constants of the model: fetched while the kernel in front still runs
         qt.load(A.kv, part, lane);
         const uint4* src = reinterpret_cast<const uint4*>(A.kv.image + M2_IMG_ROT);
         uint4* dst = reinterpret_cast<uint4*>(smem + ST_SM_ROT);
@@ -779,7 +835,7 @@ __global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_co
         const uint4* small = reinterpret_cast<const uint4*>(A.kv.image + M2_IMG_SMALL);
         for (int e = tid; e < M2_SMALL_BYTES / 16; e += ST_THREADS) reinterpret_cast<uint4*>(smem + ST_SM_SMALL)[e] = __ldg(small + e);
         const float* freq = reinterpret_cast<const float*>(A.kv.image + M2_IMG_SMALL);
-        st_rope_seed(rope, A.kv, freq, part, lane, block0 * M2_BT);
+        if (!BATCH) st_rope_seed(rope, A.kv, freq, part, lane, (cl / HKV * ST_CLUSTER + rank) * A.blocks_per_cta * M2_BT);
         if (tid < 32) {
             double th = (double)M2_BT * (double)freq[tid] * 0.3183098861837907;  // half turns
             th -= 2.0 * rint(0.5 * th);
@@ -790,6 +846,15 @@ __global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_co
     st_cluster_wait();
     pdl_wait();
     pdl_trigger();
+    if (BATCH) {
+        if (tid == 0) st_fill_item(filled, batch, cl / HKV);
+        __syncthreads();
+    }
+    const int rec = BATCH ? A.rec : cl / HKV;
+    const bool comp = BATCH ? A.comp != 0 : rec < A.n_records - 1;
+    const int block0 = BATCH ? A.block0 + rank * A.blocks_per_cta : (rec * ST_CLUSTER + rank) * A.blocks_per_cta;
+    const int nblk = comp ? min(max((A.kv.c_len + M2_BT - 1) / M2_BT - block0, 0), A.blocks_per_cta) : 0;
+    if (BATCH && nblk > 0) st_rope_seed(rope, A.kv, reinterpret_cast<const float*>(smem + ST_SM_SMALL), part, lane, block0 * M2_BT);
     float val[2][8], m[2], l[2];
     if (comp) {
         st_compressed(smem, A, block0, nblk, qt, rope, tid, kvh, part, lane, val, m, l);
@@ -841,14 +906,18 @@ __global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_co
 // one cluster of the same grid has the window (window_range).  The three warps of a kv-head are merged inside the CTA, the rest
 // is as above.  One more cluster barrier than there: the received records take the codebook's place.
 constexpr int SW_SEND = M2_SM_VQ, SW_RECV = SW_SEND + 32 * 1024;
-static_assert(HQ * ST_RECV * 4 <= 32 * 1024 && SW_RECV + HQ * ST_RECV * 4 <= M2_SM_ROPE && SW_SEND % 16 == 0, "records take the codebook's place");
-__global__ void __launch_bounds__(M2_THREADS, 1) khq_step_wide_kernel(const __grid_constant__ StepArgs A) {
+constexpr int SW_ARGS = (M2_SM_TOTAL + 15) / 16 * 16, SW_TOTAL = SW_ARGS + ST_ARGS_BYTES;  // of a batch
+static_assert(SW_TOTAL <= 226 * 1024 && HQ * ST_RECV * 4 <= 32 * 1024 && SW_RECV + HQ * ST_RECV * 4 <= M2_SM_ROPE && SW_SEND % 16 == 0, "records take the codebook's place");
+template <bool BATCH>
+__global__ void __launch_bounds__(M2_THREADS, 1) khq_step_wide_kernel(const __grid_constant__ StepArgs one, const __grid_constant__ StepBatch batch) {
     extern __shared__ __align__(128) unsigned char smem[];
+    StepArgs& filled = *reinterpret_cast<StepArgs*>(smem + SW_ARGS);
+    const StepArgs& A = BATCH ? filled : one;
     __shared__ __align__(8) uint64_t s_bar;
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31, kvh = warp & 3, sub = warp >> 2;
-    const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), rec = (int)blockIdx.x / csize, owned = HQ / csize;
-    const bool comp = rec < A.n_comp;
+    const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), cl = (int)blockIdx.x / csize, owned = HQ / csize;
+    const bool tables = BATCH || cl < A.n_records - 1;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M2_SM_BARS);
     uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + M2_SM_TMSLOT);
     if (tid == 0) {
@@ -857,25 +926,37 @@ __global__ void __launch_bounds__(M2_THREADS, 1) khq_step_wide_kernel(const __gr
         mbar_init(&s_bar, 1);
         fence_barrier_init();
         mbar_arrive_expect_tx(&s_bar, HQ * ST_RECV * 4);
+        if (BATCH) st_fill_constants(filled, batch);
     }
-    if (comp) m2_tm_alloc(tm_slot, warp);
+    if (tables) m2_tm_alloc(tm_slot, warp);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = comp ? __shfl_sync(0xFFFFFFFFu, *tm_slot, 0) : 0u;
+    const uint32_t tmem = tables ? __shfl_sync(0xFFFFFFFFu, *tm_slot, 0) : 0u;
     VInverse inv;
-    if (comp) {
-        M2QueryTables qt;
+    M2QueryTables qt;
+    if (tables) {
         m2_load_tables(smem, A.kv, tmem, tid, warp, lane);  // constants of the model: while the kernel in front still runs
         qt.load(A.kv, sub, lane);
-        pdl_wait();
-        pdl_trigger();
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (BATCH) {
+        if (tid == 0) st_fill_item(filled, batch, cl);
+        __syncthreads();
+    }
+    const int rec = BATCH ? A.rec : cl;
+    const bool comp = BATCH ? A.comp != 0 : tables;
+    if (comp) {
         unsigned blocks_done = 0;
-        const int lo = min((int)blockIdx.x * M2_BT * A.blocks_per_cta, A.kv.c_len), hi = min(lo + M2_BT * A.blocks_per_cta, A.kv.c_len);
+        const int block0 = BATCH ? A.block0 + rank * A.blocks_per_cta : (int)blockIdx.x * A.blocks_per_cta;
+        const int lo = min(M2_BT * block0, A.kv.c_len), hi = min(lo + M2_BT * A.blocks_per_cta, A.kv.c_len);
         m2_compressed_range(smem, A.q, (size_t)2 * D, A.kv, lo, hi, A.scale, blocks_done, tmem, qt, 1u, inv);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     } else {
-        pdl_wait();
-        pdl_trigger();
+        if (BATCH) {  // the tables that it has no use for: no copy outlives the kernel, none lands in what follows
+            mbar_wait_bounded(&bars[M2_BAR_SMALL], 0u, &g_status);
+            mbar_wait_bounded(&bars[M2_BAR_VQ], 0u, &g_status);
+        }
         if (rank < 3) {  // ring appends: one ring per CTA
             const size_t at = (size_t)((A.win_start + A.win_len - 1) % A.ring_cap) * HKV * D;
             const __half* src = rank == 0 ? A.new_k : rank == 1 ? A.new_v : A.new_u;
@@ -909,7 +990,7 @@ __global__ void __launch_bounds__(M2_THREADS, 1) khq_step_wide_kernel(const __gr
     }
     fence_proxy_async();
     __syncthreads();
-    if (comp) m2_tm_free(tmem, warp);
+    if (tables) m2_tm_free(tmem, warp);
     st_cluster_wait();
     float* recv = reinterpret_cast<float*>(smem + SW_RECV);
     if (tid < HQ)

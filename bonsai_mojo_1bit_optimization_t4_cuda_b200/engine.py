@@ -142,7 +142,8 @@ class BatchEngine:
         sms_plan = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 148
         tail_items = int(4 * sms_plan * (1.0 + np.log(self.tokens_per_item / 48.0))) + 16
         self.max_items = int(sum((int(c) + self.tokens_per_item - 1) // self.tokens_per_item + 2 for c in self.cap)) + tail_items
-        self.ws_bytes = int(self.lib.khq_b200_decode_workspace_bytes(self.max_items))
+        # the last bytes: counters of the step kernels (khq_b200_plan_steps), zero
+        self.ws_bytes = _align(int(self.lib.khq_b200_decode_workspace_bytes(self.max_items)), 256) + _align(self.B * H_Q * 4, 256)
         self.workspace = z(self.ws_bytes, torch.uint8)
         # a step's control block: per-sequence state, ring slots, positions, work items and, last, the runs that are
         # compressed this step (copied only when there are some); one copy per step, device and host laid out alike
@@ -288,10 +289,20 @@ class BatchEngine:
         w = (self.write_pos - self.boundary).astype(np.int32)
         first = np.empty(self.B, np.int32)
         cnt = np.empty(self.B, np.int32)
-        n = self.lib.khq_b200_plan_decode(c.ctypes.data, w.ctypes.data, self.B, self.tokens_per_item_arg,
-                                          ctl["block"].data_ptr() + self._at["items"], self.max_items, first.ctypes.data, cnt.ctypes.data)
-        if n < 0 or n > self.max_items:
-            raise _lib.KhqLaunchError("khq_b200_plan_decode", n)
+        items = ctl["block"].data_ptr() + self._at["items"]
+        # a small batch: the kernels of a single sequence's step
+        self._kernel, steps = int(self.codebook_in_smem), ctypes.c_int(0)
+        mode = 0
+        if self._kernel < 0 and self.tokens_per_item_arg == 0:
+            mode = self.lib.khq_b200_plan_steps(c.ctypes.data, w.ctypes.data, self.B, items, self.max_items, ctypes.addressof(steps),
+                                                first.ctypes.data, cnt.ctypes.data)
+        if mode > 0:
+            self._kernel, n = mode, steps.value
+        else:
+            n = self.lib.khq_b200_plan_decode(c.ctypes.data, w.ctypes.data, self.B, self.tokens_per_item_arg, items, self.max_items,
+                                              first.ctypes.data, cnt.ctypes.data)
+            if n < 0 or n > self.max_items:
+                raise _lib.KhqLaunchError("khq_b200_plan_decode", n)
         self.n_items = int(n)
         dyn["c_len"], dyn["start_pos"], dyn["win_start"], dyn["win_len"] = c, 0, c % RING, w
         dyn["first_slot"], dyn["n_slots"] = first, cnt
@@ -358,7 +369,7 @@ class BatchEngine:
         rc = self.lib.launch_khq_decode_batched_prepared_fp16(
             self.d_descs.data_ptr() + layer * self.B * SEQ_DESC.itemsize, self.d_tables.data_ptr(), self._d_images.data_ptr(), self.d_items.data_ptr(),
             self.B, self.n_items, self.workspace.data_ptr(), self.ws_bytes, self.n_items, float(scale), self.rope_theta, RING,
-            int(self.codebook_in_smem), current_stream())
+            self._kernel if self._kernel >= 5 else int(self.codebook_in_smem), current_stream())  # the items' kernel
         check("launch_khq_decode_batched_prepared_fp16", rc)
 
     def _host_buffer(self, t, name: str):
@@ -399,7 +410,7 @@ class BatchEngine:
         self._plan(ctl)
         a.h_control, a.control_bytes, a.parity = ctl["block"].data_ptr(), self._control_bytes(n_ev), parity
         a.n_items, a.n_events, a.scale = self.n_items, n_ev, float(scale)
-        a.codebook_in_smem, a.rms_eps = int(self.codebook_in_smem), self.rms_eps
+        a.codebook_in_smem, a.rms_eps = self._kernel, self.rms_eps
         if self.rope_theta != self._laid_out_theta:
             self.refresh_tables()
         given = dict(q=self.h_q, k=self.h_k, v=self.h_v, out=self.h_out)

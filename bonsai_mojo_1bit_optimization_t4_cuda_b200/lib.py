@@ -45,6 +45,7 @@ SIGNATURES = {
     "launch_khq_decode_batched_prepared_fp16": (
         c_int, [_P, _P, _P, _P, c_int, c_int, _P, c_size_t, c_int, c_float, c_float, c_int, c_int, _P]),
     "launch_khq_layer_step": (c_int, [_P] * 6 + [c_int] * 4 + [c_float, _P]),
+    "khq_b200_plan_steps": (c_int, [_P, _P, c_int, _P, c_int, _P, _P, _P]),
     "launch_khq_layer_token": (c_int, [_P] * 7 + [c_int] * 3 + [c_float, _P]),
     "launch_khq_layer_prefill": (c_int, [_P] * 6 + [c_int] * 2 + [c_float, _P]),
     "khq_b200_engine_create": (c_int, [POINTER(c_void_p)]),

@@ -301,6 +301,13 @@ typedef struct khq_layer_ctx {
 int launch_khq_layer_step(const khq_layer_ctx* ctx, const void* q_gate, const void* k_roped, const void* v_new,
                           const void* k_unroped, void* out, int c_len, int win_len, int compress, int num_splits, float scale,
                           khq_stream_t stream);
+/* A small batch for the same kernels: items for launch_khq_decode_batched_prepared_fp16 / launch_khq_engine_step with codebook_in_smem set
+ * to the returned 5 or 6, or 0 if khq_b200_plan_decode's serve the batch better (then nothing is written).  All descriptors of such a
+ * launch name the same tables; table_id, tables and images are read before the launch waits for the one in front of it.  The
+ * workspace's last ceil(n_desc * 24 * 4 / 256) * 256 bytes are counters, beyond khq_b200_decode_workspace_bytes(n_items): zero before the
+ * first such launch (each leaves them zero), workspace_bytes a multiple of 256, both -105 otherwise; -103 without images. */
+int khq_b200_plan_steps(const int* c_len, const int* win_len, int n_desc, void* items, int max_items, int* n_items, int* first_slot,
+                        int* n_slots);
 /* The same step as ONE kernel beside the event's two: the library cuts the regions by its own rule.  Needs ctx->prepared;
  * ctx->attn_partial holds (24, 32, 258) fp32 on 16 bytes; `counters`: 24 int32 on the device, zero before the first step that is
  * given them (each step leaves them zero) and, like attn_partial, not shared by steps that may run at the same time.  Returns as

@@ -224,3 +224,41 @@ def test_replaced_host_buffers(cuda_ops, form):
     torch.cuda.synchronize()
     got = torch.stack(list(got)) if form == "list" else got
     assert torch.equal(got.cpu().half(), want)
+
+
+@pytest.mark.parametrize("c_len,win,kernel", [
+    ([0, 128, 256], [1, 128, 250], 5), ([1664], [200], 5), ([1920], [130], 6), ([0, 4224, 128, 1280], [255, 129, 131, 200], 6),
+    ([16000], [200], 6), ([640] * 6, [128, 140, 150, 160, 170, 180], 6), ([40064], [200], -1), ([128] * 16, [130] * 16, -1)])
+def test_small_batches_through_the_step_kernels(cuda_ops, c_len, win, kernel):
+    """The same step through the kernels of a single sequence (khq_b200_plan_steps), where that takes the batch, and through the
+    persistent one."""
+    import torch
+
+    from bonsai_mojo_1bit_optimization_t4_cuda_b200.engine import BatchEngine
+
+    rng = np.random.default_rng(4)
+    k, v = cases.synth.make_kv(rng, 64)
+    tb = cases.synth.make_tables(rng, 3, k.reshape(-1, D), v.reshape(-1, D), vq_scale=1.0 / 16.0)
+    outs, engines = [], []
+    for gen in (-1, 2):
+        eng = BatchEngine([tb, tb], c_len, win, grow_tokens=128, codebook_in_smem=gen)
+        eng.fill_synthetic(7)
+        g = torch.Generator().manual_seed(9)
+        steps = []
+        for _ in range(3):  # the counters are left as they were
+            for h in (eng.h_q, eng.h_k, eng.h_v):
+                h.copy_(torch.randn(h.shape, generator=g).half())
+            eng.decode_step(SCALE)
+            torch.cuda.synchronize()
+            steps.append(eng.h_out.float().clone())
+        outs.append(torch.stack(steps))
+        engines.append(eng)
+    assert engines[0]._kernel == kernel and engines[1]._kernel == 2 and cuda_ops.lib.khq_b200_device_status() == 0
+    # fp32 sums in another order on both sides (some 1e-6 of the largest term), then one rounding to fp16
+    err, want = (outs[0] - outs[1]).abs(), outs[1].abs()
+    assert bool((err <= 2.0 ** -10 * want + 3e-4 * want.max()).all()), float(err.max())
+    for eng in engines:  # the resident entry, with the items of the last step
+        eng.attention_resident(0, SCALE)
+    torch.cuda.synchronize()
+    a, b = (eng.out[0].float() for eng in engines)
+    assert bool(((a - b).abs() <= 2.0 ** -10 * b.abs() + 3e-4 * b.abs().max()).all())
