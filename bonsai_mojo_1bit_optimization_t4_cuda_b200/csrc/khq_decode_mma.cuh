@@ -63,7 +63,8 @@ constexpr int M2_SM_FREQ = M2_SM_RSC + M2_THREADS / 32 * 16 * 32;      // 32 flo
 constexpr int M2_SM_DINV = M2_SM_FREQ + 128;                         // 64 floats: 1 / (256 d) of the rotary dims
 constexpr int M2_SM_C3 = M2_SM_DINV + 256;                           // 64 patches x float2: alpha_v x (mean, half the difference 0 - 1) of the two dim-3 centroids
 constexpr int M2_SM_RSTEP = M2_SM_C3 + NP * 8;                       // 32 x float2: cos / sin of M2_TT positions of each rotary pair
-constexpr int M2_SMALL_BYTES = 128 + 256 + NP * 8 + 32 * 8;
+constexpr int M2_SM_FLAGS = M2_SM_RSTEP + 32 * 8;                    // nonzero: rotor fragments have low-order parts
+constexpr int M2_SMALL_BYTES = 128 + 256 + NP * 8 + 32 * 8 + 16;
 constexpr int M2_SM_BARS = M2_SM_FREQ + M2_SMALL_BYTES;              // M2_WPK * M2_NSTAGE stages, then the image's small tables and codebook
 constexpr int M2_BAR_SMALL = M2_WPK * M2_NSTAGE, M2_BAR_VQ = M2_BAR_SMALL + 1, M2_NBARS = M2_BAR_VQ + 1;
 constexpr int M2_SM_TMSLOT = M2_SM_BARS + M2_NBARS * 8;
@@ -269,7 +270,7 @@ __device__ __forceinline__ void m2_stage_codebook(unsigned char* dst, const __ha
     }
 }
 
-// A layer's small tables to `dst` (the order of M2_SM_FREQ ..), one entry per thread.
+// A layer's small tables to `dst` (the order of M2_SM_FREQ ..), one entry per thread; without the flags.
 __device__ __forceinline__ void m2_small_tables(unsigned char* dst, const CompressedKV& P, int tid) {
     constexpr int O_DINV = M2_SM_DINV - M2_SM_FREQ, O_C3 = M2_SM_C3 - M2_SM_FREQ, O_RSTEP = M2_SM_RSTEP - M2_SM_FREQ;
     if (tid < 32) reinterpret_cast<float*>(dst)[tid] = powf(P.rope_base, -2.0f * (float)tid / 64.0f);
@@ -292,6 +293,7 @@ __device__ __forceinline__ void m2_small_tables(unsigned char* dst, const Compre
 struct M2Query {
     uint32_t tm;   // tensor-memory address of this warp's query fragments
     uint32_t rot;  // ... and of its lane quadrant's rotor fragments
+    bool low;      // the rotor fragments have low-order parts
 };
 
 __device__ __forceinline__ void m2_tm_st4f(uint32_t taddr, const float* r) {
@@ -314,6 +316,9 @@ __device__ __forceinline__ void m2_tm_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
+}
+__device__ __forceinline__ void m2_tm_ld4(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void m2_tm_st16f(uint32_t taddr, const float* r) {
     asm volatile(
@@ -415,6 +420,7 @@ __device__ __forceinline__ void m2_load_tables(unsigned char* smem, const Compre
 
 // grid = 1: the image of one layer.
 __global__ void __launch_bounds__(M2_THREADS) khq_prepare_tables_kernel(CompressedKV P, unsigned char* __restrict__ image) {
+    uint32_t low = 0;
     m2_small_tables(image + M2_IMG_SMALL, P, threadIdx.x);
     m2_stage_codebook(image + M2_IMG_VQ, P.vq, threadIdx.x);
     for (int c = threadIdx.x; c < 256; c += M2_THREADS) *reinterpret_cast<uint32_t*>(image + M2_IMG_VQ + c * M2_VQ_ROW + M2_VQ_ROW - 4) = 0u;
@@ -429,7 +435,10 @@ __global__ void __launch_bounds__(M2_THREADS) khq_prepare_tables_kernel(Compress
         uint4* o = reinterpret_cast<uint4*>(image + M2_IMG_ROT) + 2 * e;
         o[0] = make_uint4(r[0], r[1], r[2], r[3]);
         o[1] = make_uint4(r[4], r[5], r[6], r[7]);
+        low |= (r[4] | r[5] | r[6] | r[7]) & 0x7FFF7FFFu;
     }
+    const int any = __syncthreads_or((int)low);
+    if (threadIdx.x < 4) reinterpret_cast<uint32_t*>(image + M2_IMG_SMALL + (M2_SM_FLAGS - M2_SM_FREQ))[threadIdx.x] = any != 0 ? 1u : 0u;
 }
 
 // Where the query build's scratch keeps the four dims 4c .. 4c + 3 of head h: swizzled so that the eight lanes (two heads, four
@@ -644,13 +653,19 @@ __device__ __forceinline__ void m2_word(M2KRows& kr, int x, int wi, uint32_t (&t
     }
 }
 
-template <bool ANY>
+// LOW: the rotor fragments have low-order parts.  The products of an identity rotor (centroids and +-1, what a calibration leaves for
+// K) are exact in fp16, so 32 of a block's 176 products would add zeros.
+template <bool ANY, bool LOW>
 __device__ __forceinline__ void m2_k_gemm(M2KRows& kr, const M2Query& Q, const float (&ratio)[2], M2KSums& ks) {
     float (&cs)[4] = ks.cs, (&cs2)[4] = ks.cs2, (&cu)[8][4] = ks.cu;
     float cur[4];  // residual part of a rotor tile, before the row scale
     uint32_t qf[2][8], rf[2][8];  // this and the next k-step's query and rotor fragments
     m2_tm_ld8(Q.tm, qf[0]);
-    m2_tm_ld8(Q.rot, rf[0]);
+    const auto load_rot = [&](int s, uint32_t (&r)[8]) {
+        if (LOW) m2_tm_ld8(Q.rot + 8 * s, r);
+        else m2_tm_ld4(Q.rot + 8 * s, r);
+    };
+    load_rot(0, rf[0]);
 #pragma unroll
     for (int wi = 0; wi < 4; ++wi) {
         // a whole mask word (16 dims = this thread's share of four k-steps) of each of the two rows at once
@@ -666,7 +681,7 @@ __device__ __forceinline__ void m2_k_gemm(M2KRows& kr, const M2Query& Q, const f
             m2_tm_ld_wait();
             if (s + 1 < 16) {
                 m2_tm_ld8(Q.tm + 8 * (s + 1), qf[(s + 1) & 1]);
-                m2_tm_ld8(Q.rot + 8 * (s + 1), rf[(s + 1) & 1]);
+                load_rot(s + 1, rf[(s + 1) & 1]);
             }
             const uint32_t(&qq)[8] = qf[s & 1];  // q1.x, q1.y, q2.x, q2.y, then their low-order halves
             const uint32_t(&rr)[8] = rf[s & 1];  // b1.x, b1.y, b2.x, b2.y, then their low-order halves
@@ -688,8 +703,10 @@ __device__ __forceinline__ void m2_k_gemm(M2KRows& kr, const M2Query& Q, const f
             }
             m2_mma_lo(cs, a1, qq[4], qq[5]);  // low-order halves of the query operands: the code operands are exact
             m2_mma_lo(cs2, ax, qq[6], qq[7]);
-            m2_mma_lo(cu[s >> 1], a1, rr[4], rr[5]);
-            m2_mma_lo(cur, ax, rr[6], rr[7]);
+            if (LOW) {
+                m2_mma_lo(cu[s >> 1], a1, rr[4], rr[5]);
+                m2_mma_lo(cur, ax, rr[6], rr[7]);
+            }
             if (s & 1) {
                 float* c = cu[s >> 1];
                 m2_fma2(c[0], c[1], ratio[0], ratio[0], cur[0], cur[1], c[0], c[1]);
@@ -705,7 +722,7 @@ __device__ __noinline__ void m2_k_gemm_odd(const M2KRows& kr0, const M2Query& Q0
     const M2Query Q = Q0;
     M2KSums ks;
     const float ratio[2] = {ratio0, ratio1};
-    m2_k_gemm<true>(kr, Q, ratio, ks);
+    m2_k_gemm<true, true>(kr, Q, ratio, ks);
     out = ks;
 }
 
@@ -746,7 +763,8 @@ __device__ __forceinline__ void m2_block(const unsigned char* __restrict__ S, co
     const float ratio[2] = {rsc[2 * g].z, rsc[2 * (g + 8)].z};
     M2KSums ks;
     if (!__any_sync(0xFFFFFFFFu, odd)) {
-        m2_k_gemm<false>(kr, Q, ratio, ks);
+        if (Q.low) m2_k_gemm<false, true>(kr, Q, ratio, ks);
+        else m2_k_gemm<false, false>(kr, Q, ratio, ks);
     } else {  // only these have their address taken
         const M2KRows krm = kr;
         const M2Query Qm = Q;
@@ -984,6 +1002,7 @@ __device__ __forceinline__ void m2_compressed_range(unsigned char* smem, const _
     const uint32_t table_parity = (table_loads + 1u) & 1u;
     if (P.image != nullptr) mbar_wait_bounded(&table_bars[0], table_parity, &g_status);
     bool vq_ready = P.image == nullptr;
+    Q.low = P.image == nullptr || *reinterpret_cast<const uint32_t*>(smem + M2_SM_FLAGS) != 0u;
     if (nblk > 0) m2_fill_rope(rope_tab, freq_s, P, base, gtid);
     M2State st;
     st.tm_o = tmem + ((uint32_t)(32 * kvh) << 16) + M2_TM_ACC + M2_TM_ACC_WARP * (uint32_t)sub;
