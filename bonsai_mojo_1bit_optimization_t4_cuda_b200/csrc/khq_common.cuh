@@ -77,8 +77,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 // that one has completed and its writes are visible.  trigger() lets the next kernel start.
 //   * Late trigger, behind the kernel's own wait(): what starts then knows everything before its predecessor to be complete.  All
 //     kernels but those of the next point.
-//   * Early trigger, before the own wait(): the two pre-steps, the counter kernel, and the step's tail with a compressed region.  What
+//   * Early trigger, before the own wait(): the two pre-steps, the counter kernel, the ring fill, and the step's tail with a compressed region.  What
 //     starts behind one of them may run beside the kernel before that one too.
+// khq_ring_fill_kernel writes before its wait, behind kernels that trigger late or not at all, see there.
 // So before its own wait() a kernel reads nothing but constants of the model (tables, their image: launch_khq_prepare_tables and
 // the runtime order their writes) and writes nothing.  One exception: khq_window_step_kernel with a compressed region reads the step's
 // inputs and rings and appends to the rings first.  decode_step_impl launches it directly behind the attention or its

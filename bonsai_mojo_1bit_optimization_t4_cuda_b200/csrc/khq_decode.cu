@@ -1363,19 +1363,25 @@ extern "C" int launch_khq_layer_token(const khq_layer_ctx* L, void* counters, co
 
 // The newest rows of a prompt into the three rings, row by row at slot = token % ring_cap.  Grid (16-byte vectors, 3 rings).  One
 // launch instead of up to six copies: short prompts are bound by launches (a 2 KB row per token and ring, 1.5 us).
+// It copies beside the kernel before and waits for that at its end only.  launch_khq_layer_prefill puts it directly behind the attention,
+// which lets it start when everything before that is complete and shares nothing with it but inputs that both read, or behind the
+// compression, which ends before it starts.
 __global__ void __launch_bounds__(256)
 khq_ring_fill_kernel(const uint4* __restrict__ k_roped, const uint4* __restrict__ v, const uint4* __restrict__ k_unroped,
                      uint4* __restrict__ ring_k, uint4* __restrict__ ring_v, uint4* __restrict__ ring_u, int first, int tokens,
                      int ring_cap) {
     constexpr int ROW = HKV * D / 8;
-    pdl_wait();
-    pdl_trigger();
+    pdl_trigger();  // the kernel behind reads nothing but constants before its own wait
     const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= tokens * ROW) return;
+    if (i >= tokens * ROW) {
+        pdl_wait();
+        return;
+    }
     const int token = first + i / ROW;
     const uint4* src = blockIdx.y == 0 ? k_roped : blockIdx.y == 1 ? v : k_unroped;
     uint4* dst = blockIdx.y == 0 ? ring_k : blockIdx.y == 1 ? ring_v : ring_u;
     dst[(size_t)(token % ring_cap) * ROW + i % ROW] = src[(size_t)token * ROW + i % ROW];
+    pdl_wait();
 }
 
 extern "C" int launch_khq_gqa_prefill_fp16(const void*, const void*, const void*, void*, int, int, int, int, int, float, long long,

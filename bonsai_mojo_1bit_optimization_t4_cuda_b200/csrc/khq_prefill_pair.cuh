@@ -175,6 +175,7 @@ khq_gqa_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     // Everything above overlaps the kernel before; tensor memory is only taken once that kernel has finished (it may still have
     // to allocate its own on this SM).
     khq::pdl_wait();
+    khq::pdl_trigger();
     const uint32_t sbase = smem_u32(smem);
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TM_COLS) : "memory");

@@ -379,6 +379,7 @@ khq_gqa_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
     // Everything above overlaps the kernel before; tensor memory is only taken once that kernel has finished (it may still have
     // to allocate its own on this SM).
     khq::pdl_wait();
+    khq::pdl_trigger();
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "n"(TM_COLS)
@@ -842,26 +843,13 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     }
     const int forced = g_tc5_items_per_cta > 0 ? g_tc5_items_per_cta : env_forced;
     const bool pairs = use_pair(nqb, items, H_q / H_kv, sm_count[dev]);
-    CUtensorMap mq, mk, mv, mg, mo;
-    int rc = make_map(&mq, q_gate, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 4, bf16);
-    if (rc == 0) rc = make_map(&mk, k, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? 64 : BC, pairs ? 4 : 2, bf16);
-    if (rc == 0) rc = make_map(&mv, v, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? BC : 64, pairs ? 2 : 4, bf16);
-    if (rc == 0) rc = make_map(&mg, static_cast<const __half*>(q_gate) + D, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 1, bf16);
-    if (rc == 0) rc = make_map(&mo, out, T, H_q, batch, (long long)H_q * D, D, out_batch_stride, BR, 1, bf16);
-    if (rc != 0) return rc;
-    const float sl2 = scale * 1.4426950408889634f;
-    if (pairs) {
-        err = khq::launch_pdl(bf16 ? pair::khq_gqa_prefill_pair_kernel<true> : pair::khq_gqa_prefill_pair_kernel<false>, (unsigned)items, 2u, (size_t)pair::SMEM,
-                              stream, (unsigned)NTHREADS, mq, mk, mv, mg, mo, T, H_q, H_kv, sl2);
-        return (err == cudaSuccess) ? 0 : static_cast<int>(err);
-    }
     // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
     // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
     // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
     // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
     // 24 row blocks (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99), and above 16 where a CTA has few
     // items to even out its share (1 x 2500: 89 against 92 us, 1 x 3000: 116 against 122, 4 x 3000: 473 against 550).
-    long long ctas;
+    long long ctas;  // without pairs
     int group_major = 0;
     if (forced == 1 || (forced == 0 && (nqb > 24 || (nqb > 16 && items <= 16LL * sm_count[dev])))) {
         ctas = items;
@@ -871,6 +859,23 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
         if (ctas < sm_count[dev]) ctas = items < sm_count[dev] ? items : sm_count[dev];
     } else {
         ctas = items < sm_count[dev] ? items : sm_count[dev];
+    }
+    CUtensorMap mq, mk, mv, mg, mo;
+    int rc = make_map(&mq, q_gate, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 4, bf16);
+    if (rc == 0) rc = make_map(&mk, k, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? 64 : BC, pairs ? 4 : 2, bf16);
+    if (rc == 0) rc = make_map(&mv, v, T, H_kv, batch, (long long)H_kv * D, D, kv_batch_stride, pairs ? BC : 64, pairs ? 2 : 4, bf16);
+    if (!pairs && ctas == items && T <= DIRECT_MAX_T) {  // gates and outputs go without maps, which take the host some time
+        mg = mo = mq;
+    } else {
+        if (rc == 0) rc = make_map(&mg, static_cast<const __half*>(q_gate) + D, T, H_q, batch, (long long)H_q * 2 * D, 2 * D, q_batch_stride, BR, 1, bf16);
+        if (rc == 0) rc = make_map(&mo, out, T, H_q, batch, (long long)H_q * D, D, out_batch_stride, BR, 1, bf16);
+    }
+    if (rc != 0) return rc;
+    const float sl2 = scale * 1.4426950408889634f;
+    if (pairs) {
+        err = khq::launch_pdl(bf16 ? pair::khq_gqa_prefill_pair_kernel<true> : pair::khq_gqa_prefill_pair_kernel<false>, (unsigned)items, 2u, (size_t)pair::SMEM,
+                              stream, (unsigned)NTHREADS, mq, mk, mv, mg, mo, T, H_q, H_kv, sl2);
+        return (err == cudaSuccess) ? 0 : static_cast<int>(err);
     }
     const unsigned grid = (unsigned)ctas;
     const __half* qp = static_cast<const __half*>(q_gate);  // 16-bit storage; the kernel converts per its type flag

@@ -185,10 +185,8 @@ struct StepQueryTables {  // constants of the model
     }
 };
 
-__device__ __forceinline__ void st_build_query(uint32_t (&qf)[4][8], uint32_t (&qr)[2], const __half* __restrict__ q,
-                                               const StepQueryTables& qt, int kvh, int part, int lane, float* scratch) {
+__device__ __forceinline__ void st_load_query(uint4 (&qraw)[2], uint32_t (&qr)[2], const __half* __restrict__ q, int kvh, int part, int lane) {
     const int g = lane >> 2, t = lane & 3;
-    uint4 qraw[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i)  // heads part and part + 4
         if (i == 0 || part < NREP - 4) qraw[i] = *reinterpret_cast<const uint4*>(q + (size_t)(kvh * NREP + part + 4 * i) * 2 * D + lane * 8);
@@ -197,6 +195,10 @@ __device__ __forceinline__ void st_build_query(uint32_t (&qf)[4][8], uint32_t (&
         qr[0] = g < NREP ? *reinterpret_cast<const uint32_t*>(qh) : 0u;
         qr[1] = g < NREP ? *reinterpret_cast<const uint32_t*>(qh + 32) : 0u;
     }
+}
+__device__ __forceinline__ void st_build_query(uint32_t (&qf)[4][8], const uint4 (&qraw)[2], const StepQueryTables& qt, int part, int lane,
+                                               float* scratch) {
+    const int g = lane >> 2, t = lane & 3;
     float dv[8];
     const __half* hd = reinterpret_cast<const __half*>(&qt.d);
     const __half* hr = reinterpret_cast<const __half*>(qt.rotor);
@@ -601,10 +603,12 @@ __device__ __forceinline__ void st_compressed(unsigned char* smem, const StepArg
         const int tok0 = (block0 + i) * M2_BT;
         st_stage(P, smem + (i & 1) * ST_STAGE, tok0, min(M2_BT, P.c_len - tok0), kvh, A.wide != 0, tid, sc);
     };
-    if (nblk > 0) stage(0, now);
     StepFragments f;
     uint32_t qr[2];
-    st_build_query(f.qf, qr, A.q, qt, kvh, part, lane, reinterpret_cast<float*>(smem + ST_SM_X));
+    uint4 qraw[2];
+    st_load_query(qraw, qr, A.q, kvh, part, lane);  // the longer chain first
+    if (nblk > 0) stage(0, now);
+    st_build_query(f.qf, qraw, qt, part, lane, reinterpret_cast<float*>(smem + ST_SM_X));
     StepState st;
     st.init();
 #pragma unroll 1

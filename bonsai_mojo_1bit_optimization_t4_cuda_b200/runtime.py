@@ -502,15 +502,15 @@ class KhqRuntime:
         T = int(k_roped_dev.shape[0])
         # the prompt length comes from the leading dimension: refuse tensors whose sizes do not agree
         # with it before any kernel is given their addresses
-        want = {"q_gate": T * H_q * 2 * d, "k_unroped": T * kv, "k_roped": T * kv, "v": T * kv, "out": T * H_q * d}
-        have = {"q_gate": q_gate_dev.numel(), "k_unroped": k_unroped_dev.numel(), "k_roped": k_roped_dev.numel(),
-                "v": v_dev.numel(), "out": out_dev.numel()}
-        if T <= 0 or any(have[k] != want[k] for k in want):
+        n_kv, n_out = T * kv, T * H_q * d
+        if (T <= 0 or q_gate_dev.numel() != 2 * n_out or k_unroped_dev.numel() != n_kv or k_roped_dev.numel() != n_kv or v_dev.numel() != n_kv
+                or out_dev.numel() != n_out):
+            want = {"q_gate": 2 * n_out, "k_unroped": n_kv, "k_roped": n_kv, "v": n_kv, "out": n_out}
+            have = {"q_gate": q_gate_dev.numel(), "k_unroped": k_unroped_dev.numel(), "k_roped": k_roped_dev.numel(),
+                    "v": v_dev.numel(), "out": out_dev.numel()}
             raise ValueError(f"khq_prefill: tensors do not hold T={T} rows of (H_q={H_q}, H_kv={H_kv}, d={d}): {have} vs {want}")
         # the per-token path compresses chunk c when write_pos reaches 128*(c+2), capped by `cap`
-        n_chunks = 0
-        while (n_chunks + 2) * KHQ_CHUNK <= T and (n_chunks + 1) * KHQ_CHUNK <= L.cap:
-            n_chunks += 1
+        n_chunks = max(0, min(T // KHQ_CHUNK - 1, L.cap // KHQ_CHUNK))
         if self._native_prefill(L, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, T, n_chunks, scale):
             self._prefill_done(layer_idx, L, T, n_chunks)
             return True
