@@ -675,7 +675,7 @@ def run_loop(args, rank, world, local_rank):
                        "l2": "working set under 1 MB per layer: L2-resident by nature"},
             "roofline": {"bound": "hbm", "achieved": b_alg / (us * 1e-6) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": b_alg / (us * 1e-6) / 1e9 / peak, "traffic": None, "algorithmic_bytes_per_step": b_alg},
-            "loop": r, "gpu_launches": 512 * r["layers"] * 2, "clocks": clocks}
+            "loop": r, "gpu_launches": (512 + 2 * r["events_per_layer"]) * r["layers"], "clocks": clocks}
     if not args.no_extras:
         try:
             line["cpu_baseline"] = cpu_loop_baseline(min(r["layers"], 1))
