@@ -12,7 +12,7 @@
 //   * A cluster's CTAs push each head's sums into the shared memory of the CTA that owns the head (bulk copies that count on
 //     the owner's barrier: 0.7 us; pulled by loads, 24 records took 9 us), which merges them and, for the compressed region,
 //     applies the inverse V transform.
-//   * The raw window is one more cluster per kv-head of the same grid, on mma.sync as well (a warp: 64 dims of Q K^T and of P V).
+//   * The raw window is one more cluster per kv-head of the same grid: Q K^T on mma.sync, weights and P V in fp32 (st_window has the reason).
 //   * No second kernel: the clusters' records go to global memory, and for each head the warp that arrives last (a counter per
 //     head) merges them, divides and gates.  No block ever waits for another cluster.
 // khq_step_wide_kernel is the same around the throughput kernel's CTA, for contexts where a 16-token block per CTA would take
@@ -655,18 +655,21 @@ __device__ __forceinline__ void st_compressed(unsigned char* smem, const StepArg
     }
 }
 
-// The CTA's share of the raw window: blocks of 16 tokens rank, rank + ctas, ...  The order of the 64 dims in a contraction is free, so
-// a thread takes 16 contiguous dims of K (and Q) and 8 of V with 16-byte loads.  val: dims 64 part + 8g .. + 7.
+// The CTA's share of the raw window: blocks of 16 tokens rank, rank + ctas, ...  Q K^T on mma.sync (fp16 rows as they are, exact products, fp32
+// sums; the order of the 64 dims in a contraction is free, so a thread takes 16 contiguous dims of K and Q with 16-byte loads).  The
+// weights and P V stay in fp32 on the CUDA cores, lane = 4 dims of 8 of the block's tokens: as a pair of fp16 operands a weight was held to 3e-8
+// of the largest one, and where one token with a small V row takes the attention the output is the sum of just those others (200
+// tokens, relative error of the output where the others' weights are 2e-4 together: 4.2e-3, 1.7e-6: 0.27; so 2.1e-4 for both, the
+// output's own rounding; 16 layers of 384 + 128 tokens 185.5 us with the operands in fp16, 183.3 so).  out: dims 64 part + 4 (lane & 15) .. + 3
+// of heads 3 (lane >> 4) .. + 2.
+constexpr int ST_WIN_P = (M2_BT + 1) * 8;  // floats per warp: the block's weights, token by token, and the factors of the sums so far
+static_assert(ST_PARTS * ST_WIN_P * 4 <= ST_SM_X, "the window's weights take the stages' place");
 __device__ __forceinline__ void st_window(unsigned char* smem, const StepArgs& A, int rank, int ctas, int kvh, int part, int lane,
-                                          float (&val)[2][8], float (&m)[2], float (&l)[2]) {
-    const int g = lane >> 2, t = lane & 3;
+                                          float (&out)[3][4], float (&m)[2], float (&l)[2]) {
+    const int g = lane >> 2, t = lane & 3, half = lane >> 4;
     float4* xs = reinterpret_cast<float4*>(smem + ST_SM_X);
+    float* wp = reinterpret_cast<float*>(smem) + part * ST_WIN_P;
     const int blocks = (A.win_len + M2_BT - 1) / M2_BT, new_s = A.new_k != nullptr ? A.win_len - 1 : -1;
-    const auto row = [&](const __half* ring, const __half* fresh, int s) {
-        s = min(s, A.win_len - 1);  // past the end: a row that is there, weight 0
-        const __half* base = s == new_s ? fresh : ring + (size_t)((A.win_start + s) % A.ring_cap) * HKV * D;
-        return reinterpret_cast<const uint4*>(base + kvh * D);
-    };
     uint4 qv[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
     if (g < NREP) {
         const uint4* qp = reinterpret_cast<const uint4*>(A.q + (size_t)(kvh * NREP + g) * 2 * D + 64 * part + 16 * t);
@@ -675,18 +678,31 @@ __device__ __forceinline__ void st_window(unsigned char* smem, const StepArgs& A
     }
     StepState st;
     st.init();
+    float o[NREP][4];
+#pragma unroll
+    for (int h = 0; h < NREP; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[h][j] = 0.0f;
     int turn = 0;
 #pragma unroll 1
     for (int b = rank; b < blocks; b += ctas, turn ^= 1) {
-        uint4 kv[2][2], vv[4];
+        const int slot0 = (A.win_start + M2_BT * b) % A.ring_cap, last = A.win_len - 1 - M2_BT * b;
+        const auto row = [&](const __half* ring, const __half* fresh, int i) {
+            i = min(i, last);  // past the end: a row that is there, weight 0
+            int slot = slot0 + i;
+            if (slot >= A.ring_cap) slot = A.ring_cap >= M2_BT ? slot - A.ring_cap : slot % A.ring_cap;
+            return (M2_BT * b + i == new_s ? fresh : ring + (size_t)slot * HKV * D) + kvh * D + 64 * part;
+        };
+        uint4 kv[2][2];
+        uint2 vv[8];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-            const uint4* kp = row(A.ring_k, A.new_k, M2_BT * b + g + 8 * x) + (64 * part + 16 * t) / 8;
+            const uint4* kp = reinterpret_cast<const uint4*>(row(A.ring_k, A.new_k, g + 8 * x) + 16 * t);
             kv[x][0] = kp[0];
             kv[x][1] = kp[1];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) vv[i] = row(A.ring_v, A.new_v, M2_BT * b + 2 * t + (i & 1) + 8 * (i >> 1))[(64 * part + 8 * g) / 8];
+        for (int i = 0; i < 8; ++i) vv[i] = *reinterpret_cast<const uint2*>(row(A.ring_v, A.new_v, 8 * half + i) + 4 * (lane & 15));
         float s4[4];
         const uint32_t *k0 = reinterpret_cast<const uint32_t*>(kv[0]), *k1 = reinterpret_cast<const uint32_t*>(kv[1]);
         const uint32_t* qw = reinterpret_cast<const uint32_t*>(qv);
@@ -706,39 +722,57 @@ __device__ __forceinline__ void st_window(unsigned char* smem, const StepArgs& A
         bool valid[2];
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
-            valid[y] = M2_BT * b + g + 8 * y < A.win_len;
+            valid[y] = g + 8 * y <= last;
 #pragma unroll
             for (int e = 0; e < 2; ++e) sc[y][e] = valid[y] ? A.scale * tot[2 * y + e] : -1e30f;
         }
-        st_weights<4>(st, sc, valid, 0.0f, pw);
-        uint32_t pb[2], pl_[2];
+        const float before[2] = {st.m[0], st.m[1]};
+        st_weights<0>(st, sc, valid, 0.0f, pw);
+        if (t < 3) {
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-            uint32_t hi, lo;
-            m2_pack_hilo(pw[y][0], pw[y][1], hi, lo);
-            pb[y] = m2_movmatrix_t(hi);
-            pl_[y] = m2_movmatrix_t(lo);
+            for (int y = 0; y < 2; ++y) *reinterpret_cast<float2*>(wp + (g + 8 * y) * 8 + 2 * t) = make_float2(pw[y][0], pw[y][1]);
+            if (g == 0) *reinterpret_cast<float2*>(wp + M2_BT * 8 + 2 * t) = make_float2(__expf(before[0] - st.m[0]), __expf(before[1] - st.m[1]));
+        }
+        __syncwarp();
+        const auto weights = [&](int i, float (&w)[NREP]) {
+            const float4 a = *reinterpret_cast<const float4*>(wp + i * 8);
+            const float2 c = *reinterpret_cast<const float2*>(wp + i * 8 + 4);
+            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y;
+        };
+        float w[NREP];
+        if (b != rank) {
+            weights(M2_BT, w);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
+                m2_mul2(o[h][0], o[h][1], o[h][0], o[h][1], w[h], w[h]);
+                m2_mul2(o[h][2], o[h][3], o[h][2], o[h][3], w[h], w[h]);
+            }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {  // rows g and g + 8 of tile j: dims 64 part + 8g + 2j, + 1
-            const uint32_t w0 = reinterpret_cast<const uint32_t*>(&vv[0])[j], w1 = reinterpret_cast<const uint32_t*>(&vv[1])[j];
-            const uint32_t w2 = reinterpret_cast<const uint32_t*>(&vv[2])[j], w3 = reinterpret_cast<const uint32_t*>(&vv[3])[j];
-            const uint32_t a[4] = {__byte_perm(w0, w1, 0x5410), __byte_perm(w0, w1, 0x7632), __byte_perm(w2, w3, 0x5410), __byte_perm(w2, w3, 0x7632)};
-            m2_mma(st.o[j], a, pb[0], pb[1]);
-            m2_mma_lo(st.o[j], a, pl_[0], pl_[1]);
+        for (int i = 0; i < 8; ++i) {
+            weights(8 * half + i, w);
+            const float2 va = __half22float2(*reinterpret_cast<const __half2*>(&vv[i].x)), vb = __half22float2(*reinterpret_cast<const __half2*>(&vv[i].y));
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
+                m2_fma2(o[h][0], o[h][1], va.x, va.y, w[h], w[h], o[h][0], o[h][1]);
+                m2_fma2(o[h][2], o[h][3], vb.x, vb.y, w[h], w[h], o[h][2], o[h][3]);
+            }
         }
     }
+    // both halves of the tokens: three heads each
+#pragma unroll
+    for (int h = 0; h < 3; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float other = __shfl_xor_sync(0xFFFFFFFFu, half ? o[h][j] : o[h + 3][j], 16);
+            out[h][j] = (half ? o[h + 3][j] : o[h][j]) + other;
+        }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
 #pragma unroll
         for (int y = 4; y <= 16; y <<= 1) st.l[e] += __shfl_xor_sync(0xFFFFFFFFu, st.l[e], y);
         m[e] = st.m[e];
         l[e] = st.l[e];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            val[e][2 * j] = st.o[j][e];
-            val[e][2 * j + 1] = st.o[j][2 + e];
-        }
     }
 }
 
@@ -859,7 +893,7 @@ __global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_co
     const int block0 = BATCH ? A.block0 + rank * A.blocks_per_cta : (rec * ST_CLUSTER + rank) * A.blocks_per_cta;
     const int nblk = comp ? min(max((A.kv.c_len + M2_BT - 1) / M2_BT - block0, 0), A.blocks_per_cta) : 0;
     if (BATCH && nblk > 0) st_rope_seed(rope, A.kv, reinterpret_cast<const float*>(smem + ST_SM_SMALL), part, lane, block0 * M2_BT);
-    float val[2][8], m[2], l[2];
+    float val[2][8], win[3][4], m[2], l[2];
     if (comp) {
         st_compressed(smem, A, block0, nblk, qt, rope, tid, kvh, part, lane, val, m, l);
     } else {
@@ -869,23 +903,30 @@ __global__ void __launch_bounds__(ST_THREADS, 4) khq_step_kernel(const __grid_co
             __half* dst = rank == 0 ? A.ring_k : rank == 1 ? A.ring_v : A.ring_u;
             if (tid < D / 8 && src != nullptr && dst != nullptr) reinterpret_cast<uint4*>(dst + at)[tid] = reinterpret_cast<const uint4*>(src + kvh * D)[tid];
         }
-        st_window(smem, A, rank, ST_CLUSTER, kvh, part, lane, val, m, l);
+        st_window(smem, A, rank, ST_CLUSTER, kvh, part, lane, win, m, l);
     }
     // ---- each head's sums to the CTA that owns it ------------------------------------------------
     const int g = lane >> 2, t = lane & 3;
     float* send = reinterpret_cast<float*>(smem + ST_SM_SEND);
     __syncthreads();  // the records alias what the last block was read from
-    if (t < 3) {
-        const int d0 = comp ? 32 * g + 8 * part : 64 * part + 8 * g;
+    if (comp) {
+        const int d0 = 32 * g + 8 * part;
+        if (t < 3)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float* r = send + (2 * t + e) * ST_RECV;
-            float4* to = reinterpret_cast<float4*>(r + d0 + 4 * (d0 >> 5));
-            to[0] = make_float4(val[e][0], val[e][1], val[e][2], val[e][3]);
-            to[1] = make_float4(val[e][4], val[e][5], val[e][6], val[e][7]);
-            if (g == 0 && part == 0) *reinterpret_cast<float2*>(r + ST_REC) = make_float2(m[e], l[e]);
-        }
+            for (int e = 0; e < 2; ++e) {
+                float4* to = reinterpret_cast<float4*>(send + (2 * t + e) * ST_RECV + d0 + 4 * (d0 >> 5));
+                to[0] = make_float4(val[e][0], val[e][1], val[e][2], val[e][3]);
+                to[1] = make_float4(val[e][4], val[e][5], val[e][6], val[e][7]);
+            }
+    } else {
+        const int d0 = 64 * part + 4 * (lane & 15);
+#pragma unroll
+        for (int h = 0; h < 3; ++h)
+            *reinterpret_cast<float4*>(send + (3 * (lane >> 4) + h) * ST_RECV + d0 + 4 * (d0 >> 5)) = make_float4(win[h][0], win[h][1], win[h][2], win[h][3]);
     }
+    if (t < 3 && g == 0 && part == 0)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) *reinterpret_cast<float2*>(send + (2 * t + e) * ST_RECV + ST_REC) = make_float2(m[e], l[e]);
     fence_proxy_async();
     __syncthreads();
     if (tid < NREP) st_push(st_map(recv + rank * ST_RECV, tid), send + tid * ST_RECV, ST_RECV * 4, st_map(bar, tid));

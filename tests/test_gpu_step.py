@@ -123,3 +123,36 @@ def test_refused(cuda_ops, state):
     ctypes.memmove(ctypes.addressof(bare), ctx[1], ctypes.sizeof(bare))
     bare.prepared = None
     assert f(ctypes.addressof(bare), c, q, 0, 0, 0, out, 128, 10, 0, SCALE, stream) == -100
+
+
+@pytest.mark.parametrize("v_scale,gap", [(1.0, 0.0), (200.0, 14.3), (2000.0, 19.1), (30000.0, 24.0)])
+@pytest.mark.parametrize("win_len", [17, 200, 256])
+def test_window_with_one_dominant_token(cuda_ops, state, win_len, v_scale, gap):
+    """The raw window against 64 bits, its first token with all but e^-gap of each other token's weight and V = 0, as the first token of a
+    conversation has it: the output is the others' sum, so their small weights have to be as exact as large ones."""
+    import torch
+
+    L, ctx = state["plain"]
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    q, k, v = rnd(HQ, 2 * D), rnd(win_len, HKV, D), v_scale * rnd(win_len, HKV, D).clamp(-2.0, 2.0)
+    q[:, D:] = 20.0  # open gates
+    q[:, 255], k[:, :, 255] = 16.0, 0.0
+    if gap:
+        k[0], v[0] = 0.0, 0.0
+        k[0, :, 255] = gap
+    q, k, v = q.half(), k.half(), v.half()
+    for ring, rows in (("ring_k", k), ("ring_v", v)):
+        L.t[ring].view(RING, HKV, D)[:win_len] = rows
+    out = torch.empty(HQ * D, dtype=torch.float16, device="cuda")
+    cuda_ops.layer_step(ctx, q.reshape(-1), k[-1].reshape(-1), v[-1].reshape(-1), None, out, 0, win_len, False, 1, SCALE)
+    qd, kd, vd = q[:, :D].double().view(HKV, 6, D), k.double(), v.double()
+    w = torch.softmax(SCALE * torch.einsum("jhd,sjd->jhs", qd, kd), dim=-1)
+    gate = torch.sigmoid(q[:, D:].double())
+    want = torch.einsum("jhs,sjd->jhd", w, vd).reshape(HQ, D) * gate
+    terms = torch.einsum("jhs,sjd->jhd", w, vd.abs()).reshape(HQ, D) * gate
+    err = (out.view(HQ, D).double() - want).abs()
+    # the output's own rounding, and scores of up to 32 (4e-6) and their exponentials in fp32
+    assert cuda_ops.lib.khq_b200_device_status() == 0
+    assert bool((err <= 2.0 ** -11 * want.abs() + 2.0 ** -25 + 1e-5 * terms).all()), (float((err / terms).max()), float(err.norm() / want.norm()))
+    print(f"win {win_len} gap {gap}: {float(err.norm() / want.norm()):.2e}")
