@@ -793,6 +793,7 @@ __device__ __forceinline__ void st_finish_head(const StepArgs& A, int h, int rec
             order = atomicAdd(A.counters + h, 1);
             __threadfence();
         }
+        __syncwarp();  // the other lanes read the records behind lane 0's fence (a shuffle orders no memory)
         if (__shfl_sync(0xFFFFFFFFu, order, 0) != n - 1) return;
         if (lane == 0) A.counters[h] = 0;
         constexpr int AHEAD = 6;  // records whose sums are on their way beside the maxima

@@ -156,3 +156,18 @@ def test_window_with_one_dominant_token(cuda_ops, state, win_len, v_scale, gap):
     assert cuda_ops.lib.khq_b200_device_status() == 0
     assert bool((err <= 2.0 ** -11 * want.abs() + 2.0 ** -25 + 1e-5 * terms).all()), (float((err / terms).max()), float(err.norm() / want.norm()))
     print(f"win {win_len} gap {gap}: {float(err.norm() / want.norm()):.2e}")
+
+
+@pytest.mark.parametrize("c_len", [1792, 1793, 16999])
+def test_the_last_warp_merges_every_record(cuda_ops, state, c_len):
+    """A head's records are merged in their own order by whichever warp arrives last: the same bits in each of many steps back to back
+    (15 records of khq_step_kernel, 9 and 31 of khq_step_wide_kernel), and the counters are left at zero."""
+    import torch
+
+    L, ctx = state["plain"]
+    k, v, u = state["new"]
+    outs = torch.empty(400, HQ * D, dtype=torch.float16, device="cuda")
+    for o in outs:
+        cuda_ops.layer_step(ctx, state["q"], k, v, u, o, c_len, 130, False, 1, SCALE)
+    assert bool((outs == outs[0]).all()) and int(ctx[3].abs().sum()) == 0
+    assert cuda_ops.lib.khq_b200_device_status() == 0
