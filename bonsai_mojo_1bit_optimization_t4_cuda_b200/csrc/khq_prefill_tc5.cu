@@ -795,9 +795,10 @@ namespace {
 // the epilogue of one item runs beside the tiles of others (T = 1531: one prompt 41.5 us against 39.1, two 85.0 against 85.8, nine
 // 355 against 373; one of 2000: 58 against 62; 8 x 2048: 492 against 533; 4 x 8192 in a row, both at the power limit: 2.45 to 2.84 ms
 // against 2.65 to 2.97).
-bool use_pair(int row_blocks, long long items, int n_rep, int sms) {
+// A work distribution of the single-CTA kernel that was asked for (`forced`) asks for that kernel; only khq_b200_prefill_pairs(1) is stronger.
+bool use_pair(int row_blocks, long long items, int n_rep, int sms, int forced) {
     if (n_rep % 2 != 0 || g_tc5_pairs == 2) return false;
-    return g_tc5_pairs == 1 || (row_blocks > 8 && 4 * items > 9LL * sms);
+    return g_tc5_pairs == 1 || (forced == 0 && row_blocks > 8 && 4 * items > 9LL * sms);
 }
 
 int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int batch, int T, int H_q, int H_kv, int d,
@@ -833,7 +834,7 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     }
     const int nqb = (T + BR - 1) / BR;
     const long long items = (long long)nqb * H_q * batch;
-    // khq_b200_prefill_tc5_items_per_cta(n) or KHQ_PREFILL_ITEMS_PER_CTA (read once) force a mode of the kernel without pairs, for prompts that pairs do not take:
+    // khq_b200_prefill_tc5_items_per_cta(n) or KHQ_PREFILL_ITEMS_PER_CTA (read once) ask for the kernel without pairs and its mode:
     // 1 = one item per CTA, larger = that many items per CTA (the setter wins; 0 = automatic).
     static int env_forced = -1;
     if (env_forced < 0) {
@@ -842,7 +843,7 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
         if (env_forced < 0) env_forced = 0;
     }
     const int forced = g_tc5_items_per_cta > 0 ? g_tc5_items_per_cta : env_forced;
-    const bool pairs = use_pair(nqb, items, H_q / H_kv, sm_count[dev]);
+    const bool pairs = use_pair(nqb, items, H_q / H_kv, sm_count[dev], forced);
     // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
     // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
     // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the

@@ -395,12 +395,12 @@ int launch_khq_gqa_prefill_bf16(const void* q_gate, const void* k, const void* v
                                 int H_q, int H_kv, int d, float scale, long long q_batch_stride,
                                 long long kv_batch_stride, long long out_batch_stride, khq_stream_t stream);
 int khq_b200_prefill_select(int which);
-/* Work distribution of the _tc5_ kernel, for prompts that CTA pairs do not take (below): 0 = by prompt length (persistent CTAs up to 24 row blocks of
- * 128 rows, one CTA per 128-row item beyond), 1 = one item per CTA, n > 1 = n items per CTA (a large
+/* Work distribution of the _tc5_ kernel: 0 = by the prompts' sizes, CTA pairs among the choices (default); any other value asks for one CTA
+ * per 128-row item at a time, whatever the sizes: 1 = one item per CTA, n > 1 = n items per CTA (a large
  * n gives one persistent CTA per SM).  Returns -100 for a negative n. */
 int khq_b200_prefill_tc5_items_per_cta(int n);
-/* CTA pairs that take neighbouring query heads together: 0 = by the prompts' sizes (default), 1 = wherever H_q / H_kv is even,
- * 2 = never. */
+/* CTA pairs that take neighbouring query heads together: 0 = by the prompts' sizes unless a work distribution is asked for (default),
+ * 1 = wherever H_q / H_kv is even, 2 = never. */
 int khq_b200_prefill_pairs(int mode);
 int khq_b200_prefill_status(void);
 

@@ -8,7 +8,7 @@ from cases import D, H_KV, H_Q, SCALE
 pytestmark = pytest.mark.gpu
 
 
-# tcgen05 / tensor-memory kernel (the default; also forced into each of its two work distributions)
+# tcgen05 / tensor-memory kernel (the default; also forced into each of its two work distributions, and onto CTA pairs)
 # and the warp-level mma.sync kernel
 KERNELS = ["tc5", "mma", "tc5-one-item-per-cta", "tc5-persistent", "tc5-pairs"]
 
@@ -19,7 +19,7 @@ def _run(cuda_ops, qg, k, v, B, T, H_q=H_Q, H_kv=H_KV, kernel="tc5"):
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     out = torch.full((B, T, H_q, D), float("nan"), dtype=torch.float16, device="cuda")
     assert cuda_ops.lib.khq_b200_prefill_select(1 if kernel == "mma" else 0) == 0
-    assert cuda_ops.lib.khq_b200_prefill_pairs(1 if kernel == "tc5-pairs" else 0) == 0
+    assert cuda_ops.lib.khq_b200_prefill_pairs({"tc5-pairs": 1, "tc5-single": 2}.get(kernel, 0)) == 0
     assert cuda_ops.lib.khq_b200_prefill_tc5_items_per_cta({"tc5-one-item-per-cta": 1, "tc5-persistent": 1 << 20}.get(kernel, 0)) == 0
     try:
         cuda_ops.gqa_prefill(dev(qg), dev(k), dev(v), out, B, T, H_q, H_kv, D, SCALE)
@@ -186,12 +186,15 @@ def test_prefill_honours_batch_strides(cuda_ops, oracle, entry):
 
 @pytest.mark.parametrize("B,T", [(1, 2048), (1, 2049), (1, 3073)])
 def test_prefill_either_side_of_the_grid_rule(cuda_ops, B, T):
-    """The automatic choice between a persistent grid and one CTA per item does not show in the results."""
+    """The single-CTA kernel's automatic choice between a persistent grid and one CTA per item does not show in the results; nor do
+    pairs, the default at these sizes, take a prompt from a work distribution that was asked for."""
     rng = np.random.default_rng(T)
     qg = rng.standard_normal((B, T, H_Q, 2 * D)).astype(np.float16)
     k, v = (rng.standard_normal((B, T, H_KV, D)) * 0.25).astype(np.float16), rng.standard_normal((B, T, H_KV, D)).astype(np.float16)
-    auto, one, many = (_run(cuda_ops, qg, k, v, B, T, kernel=m) for m in ("tc5", "tc5-one-item-per-cta", "tc5-persistent"))
-    assert np.array_equal(auto, one) and np.array_equal(auto, many)
+    single, one, many, auto, pairs = (_run(cuda_ops, qg, k, v, B, T, kernel=m)
+                                      for m in ("tc5-single", "tc5-one-item-per-cta", "tc5-persistent", "tc5", "tc5-pairs"))
+    assert np.array_equal(single, one) and np.array_equal(single, many)
+    assert np.array_equal(auto, pairs) and not np.array_equal(auto, single)  # the kernels add up in another order
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
