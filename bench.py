@@ -562,7 +562,7 @@ class _RefKernelOps:
 
 def loop_measure(args, dev, n_layers, with_reference_kernels=True):
     """Configuration 1 of the benchmark specification, the loop the reference's own measurement runs (README.md:27-47): a
-    56-token prompt + 512 decode steps over `n_layers` attention layers, 8 splits, compression events
+    56-token prompt + 512 decode steps over `n_layers` attention layers, compression events
     at tokens 256, 384 and 512 on every layer, all inside the timed region.  This library: the prompt
     through khq_prefill (one prefill launch + appends), the decode steps through khq_step_fused.  The
     like-for-like leg drives the reference's kernels (recompiled for sm_100a) through the same state
@@ -628,7 +628,7 @@ def loop_measure(args, dev, n_layers, with_reference_kernels=True):
     ours_ops = CudaOps()
     run(ours_ops, True)  # warm-up pass (kernel attributes, caches, allocator)
     ms_prompt, ms_decode, o_ours = run(ours_ops, True)
-    res = {"layers": n_layers, "prompt_tokens": prompt, "decode_steps": decode, "splits": 8, "events_per_layer": 3,
+    res = {"layers": n_layers, "prompt_tokens": prompt, "decode_steps": decode, "splits": "the step's own rule; 8 in the reference-kernel leg", "events_per_layer": 3,
            "ours": {"prompt_ms": ms_prompt, "decode_ms": ms_decode,
                     "us_per_layer_step": 1e3 * ms_decode / (decode * n_layers),
                     "tok_s": decode / (ms_decode * 1e-3), "path": "khq_prefill (tcgen05 prefill + appends) then khq_step_fused"},
@@ -670,8 +670,9 @@ def run_loop(args, rank, world, local_rank):
     line = {"metric": "KHQ decode loop latency (56-token prompt + 512 steps)", "value": us, "unit": "us/layer-step", "n_gpus": world,
             "steps": 512, "warmup": 1, "ms_per_step": us * r["layers"] / 1e3, "higher_is_better": False, "scaling": "replicas only",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-            "config": {"workload": "BASELINE configs[1]: %d attention layers, batch 1, 56-token prompt + 512 decode steps, splits 8, "
+            "config": {"workload": "BASELINE configs[1]: %d attention layers, batch 1, 56-token prompt + 512 decode steps, "
                                    "compression events at tokens 256/384/512 inside the timed region" % r["layers"],
+                       "splits": r["splits"],
                        "l2": "working set under 1 MB per layer: L2-resident by nature"},
             "roofline": {"bound": "hbm", "achieved": b_alg / (us * 1e-6) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": b_alg / (us * 1e-6) / 1e9 / peak, "traffic": None, "algorithmic_bytes_per_step": b_alg},

@@ -98,7 +98,7 @@ class CudaOps:
             int(num_splits), float(scale), float(alpha_k), float(alpha_v), float(rope_base), current_stream())
         check("launch_khq_decode_step_fp16", rc)
 
-    # -- launch_khq_layer_step: one layer's step from a context that keeps its addresses -------------
+    # -- launch_khq_layer_token: one layer's step from a context that keeps its addresses ------------
     def layer_ctx(self, L, ring_cap, rope_base):
         """The context of a ``runtime.KhqLayer``; it holds raw addresses of the tensors in ``L.t``."""
         c = _lib.LayerCtx()
@@ -125,7 +125,7 @@ class CudaOps:
         return c, ctypes.addressof(c), image, counters, counters.data_ptr(), scratch
 
     def layer_step(self, ctx, q_gate, k_roped, v_new, k_unroped, out, c_len, win_len, compress, num_splits, scale):
-        """``num_splits`` is not used: the launch cuts the compressed region by its own rule."""
+        """``num_splits`` is not used: the launch cuts the compressed region by its length."""
         rc = self.lib.launch_khq_layer_token(ctx[1], ctx[4], ptr(q_gate), ptr(k_roped), ptr(v_new), ptr(k_unroped), ptr(out), c_len, win_len,
                                              compress, scale, current_stream())
         if rc != 0:

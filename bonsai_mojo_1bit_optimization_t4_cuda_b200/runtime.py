@@ -252,6 +252,8 @@ class KhqRuntime:
 
     # ------------------------------------------------------------------ split policy
     def _khq_split_count(self, c_len: int) -> int:
+        """Splits of the compressed region in the call-by-call sequence (``splits``, BONSAI_KHQ_SPLITS).  The native step has no such
+        number: its launch cuts the region into blocks by the length."""
         if self.splits <= 1 or c_len <= 0:
             return 1
         eff = max(c_len // KHQ_MIN_TOKENS_PER_SPLIT, 1)
@@ -351,8 +353,7 @@ class KhqRuntime:
         c_len = L.boundary
         event = window >= KHQ_WATERMARK and c_len + KHQ_CHUNK <= L.cap
         c_after = c_len + KHQ_CHUNK if event else c_len
-        self.ops.layer_step(ctx, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, c_len, window, event,
-                            self._khq_split_count(c_after), scale)
+        self.ops.layer_step(ctx, q_gate_dev, k_roped_dev, v_dev, k_unroped_dev, out_dev, c_len, window, event, 0, scale)
         L.write_pos += 1
         if event:
             L.boundary = c_after
@@ -460,9 +461,9 @@ class KhqRuntime:
 
     # ------------------------------------------------------------------ fused step (addition)
     def khq_step_fused(self, layer_idx: int, q_gate_dev, k_unroped_dev, k_roped_dev, v_dev, out_dev, scale: float) -> bool:
-        """``khq_capture_unroped`` + ``khq_step`` of one token through ``launch_khq_layer_step``:
+        """``khq_capture_unroped`` + ``khq_step`` of one token through ``launch_khq_layer_token``:
         the compression event if it is due, the three ring appends, both attention regions, the merge and
-        the gate in one host call and two launches (four with an event) instead of seven.  A step whose window
+        the gate in one host call and one launch (three with an event) instead of seven.  A step whose window
         would exceed the ring takes the classic sequence (compressed capacity exhausted: the reference keeps
         stepping with window > 256, ``README.md:259``, and so does ``khq_step``), and so does one whose rows are
         not contiguous fp16 on 16 bytes.  The state afterwards

@@ -95,3 +95,17 @@ def test_wrong_size_and_unaligned_output(fused):
     off = next(i for i in range(1, 8) if out[i:].data_ptr() % 16)
     assert step(plain, out[off:off + H_Q * D])
     assert not [c for c in rt.ops.calls if c[0] == "native"] and rt.ops.calls[-1] == ("merge", True, False)
+
+
+@pytest.mark.parametrize("splits", [1, 8])
+def test_native_step_has_no_split_count(monkeypatch, splits):
+    """The native launch cuts the compressed region itself: the same call whatever `splits` is, and nothing computed for it."""
+    rt = _runtime()
+    rt.splits = splits
+    monkeypatch.setattr(rt, "_khq_split_count", lambda c_len: pytest.fail("not used by the native step"))
+    seen = []
+    monkeypatch.setattr(rt.ops, "layer_step", lambda *args: seen.append(args[6:]))
+    q, out = torch.zeros(H_Q * 2 * D, dtype=torch.float16), torch.zeros(H_Q * D, dtype=torch.float16)
+    rt.layers[3].write_pos, rt.layers[3].boundary = 300, 128
+    assert rt.khq_step_fused(3, q, _rows("plain"), _rows("plain"), _rows("plain"), out, SCALE)
+    assert seen == [(128, 173, False, 0, SCALE)]
