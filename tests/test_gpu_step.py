@@ -171,3 +171,33 @@ def test_the_last_warp_merges_every_record(cuda_ops, state, c_len):
         cuda_ops.layer_step(ctx, state["q"], k, v, u, o, c_len, 130, False, 1, SCALE)
     assert bool((outs == outs[0]).all()) and int(ctx[3].abs().sum()) == 0
     assert cuda_ops.lib.khq_b200_device_status() == 0
+
+
+@pytest.mark.parametrize("c_len,splits", [(0, 1), (1, 1), (129, 8), (385, 32), (1793, 16), (5377, 33)])
+def test_two_kernel_step_matches_the_separate_launches(cuda_ops, state, c_len, splits):
+    """launch_khq_layer_step, the step as an attention launch and a tail (up to 32 splits: the tail merges their records)."""
+    import torch
+
+    L, ctx = state["plain"]
+    k, v, u = state["new"]
+    q, out = state["q"], torch.empty(HQ * D, dtype=torch.float16, device="cuda")
+    c = type(ctx[0])()
+    ctypes.memmove(ctypes.addressof(c), ctx[1], ctypes.sizeof(c))
+    partial = torch.empty(HQ * splits * 258, dtype=torch.float32, device="cuda")
+    c.attn_partial = partial.data_ptr()
+    f = cuda_ops.lib.launch_khq_layer_step
+    stream = torch.cuda.current_stream().cuda_stream
+    for win_len in (17, 256):
+        rows = [t.data_ptr() for t in (k, v, u)]
+        assert f(ctypes.addressof(c), q.data_ptr(), *rows, out.data_ptr(), c_len, win_len, 0, splits, SCALE, stream) == 0
+        slot = (c_len + win_len - 1) % RING
+        assert all(torch.equal(L.t[n].view(RING, -1)[slot], x) for n, x in (("ring_k", k), ("ring_v", v), ("ring_u", u)))
+        want = _separate(cuda_ops, L, q, c_len, win_len).float()
+        again = torch.empty_like(out)  # the token is in the rings now
+        assert f(ctypes.addressof(c), q.data_ptr(), 0, 0, 0, again.data_ptr(), c_len, win_len, 0, splits, SCALE, stream) == 0
+        torch.cuda.synchronize()
+        assert cuda_ops.lib.khq_b200_device_status() == 0 and torch.equal(out, again)
+        err = (out.float() - want).abs()  # as above
+        assert bool((err <= 2.0 ** -10 * want.abs() + 3e-4 * want.abs().max()).all()), (c_len, win_len, float(err.max()), float(want.abs().max()))
+    assert f(ctypes.addressof(c), q.data_ptr(), 0, 0, 0, out.data_ptr(), c_len, 257, 0, splits, SCALE, stream) == -103
+    assert f(ctypes.addressof(c), q.data_ptr(), rows[0], 0, 0, out.data_ptr(), c_len, 17, 0, splits, SCALE, stream) == -100
