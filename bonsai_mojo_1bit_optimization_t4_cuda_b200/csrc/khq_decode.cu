@@ -1690,8 +1690,7 @@ extern "C" int khq_b200_plan_decode(const int* c_len, const int* win_len, int n_
     return n;  // > max_items means the items buffer was too small
 }
 
-// The item counter of a persistent launch.  A kernel, because a memset between two kernels keeps the launch of the second one from
-// overlapping the end of the first.
+// The counters of a batch's step kernels at the end of its workspace: one per problem and head.
 static size_t step_counter_bytes(int n_desc) { return ((size_t)n_desc * HQ * sizeof(int) + 255) / 256 * 256; }
 
 // A small batch as clusters of the step kernels (khq_step.cuh), mirrored in include/khq_b200.h: where every CTA has one block
@@ -1706,11 +1705,8 @@ extern "C" int khq_b200_plan_steps(const int* c_len, const int* win_len, int n_d
                                    int* n_slots) {
     if (!c_len || !win_len || n_desc <= 0 || !items || !n_items || !first_slot || !n_slots) return -100;
     const int most = plan_sm_count() / 8 - 3;  // clusters of eight CTAs that run side by side; as many sets of four clusters of khq_step_kernel
-    int total = 0;
-    for (int i = 0; i < n_desc; ++i) {
+    for (int i = 0; i < n_desc; ++i)
         if (c_len[i] < 0 || win_len[i] <= 0) return 0;
-        total += (c_len[i] + M2_BT - 1) / M2_BT;
-    }
     int mode = 0, per = 0;
     const auto clusters = [&](int p) {
         int n = 0;
@@ -1737,6 +1733,8 @@ extern "C" int khq_b200_plan_steps(const int* c_len, const int* win_len, int n_d
     return mode;
 }
 
+// The item counter of a persistent launch.  A kernel, because a memset between two kernels keeps the launch of the second one from
+// overlapping the end of the first.
 __global__ void khq_zero_counter_kernel(int* counter) {
     pdl_trigger();
     pdl_wait();

@@ -844,12 +844,13 @@ int launch_tc5(const void* q_gate, const void* k, const void* v, void* out, int 
     }
     const int forced = g_tc5_items_per_cta > 0 ? g_tc5_items_per_cta : env_forced;
     const bool pairs = use_pair(nqb, items, H_q / H_kv, sm_count[dev], forced);
-    // Short prompts: a persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with
-    // the next one's first tiles (32 x 300: 170 us against 215; 4 x 1000: 96 against 109; 8 x 2048: 490 against 568).  Longer
-    // ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of the
-    // triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
-    // 24 row blocks (4 x 4096: 0.78 ms against 0.81; 4 x 8192: 2.72 against 2.99), and above 16 where a CTA has few
-    // items to even out its share (1 x 2500: 89 against 92 us, 1 x 3000: 116 against 122, 4 x 3000: 473 against 550).
+    // The kernel without pairs, for what those leave (short prompts, few items, odd numbers of query heads per kv head).  Short prompts: a
+    // persistent grid of one CTA per SM, each working through its items and overlapping one item's epilogue with the next one's first
+    // tiles.  Longer ones: one CTA per item, one (batch, kv head) group after the other, heaviest first, which leaves the balancing of
+    // the triangular workload to the hardware's dynamic CTA scheduler and runs the leaner instantiation of the kernel.  It wins above
+    // 24 row blocks, and above 16 where a CTA has few items to even out its share.  Persistent / one per item, us, 20 query heads on
+    // 4 kv heads: 32 x 300: 130 / 168; 4 x 1000: 74 / 82; 8 x 2048: 406 / 408; 2 x 2300: 132 / 136; 1 x 2500: 83 / 77; 1 x 3000:
+    // 105 / 97; 4 x 3000: 435 / 411; 1 x 4000: 185 / 170; 4 x 4096: 757 / 716; 2 x 8192: 1413 / 1187.
     long long ctas;  // without pairs
     int group_major = 0;
     if (forced == 1 || (forced == 0 && (nqb > 24 || (nqb > 16 && items <= 16LL * sm_count[dev])))) {
