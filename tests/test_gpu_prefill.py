@@ -221,3 +221,37 @@ def test_prompts_of_many_row_blocks_pair_against_single(cuda_ops, B, T, dtype):
     # the weights are 16-bit operands too: half a unit each, relative to the row's largest terms
     assert bool(((outs[0] - outs[1]).abs() <= eps * outs[1].abs() + 2 * eps * outs[1].abs().amax(-1, keepdim=True)).all())
     assert cuda_ops.lib.khq_b200_prefill_pairs(3) == -100
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("H_q,H_kv", [(24, 4), (8, 2), (4, 2)])
+@pytest.mark.parametrize("B,T,S", [(2, 63, 64), (3, 150, 256), (2, 257, 300), (1, 1300, 1300)])
+def test_pairs_in_slabs_vs_torch_fp32(cuda_ops, B, T, S, H_q, H_kv, dtype):
+    """CTA pairs with six, four and two query heads per kv head, prompts in slabs of S rows whose rest is NaN: a plain PyTorch fp32 reference
+    of the same op on the same inputs, at the storage type's bar; the rest of the output's slabs stays as it is."""
+    import torch
+
+    dt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(T + H_q)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    qg, k, v = rnd(B, S, H_q, 2 * D).to(dt), (0.25 * rnd(B, S, H_kv, D)).to(dt), rnd(B, S, H_kv, D).to(dt)
+    k[:, :T:7] *= 3.0  # scores that move the reference
+    for t in (qg, k, v):
+        t[:, T:] = float("nan")
+    out = torch.full((B, S, H_q, D), -7.0, dtype=dt, device="cuda")
+    lib = cuda_ops.lib
+    assert lib.khq_b200_prefill_pairs(1) == 0
+    fn = lib.launch_khq_gqa_prefill_tc5_fp16 if dtype == "float16" else lib.launch_khq_gqa_prefill_bf16
+    rc = fn(qg.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, T, H_q, H_kv, D, SCALE, S * H_q * 2 * D, S * H_kv * D, S * H_q * D,
+            torch.cuda.current_stream().cuda_stream)
+    lib.khq_b200_prefill_pairs(0)
+    assert rc == 0 and lib.khq_b200_prefill_status() == 0
+    assert bool((out[:, T:] == -7.0).all())
+    heads = lambda x: x[:, :T].float().transpose(1, 2)
+    kk, vv = (heads(x).repeat_interleave(H_q // H_kv, dim=1) for x in (k, v))
+    s = heads(qg[..., :D]) @ kk.transpose(-1, -2) * SCALE
+    s = s.masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    ref = torch.softmax(s, dim=-1) @ vv * torch.sigmoid(heads(qg[..., D:]))
+    err = (heads(out) - ref).abs()
+    lim = 2e-3 + 1e-2 * ref.abs() if dtype == "float16" else 4e-3 + 2e-2 * ref.abs()
+    assert bool((err <= lim).all()), (float(err.max()), float((err - lim).max()))
